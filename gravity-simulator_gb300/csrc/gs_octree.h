@@ -17,8 +17,8 @@ enum OctCtr {
     CTR_N = 3,          // particle count (for device-count kernels)
     CTR_SAFE_INTERNAL = 4,   // internal nodes for the kernels after the expansion:
                              // CTR_INTERNAL, or 0 once the node capacity overflowed
-    CTR_LVL = 8,        // CTR_LVL + d: first internal index of depth d (d = 0..22)
-    CTR_SIZE = 40
+    CTR_DONE = 5,       // finished CTAs of a kernel whose last CTA scans (0 between kernels)
+    CTR_SIZE = 8
 };
 
 #ifdef __CUDACC__
@@ -55,17 +55,18 @@ struct OctreeDevice {
     DBuf frame;               // double[8]: cx, cy, cz, width, box_length
     DBuf bbox_part;           // double[blocks * 6]
     DBuf keys, sidx;          // uint64[n] sorted Morton keys, int[n] particle ids
-    // construction lists (unordered)
-    DBuf nd_start, nd_count, nd_depth, nd_parent, nd_rank, nd_int;   // int[cap]
-    DBuf in_node, in_nchild, in_fc, in_id;                           // int[cap]
-    DBuf in_key;                                                     // uint64[cap]
-    DBuf in_order;                                                   // int[cap]
+    // internal nodes in depth-first pre-order, the order of (first particle, depth)
+    DBuf pre_of;              // int[n]: internal nodes that start before particle i
+    DBuf in_sd;               // int2[cap]: (first particle, depth)
+    DBuf in_end;              // int[8 * cap]: sorted index at which each octant ends
+    DBuf in_nch;              // int[cap]: children
+    DBuf in_rec;              // int4[cap]: (first child, children | inner mask << 8, parent, id)
     DBuf scan_tiles;                                                 // unsigned[...]
     // final node arrays in the reference's numbering
     DBuf t_np, t_nc, t_fp, t_fc, t_depth, t_int;                     // int[cap]
     DBuf t_mass;                                                     // double[cap]
     DBuf t_com;                                                      // double[3*cap]
-    DBuf in_sum;                                                     // double[4*cap]
+    DBuf t_sum;                                                      // double[4*cap] (internal)
     DBuf in_arrive;   // int[cap]: children whose multipoles are done (bottom-up pass)
     // walk arrays (frame-centred double-float positions)
     DBuf w_na, w_nb;          // float4[cap]: (com_hi, mass), (com_lo, (cell side)^2)
@@ -89,13 +90,6 @@ struct OctreeDevice {
     ErrorStatus build(const double *d_x, const double *d_m, cudaStream_t s,
                       const double *box_center = nullptr, double box_width = -1.0);
     int launches_per_build() const;
-    // Bits of the internal-node sort key (first particle << 5 | depth).
-    int internal_key_bits() const
-    {
-        int b = 1;
-        while (b < 31 && (1 << b) <= n) ++b;
-        return b + 5;
-    }
     // Host copies: number of nodes, status word.
     ErrorStatus read_counts(cudaStream_t s, int *nodes, unsigned *status);
     // Clears the status word once the host has reported it.

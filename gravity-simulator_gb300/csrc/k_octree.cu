@@ -10,19 +10,18 @@
 //                  21-bit mask (a coordinate at the box maximum wraps to 0,
 //                  as in the reference), bit interleave.
 //   sort           RadixSorter (stable LSD, 8-bit digits, one sweep per digit) of (key, id).
-//   topology       level-synchronous: k_tree_expand(d) splits every internal
-//                  node of depth d into its non-empty octants (binary search
-//                  on the sorted keys), appending children to an unordered
-//                  node list; a child is internal when it holds more than
-//                  leaf_max particles and is above depth 21.
+//   topology       from the sorted keys alone: which internal nodes start at a
+//                  particle follows from three keys (k_tree_count, k_tree_emit);
+//                  a child is internal when it holds more than leaf_max particles
+//                  and is above depth 21.  k_tree_children finds each node's
+//                  octants by binary search.
 //   numbering      the reference numbers nodes in creation order: all
 //                  children of a node get consecutive ids when the node is
 //                  expanded, and nodes are expanded in depth-first pre-order.
 //                  Pre-order of internal nodes is the order of (first
-//                  particle, depth), so internal nodes are radix-sorted by
-//                  that key and an exclusive scan of their child counts gives
-//                  each one's first-child id; a node's id is then its
-//                  parent's first-child id plus its octant rank.
+//                  particle, depth), the order in which they are emitted, so an
+//                  exclusive scan of their child counts gives each one's
+//                  first-child id (k_tree_nodes).
 //   multipoles     bottom-up in one launch (arrival counters): an internal
 //                  node adds, child by child in octant order, the particles
 //                  of leaf children (sorted order) and the running sums of
@@ -44,7 +43,6 @@ namespace gs {
 
 constexpr int OT_THREADS = 256;
 constexpr int BBOX_BLOCKS = 512;
-constexpr int SCAN_TILE = 4096;
 
 __device__ __forceinline__ double dmin(double a, double b) { return fmin(a, b); }
 __device__ __forceinline__ double dmax(double a, double b) { return fmax(a, b); }
@@ -194,326 +192,311 @@ __global__ void k_morton(const double *__restrict__ x, int n, const double *__re
     misplaced[i] = out ? 1 : 0;
 }
 
-__global__ void k_tree_init(int *__restrict__ ctr, int n, int *__restrict__ nd_start,
-                            int *__restrict__ nd_count, int *__restrict__ nd_depth,
-                            int *__restrict__ nd_parent, int *__restrict__ nd_rank,
-                            int *__restrict__ nd_int, int *__restrict__ in_node)
+// ---- topology ---------------------------------------------------------------
+// A cell of depth d that starts at sorted particle i is internal when the keys
+// i .. i + leaf_max share its prefix, so the internal nodes that start at i are
+// the depths from (levels shared with key i - 1) + 1 to (levels shared with key
+// i + leaf_max), and their number needs three keys.  Their order by (first
+// particle, depth) is the reference's depth-first pre-order, so an exclusive
+// scan of those numbers over the particles gives every internal node its index:
+// no level-by-level expansion and no sort of the nodes.
+constexpr int TC_ITEMS = 8;
+constexpr int TC_TILE = OT_THREADS * TC_ITEMS;   // particles per scan tile
+constexpr int TN_TILE = OT_THREADS;              // internal nodes per scan tile
+
+// Levels (octant digits) shared by two 63-bit keys.
+__device__ __forceinline__ int shared_levels(uint64_t a, uint64_t b)
 {
-    if (threadIdx.x != 0) return;
-    ctr[CTR_NODES] = 1;
-    ctr[CTR_INTERNAL] = 1;
-    ctr[CTR_N] = n;
-    ctr[CTR_LVL + 0] = 0;
-    ctr[CTR_LVL + 1] = 1;
-    nd_start[0] = 0;
-    nd_count[0] = n;
-    nd_depth[0] = 0;
-    nd_parent[0] = -1;
-    nd_rank[0] = 0;
-    nd_int[0] = 0;
-    in_node[0] = 0;
+    const uint64_t x = a ^ b;
+    return x ? (62 - (63 - __clzll((long long)x))) / 3 : OCT_MAX_LEVEL;
 }
 
-// First index in [lo, hi) whose octant digit at `shift` exceeds o.
-__device__ __forceinline__ int octant_end(const uint64_t *__restrict__ keys, int lo, int hi,
-                                          int shift, int o)
+// Depths [lo, hi] of the internal nodes that start at particle i (none when
+// hi < lo).  The root is internal whatever its count.
+__device__ __forceinline__ void internal_depths(const uint64_t *__restrict__ keys, int n,
+                                                int leaf_max, int i, int &lo, int &hi)
 {
+    const uint64_t k = keys[i];
+    lo = i == 0 ? 0 : shared_levels(keys[i - 1], k) + 1;
+    hi = leaf_max < n - i ? min(OCT_MAX_LEVEL - 1, shared_levels(k, keys[i + leaf_max])) : -1;
+    if (i == 0) hi = max(hi, 0);
+}
+
+// Exclusive prefix of v over the CTA's threads; every thread also gets the sum.
+__device__ __forceinline__ unsigned block_exclusive(unsigned v, unsigned &sum)
+{
+    __shared__ unsigned wsum[OT_THREADS / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned incl = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) wsum[w] = incl;
+    __syncthreads();
+    unsigned before = 0;
+    sum = 0;
+    for (int q = 0; q < OT_THREADS / 32; ++q) {
+        before += q < w ? wsum[q] : 0u;
+        sum += wsum[q];
+    }
+    __syncthreads();
+    return before + incl - v;
+}
+
+// The CTA that is the last of the grid to come here returns true in all its
+// threads (and sees what the others wrote before); the counter is left at 0.
+__device__ __forceinline__ bool last_block(int *counter)
+{
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(counter, 1) == (int)gridDim.x - 1;
+        if (last) *counter = 0;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
+// tile[0 .. tiles) -> its exclusive scan, by one CTA; returns the total.
+__device__ unsigned long long scan_tiles_inplace(unsigned *tile, int tiles)
+{
+    unsigned long long run = 0;
+    for (int b = 0; b < tiles; b += OT_THREADS) {
+        const int t = b + (int)threadIdx.x;
+        unsigned sum;
+        const unsigned before = block_exclusive(t < tiles ? __ldcg(tile + t) : 0u, sum);
+        if (t < tiles) tile[t] = (unsigned)run + before;   // meaningful while the total fits
+        run += sum;
+    }
+    return run;
+}
+
+// Internal nodes per tile of particles, and their scan by the last CTA.
+__global__ void __launch_bounds__(OT_THREADS)
+k_tree_count(const uint64_t *__restrict__ keys, int n, int leaf_max, int cap,
+             unsigned *__restrict__ tile_sum, int *__restrict__ ctr)
+{
+    unsigned c = 0;
+#pragma unroll
+    for (int k = 0; k < TC_ITEMS; ++k) {
+        const int i = blockIdx.x * TC_TILE + k * OT_THREADS + threadIdx.x;
+        if (i < n) {
+            int lo, hi;
+            internal_depths(keys, n, leaf_max, i, lo, hi);
+            c += max(0, hi - lo + 1);
+        }
+    }
+    unsigned sum;
+    (void)block_exclusive(c, sum);
+    if (threadIdx.x == 0) tile_sum[blockIdx.x] = sum;
+    if (!last_block(&ctr[CTR_DONE])) return;
+    const unsigned long long total = scan_tiles_inplace(tile_sum, gridDim.x);
+    if (threadIdx.x == 0) {
+        // every internal node but the root is a node, and has a child
+        if (total >= (unsigned long long)cap)
+            atomicOr((unsigned *)&ctr[CTR_STATUS], ST_TREE_OVERFLOW);
+        const bool failed = tree_failed(ctr);
+        ctr[CTR_INTERNAL] = failed ? 0 : (int)total;
+        ctr[CTR_SAFE_INTERNAL] = failed ? 0 : (int)total;
+    }
+}
+
+// Index of the first internal node at or after each particle (pre_of), and
+// each internal node's (first particle, depth).
+__global__ void __launch_bounds__(OT_THREADS)
+k_tree_emit(const uint64_t *__restrict__ keys, int n, int leaf_max,
+            const unsigned *__restrict__ tile_off, const int *__restrict__ ctr,
+            int *__restrict__ pre_of, int2 *__restrict__ in_sd)
+{
+    if (tree_failed(ctr)) return;
+    const int i0 = blockIdx.x * TC_TILE + threadIdx.x * TC_ITEMS;
+    int lo[TC_ITEMS], cnt[TC_ITEMS];
+    unsigned c = 0;
+#pragma unroll
+    for (int k = 0; k < TC_ITEMS; ++k) {
+        lo[k] = cnt[k] = 0;
+        if (i0 + k < n) {
+            int hi;
+            internal_depths(keys, n, leaf_max, i0 + k, lo[k], hi);
+            cnt[k] = max(0, hi - lo[k] + 1);
+        }
+        c += cnt[k];
+    }
+    unsigned sum;
+    int at = (int)(tile_off[blockIdx.x] + block_exclusive(c, sum));
+#pragma unroll
+    for (int k = 0; k < TC_ITEMS; ++k) {
+        if (i0 + k >= n) break;
+        pre_of[i0 + k] = at;
+        for (int q = 0; q < cnt[k]; ++q) in_sd[at + q] = make_int2(i0 + k, lo[k] + q);
+        at += cnt[k];
+    }
+}
+
+// First index after s whose key, shifted, exceeds `limit`: steps of a factor
+// of eight from s (most nodes hold few particles), then a binary search.
+__device__ __forceinline__ int prefix_end(const uint64_t *__restrict__ keys, int s, int n,
+                                          int shift, uint64_t limit)
+{
+    int lo = s, hi = n;   // the answer lies in [lo, hi]
+    for (long long step = 8;; step *= 8) {
+        const long long at = s + step;
+        if (at >= n) break;
+        if ((keys[at] >> shift) > limit) {
+            hi = (int)at;
+            break;
+        }
+        lo = (int)at + 1;
+    }
     while (lo < hi) {
         const int mid = lo + ((hi - lo) >> 1);
-        const int dig = (int)((keys[mid] >> shift) & 7ull);
-        if (dig <= o)
-            lo = mid + 1;
-        else
+        if ((keys[mid] >> shift) > limit)
             hi = mid;
+        else
+            lo = mid + 1;
     }
     return lo;
 }
 
-// src/linear_octree.c:342-576 for all internal nodes of depth d at once.
-// Levels with few nodes (the top of the tree, where a node's binary
-// searches are long) use eight lanes per node, one per octant: each finds
-// where its octant ends by its own binary search over the node's sorted
-// keys (the searches are independent: the keys of a node are sorted by
-// their octant digit), the eight ends are combined by shuffles within the
-// 8-lane group, and each lane writes its own child.  Levels with many nodes
-// use one thread per node.  Node ids come from an atomic counter; the
-// reference's numbering is recovered later by k_tree_number.
-constexpr int EXPAND_WIDE_NODES = 16384;
+// Children of every internal node (src/linear_octree.c:342-576): eight lanes
+// per node, one per octant, each finds where its octant ends.  in_end[8 ii + o]
+// receives the ends, in_nch[ii] the non-empty octants; the last CTA scans the
+// children over the tiles of nodes, which gives the node total.
 __global__ void __launch_bounds__(OT_THREADS)
-k_tree_expand(int d, int leaf_max, int cap, const uint64_t *__restrict__ keys, int *__restrict__ ctr,
-              int *__restrict__ nd_start, int *__restrict__ nd_count, int *__restrict__ nd_depth,
-              int *__restrict__ nd_parent, int *__restrict__ nd_rank, int *__restrict__ nd_int,
-              int *__restrict__ in_node, int *__restrict__ in_nchild)
+k_tree_children(const uint64_t *__restrict__ keys, int n, int cap, const int2 *__restrict__ in_sd,
+                int *__restrict__ in_end, int *__restrict__ in_nch,
+                unsigned *__restrict__ tile_sum, int *__restrict__ ctr)
 {
-    if (tree_failed(ctr)) return;   // an earlier level overflowed
-    const int lo = ctr[CTR_LVL + d];
-    const int hi = ctr[CTR_LVL + d + 1];
-    const int cd = d + 1;
-    const int shift = 3 * (OCT_MAX_LEVEL - cd);
-    if (hi - lo > EXPAND_WIDE_NODES) {
-        // many nodes (deep levels, few particles each): one thread per node,
-        // its eight searches over shrinking ranges
-        for (int ii = lo + blockIdx.x * OT_THREADS + threadIdx.x; ii < hi;
-             ii += gridDim.x * OT_THREADS) {
-            const int q = in_node[ii];
-            const int s = nd_start[q];
-            const int e = s + nd_count[q];
-            int ends[8];
-            int nch = 0;
-            int prev = s;
-            for (int o = 0; o < 8; ++o) {
-                ends[o] = octant_end(keys, prev, e, shift, o);
-                if (ends[o] > prev) ++nch;
-                prev = ends[o];
+    const int ni = ctr[CTR_SAFE_INTERNAL];
+    const int lane = threadIdx.x & 31, o = lane & 7, g0 = lane & ~7;
+    const int tiles = (ni + TN_TILE - 1) / TN_TILE;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        unsigned mine = 0;
+        for (int q = 0; q < TN_TILE; q += OT_THREADS / 8) {
+            const int ii = tile * TN_TILE + q + (threadIdx.x >> 3);
+            const bool act = ii < ni;
+            int s = 0, end = 0;
+            if (act) {
+                const int2 sd = in_sd[ii];
+                s = sd.x;
+                const int shift = 3 * (OCT_MAX_LEVEL - 1 - sd.y);
+                end = prefix_end(keys, s, n, shift, ((keys[s] >> shift) & ~7ull) | (uint64_t)o);
+                in_end[8 * (size_t)ii + o] = end;
             }
-            const int base = atomicAdd(&ctr[CTR_NODES], nch);
-            if (base + nch > cap) {
-                atomicOr((unsigned *)&ctr[CTR_STATUS], ST_TREE_OVERFLOW);
-                in_nchild[ii] = 0;
-                continue;
+            const int up = __shfl_up_sync(0xffffffffu, end, 1, 8);
+            const bool has = act && end > (o == 0 ? s : up);
+            const int nch = __popc((__ballot_sync(0xffffffffu, has) >> g0) & 0xffu);
+            if (act && o == 0) {
+                in_nch[ii] = nch;
+                mine += nch;
             }
-            int r = 0;
-            prev = s;
-            for (int o = 0; o < 8; ++o) {
-                const int cnt = ends[o] - prev;
-                if (cnt > 0) {
-                    const int c = base + r;
-                    nd_start[c] = prev;
-                    nd_count[c] = cnt;
-                    nd_depth[c] = cd;
-                    nd_parent[c] = ii;
-                    nd_rank[c] = r;
-                    int slot = -1;
-                    if (cnt > leaf_max && cd < OCT_MAX_LEVEL) {
-                        slot = atomicAdd(&ctr[CTR_INTERNAL], 1);
-                        if (slot >= cap) {
-                            atomicOr((unsigned *)&ctr[CTR_STATUS], ST_TREE_OVERFLOW);
-                            slot = -1;
-                        } else {
-                            in_node[slot] = c;
-                        }
-                    }
-                    nd_int[c] = slot;
-                    ++r;
-                }
-                prev = ends[o];
-            }
-            in_nchild[ii] = nch;
         }
-        return;
+        unsigned sum;
+        (void)block_exclusive(mine, sum);
+        if (threadIdx.x == 0) tile_sum[tile] = sum;
     }
-    const int lane = threadIdx.x & 31;
-    const int o = lane & 7;
-    const int g0 = lane & ~7;   // first lane of this node's group
-    for (int wt = blockIdx.x * OT_THREADS + (threadIdx.x & ~31);; wt += gridDim.x * OT_THREADS) {
-        if (lo + (wt >> 3) >= hi) break;   // warp-uniform
-        const int ii = lo + ((wt + lane) >> 3);
-        const bool act = ii < hi;
-        int s = 0, e = 0;
-        if (act) {
-            const int q = in_node[ii];
-            s = nd_start[q];
-            e = s + nd_count[q];
-        }
-        const int endo = act ? octant_end(keys, s, e, shift, o) : 0;
-        const int up = __shfl_up_sync(0xffffffffu, endo, 1, 8);
-        const int prev = (o == 0) ? s : up;
-        const int cnt = act ? endo - prev : 0;
-        const unsigned m8 = (__ballot_sync(0xffffffffu, cnt > 0) >> g0) & 0xffu;
-        const int nch = __popc(m8);
-        const int rank = __popc(m8 & ((1u << o) - 1u));
-        int base = 0;
-        if (act && o == 0) base = atomicAdd(&ctr[CTR_NODES], nch);
-        base = __shfl_sync(0xffffffffu, base, g0);
-        if (!act) continue;
-        if (base + nch > cap) {
-            if (o == 0) {
-                atomicOr((unsigned *)&ctr[CTR_STATUS], ST_TREE_OVERFLOW);
-                in_nchild[ii] = 0;
-            }
-            continue;
-        }
-        if (cnt > 0) {
-            const int c = base + rank;
-            nd_start[c] = prev;
-            nd_count[c] = cnt;
-            nd_depth[c] = cd;
-            nd_parent[c] = ii;
-            nd_rank[c] = rank;
-            int slot = -1;
-            if (cnt > leaf_max && cd < OCT_MAX_LEVEL) {
-                slot = atomicAdd(&ctr[CTR_INTERNAL], 1);
-                if (slot >= cap) {
-                    atomicOr((unsigned *)&ctr[CTR_STATUS], ST_TREE_OVERFLOW);
-                    slot = -1;
-                } else {
-                    in_node[slot] = c;
-                }
-            }
-            nd_int[c] = slot;
-        }
-        if (o == 0) in_nchild[ii] = nch;
-    }
-}
-
-__global__ void k_tree_mark(int d, int *__restrict__ ctr)
-{
+    if (!last_block(&ctr[CTR_DONE])) return;
+    const unsigned long long total = scan_tiles_inplace(tile_sum, tiles) + 1ull;
     if (threadIdx.x == 0) {
-        ctr[CTR_LVL + d + 2] = ctr[CTR_INTERNAL];
-        ctr[CTR_SAFE_INTERNAL] = tree_failed(ctr) ? 0 : ctr[CTR_INTERNAL];
+        if (total > (unsigned long long)cap) {
+            atomicOr((unsigned *)&ctr[CTR_STATUS], ST_TREE_OVERFLOW);
+            ctr[CTR_SAFE_INTERNAL] = 0;
+        }
+        ctr[CTR_NODES] = tree_failed(ctr) ? 1 : (int)total;
     }
 }
 
-// Sort key of an internal node: pre-order = (first particle, depth).
-__global__ void k_internal_keys(const int *__restrict__ ctr, const int *__restrict__ in_node,
-                                const int *__restrict__ nd_start, const int *__restrict__ nd_depth,
-                                uint64_t *__restrict__ in_key, int *__restrict__ in_order,
-                                int *__restrict__ in_arrive)
-{
-    const int ni = ctr[CTR_SAFE_INTERNAL];
-    for (int ii = blockIdx.x * blockDim.x + threadIdx.x; ii < ni; ii += gridDim.x * blockDim.x) {
-        const int q = in_node[ii];
-        in_key[ii] = ((uint64_t)nd_start[q] << 5) | (uint64_t)nd_depth[q];
-        in_order[ii] = ii;
-        in_arrive[ii] = 0;
-    }
-}
-
-// Tile sums of child counts in pre-order.
+// Node arrays by id: the children of internal node ii take the ids from
+// first child = 1 + (children of the internal nodes before it), in octant
+// order, which is the reference's creation order.  in_rec[ii] is (first child,
+// children | internal ones' mask << 8, parent, id); a child's half of it is
+// written by its parent.
 __global__ void __launch_bounds__(OT_THREADS)
-k_fc_tile_sums(const int *__restrict__ ctr, const int *__restrict__ in_order,
-               const int *__restrict__ in_nchild, unsigned *__restrict__ tile_sum)
+k_tree_nodes(int n, int leaf_max, const unsigned *__restrict__ tile_off,
+             const int *__restrict__ ctr, const int2 *__restrict__ in_sd,
+             const int *__restrict__ in_end, const int *__restrict__ in_nch,
+             const int *__restrict__ pre_of, int4 *__restrict__ in_rec, int *__restrict__ in_arrive,
+             int *__restrict__ t_np, int *__restrict__ t_fp, int *__restrict__ t_depth,
+             int *__restrict__ t_int)
 {
-    __shared__ unsigned red[OT_THREADS];
+    __shared__ int s_fc[TN_TILE];
     const int ni = ctr[CTR_SAFE_INTERNAL];
-    const int base = blockIdx.x * SCAN_TILE;
-    unsigned s = 0;
-    for (int k = threadIdx.x; k < SCAN_TILE; k += OT_THREADS) {
-        const int e = base + k;
-        if (e < ni) s += (unsigned)in_nchild[in_order[e]];
-    }
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = OT_THREADS / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+    const int lane = threadIdx.x & 31, o = lane & 7, g0 = lane & ~7;
+    const int tiles = (ni + TN_TILE - 1) / TN_TILE;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int mine = tile * TN_TILE + (int)threadIdx.x;
+        unsigned sum;
+        const unsigned before = block_exclusive(mine < ni ? (unsigned)in_nch[mine] : 0u, sum);
+        s_fc[threadIdx.x] = 1 + (int)(tile_off[tile] + before);
         __syncthreads();
-    }
-    if (threadIdx.x == 0) tile_sum[blockIdx.x] = red[0];
-}
-
-__global__ void __launch_bounds__(1024) k_scan_small(unsigned *__restrict__ v, int len)
-{
-    __shared__ unsigned part[1024];
-    const int per = (len + 1023) / 1024;
-    const int b = threadIdx.x * per;
-    const int e = min(len, b + per);
-    unsigned s = 0;
-    for (int i = b; i < e; ++i) s += v[i];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-        const unsigned t = threadIdx.x >= off ? part[threadIdx.x - off] : 0u;
-        __syncthreads();
-        part[threadIdx.x] += t;
-        __syncthreads();
-    }
-    unsigned run = threadIdx.x ? part[threadIdx.x - 1] : 0u;
-    for (int i = b; i < e; ++i) {
-        const unsigned c = v[i];
-        v[i] = run;
-        run += c;
-    }
-}
-
-// First-child id of each internal node: 1 + exclusive scan in pre-order.
-__global__ void __launch_bounds__(OT_THREADS)
-k_fc_apply(const int *__restrict__ ctr, const int *__restrict__ in_order,
-           const int *__restrict__ in_nchild, const unsigned *__restrict__ tile_off,
-           int *__restrict__ in_fc)
-{
-    constexpr int PER = SCAN_TILE / OT_THREADS;   // 16 consecutive per thread
-    __shared__ unsigned part[OT_THREADS];
-    const int ni = ctr[CTR_SAFE_INTERNAL];
-    const int base = blockIdx.x * SCAN_TILE + threadIdx.x * PER;
-    unsigned v[PER];
-    unsigned s = 0;
-    for (int k = 0; k < PER; ++k) {
-        const int e = base + k;
-        v[k] = e < ni ? (unsigned)in_nchild[in_order[e]] : 0u;
-        s += v[k];
-    }
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (int off = 1; off < OT_THREADS; off <<= 1) {
-        const unsigned t = threadIdx.x >= off ? part[threadIdx.x - off] : 0u;
-        __syncthreads();
-        part[threadIdx.x] += t;
-        __syncthreads();
-    }
-    unsigned run = tile_off[blockIdx.x] + (threadIdx.x ? part[threadIdx.x - 1] : 0u);
-    for (int k = 0; k < PER; ++k) {
-        const int e = base + k;
-        if (e < ni) in_fc[in_order[e]] = 1 + (int)run;
-        run += v[k];
-    }
-}
-
-// Final node arrays by id.
-__global__ void k_tree_number(const int *__restrict__ ctr, int compat,
-                              const int *__restrict__ nd_start, const int *__restrict__ nd_count,
-                              const int *__restrict__ nd_depth, const int *__restrict__ nd_parent,
-                              const int *__restrict__ nd_rank, const int *__restrict__ nd_int,
-                              const int *__restrict__ in_nchild, const int *__restrict__ in_fc,
-                              int *__restrict__ in_id, int *__restrict__ t_np,
-                              int *__restrict__ t_nc, int *__restrict__ t_fp,
-                              int *__restrict__ t_fc, int *__restrict__ t_depth,
-                              int *__restrict__ t_int, double *__restrict__ t_mass,
-                              double *__restrict__ t_com)
-{
-    const int nn = tree_nodes(ctr);
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nn; q += gridDim.x * blockDim.x) {
-        const int id = (q == 0) ? 0 : in_fc[nd_parent[q]] + nd_rank[q];
-        t_np[id] = nd_count[q];
-        t_fp[id] = nd_start[q];
-        t_depth[id] = nd_depth[q];
-        const int ii = nd_int[q];
-        t_int[id] = ii;
-        if (ii >= 0) {
-            t_nc[id] = in_nchild[ii];
-            t_fc[id] = in_fc[ii];
-            in_id[ii] = id;
-        } else {
-            t_nc[id] = 0;
-            t_fc[id] = -1;
-            if (compat) {
-                t_mass[id] = 0.0;
-                t_com[3 * id + 0] = 0.0;
-                t_com[3 * id + 1] = 0.0;
-                t_com[3 * id + 2] = 0.0;
+        for (int q = 0; q < TN_TILE; q += OT_THREADS / 8) {
+            const int local = q + (int)(threadIdx.x >> 3);
+            const int ii = tile * TN_TILE + local;
+            const bool act = ii < ni;
+            int2 sd = make_int2(0, 0);
+            int end = 0;
+            if (act) {
+                sd = in_sd[ii];
+                end = in_end[8 * (size_t)ii + o];
+            }
+            const int up = __shfl_up_sync(0xffffffffu, end, 1, 8);
+            const int start = o == 0 ? sd.x : up;
+            const int cnt = act ? end - start : 0;
+            const int cd = sd.y + 1;
+            const bool inner = cnt > leaf_max && cd < OCT_MAX_LEVEL;
+            const unsigned m8 = (__ballot_sync(0xffffffffu, cnt > 0) >> g0) & 0xffu;
+            const int rank = __popc(m8 & ((1u << o) - 1u));
+            unsigned imask = inner ? 1u << rank : 0u;
+            for (int w = 1; w < 8; w <<= 1) imask |= __shfl_xor_sync(0xffffffffu, imask, w, 8);
+            if (!act) continue;
+            const int fc = s_fc[local];
+            int2 *rec = reinterpret_cast<int2 *>(in_rec);
+            if (o == 0) {
+                rec[2 * (size_t)ii] = make_int2(fc, __popc(m8) | (int)(imask << 8));
+                in_arrive[ii] = 0;
+                if (ii == 0) {
+                    rec[1] = make_int2(-1, 0);
+                    t_np[0] = n;
+                    t_fp[0] = 0;
+                    t_depth[0] = 0;
+                    t_int[0] = 0;
+                }
+            }
+            if (cnt > 0) {
+                const int id = fc + rank;
+                // the child's own index: the next one when it starts where
+                // this node does, else the first one of its first particle
+                const int ci = start == sd.x ? ii + 1 : pre_of[start];
+                t_np[id] = cnt;
+                t_fp[id] = start;
+                t_depth[id] = cd;
+                t_int[id] = inner ? ci : -1;
+                if (inner) rec[2 * (size_t)ci + 1] = make_int2(ii, id);
             }
         }
+        __syncthreads();
     }
 }
 
 // Parent id of every node and the leaf of every sorted particle (used by
 // the learned method's features).
-__global__ void k_tree_links(const int *__restrict__ ctr, const int *__restrict__ nd_start,
-                             const int *__restrict__ nd_count, const int *__restrict__ nd_parent,
-                             const int *__restrict__ nd_rank, const int *__restrict__ nd_int,
-                             const int *__restrict__ in_node, const int *__restrict__ in_fc,
-                             int *__restrict__ t_parent, int *__restrict__ leaf_of)
+__global__ void k_tree_links(const int *__restrict__ ctr, const int4 *__restrict__ in_rec,
+                             const int *__restrict__ t_np, const int *__restrict__ t_fp,
+                             const int *__restrict__ t_int, int *__restrict__ t_parent,
+                             int *__restrict__ leaf_of)
 {
-    const int nn = tree_nodes(ctr);
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nn; q += gridDim.x * blockDim.x) {
-        int id = 0, parent = -1;
-        if (q != 0) {
-            id = in_fc[nd_parent[q]] + nd_rank[q];
-            const int pq = in_node[nd_parent[q]];
-            parent = (pq == 0) ? 0 : in_fc[nd_parent[pq]] + nd_rank[pq];
+    const int ni = ctr[CTR_SAFE_INTERNAL];
+    for (int ii = blockIdx.x * blockDim.x + threadIdx.x; ii < ni; ii += gridDim.x * blockDim.x) {
+        const int4 r = in_rec[ii];
+        if (ii == 0) t_parent[0] = -1;
+        for (int c = r.x; c < r.x + (r.y & 255); ++c) {
+            t_parent[c] = r.w;
+            if (t_int[c] < 0)
+                for (int p = t_fp[c]; p < t_fp[c] + t_np[c]; ++p) leaf_of[p] = c;
         }
-        t_parent[id] = parent;
-        if (nd_int[q] < 0)
-            for (int p = nd_start[q]; p < nd_start[q] + nd_count[q]; ++p) leaf_of[p] = id;
     }
 }
 
@@ -596,60 +579,83 @@ __device__ __forceinline__ float df_offset(float ph, float pl, float ch, float c
 
 struct MultipoleArgs {
     const double *xm;   // sorted (x, y, z, m) records
-    const int *sidx, *in_node, *nd_parent, *in_id, *in_fc, *in_nchild;
-    const int *t_np, *t_nc, *t_fp, *t_int, *t_depth;
+    const int4 *in_rec; // internal nodes: (first child, children | inner mask << 8, parent, id)
+    const int4 *nc;     // nodes: (first child, children, first particle, particles)
+    const int *t_depth;
     const double *frame;
     int *in_arrive;
-    double *in_sum, *t_mass, *t_com;
+    double *t_sum, *t_mass, *t_com;   // t_sum: (m, m x, m y, m z) of internal nodes by id
     float4 *na, *nb, *nq;   // nq null: no quadrupoles
 };
 
-// Multipoles of internal node ii from its children (reference :652-735): mass
-// and the mass-weighted coordinate sums in child order, the centre of mass by
-// division, its walk record, and, when nq is not null, the quadrupole from the
-// children's by the parallel-axis shift Q = sum_c [Q_c + M_c (3 s s^T - |s|^2 I)],
-// s = com_c - com, in FP32 from the children's walk records (FP64 runs at 1/64
-// of the FP32 rate here, and the walk uses FP32 quadrupoles).  Children's
-// values written by other threads of the same launch are read through L2
-// (__ldcg), after the fence that follows the arrival counter.
+// Multipoles of the internal node of record rec from its children (reference
+// :652-735): mass and the mass-weighted coordinate sums in child order, the
+// centre of mass by division, its walk record, and, when nq is not null, the
+// quadrupole from the children's by the parallel-axis shift
+// Q = sum_c [Q_c + M_c (3 s s^T - |s|^2 I)], s = com_c - com, in FP32 from the
+// children's walk records (FP64 runs at 1/64 of the FP32 rate here, and the walk
+// uses FP32 quadrupoles).  Children's values written by other threads of the
+// same launch are read through L2 (__ldcg), after the fence that follows the
+// arrival counter.
 //
 // A node is computed by the four lanes of a group: lane j keeps one of the
 // four ordered sums (j = 0 the mass, j = 1..3 the sums of m x, m y, m z), so
 // a particle costs one FP64 multiply and one add for all four sums (lane 0
 // multiplies the mass by 1.0, which is exact: its sum is the plain mass sum),
-// and the three quotients are one division.  An FP64 warp instruction costs
-// the pipe a whole warp's time however few lanes it carries, and near the
-// root a single group climbs alone: this cuts the FP64 instructions on that
-// path from 7 to 2 per particle.  Each sum sees the same operands in the same
-// order as a one-thread loop would, so the values are the same bit for bit.
-__device__ void multipole_node4(int ii, int j, unsigned gmask, const MultipoleArgs &A)
+// and the three quotients are one division.  Each sum sees the same operands in
+// the same order as a one-thread loop would, so the values are the same bit for
+// bit.
+//
+// Near the root a single group climbs alone, and what bounds it is the chain of
+// dependent loads of each level.  The record and the sums are laid out so that
+// a level is one round of loads: the record says which children are internal,
+// their sums are indexed by node id, and all of them (and the leaf children's
+// particle ranges) are issued before the first is used; the caller loads the
+// parent's record meanwhile.  With child type, index and sums each behind the
+// other, eight times in a row, a level took about 17 us and the kernel 309 us
+// at N = 60,000 and 311 us at N = 1,048,576.
+__device__ void multipole_node4(const int4 rec, int j, unsigned gmask, const MultipoleArgs &A)
 {
-    const int fc = A.in_fc[ii];
-    const int end = fc + A.in_nchild[ii];
+    const int fc = rec.x, nch = rec.y & 255, inner = rec.y >> 8, id = rec.w;
+    const int end = fc + nch;
+    double v[8];
+    int2 leaf[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        v[r] = 0.0;
+        leaf[r] = make_int2(0, 0);
+        if (r < nch) {
+            if ((inner >> r) & 1)
+                v[r] = __ldcg(A.t_sum + 4 * (size_t)(fc + r) + j);
+            else
+                leaf[r] = reinterpret_cast<const int2 *>(A.nc + fc + r)[1];
+        }
+    }
     double acc = 0.0;
-    for (int c = fc; c < end; ++c) {
-        if (A.t_nc[c] > 0) {
-            acc = __dadd_rn(acc, __ldcg(A.in_sum + 4 * (size_t)A.t_int[c] + j));
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        if (r >= nch) break;
+        if ((inner >> r) & 1) {
+            acc = __dadd_rn(acc, v[r]);
         } else {
-            const int p1 = A.t_fp[c] + A.t_np[c];
+            const int p1 = leaf[r].x + leaf[r].y;
 #pragma unroll 4
-            for (int p = A.t_fp[c]; p < p1; ++p) {
-                const double *r = A.xm + 4 * (size_t)p;
-                const double mp = __ldg(r + 3);
-                const double xv = j == 0 ? 1.0 : __ldg(r + j - 1);
+            for (int p = leaf[r].x; p < p1; ++p) {
+                const double *q = A.xm + 4 * (size_t)p;
+                const double mp = __ldg(q + 3);
+                const double xv = j == 0 ? 1.0 : __ldg(q + j - 1);
                 acc = __dadd_rn(acc, __dmul_rn(mp, xv));
             }
         }
     }
-    A.in_sum[4 * (size_t)ii + j] = acc;
+    A.t_sum[4 * (size_t)id + j] = acc;
     const double M = __shfl_sync(gmask, acc, 0, 4);
     const double cj = __ddiv_rn(acc, M);   // lanes 1..3: coordinate j - 1 of the centre
-    const int id = A.in_id[ii];
     float hj = 0.0f, lj = 0.0f;
     if (j == 0) {
         A.t_mass[id] = M;
     } else {
-        A.t_com[3 * id + j - 1] = cj;
+        A.t_com[3 * (size_t)id + j - 1] = cj;
         split_df(__dsub_rn(cj, A.frame[j - 1]), hj, lj);
     }
     float h[3], l[3];
@@ -665,6 +671,7 @@ __device__ void multipole_node4(int ii, int j, unsigned gmask, const MultipoleAr
     if (A.nq) {
         // every lane of the group forms the same sums; lane 0 stores them
         float Q[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
         for (int c = fc; c < end; ++c) {
             const float4 ca = __ldcg(A.na + c), cb = __ldcg(A.nb + c);
             const float4 qa = __ldcg(A.nq + 2 * (size_t)c), qb = __ldcg(A.nq + 2 * (size_t)c + 1);
@@ -698,50 +705,63 @@ __global__ void __launch_bounds__(OT_THREADS) k_multipole_up(const int *__restri
     const unsigned gmask = 0xFu << ((threadIdx.x & 31) & ~3);
     const int groups = (gridDim.x * blockDim.x) >> 2;
     for (int i0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; i0 < ni; i0 += groups) {
-        const int fc0 = A.in_fc[i0];
-        const int nch0 = A.in_nchild[i0];
-        bool bottom = true;
-        for (int c = fc0; c < fc0 + nch0; ++c) bottom = bottom && A.t_nc[c] == 0;
-        if (!bottom) continue;
-        int ii = i0;
+        int4 rec = A.in_rec[i0];
+        if (rec.y >> 8) continue;   // has internal children
         for (;;) {
-            multipole_node4(ii, j, gmask, A);
-            const int p = A.nd_parent[A.in_node[ii]];
+            const int p = rec.z;
+            const int4 up = p >= 0 ? A.in_rec[p] : make_int4(0, 0, 0, 0);
+            multipole_node4(rec, j, gmask, A);
             if (p < 0) break;
-            const int fc = A.in_fc[p];
-            const int nch = A.in_nchild[p];
-            int internal = 0;
-            for (int c = fc; c < fc + nch; ++c) internal += A.t_nc[c] > 0 ? 1 : 0;
             // each lane's writes are visible before lane 0 counts the group in
             __threadfence();
             __syncwarp(gmask);
             int arrived = 0;
             if (j == 0) arrived = atomicAdd(&A.in_arrive[p], 1);
             arrived = __shfl_sync(gmask, arrived, 0, 4);
-            if (arrived != internal - 1) break;
+            if (arrived != __popc(up.y >> 8) - 1) break;
             __threadfence();
-            ii = p;
+            rec = up;
         }
     }
 }
 
-// Leaves with their own mass and centre of mass (non-compat trees), their walk
-// records, and, when nq is not null, their quadrupole sum_p m (3 d d^T - |d|^2 I)
-// about the centre of mass, from the particles' (hi, lo) FP32 pairs.
-__global__ void k_leaf_multipoles(const int *__restrict__ ctr, MultipoleArgs A,
-                                  const float4 *__restrict__ pa, const float4 *__restrict__ pb)
+// Every node: its walk record (first child, children, first particle,
+// particles) and the membership key the per-particle walks read.
+// Leaves get their own mass and centre of mass (non-compat trees; zero in a
+// compat tree), their walk records, and, when nq is not null, their quadrupole
+// sum_p m (3 d d^T - |d|^2 I) about the centre of mass, from the particles'
+// (hi, lo) FP32 pairs.
+__global__ void k_leaf_multipoles(const int *__restrict__ ctr, int compat, MultipoleArgs A,
+                                  const float4 *__restrict__ pa, const float4 *__restrict__ pb,
+                                  const uint64_t *__restrict__ keys, const int *__restrict__ sidx,
+                                  const int *__restrict__ t_np, const int *__restrict__ t_fp,
+                                  const int *__restrict__ t_int, int *__restrict__ t_nc,
+                                  int *__restrict__ t_fc, int4 *__restrict__ nc,
+                                  uint64_t *__restrict__ nkey)
 {
     const int nn = tree_nodes(ctr);
     for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < nn; id += gridDim.x * blockDim.x) {
-        if (A.t_nc[id] > 0) continue;
-        const int fp = A.t_fp[id], np = A.t_np[id];
-        double M = 0.0, S0 = 0.0, S1 = 0.0, S2 = 0.0;
-        add_particles(A.xm, fp, np, M, S0, S1, S2);
-        const double c0 = __ddiv_rn(S0, M), c1 = __ddiv_rn(S1, M), c2 = __ddiv_rn(S2, M);
+        const int fp = t_fp[id], np = t_np[id], ii = t_int[id];
+        const int2 kids = ii >= 0 ? *reinterpret_cast<const int2 *>(A.in_rec + ii) : make_int2(-1, 0);
+        t_fc[id] = kids.x;
+        t_nc[id] = kids.y & 255;
+        nc[id] = make_int4(kids.x, kids.y & 255, fp, np);
+        // the reference's membership test reads keys[sorted_indices[first]]
+        // from the sorted key array (src/acceleration_barnes_hut.c:145)
+        nkey[id] = compat ? keys[sidx[fp]] : keys[fp];
+        if (ii >= 0) continue;
+        double M = 0.0, c0 = 0.0, c1 = 0.0, c2 = 0.0;
+        if (!compat) {
+            double S0 = 0.0, S1 = 0.0, S2 = 0.0;
+            add_particles(A.xm, fp, np, M, S0, S1, S2);
+            c0 = __ddiv_rn(S0, M);
+            c1 = __ddiv_rn(S1, M);
+            c2 = __ddiv_rn(S2, M);
+        }
         A.t_mass[id] = M;
-        A.t_com[3 * id + 0] = c0;
-        A.t_com[3 * id + 1] = c1;
-        A.t_com[3 * id + 2] = c2;
+        A.t_com[3 * (size_t)id + 0] = c0;
+        A.t_com[3 * (size_t)id + 1] = c1;
+        A.t_com[3 * (size_t)id + 2] = c2;
         float h[3], l[3];
         write_node_record(id, M, c0, c1, c2, A.t_depth[id], A.frame, A.na, A.nb, h, l);
         if (A.nq) {
@@ -754,34 +774,6 @@ __global__ void k_leaf_multipoles(const int *__restrict__ ctr, MultipoleArgs A,
             }
             store_quad(A.nq, id, Q);
         }
-    }
-}
-
-// Walk arrays of every node: (first child, children, first particle,
-// particles), the membership key, and the records of the nodes whose
-// multipoles the kernels above did not compute -- the zero-mass leaves of a
-// compat tree.
-__global__ void k_walk_nodes(const int *__restrict__ ctr, int compat, const double *__restrict__ frame,
-                             const uint64_t *__restrict__ keys, const int *__restrict__ sidx,
-                             const int *__restrict__ t_np, const int *__restrict__ t_nc,
-                             const int *__restrict__ t_fp, const int *__restrict__ t_fc,
-                             const int *__restrict__ t_depth,
-                             const double *__restrict__ t_mass, const double *__restrict__ t_com,
-                             float4 *__restrict__ na, float4 *__restrict__ nb, int4 *__restrict__ nc,
-                             uint64_t *__restrict__ nkey)
-{
-    const int nn = tree_nodes(ctr);
-    for (int id = blockIdx.x * blockDim.x + threadIdx.x; id < nn; id += gridDim.x * blockDim.x) {
-        if (compat && t_nc[id] == 0) {
-            float h[3], l[3];
-            write_node_record(id, t_mass[id], t_com[3 * id], t_com[3 * id + 1], t_com[3 * id + 2],
-                              t_depth[id], frame, na, nb, h, l);
-        }
-        const int fp = t_fp[id];
-        nc[id] = make_int4(t_fc[id], t_nc[id], fp, t_np[id]);
-        // the reference's membership test reads keys[sorted_indices[first]]
-        // from the sorted key array (src/acceleration_barnes_hut.c:145)
-        nkey[id] = compat ? keys[sidx[fp]] : keys[fp];
     }
 }
 
@@ -822,21 +814,25 @@ ErrorStatus OctreeDevice::setup(int n_, int leaf_max_, bool compat_, bool quad_)
     cap_nodes = cap;
     const size_t ci = (size_t)cap * sizeof(int);
     GS_TRY(ctr.reserve(CTR_SIZE * sizeof(int)));
-    GS_CUDA(cudaMemset(ctr.p, 0, CTR_SIZE * sizeof(int)));   // status word starts clear
+    int c0[CTR_SIZE] = {};   // status word clear, no CTA counted
+    c0[CTR_N] = n;
+    GS_CUDA(cudaMemcpy(ctr.p, c0, sizeof(c0), cudaMemcpyHostToDevice));
     GS_TRY(frame.reserve(8 * sizeof(double)));
     GS_TRY(bbox_part.reserve((size_t)BBOX_BLOCKS * 6 * sizeof(double)));
     GS_TRY(keys.reserve((size_t)n * sizeof(uint64_t)));
     GS_TRY(sidx.reserve((size_t)n * sizeof(int)));
-    DBuf *ints[] = {&nd_start, &nd_count, &nd_depth, &nd_parent, &nd_rank, &nd_int, &in_node,
-                    &in_nchild, &in_fc, &in_id, &in_order, &t_np, &t_nc, &t_fp, &t_fc, &t_depth,
-                    &t_int};
+    DBuf *ints[] = {&in_nch, &in_arrive, &t_np, &t_nc, &t_fp, &t_fc, &t_depth, &t_int};
     for (DBuf *b : ints) GS_TRY(b->reserve(ci));
-    GS_TRY(in_key.reserve((size_t)cap * sizeof(uint64_t)));
-    GS_TRY(scan_tiles.reserve((size_t)((cap + SCAN_TILE - 1) / SCAN_TILE + 1) * sizeof(unsigned)));
+    GS_TRY(pre_of.reserve((size_t)n * sizeof(int)));
+    GS_TRY(in_sd.reserve((size_t)cap * sizeof(int2)));
+    GS_TRY(in_end.reserve((size_t)cap * 8 * sizeof(int)));
+    GS_TRY(in_rec.reserve((size_t)cap * sizeof(int4)));
+    GS_TRY(scan_tiles.reserve(
+        (size_t)(std::max((n + TC_TILE - 1) / TC_TILE, (cap + TN_TILE - 1) / TN_TILE) + 1) *
+        sizeof(unsigned)));
     GS_TRY(t_mass.reserve((size_t)cap * sizeof(double)));
     GS_TRY(t_com.reserve((size_t)cap * 3 * sizeof(double)));
-    GS_TRY(in_sum.reserve((size_t)cap * 4 * sizeof(double)));
-    GS_TRY(in_arrive.reserve(ci));
+    GS_TRY(t_sum.reserve((size_t)cap * 4 * sizeof(double)));
     GS_TRY(w_na.reserve((size_t)cap * sizeof(float4)));
     GS_TRY(w_nb.reserve((size_t)cap * sizeof(float4)));
     GS_TRY(w_nc.reserve((size_t)cap * sizeof(int4)));
@@ -853,18 +849,15 @@ ErrorStatus OctreeDevice::setup(int n_, int leaf_max_, bool compat_, bool quad_)
         GS_TRY(t_parent.reserve((size_t)cap * sizeof(int)));
         GS_TRY(leaf_of.reserve((size_t)n * sizeof(int)));
     }
-    GS_TRY(sorter.reserve(std::max(n, cap)));
+    GS_TRY(sorter.reserve(n));
     return ok();
 }
 
 int OctreeDevice::launches_per_build() const
 {
-    // bbox 2, morton 1, sort, init 1, levels 2*21, keys 1, sort, fc 3,
-    // number 1, multipoles 1 (+1 leaves; quadrupoles in the same launches),
-    // walk arrays 2
-    return 2 + 1 + RadixSorter::launches(63) + 1 + 42 + 1 +
-           RadixSorter::launches(internal_key_bits()) + 3 + 1 +
-           1 + (compat ? 0 : 1) + 2 + (links ? 1 : 0);
+    // bbox 2, morton 1, sort, topology 4, walk particles 1, leaves 1,
+    // multipoles 1
+    return 2 + 1 + RadixSorter::launches(63) + 4 + 1 + 1 + 1 + (links ? 1 : 0);
 }
 
 ErrorStatus OctreeDevice::build(const double *d_x, const double *d_m, cudaStream_t s,
@@ -881,9 +874,6 @@ ErrorStatus OctreeDevice::build(const double *d_x, const double *d_m, cudaStream
     k_morton<<<pb, OT_THREADS, 0, s>>>(d_x, n, frame.as<double>(), keys.as<uint64_t>(),
                                        sidx.as<int>(), misplaced.as<unsigned char>());
     if (tm_morton) GS_TRY(tm_morton->end(s));
-    k_tree_init<<<1, 32, 0, s>>>(ctr.as<int>(), n, nd_start.as<int>(), nd_count.as<int>(),
-                                 nd_depth.as<int>(), nd_parent.as<int>(), nd_rank.as<int>(),
-                                 nd_int.as<int>(), in_node.as<int>());
     GS_CUDA(cudaGetLastError());
     if (tm_sort) GS_TRY(tm_sort->begin(s));
     GS_TRY(sorter.sort(keys.as<uint64_t>(), sidx.as<int>(), ctr.as<int>() + CTR_N, n, 63,
@@ -892,58 +882,36 @@ ErrorStatus OctreeDevice::build(const double *d_x, const double *d_m, cudaStream
 
     const DeviceInfo *dev = nullptr;
     GS_TRY(device_info(&dev));
-    // Grid-stride kernels: two CTAs per SM cover the largest levels, and a
-    // small grid keeps the launches of the many small levels cheap.
-    const int grid = dev->sm_count * 2;
-    for (int d = 0; d < OCT_MAX_LEVEL; ++d) {
-        k_tree_expand<<<grid, OT_THREADS, 0, s>>>(
-            d, leaf_max, cap_nodes, keys.as<uint64_t>(), ctr.as<int>(), nd_start.as<int>(),
-            nd_count.as<int>(), nd_depth.as<int>(), nd_parent.as<int>(), nd_rank.as<int>(),
-            nd_int.as<int>(), in_node.as<int>(), in_nchild.as<int>());
-        k_tree_mark<<<1, 32, 0, s>>>(d, ctr.as<int>());
-    }
-    GS_CUDA(cudaGetLastError());
-    k_internal_keys<<<grid, OT_THREADS, 0, s>>>(ctr.as<int>(), in_node.as<int>(), nd_start.as<int>(),
-                                                nd_depth.as<int>(), in_key.as<uint64_t>(),
-                                                in_order.as<int>(), in_arrive.as<int>());
-    GS_TRY(sorter.sort(in_key.as<uint64_t>(), in_order.as<int>(), ctr.as<int>() + CTR_SAFE_INTERNAL,
-                       cap_nodes, internal_key_bits(),
-                       reinterpret_cast<unsigned *>(ctr.as<int>() + CTR_STATUS), s));
-    const int tiles = (cap_nodes + SCAN_TILE - 1) / SCAN_TILE;
-    k_fc_tile_sums<<<tiles, OT_THREADS, 0, s>>>(ctr.as<int>(), in_order.as<int>(),
-                                                in_nchild.as<int>(), scan_tiles.as<unsigned>());
-    k_scan_small<<<1, 1024, 0, s>>>(scan_tiles.as<unsigned>(), tiles);
-    k_fc_apply<<<tiles, OT_THREADS, 0, s>>>(ctr.as<int>(), in_order.as<int>(), in_nchild.as<int>(),
-                                            scan_tiles.as<unsigned>(), in_fc.as<int>());
-    k_tree_number<<<grid, OT_THREADS, 0, s>>>(
-        ctr.as<int>(), compat ? 1 : 0, nd_start.as<int>(), nd_count.as<int>(), nd_depth.as<int>(),
-        nd_parent.as<int>(), nd_rank.as<int>(), nd_int.as<int>(), in_nchild.as<int>(),
-        in_fc.as<int>(), in_id.as<int>(), t_np.as<int>(), t_nc.as<int>(), t_fp.as<int>(),
-        t_fc.as<int>(), t_depth.as<int>(), t_int.as<int>(), t_mass.as<double>(),
-        t_com.as<double>());
+    // Kernels over internal nodes or nodes, whose count only the device knows,
+    // stride over them: a grid for the capacity would be mostly empty CTAs.
+    const int grid = dev->sm_count * 4;
+    const int ptiles = (n + TC_TILE - 1) / TC_TILE;
+    unsigned *tiles = scan_tiles.as<unsigned>();
+    k_tree_count<<<ptiles, OT_THREADS, 0, s>>>(keys.as<uint64_t>(), n, leaf_max, cap_nodes, tiles,
+                                               ctr.as<int>());
+    k_tree_emit<<<ptiles, OT_THREADS, 0, s>>>(keys.as<uint64_t>(), n, leaf_max, tiles,
+                                              ctr.as<int>(), pre_of.as<int>(), in_sd.as<int2>());
+    k_tree_children<<<grid, OT_THREADS, 0, s>>>(keys.as<uint64_t>(), n, cap_nodes,
+                                                in_sd.as<int2>(), in_end.as<int>(),
+                                                in_nch.as<int>(), tiles, ctr.as<int>());
+    k_tree_nodes<<<grid, OT_THREADS, 0, s>>>(n, leaf_max, tiles, ctr.as<int>(), in_sd.as<int2>(),
+                                             in_end.as<int>(), in_nch.as<int>(), pre_of.as<int>(),
+                                             in_rec.as<int4>(), in_arrive.as<int>(),
+                                             t_np.as<int>(), t_fp.as<int>(), t_depth.as<int>(),
+                                             t_int.as<int>());
     GS_CUDA(cudaGetLastError());
     if (links)
-        k_tree_links<<<grid, OT_THREADS, 0, s>>>(ctr.as<int>(), nd_start.as<int>(),
-                                                 nd_count.as<int>(), nd_parent.as<int>(),
-                                                 nd_rank.as<int>(), nd_int.as<int>(),
-                                                 in_node.as<int>(), in_fc.as<int>(),
+        k_tree_links<<<grid, OT_THREADS, 0, s>>>(ctr.as<int>(), in_rec.as<int4>(), t_np.as<int>(),
+                                                 t_fp.as<int>(), t_int.as<int>(),
                                                  t_parent.as<int>(), leaf_of.as<int>());
     MultipoleArgs A;
     A.xm = xm.as<double>();
-    A.sidx = sidx.as<int>();
-    A.in_node = in_node.as<int>();
-    A.nd_parent = nd_parent.as<int>();
-    A.in_id = in_id.as<int>();
-    A.in_fc = in_fc.as<int>();
-    A.in_nchild = in_nchild.as<int>();
-    A.t_np = t_np.as<int>();
-    A.t_nc = t_nc.as<int>();
-    A.t_fp = t_fp.as<int>();
-    A.t_int = t_int.as<int>();
+    A.in_rec = in_rec.as<int4>();
+    A.nc = w_nc.as<int4>();
     A.t_depth = t_depth.as<int>();
     A.frame = frame.as<double>();
     A.in_arrive = in_arrive.as<int>();
-    A.in_sum = in_sum.as<double>();
+    A.t_sum = t_sum.as<double>();
     A.t_mass = t_mass.as<double>();
     A.t_com = t_com.as<double>();
     A.na = w_na.as<float4>();
@@ -955,17 +923,13 @@ ErrorStatus OctreeDevice::build(const double *d_x, const double *d_m, cudaStream
                                                w_pa.as<float4>(), w_pb.as<float4>(),
                                                xm.as<double>(), misplaced.as<unsigned char>(),
                                                mlist.as<int>());
-    if (!compat)
-        k_leaf_multipoles<<<grid, OT_THREADS, 0, s>>>(ctr.as<int>(), A, w_pa.as<float4>(),
-                                                      w_pb.as<float4>());
+    k_leaf_multipoles<<<grid, OT_THREADS, 0, s>>>(
+        ctr.as<int>(), compat ? 1 : 0, A, w_pa.as<float4>(), w_pb.as<float4>(),
+        keys.as<uint64_t>(), sidx.as<int>(), t_np.as<int>(), t_fp.as<int>(), t_int.as<int>(),
+        t_nc.as<int>(), t_fc.as<int>(), w_nc.as<int4>(), w_nkey.as<uint64_t>());
     // four lanes per internal node: a larger grid, so that every node of a
     // tree of up to about 2^16 internal nodes starts at once
     k_multipole_up<<<dev->sm_count * 8, OT_THREADS, 0, s>>>(ctr.as<int>(), A);
-    k_walk_nodes<<<grid, OT_THREADS, 0, s>>>(
-        ctr.as<int>(), compat ? 1 : 0, frame.as<double>(), keys.as<uint64_t>(), sidx.as<int>(),
-        t_np.as<int>(), t_nc.as<int>(), t_fp.as<int>(), t_fc.as<int>(), t_depth.as<int>(),
-        t_mass.as<double>(), t_com.as<double>(), w_na.as<float4>(), w_nb.as<float4>(),
-        w_nc.as<int4>(), w_nkey.as<uint64_t>());
     GS_CUDA(cudaGetLastError());
     return ok();
 }

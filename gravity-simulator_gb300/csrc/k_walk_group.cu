@@ -114,41 +114,42 @@ __global__ void k_group_list(const int *__restrict__ ctr, const int4 *__restrict
                              const int *__restrict__ mlist, int2 *__restrict__ groups,
                              int *__restrict__ gctr)
 {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= tree_nodes(ctr)) return;   // no groups from an overflowed build
     const double bl = frame[4];
     const int nmis = mlist[0];
-    const int4 ci = nc[c];   // (first child, children, first particle, particles)
-    if (ci.w <= 0) return;
-    const int d = depth[c];
-    if (c == 0 && ci.w <= GW_GROUP) {
-        put_group(groups, gctr, ci.z, ci.w, d, pa, pb, bl, mlist, nmis);
-        return;
-    }
-    if (ci.w <= GW_GROUP) return;   // its own parent groups it
-    if (ci.y <= 0) {                // oversized leaf (depth limit): runs of GW_GROUP
-        for (int b = 0; b < ci.w; b += GW_GROUP)
-            put_group(groups, gctr, ci.z + b, min(GW_GROUP, ci.w - b), d, pa, pb, bl, mlist, nmis);
-        return;
-    }
-    // Runs of consecutive children of at most GW_GROUP particles each are
-    // contiguous in sorted order and lie in this cell: each run is cut into
-    // pieces of GW_GROUP particles (the last one shorter), so that groups
-    // fill the warp's lanes (children of 20, 20 and 20 particles make groups
-    // of 32 and 28, not three of 20).
-    int first = 0, count = 0;
-    for (int k = 0; k <= ci.y; ++k) {
-        const int4 ch = k < ci.y ? nc[ci.x + k] : make_int4(0, 0, 0, GW_GROUP + 1);
-        if (ch.w > GW_GROUP) {   // a child walked as its own cell, or the end
-            for (int b = 0; b < count; b += GW_GROUP)
-                put_group(groups, gctr, first + b, min(GW_GROUP, count - b), d, pa, pb, bl, mlist,
-                          nmis);
-            count = 0;
+    const int nodes = tree_nodes(ctr);   // none in an overflowed build
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nodes; c += gridDim.x * blockDim.x) {
+        const int4 ci = nc[c];   // (first child, children, first particle, particles)
+        if (ci.w <= 0) continue;
+        const int d = depth[c];
+        if (c == 0 && ci.w <= GW_GROUP) {
+            put_group(groups, gctr, ci.z, ci.w, d, pa, pb, bl, mlist, nmis);
             continue;
         }
-        if (ch.w <= 0) continue;
-        if (count == 0) first = ch.z;
-        count += ch.w;
+        if (ci.w <= GW_GROUP) continue;   // its own parent groups it
+        if (ci.y <= 0) {                  // oversized leaf (depth limit): runs of GW_GROUP
+            for (int b = 0; b < ci.w; b += GW_GROUP)
+                put_group(groups, gctr, ci.z + b, min(GW_GROUP, ci.w - b), d, pa, pb, bl, mlist, nmis);
+            continue;
+        }
+        // Runs of consecutive children of at most GW_GROUP particles each are
+        // contiguous in sorted order and lie in this cell: each run is cut into
+        // pieces of GW_GROUP particles (the last one shorter), so that groups
+        // fill the warp's lanes (children of 20, 20 and 20 particles make groups
+        // of 32 and 28, not three of 20).
+        int first = 0, count = 0;
+        for (int k = 0; k <= ci.y; ++k) {
+            const int4 ch = k < ci.y ? nc[ci.x + k] : make_int4(0, 0, 0, GW_GROUP + 1);
+            if (ch.w > GW_GROUP) {   // a child walked as its own cell, or the end
+                for (int b = 0; b < count; b += GW_GROUP)
+                    put_group(groups, gctr, first + b, min(GW_GROUP, count - b), d, pa, pb, bl, mlist,
+                              nmis);
+                count = 0;
+                continue;
+            }
+            if (ch.w <= 0) continue;
+            if (count == 0) first = ch.z;
+            count += ch.w;
+        }
     }
 }
 
@@ -634,19 +635,19 @@ ErrorStatus launch_bh_group_walk(const OctreeDevice &t, double theta, double eps
     w.gate = gate;
     w.groups = t.g_list.as<int2>();
     w.gctr = t.g_ctr.as<int>();
+    const DeviceInfo *dev = nullptr;
+    GS_TRY(device_info(&dev));
     if (reuse_groups) {
         // the list and its count stay; only the work-queue head restarts
         GS_CUDA(cudaMemsetAsync(w.gctr + 1, 0, sizeof(int), s));
     } else {
         GS_CUDA(cudaMemsetAsync(t.g_ctr.p, 0, 2 * sizeof(int), s));
-        k_group_list<<<(t.cap_nodes + 255) / 256, 256, 0, s>>>(
+        k_group_list<<<dev->sm_count * 8, 256, 0, s>>>(
             t.ctr.as<int>(), t.w_nc.as<int4>(), t.t_depth.as<int>(), t.w_pa.as<float4>(),
             t.w_pb.as<float4>(), t.frame.as<double>(), t.mlist.as<int>(), t.g_list.as<int2>(),
             w.gctr);
     }
     // persistent: every SM filled once (computed once per device)
-    const DeviceInfo *dev = nullptr;
-    GS_TRY(device_info(&dev));
     static std::atomic<int> grid_cache[kMaxDevices];
     int grid = grid_cache[dev->id].load(std::memory_order_acquire);
     if (grid == 0) {

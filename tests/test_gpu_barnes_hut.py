@@ -79,6 +79,19 @@ def test_octree_bitexact_fresh(lib, g, orc, wl, n, leaf):
     assert np.array_equal(gf["mass"], rf["mass"]) and np.array_equal(gf["com"], rf["com"])
 
 
+@pytest.mark.parametrize("n", [2047, 2048, 2049, 4097])
+@pytest.mark.parametrize("leaf", [1, 6, 5000])
+def test_octree_bitexact_at_scan_tile_edges(lib, g, orc, wl, n, leaf):
+    """Particle counts next to the 2,048-particle tile of the topology scans (leaf 6: internal
+    nodes on both sides of its 256-node tile; leaf 5000: the root's children are all leaves), with
+    coincident particles, whose chains of nodes reach depth 21, on both sides of a tile's end."""
+    x, v, m = wl.plummer(n, n + leaf)
+    order = np.argsort(orc.morton(x, *orc.bbox(x)), kind="stable")
+    x[order[2040:2046]] = x[order[2040]]
+    gt = gpu_octree(lib, g, x, m, leaf)
+    assert_same_tree(gt, orc.build_tree(x, m, leaf, True))
+
+
 def test_octree_bitexact_galaxy_collision_2097152(lib, g, orc, wl):
     """Morton keys, order and tree of the galaxy-collision workload at full
     size, bit-exact."""
