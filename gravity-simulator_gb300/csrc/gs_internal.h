@@ -177,10 +177,6 @@ class DirectRows {
     static constexpr int kernels() { return 4; }
 
   private:
-    // j-split of a launch over i_tiles row tiles: the whole number of waves
-    // of resident CTAs that needs the fewest tiles per CTA, with at most
-    // max_splits chunks.
-    void split_for(int i_tiles, int max_splits, int *splits, int *chunk) const;
     int nj_ = 0, nj_pad_ = 0, ni_pad_ = 0, jt_total_ = 0;
     long slots_ = 1;
     size_t partial_rows_ = 0;   // capacity of partial_ in (split, row) pairs

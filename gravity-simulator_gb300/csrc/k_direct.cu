@@ -14,10 +14,15 @@
 //   * each pair term is 3 FADD + 3 FFMA + rsqrt + 3 FMUL + 3 FFMA in FP32;
 //     each partial sum of 128 pair terms is added into a Kahan-compensated FP32
 //     accumulator;
-//   * the (i-tile, j-chunk) work units are sized so that their count is a
-//     whole number of waves of resident CTAs (152 SMs x occupancy); partial
-//     sums go to an FP64 scratch array [split][3][N] that a second kernel
-//     reduces in fixed order and scales by G.
+//   * the j-particles are divided in granules of 128 (the length of a plain
+//     partial sum), and a row tile's granules into units so that the last wave of
+//     resident CTAs is as full as it gets (choose_per); the units' Kahan pairs go
+//     to scratch [split][3][N], which a second kernel adds in fixed order with the
+//     FP32 rounding errors kept, and scales by G;
+//   * up to 20,480 particles the units are 64 rows by 1,024 or 2,048 terms
+//     (k_direct_run).
+//   Measured at N = 100,000: 3.76 -> 3.51 ms (57 TFLOP/s at 20 per pair term, 0.74
+//   of the FP32 FMA peak; the pair term's own ceiling is 20/24 of it).
 //
 // GRAV_GPU_PAIRWISE_FP64 (reference order): a warp per ten particles forms
 // the pair terms of all other particles, 32 at a time, and sums them in index
@@ -41,7 +46,15 @@ constexpr int DS_ITILE = DS_THREADS * DS_IPT;  // 1024
 constexpr int DS_JTILE = 1024;                 // 16 KiB of float4
 constexpr int DS_STAGES = 3;
 constexpr int DS_SMEM = DS_STAGES * DS_JTILE * 16;
-constexpr int DS_KAHAN_CHUNK = 128;            // plain FP32 partials of 128 terms
+constexpr int DS_GRANULE = 128;                // plain FP32 partials of 128 terms
+constexpr int DS_SMALL_ITILE = 2 * DS_THREADS; // rows of a unit of k_direct_small
+constexpr int DS_TILE_GRANULES = DS_JTILE / DS_GRANULE;
+constexpr int DR_WARPS = 8;                    // k_direct_run
+constexpr int DR_THREADS = 32 * DR_WARPS;
+constexpr int DR_ROWS = 64;
+// k_direct_run up to here, k_direct_sum above: at N = 20,000 159 against 164 us, at
+// 24,000 223 against 219 us.
+constexpr int DS_RUN_N = 20 * DS_JTILE;
 static_assert(DS_ITILE == DS_JTILE, "i and j tiles share the padding unit");
 
 // Padding particle: massless and far from everything (its pair terms are 0).
@@ -85,8 +98,6 @@ __device__ __forceinline__ void pair_term(const float4 q, float xi, float yi, fl
     az = fmaf(dz, s, az);
 }
 
-// One (i-tile, j-chunk) work unit: the 1024 i-particles start at pi_tile;
-// partial sums go to partial[split][3][plane] at rows itile*1024 + ...
 // Two i-particles per instruction: Blackwell's paired FP32 operations
 // (add / mul / fma on float2, each lane rounded as the scalar operation)
 // carry the pair terms of particles (k, k+1) together, halving the FP32
@@ -115,17 +126,21 @@ __device__ __forceinline__ void pair_term2(const float4 q, float2 nxi, float2 ny
     az = __ffma2_rn(dz, sc, az);
 }
 
+// One work unit: the IPT * 128 i-particles from pi_tile against the j-particles
+// of granules [g0, g1) (128 particles each, the length of a plain FP32 partial
+// sum); the unit compensates over its granules, and its Kahan pairs go to
+// partial[split][3][plane] at rows row0 + ...
 template <bool SOFT>
 __device__ __forceinline__ void direct_sum_unit(const float4 *__restrict__ pi_tile,
                                                 const float4 *__restrict__ pj, int plane,
-                                                int itile, int split, int jt_per_chunk,
-                                                int jt_total, float eps2,
-                                                double *__restrict__ partial,
+                                                int row0, int split, int g0, int g1, float eps2,
+                                                float2 *__restrict__ partial,
                                                 unsigned *__restrict__ status, float4 *sj,
                                                 uint64_t *full_bar)
 {
-    const int jt0 = split * jt_per_chunk;
-    const int ntiles = min(jt_total, jt0 + jt_per_chunk) - jt0;
+    const int nj = (g1 - g0) * DS_GRANULE;
+    const int ntiles = (nj + DS_JTILE - 1) / DS_JTILE;
+    const float4 *src = pj + (size_t)g0 * DS_GRANULE;
 
     float xi[DS_IPT], yi[DS_IPT], zi[DS_IPT];
 #pragma unroll
@@ -141,14 +156,17 @@ __device__ __forceinline__ void direct_sum_unit(const float4 *__restrict__ pi_ti
         mbar_fence_init();
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        const int pre = min(DS_STAGES, ntiles);
-        for (int s = 0; s < pre; ++s) {
-            mbar_expect_tx(&full_bar[s], DS_JTILE * 16);
-            bulk_g2s(sj + s * DS_JTILE, pj + (size_t)(jt0 + s) * DS_JTILE, DS_JTILE * 16,
-                     &full_bar[s]);
-        }
-    }
+    // tile u: DS_JTILE particles, or what is left (whole granules, so every
+    // copy is a multiple of 2 KiB)
+    auto fetch = [&](int u) {
+        const unsigned bytes = (unsigned)min(DS_JTILE, nj - u * DS_JTILE) * 16u;
+        mbar_expect_tx(&full_bar[u % DS_STAGES], bytes);
+        bulk_g2s(sj + (u % DS_STAGES) * DS_JTILE, src + (size_t)u * DS_JTILE, bytes,
+                 &full_bar[u % DS_STAGES]);
+    };
+    int issued = min(DS_STAGES, ntiles);
+    if (threadIdx.x == 0)
+        for (int u = 0; u < issued; ++u) fetch(u);
 
     float sx[DS_IPT], sy[DS_IPT], sz[DS_IPT], cx[DS_IPT], cy[DS_IPT], cz[DS_IPT];
 #pragma unroll
@@ -166,7 +184,6 @@ __device__ __forceinline__ void direct_sum_unit(const float4 *__restrict__ pi_ti
     }
     const float2 eps2v = make_float2(eps2, eps2);
 
-    int issued = min(DS_STAGES, ntiles);
     int t = 0;
     for (; t < ntiles; ++t) {
         const int st = t % DS_STAGES;
@@ -177,13 +194,14 @@ __device__ __forceinline__ void direct_sum_unit(const float4 *__restrict__ pi_ti
             break;
         }
         const float4 *tile = sj + st * DS_JTILE;
-        for (int j0 = 0; j0 < DS_JTILE; j0 += DS_KAHAN_CHUNK) {
+        const int jn = min(DS_JTILE, nj - t * DS_JTILE);
+        for (int j0 = 0; j0 < jn; j0 += DS_GRANULE) {
             float2 ax[DS_IPT / 2], ay[DS_IPT / 2], az[DS_IPT / 2];
 #pragma unroll
             for (int k = 0; k < DS_IPT / 2; ++k)
                 ax[k] = ay[k] = az[k] = make_float2(0.0f, 0.0f);
 #pragma unroll 8
-            for (int j = j0; j < j0 + DS_KAHAN_CHUNK; ++j) {
+            for (int j = j0; j < j0 + DS_GRANULE; ++j) {
                 const float4 q = tile[j];
 #pragma unroll
                 for (int k = 0; k < DS_IPT / 2; ++k)
@@ -200,10 +218,8 @@ __device__ __forceinline__ void direct_sum_unit(const float4 *__restrict__ pi_ti
             }
         }
         __syncthreads();   // every thread is done with stage st
-        if (threadIdx.x == 0 && issued < ntiles) {
-            mbar_expect_tx(&full_bar[st], DS_JTILE * 16);
-            bulk_g2s(sj + st * DS_JTILE, pj + (size_t)(jt0 + issued) * DS_JTILE, DS_JTILE * 16,
-                     &full_bar[st]);
+        if (issued < ntiles) {
+            if (threadIdx.x == 0) fetch(issued);
             ++issued;
         }
     }
@@ -217,29 +233,112 @@ __device__ __forceinline__ void direct_sum_unit(const float4 *__restrict__ pi_ti
         return;
     }
 
-    double *out = partial + (size_t)split * 3 * (size_t)plane;
+    float2 *out = partial + (size_t)split * 3 * (size_t)plane;
 #pragma unroll
     for (int k = 0; k < DS_IPT; ++k) {
-        const size_t i = (size_t)itile * DS_ITILE + k * DS_THREADS + threadIdx.x;
-        out[0 * (size_t)plane + i] = (double)sx[k] - (double)cx[k];
-        out[1 * (size_t)plane + i] = (double)sy[k] - (double)cy[k];
-        out[2 * (size_t)plane + i] = (double)sz[k] - (double)cz[k];
+        const size_t i = (size_t)row0 + k * DS_THREADS + threadIdx.x;
+        out[0 * (size_t)plane + i] = make_float2(sx[k], cx[k]);
+        out[1 * (size_t)plane + i] = make_float2(sy[k], cy[k]);
+        out[2 * (size_t)plane + i] = make_float2(sz[k], cz[k]);
     }
 }
 
+// A unit's Kahan pair (s, c), whose value is s - c, added to the running sum
+// h + l by Knuth's two-sum (exact), the small parts gathered in l.
+__device__ __forceinline__ void add_pair(float &h, float &l, const float2 sc)
+{
+    const float t = __fadd_rn(h, sc.x);
+    const float b = __fsub_rn(t, h);
+    const float e = __fadd_rn(__fsub_rn(h, __fsub_rn(t, b)), __fsub_rn(sc.x, b));
+    l = __fadd_rn(l, __fsub_rn(e, sc.y));
+    h = t;
+}
+
+// Work units: unit (itile, split) takes granules [split * per, (split + 1) * per).
 template <bool SOFT>
 __global__ void __launch_bounds__(DS_THREADS, 2)
-k_direct_sum(const float4 *__restrict__ pj, int n_pad, int i_tiles, int jt_per_chunk,
-             int jt_total, float eps2, double *__restrict__ partial,
-             unsigned *__restrict__ status)
+k_direct_sum(const float4 *__restrict__ pj, int n_pad, int i_tiles, int per, int granules,
+             float eps2, float2 *__restrict__ partial, unsigned *__restrict__ status)
 {
     extern __shared__ __align__(128) unsigned char ds_smem[];
     __shared__ __align__(8) uint64_t full_bar[DS_STAGES];
     const int itile = blockIdx.x % i_tiles;
     const int split = blockIdx.x / i_tiles;
-    direct_sum_unit<SOFT>(pj + (size_t)itile * DS_ITILE, pj, n_pad, itile, split, jt_per_chunk,
-                          jt_total, eps2, partial, status, reinterpret_cast<float4 *>(ds_smem),
-                          full_bar);
+    const int row0 = itile * DS_ITILE;
+    direct_sum_unit<SOFT>(pj + row0, pj, n_pad, row0, split, split * per,
+                          min(granules, (split + 1) * per), eps2, partial, status,
+                          reinterpret_cast<float4 *>(ds_smem), full_bar);
+}
+
+// Direct sum of a system too small to give every SM units of 1024 rows.  A
+// unit is 64 rows (two per lane) by one compensated run of `run` granules: the
+// eight warps take a granule each, and the run is then added up in granule order
+// from shared memory, so that the Kahan sequence of a row is that of a thread that
+// takes the granules one after the other, and the units are small enough to fill
+// the GPU (12,000 particles: 2,256 units where units of 1024 x 1024 made 144).
+// Two rows per lane beat four and eight at every size (58 against 62 and 63 us at
+// N = 12,000): the FP32 pipe has enough warps, and smaller units waste less at the
+// end.  With packing and reduction, in a graph: 10.1 us at N = 1,500 (72 before),
+// 22 at 6,000, 62.5 at 12,000 (76 before), 159 at 20,000 (k_direct_sum: 164).
+template <bool SOFT>
+__global__ void __launch_bounds__(DR_THREADS)
+k_direct_run(const float4 *__restrict__ pj, int n_pad, int i_tiles, int run, int granules,
+             float eps2, float2 *__restrict__ partial, unsigned *__restrict__ status)
+{
+    __shared__ __align__(128) float4 sj[DS_JTILE];
+    __shared__ float part[DR_WARPS][3][DR_ROWS];
+    __shared__ __align__(8) uint64_t bar;
+    static_assert(DR_WARPS * DS_GRANULE == DS_JTILE && 3 * DR_ROWS <= DR_THREADS,
+                  "a granule per warp, a thread per row and component");
+    const int itile = blockIdx.x % i_tiles, r = blockIdx.x / i_tiles;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int row0 = itile * DR_ROWS;
+    const int g0 = r * run, g1 = min(granules, g0 + run);
+    if (threadIdx.x == 0) {
+        mbar_init(&bar, 1);
+        mbar_fence_init();
+    }
+    __syncthreads();
+    const float4 p0 = pj[row0 + lane], p1 = pj[row0 + 32 + lane];
+    const float2 nx = make_float2(-p0.x, -p1.x), ny = make_float2(-p0.y, -p1.y),
+                 nz = make_float2(-p0.z, -p1.z), e2 = make_float2(eps2, eps2);
+    const int e = threadIdx.x;   // this thread's component and row of the run's sums
+    float s = 0.0f, c = 0.0f;
+    unsigned parity = 0;
+    for (int g = g0; g < g1; g += DR_WARPS, parity ^= 1u) {
+        const int here = min(DR_WARPS, g1 - g);
+        if (threadIdx.x == 0) {
+            mbar_expect_tx(&bar, here * DS_GRANULE * 16);
+            bulk_g2s(sj, pj + (size_t)g * DS_GRANULE, here * DS_GRANULE * 16, &bar);
+        }
+        const bool ready = mbar_wait(&bar, parity);
+        if (!__syncthreads_and(ready)) {
+            if (threadIdx.x == 0) atomicOr(status, ST_WAIT_TIMEOUT);
+            // the copy lands before the CTA exits
+            if (threadIdx.x == 0) (void)mbar_wait(&bar, parity);
+            __syncthreads();
+            return;
+        }
+        if (w < here) {
+            float2 ax = make_float2(0.f, 0.f), ay = ax, az = ax;
+            const float4 *tile = sj + w * DS_GRANULE;
+#pragma unroll 8
+            for (int j = 0; j < DS_GRANULE; ++j) pair_term2<SOFT>(tile[j], nx, ny, nz, e2, ax, ay, az);
+            part[w][0][lane] = ax.x;
+            part[w][0][32 + lane] = ax.y;
+            part[w][1][lane] = ay.x;
+            part[w][1][32 + lane] = ay.y;
+            part[w][2][lane] = az.x;
+            part[w][2][32 + lane] = az.y;
+        }
+        __syncthreads();
+        if (e < 3 * DR_ROWS)
+            for (int q = 0; q < here; ++q) kahan_add(s, c, part[q][e / DR_ROWS][e % DR_ROWS]);
+        __syncthreads();   // the tile and the partials are free again
+    }
+    if (e < 3 * DR_ROWS)
+        partial[((size_t)r * 3 + e / DR_ROWS) * (size_t)n_pad + row0 + e % DR_ROWS] =
+            make_float2(s, c);
 }
 
 // Direct sum for a separate list of target particles pi [ni_pad] (padded to
@@ -248,35 +347,40 @@ k_direct_sum(const float4 *__restrict__ pj, int n_pad, int i_tiles, int jt_per_c
 template <bool SOFT>
 __global__ void __launch_bounds__(DS_THREADS, 2)
 k_direct_rows(const float4 *__restrict__ pi, int ni_pad, const float4 *__restrict__ pj,
-              int i_tiles, int jt_per_chunk, int jt_total, float eps2,
-              double *__restrict__ partial, unsigned *__restrict__ status)
+              int i_tiles, int per, int granules, float eps2, float2 *__restrict__ partial,
+              unsigned *__restrict__ status)
 {
     extern __shared__ __align__(128) unsigned char ds_smem[];
     __shared__ __align__(8) uint64_t full_bar[DS_STAGES];
     const int itile = blockIdx.x % i_tiles;
     const int split = blockIdx.x / i_tiles;
-    direct_sum_unit<SOFT>(pi + (size_t)itile * DS_ITILE, pj, ni_pad, itile, split, jt_per_chunk,
-                          jt_total, eps2, partial, status, reinterpret_cast<float4 *>(ds_smem),
-                          full_bar);
+    const int row0 = itile * DS_ITILE;
+    direct_sum_unit<SOFT>(pi + row0, pj, ni_pad, row0, split, split * per,
+                          min(granules, (split + 1) * per), eps2, partial, status,
+                          reinterpret_cast<float4 *>(ds_smem), full_bar);
 }
 
-// a_i = G * sum_s partial[s][.][i], summed in split order.
-__global__ void k_reduce_splits(const double *__restrict__ partial, int splits, int n,
+// Sum over the splits, in split order, of component k of row i.  The pairs
+// are added in FP32 with their rounding errors kept: FP64 conversions and adds
+// cost a whole warp's time on a pipe of 1/64 of the FP32 rate (72 of them per
+// thread in a unit's epilogue took 4 us of a 65 us launch at N = 12,000).
+__device__ __forceinline__ double reduce_row(const float2 *__restrict__ partial, int splits,
+                                             size_t plane, int k, int i)
+{
+    const float2 *p = partial + k * plane + i;
+    float h = 0.0f, l = 0.0f;
+#pragma unroll 8
+    for (int q = 0; q < splits; ++q) add_pair(h, l, p[(size_t)q * 3 * plane]);
+    return (double)h + (double)l;
+}
+
+// a_i = G * sum_s partial[s][.][i]; a thread per component.
+__global__ void k_reduce_splits(const float2 *__restrict__ partial, int splits, int n,
                                 int n_pad, double G, double *__restrict__ a)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const size_t plane = (size_t)n_pad;
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-    for (int s = 0; s < splits; ++s) {
-        const double *p = partial + (size_t)s * 3 * plane;
-        s0 += p[i];
-        s1 += p[plane + i];
-        s2 += p[2 * plane + i];
-    }
-    a[3 * i + 0] = G * s0;
-    a[3 * i + 1] = G * s1;
-    a[3 * i + 2] = G * s2;
+    const int k = blockIdx.y;
+    if (i < n) a[3 * (size_t)i + k] = G * reduce_row(partial, splits, n_pad, k, i);
 }
 
 // FP64, reference operation order (see file comment).  One warp per PER
@@ -349,6 +453,62 @@ k_direct_fp64_reference_order(const double *__restrict__ x, const double *__rest
 // ------------------------------------------------------------------------
 namespace {
 
+// Granules per unit of a direct sum: the row tiles' granules are divided by the
+// time a unit takes.  Whole waves of resident CTAs take a unit each; in the last,
+// partial wave an SM whose slots are not all taken gives the CTAs it has a larger
+// share of its pipes, so a wave that is a quarter full costs less than a full one.
+// A unit is charged 0.15 granules to start and end; every split adds the traffic
+// of its partial sums (48 bytes a row, written and read) where it has its own.
+// One granule of a full wave takes 13.9 us, and this form follows the sweep of 1
+// to 64 splits at N = 12,000 to 100,000 within 3 %.  (Counting whole waves only
+// took 232 us instead of 220 at N = 24,000.)
+int choose_per(int i_tiles, int granules, int per_sm, long slots, double split_cost)
+{
+    int best_per = granules;
+    double best = 1e300;
+    for (int s = 1; s <= std::min(granules, 64); ++s) {
+        const int per = (granules + s - 1) / s;
+        const int used = (granules + per - 1) / per;
+        const long units = (long)i_tiles * used;
+        const long left = units % slots;
+        const double filled = std::ceil((double)left / (double)slots * per_sm) / per_sm;
+        const double waves = (double)(units / slots) + (left ? 0.1 + 0.9 * filled : 0.0);
+        const double cost = waves * (0.5 * (per + (double)granules / used) + 0.15) + split_cost * used;
+        if (cost < best - 1e-9) {
+            best = cost;
+            best_per = per;
+        }
+    }
+    return best_per;
+}
+
+// Splits and source tiles per split where a unit takes whole tiles: the whole
+// number of waves that needs the fewest tiles per CTA.
+void choose_tiles(int i_tiles, int tiles, long slots, int max_splits, int *splits, int *chunk)
+{
+    double best = 1e300;
+    for (int s = 1; s <= std::min(tiles, max_splits); ++s) {
+        const int c = (tiles + s - 1) / s;
+        const int used = (tiles + c - 1) / c;
+        const double cost = (double)(((long)i_tiles * used + slots - 1) / slots) * (c + 0.25);
+        if (cost < best - 1e-9) {
+            best = cost;
+            *splits = used;
+            *chunk = c;
+        }
+    }
+}
+
+// Resident CTAs of a kernel on the current device.
+template <class Kernel>
+ErrorStatus resident_ctas(Kernel kernel, int *per_sm)
+{
+    GS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DS_SMEM));
+    GS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, DS_THREADS, DS_SMEM));
+    *per_sm = std::max(*per_sm, 1);
+    return ok();
+}
+
 class DirectEngine final : public Engine {
   public:
     explicit DirectEngine(bool fp64) : fp64_(fp64) {}
@@ -361,38 +521,22 @@ class DirectEngine final : public Engine {
         if (fp64_) return ok();
         const DeviceInfo *dev = nullptr;
         GS_TRY(device_info(&dev));
-        n_pad_ = ((n + DS_JTILE - 1) / DS_JTILE) * DS_JTILE;
-        i_tiles_ = n_pad_ / DS_ITILE;
-        jt_total_ = n_pad_ / DS_JTILE;
-        int per_sm = 0;
-        GS_CUDA(cudaFuncSetAttribute(k_direct_sum<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     DS_SMEM));
-        GS_CUDA(cudaFuncSetAttribute(k_direct_sum<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     DS_SMEM));
-        GS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_direct_sum<true>, DS_THREADS,
-                                                              DS_SMEM));
-        per_sm = std::max(per_sm, 1);
-        const long slots = (long)dev->sm_count * per_sm;
-        // Choose the j-split count: minimise (waves x tiles per unit) with a
-        // small per-unit overhead, so the last wave is (nearly) full.
-        int best_s = 1;
-        double best_cost = 1e300;
-        const int max_s = std::min(jt_total_, 64);
-        for (int s = 1; s <= max_s; ++s) {
-            const int chunk = (jt_total_ + s - 1) / s;
-            const int used = (jt_total_ + chunk - 1) / chunk;   // non-empty splits
-            const long units = (long)i_tiles_ * used;
-            const long waves = (units + slots - 1) / slots;
-            const double cost = (double)waves * (chunk + 0.25);
-            if (cost < best_cost - 1e-9) {
-                best_cost = cost;
-                best_s = used;
-                jt_per_chunk_ = chunk;
-            }
+        n_pad_ = ((n + DS_ITILE - 1) / DS_ITILE) * DS_ITILE;
+        granules_ = (n + DS_GRANULE - 1) / DS_GRANULE;
+        if (n <= DS_RUN_N) {
+            // compensated runs of 1,024 terms, 2,048 from 17,409 particles on
+            per_ = (n <= 17 * DS_JTILE ? 1 : 2) * DS_TILE_GRANULES;
+            i_tiles_ = (n + DR_ROWS - 1) / DR_ROWS;
+        } else {
+            int per_sm = 1;
+            GS_TRY(resident_ctas(k_direct_sum<true>, &per_sm));
+            GS_TRY(resident_ctas(k_direct_sum<false>, &per_sm));
+            i_tiles_ = n_pad_ / DS_ITILE;
+            per_ = choose_per(i_tiles_, granules_, per_sm, (long)dev->sm_count * per_sm, 7e-7 * n);
         }
-        splits_ = best_s;
+        splits_ = (granules_ + per_ - 1) / per_;
         GS_TRY(pj_.reserve((size_t)n_pad_ * sizeof(float4)));
-        GS_TRY(partial_.reserve((size_t)splits_ * 3 * n_pad_ * sizeof(double)));
+        GS_TRY(partial_.reserve((size_t)splits_ * 3 * n_pad_ * sizeof(float2)));
         GS_TRY(status_.reserve(sizeof(unsigned)));
         GS_CUDA(cudaMemset(status_.p, 0, sizeof(unsigned)));
         return ok();
@@ -421,24 +565,27 @@ class DirectEngine final : public Engine {
             if (timer) GS_TRY(timer->end(s));
             return ok();
         }
+        const float eps2 = (float)(eps_ * eps_);
+        const int grid = i_tiles_ * splits_;
+        const bool soft = eps2 > 0.0f;
         k_pack_float4<<<(n_pad_ + 255) / 256, 256, 0, s>>>(d_x, d_m, n_, n_pad_, c_[0], c_[1], c_[2],
                                                            pj_.as<float4>());
         GS_CUDA(cudaGetLastError());
-        const float eps2 = (float)(eps_ * eps_);
-        const int grid = i_tiles_ * splits_;
         if (timer) GS_TRY(timer->begin(s));
-        if (eps2 > 0.0f)
-            k_direct_sum<true><<<grid, DS_THREADS, DS_SMEM, s>>>(
-                pj_.as<float4>(), n_pad_, i_tiles_, jt_per_chunk_, jt_total_, eps2,
-                partial_.as<double>(), status_.as<unsigned>());
-        else
-            k_direct_sum<false><<<grid, DS_THREADS, DS_SMEM, s>>>(
-                pj_.as<float4>(), n_pad_, i_tiles_, jt_per_chunk_, jt_total_, eps2,
-                partial_.as<double>(), status_.as<unsigned>());
+        if (n_ <= DS_RUN_N) {
+            auto run = soft ? k_direct_run<true> : k_direct_run<false>;
+            run<<<grid, DR_THREADS, 0, s>>>(pj_.as<float4>(), n_pad_, i_tiles_, per_, granules_, eps2,
+                                            partial_.as<float2>(), status_.as<unsigned>());
+        } else {
+            auto sum = soft ? k_direct_sum<true> : k_direct_sum<false>;
+            sum<<<grid, DS_THREADS, DS_SMEM, s>>>(pj_.as<float4>(), n_pad_, i_tiles_, per_, granules_,
+                                                  eps2, partial_.as<float2>(),
+                                                  status_.as<unsigned>());
+        }
         GS_CUDA(cudaGetLastError());
         if (timer) GS_TRY(timer->end(s));
-        k_reduce_splits<<<(n_ + 255) / 256, 256, 0, s>>>(partial_.as<double>(), splits_, n_, n_pad_,
-                                                         G_, d_a);
+        k_reduce_splits<<<dim3((n_ + 127) / 128, 3), 128, 0, s>>>(partial_.as<float2>(), splits_, n_,
+                                                                  n_pad_, G_, d_a);
         GS_CUDA(cudaGetLastError());
         return ok();
     }
@@ -458,7 +605,7 @@ class DirectEngine final : public Engine {
 
   private:
     bool fp64_;
-    int n_ = 0, n_pad_ = 0, i_tiles_ = 0, jt_total_ = 0, jt_per_chunk_ = 1, splits_ = 1;
+    int n_ = 0, n_pad_ = 0, i_tiles_ = 0, granules_ = 1, per_ = 1, splits_ = 1;
     double G_ = 1.0, eps_ = 0.0;
     double c_[3] = {0.0, 0.0, 0.0};
     DBuf pj_, partial_, status_;
@@ -498,50 +645,29 @@ __global__ void k_gather_rows(const float4 *__restrict__ pj, const int *__restri
     pi[r] = r < nrows ? pj[rows[r]] : make_float4(kPadPos, kPadPos, kPadPos, 0.0f);
 }
 
-void DirectRows::split_for(int i_tiles, int max_splits, int *splits, int *chunk) const
-{
-    double best = 1e300;
-    *splits = 1;
-    *chunk = jt_total_;
-    for (int s = 1; s <= std::min(jt_total_, max_splits); ++s) {
-        const int c = (jt_total_ + s - 1) / s;
-        const int used = (jt_total_ + c - 1) / c;
-        const long units = (long)i_tiles * used;
-        const double cost = (double)((units + slots_ - 1) / slots_) * (c + 0.25);
-        if (cost < best - 1e-9) {
-            best = cost;
-            *splits = used;
-            *chunk = c;
-        }
-    }
-}
-
 ErrorStatus DirectRows::setup(int nj, int max_rows)
 {
     const DeviceInfo *dev = nullptr;
     GS_TRY(device_info(&dev));
     nj_ = nj;
     nj_pad_ = ((nj + DS_JTILE - 1) / DS_JTILE) * DS_JTILE;
-    ni_pad_ = ((max_rows + DS_ITILE - 1) / DS_ITILE) * DS_ITILE;
     jt_total_ = nj_pad_ / DS_JTILE;
-    int per_sm = 0;
-    GS_CUDA(cudaFuncSetAttribute(k_direct_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 DS_SMEM));
-    GS_CUDA(cudaFuncSetAttribute(k_direct_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 DS_SMEM));
-    GS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_direct_rows<true>, DS_THREADS,
-                                                          DS_SMEM));
-    slots_ = (long)dev->sm_count * std::max(per_sm, 1);
+    ni_pad_ = ((max_rows + DS_ITILE - 1) / DS_ITILE) * DS_ITILE;
+    int per_sm = 1;
+    GS_TRY(resident_ctas(k_direct_rows<false>, &per_sm));
+    GS_TRY(resident_ctas(k_direct_rows<true>, &per_sm));
+    slots_ = (long)dev->sm_count * per_sm;
     // Partial sums sized for the largest launch and for a launch of a single
     // row tile, which splits the j range most finely.
+    const int i_tiles = ni_pad_ / DS_ITILE;
     int sp = 1, ch = 1;
-    split_for(ni_pad_ / DS_ITILE, 128, &sp, &ch);
+    choose_tiles(i_tiles, jt_total_, slots_, 128, &sp, &ch);
     partial_rows_ = (size_t)sp * ni_pad_;
-    split_for(1, 128, &sp, &ch);
+    choose_tiles(1, jt_total_, slots_, 128, &sp, &ch);
     partial_rows_ = std::max(partial_rows_, (size_t)sp * DS_ITILE);
     GS_TRY(pj_.reserve((size_t)nj_pad_ * sizeof(float4)));
     GS_TRY(pi_.reserve((size_t)ni_pad_ * sizeof(float4)));
-    GS_TRY(partial_.reserve(partial_rows_ * 3 * sizeof(double)));
+    GS_TRY(partial_.reserve(partial_rows_ * 3 * sizeof(float2)));
     GS_TRY(status_.reserve(sizeof(unsigned)));
     GS_CUDA(cudaMemset(status_.p, 0, sizeof(unsigned)));
     return ok();
@@ -564,19 +690,17 @@ ErrorStatus DirectRows::compute(const double *d_x, const double *d_m, const doub
     // the split is chosen for this launch's row count (few rows: many
     // j-chunks, so that the launch still fills every SM)
     int splits = 1, chunk = jt_total_;
-    split_for(i_tiles, (int)std::min<size_t>(128, partial_rows_ / nr_pad), &splits, &chunk);
+    choose_tiles(i_tiles, jt_total_, slots_, (int)std::min<size_t>(128, partial_rows_ / nr_pad),
+                 &splits, &chunk);
+    auto kernel = eps2 > 0.0f ? k_direct_rows<true> : k_direct_rows<false>;
     if (timer) GS_TRY(timer->begin(s));
-    if (eps2 > 0.0f)
-        k_direct_rows<true><<<i_tiles * splits, DS_THREADS, DS_SMEM, s>>>(
-            pi_.as<float4>(), nr_pad, pj_.as<float4>(), i_tiles, chunk, jt_total_, eps2,
-            partial_.as<double>(), status_.as<unsigned>());
-    else
-        k_direct_rows<false><<<i_tiles * splits, DS_THREADS, DS_SMEM, s>>>(
-            pi_.as<float4>(), nr_pad, pj_.as<float4>(), i_tiles, chunk, jt_total_, eps2,
-            partial_.as<double>(), status_.as<unsigned>());
+    kernel<<<i_tiles * splits, DS_THREADS, DS_SMEM, s>>>(
+        pi_.as<float4>(), nr_pad, pj_.as<float4>(), i_tiles, chunk * DS_TILE_GRANULES,
+        jt_total_ * DS_TILE_GRANULES, eps2, partial_.as<float2>(), status_.as<unsigned>());
+    GS_CUDA(cudaGetLastError());
     if (timer) GS_TRY(timer->end(s));
-    k_reduce_splits<<<(nrows + 255) / 256, 256, 0, s>>>(partial_.as<double>(), splits, nrows,
-                                                        nr_pad, G, d_a_rows);
+    k_reduce_splits<<<dim3((nrows + 255) / 256, 3), 256, 0, s>>>(partial_.as<float2>(), splits,
+                                                                 nrows, nr_pad, G, d_a_rows);
     GS_CUDA(cudaGetLastError());
     return ok();
 }
@@ -619,7 +743,7 @@ constexpr int NOALLOC_MAX_N = 32768;      // largest particle count accepted
 constexpr int NOALLOC_MAX_SPLITS = 8;
 constexpr size_t NOALLOC_PJ_BYTES = (size_t)NOALLOC_MAX_N * sizeof(float4);
 constexpr size_t NOALLOC_PARTIAL_BYTES =
-    (size_t)NOALLOC_MAX_SPLITS * 3 * NOALLOC_MAX_N * sizeof(double);
+    (size_t)NOALLOC_MAX_SPLITS * 3 * NOALLOC_MAX_N * sizeof(float2);
 constexpr size_t NOALLOC_BYTES = NOALLOC_PJ_BYTES + NOALLOC_PARTIAL_BYTES + 256;
 static_assert(NOALLOC_MAX_N % DS_JTILE == 0, "capacity must be whole tiles");
 // The last 256 bytes: the status word at offset 0, the FP64 frame centre at 64.
@@ -672,30 +796,15 @@ k_noalloc_frame(const double *__restrict__ x, int n, double *__restrict__ frame)
 // k_reduce_splits for this entry point: when a tile wait of k_direct_sum
 // ran out (status bit ST_WAIT_TIMEOUT), some partial sums were never
 // written, and every row gets NaN instead of a wrong finite value.
-__global__ void k_noalloc_reduce(const double *__restrict__ partial, int splits, int n, int n_pad,
+__global__ void k_noalloc_reduce(const float2 *__restrict__ partial, int splits, int n, int n_pad,
                                  double G, const unsigned *__restrict__ status,
                                  double *__restrict__ a)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = blockIdx.y;
     if (i >= n) return;
-    if (*status & ST_WAIT_TIMEOUT) {
-        const double nan = __longlong_as_double(0x7ff8000000000000LL);
-        a[3 * i + 0] = nan;
-        a[3 * i + 1] = nan;
-        a[3 * i + 2] = nan;
-        return;
-    }
-    const size_t plane = (size_t)n_pad;
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-    for (int s = 0; s < splits; ++s) {
-        const double *p = partial + (size_t)s * 3 * plane;
-        s0 += p[i];
-        s1 += p[plane + i];
-        s2 += p[2 * plane + i];
-    }
-    a[3 * i + 0] = G * s0;
-    a[3 * i + 1] = G * s1;
-    a[3 * i + 2] = G * s2;
+    a[3 * i + k] = (*status & ST_WAIT_TIMEOUT) ? __longlong_as_double(0x7ff8000000000000LL)
+                                               : G * reduce_row(partial, splits, n_pad, k, i);
 }
 
 namespace {
@@ -757,43 +866,29 @@ extern "C" int gsgpu_pairwise_acceleration_noalloc(const double *d_x, const doub
     int dev = 0, sms = 0, per_sm = 0;
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const float eps2 = (float)(softening_length * softening_length);
+    auto kernel = eps2 > 0.0f ? k_direct_sum<true> : k_direct_sum<false>;
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_direct_sum<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 DS_SMEM);
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DS_SMEM);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_direct_sum<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 DS_SMEM);
-    if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_direct_sum<true>, DS_THREADS,
-                                                          DS_SMEM);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, DS_THREADS, DS_SMEM);
     if (e != cudaSuccess) {
         std::fprintf(stderr, "gsgpu_pairwise_acceleration_noalloc: %s\n", cudaGetErrorString(e));
         return GRAV_FAILURE;
     }
     unsigned char *scratch = static_cast<unsigned char *>(base);
     float4 *pj = reinterpret_cast<float4 *>(scratch);
-    double *partial = reinterpret_cast<double *>(scratch + NOALLOC_PJ_BYTES);
+    float2 *partial = reinterpret_cast<float2 *>(scratch + NOALLOC_PJ_BYTES);
     unsigned *status = reinterpret_cast<unsigned *>(scratch + NOALLOC_STATUS_OFF);
     double *frame = reinterpret_cast<double *>(scratch + NOALLOC_FRAME_OFF);
 
-    // Same work split as the allocating engine, with at most 8 j-chunks.
+    // Units of whole source tiles, at most NOALLOC_MAX_SPLITS of them per row.
     const int n_pad = ((num_particles + DS_JTILE - 1) / DS_JTILE) * DS_JTILE;
     const int i_tiles = n_pad / DS_ITILE;
     const int jt_total = n_pad / DS_JTILE;
     const long slots = (long)sms * (per_sm > 0 ? per_sm : 1);
-    int splits = 1, jt_per_chunk = jt_total;
-    double best = 1e300;
-    for (int sp = 1; sp <= std::min(jt_total, NOALLOC_MAX_SPLITS); ++sp) {
-        const int chunk = (jt_total + sp - 1) / sp;
-        const int used = (jt_total + chunk - 1) / chunk;
-        const long units = (long)i_tiles * used;
-        const double cost = (double)((units + slots - 1) / slots) * (chunk + 0.25);
-        if (cost < best - 1e-9) {
-            best = cost;
-            splits = used;
-            jt_per_chunk = chunk;
-        }
-    }
+    int splits = 1, chunk = jt_total;
+    choose_tiles(i_tiles, jt_total, slots, NOALLOC_MAX_SPLITS, &splits, &chunk);
 
     // The status word must start at zero; the frame centre, the packed array
     // and the partial sums are fully rewritten by every call.
@@ -802,14 +897,10 @@ extern "C" int gsgpu_pairwise_acceleration_noalloc(const double *d_x, const doub
         k_noalloc_frame<<<1, NA_FRAME_THREADS, 0, s>>>(d_x, num_particles, frame);
         k_pack_frame<<<(n_pad + 255) / 256, 256, 0, s>>>(d_x, d_m, num_particles, n_pad, frame,
                                                          pj);
-        const float eps2 = (float)(softening_length * softening_length);
-        if (eps2 > 0.0f)
-            k_direct_sum<true><<<i_tiles * splits, DS_THREADS, DS_SMEM, s>>>(
-                pj, n_pad, i_tiles, jt_per_chunk, jt_total, eps2, partial, status);
-        else
-            k_direct_sum<false><<<i_tiles * splits, DS_THREADS, DS_SMEM, s>>>(
-                pj, n_pad, i_tiles, jt_per_chunk, jt_total, eps2, partial, status);
-        k_noalloc_reduce<<<(num_particles + 255) / 256, 256, 0, s>>>(
+        kernel<<<i_tiles * splits, DS_THREADS, DS_SMEM, s>>>(
+            pj, n_pad, i_tiles, chunk * DS_TILE_GRANULES, jt_total * DS_TILE_GRANULES, eps2,
+            partial, status);
+        k_noalloc_reduce<<<dim3((num_particles + 255) / 256, 3), 256, 0, s>>>(
             partial, splits, num_particles, n_pad, G, status, d_a);
         e = cudaGetLastError();
     }

@@ -67,6 +67,21 @@ def test_fp32_sizes(lib, g, orc, wl, n):
     check_fp32(a, orc.pairwise(x, m, 1.0, 0.01), orc.abs_sum_rows(x, m, 1.0, 0.01))
 
 
+@pytest.mark.parametrize("n", [1, 127, 129, 257, 2048, 2049, 4097, 17408, 17409, 20480, 20481])
+@pytest.mark.parametrize("eps", [0.0, 0.01])
+def test_fp32_at_granule_and_dispatch_edges(lib, g, orc, wl, n, eps):
+    """Counts next to a 128-particle granule, a row tile, and the counts at which the
+    compensated runs grow and the units of 64 rows end.  The oracle sums the
+    positions the kernel works on (FP32, relative to the bounding-box centre), so the bound
+    is that of the pair terms alone: a few roundings of 6e-8 and three times the reciprocal
+    square root's 2e-7, held to 1e-5 of the terms' magnitudes."""
+    x, v, m = wl.plummer(n, 900 + n)
+    a = g.acceleration(lib, x, m, 1.0, g.METHOD_GPU_PAIRWISE, softening_length=eps)
+    xr = (x - 0.5 * (x.min(0) + x.max(0))).astype(np.float32).astype(np.float64)
+    diff = np.linalg.norm(a - orc.pairwise(xr, m, 1.0, eps), axis=1)
+    assert np.all(diff <= 1e-5 * orc.abs_sum_rows(xr, m, 1.0, eps) + 1e-300)
+
+
 def test_fp32_unsoftened_and_offset_frame(lib, g, orc, wl):
     x, v, m = wl.plummer(5000, 77)
     x = x + np.array([100.0, -50.0, 25.0])    # far from the origin
