@@ -28,6 +28,7 @@
 // not read its uninitialised a[0] / aux, taken as zero here).
 #include "gs_internal.h"
 #include "gs_ptx.cuh"
+#include "gs_whfast.cuh"
 
 #include <algorithm>
 #include <cstdio>
@@ -35,61 +36,7 @@
 
 namespace gs {
 
-// Ensemble integrator / acceleration variants.
-enum { WH_MASSLESS = 0, WH_PAIRWISE = 1 };
-
-// Largest system of an ensemble: the per-system sort holds 12 bytes per
-// slot of the next power of two in shared memory (192 KiB at 16384).
-constexpr int kEnsembleMaxSystem = 16384;
-
-// Shared pair sums of the interaction acceleration (k_wh_pairs): used when a
-// system has at most kPairMax massive bodies.
-constexpr int kPairMax = 32;
-constexpr int kPairSlots = kPairMax + 1;
-
-struct EnsDev {
-    int S;
-    const int *off;      // [S+1]
-    int *cnt;            // [S]
-    const int *sys_of;   // [P]
-    int *ids;
-    double *x, *v, *m, *jx, *jv, *a, *eta;
-    int *hv;             // massive-body list (indices within the system), per system at off[s]
-    int *nh;             // [S]
-    int *rm;             // [P] removal marks
-    int *nrm;            // [S]
-    double *pairs;       // [S][2 * kPairSlots][3] shared pair sums
-    // Jacobi -> Cartesian pass (k_wh_seq_scan / _chain / _fill)
-    int *seq_nmass;      // [S] massive particles (run path), -1: whole chain, -2: empty
-    int *seq_runs;       // [S] massless runs recorded
-    int *run_lo, *run_hi;   // [S][kSeqMassMax + 1] first / last slot of a run
-    double *run_y;       // [S][kSeqMassMax + 1][6] offsets of a run's x and v
-    // scratch for the permutation
-    int *t_ids;
-    double *t_x, *t_v, *t_m;
-    unsigned *status;
-    double G, eps;
-    int variant;
-    int remove_invalid;
-};
-
-__device__ __forceinline__ double dot3(const double *a, const double *b)
-{
-    return __dadd_rn(__dadd_rn(__dmul_rn(a[0], b[0]), __dmul_rn(a[1], b[1])), __dmul_rn(a[2], b[2]));
-}
-
-__device__ __forceinline__ double norm3d(const double *a) { return __dsqrt_rn(dot3(a, a)); }
-
 // ---- sort by distance ----------------------------------------------------
-// Sort key of a distance: its bit pattern (distances are >= 0, so the
-// patterns order like the values), NaN after +inf, padding after all.
-// This keeps the comparison a total order whatever the input, so every
-// live slot receives a live index.
-__device__ __forceinline__ unsigned long long dist_key(double d)
-{
-    return isnan(d) ? 0x7ff8000000000000ull : (unsigned long long)__double_as_longlong(fabs(d));
-}
-
 // eta_i = m_0 + m_1 + ... + m_i, added one by one in slot order
 // (src/integrator_whfast.c:1266-1279), from the masses in ms[0..n), by warp
 // 0 of the block.  The warp walks the slots 32 at a time and performs only
@@ -302,11 +249,6 @@ struct SeqRuns {
     double y[kSeqMassMax + 1][6];
     int nruns;
 };
-
-__device__ __forceinline__ bool neg_zero(double v)
-{
-    return __double_as_longlong(v) == (long long)0x8000000000000000ull;
-}
 
 // One exact chain step of src/integrator_whfast.c:744-760 for particle i;
 // y[6] receives the offsets added to jx_i / jv_i.
@@ -730,38 +672,6 @@ __global__ void __launch_bounds__(32 * PAIR_WARPS) k_wh_pairs(EnsDev E)
 
 // ---- Kepler drift -------------------------------------------------------------
 // src/integrator_whfast.c:774-815
-// Quotients x / d by the divisors d of the Stumpff series, correctly
-// rounded without a division.  zh = RN(1/d) and zl = RN(1/d - zh) (exact
-// rationals rounded once); q = RN(x zh + RN(x zl)) is within an ulp of x/d
-// (Brisebarre, Muller and Raina, "Accelerating correctly rounded
-// floating-point division when the divisor is known in advance", IEEE
-// Trans. Computers 53(8), 2004), and one correction with the exact remainder
-// r = x - q d gives RN(q + r zh) = RN(x/d) (Markstein, IBM J. Res. Dev.
-// 34(1), 1990: a faithful quotient and a correctly rounded reciprocal).
-// The remainder is exact while its last bit stays above the subnormal
-// range, so |x| outside [2^-960, 2^960] (zeros, subnormals, infinities,
-// NaN) takes the division itself.  Checked against __ddiv_rn bit for bit
-// by gsgpu_stumpff_division_selftest.
-struct StumpffDiv {
-    double d, zh, zl;
-};
-enum { SD6, SD12, SD20, SD30, SD42, SD56, SD72, SD90, SD110, SD132, SD156, SD182, SD210, kStumpffDivs };
-__constant__ StumpffDiv kStumpffDiv[kStumpffDivs] = {
-    {6.0, 0x1.5555555555555p-3, 0x1.5555555555555p-57},
-    {12.0, 0x1.5555555555555p-4, 0x1.5555555555555p-58},
-    {20.0, 0x1.999999999999ap-5, -0x1.999999999999ap-59},
-    {30.0, 0x1.1111111111111p-5, 0x1.1111111111111p-61},
-    {42.0, 0x1.8618618618618p-6, 0x1.8618618618618p-60},
-    {56.0, 0x1.2492492492492p-6, 0x1.2492492492492p-60},
-    {72.0, 0x1.c71c71c71c71cp-7, 0x1.c71c71c71c71cp-61},
-    {90.0, 0x1.6c16c16c16c17p-7, -0x1.f49f49f49f49fp-62},
-    {110.0, 0x1.29e4129e4129ep-7, 0x1.04a7904a7904ap-61},
-    {132.0, 0x1.f07c1f07c1f08p-8, -0x1.f07c1f07c1f08p-63},
-    {156.0, 0x1.a41a41a41a41ap-8, 0x1.0690690690690p-62},
-    {182.0, 0x1.6816816816817p-8, -0x1.fa5fa5fa5fa60p-62},
-    {210.0, 0x1.3813813813814p-8, -0x1.fb1fb1fb1fb20p-62},
-};
-
 template <int K> __device__ __forceinline__ double sdiv(double x)
 {
     const double d = kStumpffDiv[K].d, zh = kStumpffDiv[K].zh, zl = kStumpffDiv[K].zl;
@@ -1180,6 +1090,12 @@ struct gsgpu_ensemble {
     // half its largest system's power of two); chosen by autotune()
     int sort_tpb[kSortClasses] = {0, 0, 0};
     bool tuned = false;
+    // WHFast of at most one small system per SM: k_wh_small, a batch of steps per
+    // launch (16 us a step for the Sun and eight planets, 119 us by the launches
+    // below).  With more systems the FP64 pipes are full and the dense lanes of the
+    // per-particle kernels win.  Set by upload, which sees the masses.
+    bool small = false;
+    bool batched() const { return small && !timing; }
     int grid_for(int t) const { return (P + t - 1) / t; }
 
     // Thread-block sizes of the per-particle kernels, timed once on this
@@ -1328,7 +1244,18 @@ struct gsgpu_ensemble {
         }
         GS_CUDA(cudaGetLastError());
         primed = true;
-        GS_TRY(autotune());
+        if (!small) GS_TRY(autotune());
+        return ok();
+    }
+
+    // Enqueue `steps` steps of h of a small ensemble.
+    ErrorStatus run_batch(int64_t steps, double h)
+    {
+        constexpr int64_t kPerLaunch = 64;   // about a millisecond
+        for (; steps > 0; steps -= kPerLaunch)
+            launch_wh_small(E, (int)std::min(steps, kPerLaunch), h, stream);
+        GS_CUDA(cudaGetLastError());
+        last_dt = h;
         return ok();
     }
 
@@ -1360,7 +1287,11 @@ struct gsgpu_ensemble {
         for (int c = 0; c < kSortClasses; ++c) k += sort_first[c + 1] > sort_first[c] ? 1 : 0;
         return k;
     }
-    int kernels_per_step() const { return integrator == INTEGRATOR_WHFAST ? 7 + sort_launches() : 3; }
+    int kernels_per_step() const
+    {
+        if (batched()) return 1;   // at most: a launch takes several steps
+        return integrator == INTEGRATOR_WHFAST ? 7 + sort_launches() : 3;
+    }
 
     // Snapshot of system 0 (a launch_simulation run holds one system): E.x
     // and the velocity array dv with the ids and masses of its live slots.
@@ -1584,6 +1515,15 @@ ErrorStatus ensemble_upload(gsgpu_ensemble *e, const int *ids, const double *x, 
     GS_CUDA(cudaMemcpyAsync(e->m.p, m, P * sizeof(double), cudaMemcpyHostToDevice, e->stream));
     GS_CUDA(cudaMemsetAsync(e->xe.p, 0, P * 3 * sizeof(double), e->stream));
     GS_CUDA(cudaMemsetAsync(e->ve.p, 0, P * 3 * sizeof(double), e->stream));
+    const DeviceInfo *dev = nullptr;
+    GS_TRY(device_info(&dev));
+    e->small = e->integrator == INTEGRATOR_WHFAST && e->S <= dev->sm_count && e->max_n <= kSmallMax;
+    for (int s = 0; s < e->S && e->small; ++s) {
+        int nh = 0;
+        for (int p = e->h_off[s]; p < e->h_off[s + 1]; ++p)
+            nh += e->E.variant == WH_PAIRWISE || m[p] != 0.0;
+        e->small = nh <= kSmallMassive;
+    }
     e->primed = false;
     return ok();
 }
@@ -1609,11 +1549,26 @@ ErrorStatus ensemble_run_until(gsgpu_ensemble *e, double tf, SimulationStatus *s
     while (steps < total) {
         if (t + dt > tf) dt = tf - t;
         if (status) status->dt = dt;
-        GS_TRY(e->step_graph(dt));
-        ++steps;
-        t = (double)steps * dt;
-        if (oc && oc->due(t)) GS_TRY(e->whfast_snapshot(oc, t, dt));
-        if ((steps & 31) == 0) GS_TRY(e->check());
+        if (e->batched()) {
+            // Up to 32 steps (half a millisecond) at once, not past a step that
+            // is clamped or takes a snapshot; one when the run is to end.
+            int64_t k = 1;
+            while (k < 32 && steps + k < total && !(is_exit && *is_exit) &&
+                   !(oc && oc->due((double)(steps + k) * dt)) &&
+                   !((double)(steps + k) * dt + dt > tf))
+                ++k;
+            GS_TRY(e->run_batch(k, dt));
+            steps += k;
+            t = (double)steps * dt;
+            if (oc && oc->due(t)) GS_TRY(e->whfast_snapshot(oc, t, dt));
+            GS_TRY(e->check());
+        } else {
+            GS_TRY(e->step_graph(dt));
+            ++steps;
+            t = (double)steps * dt;
+            if (oc && oc->due(t)) GS_TRY(e->whfast_snapshot(oc, t, dt));
+            if ((steps & 31) == 0) GS_TRY(e->check());
+        }
         if (is_exit && *is_exit) break;
     }
     if (status) {
@@ -1685,6 +1640,10 @@ int gsgpu_ensemble_run(gsgpu_ensemble *e, int64_t num_steps)
 {
     if (!e) return GRAV_POINTER_ERROR;
     ErrorStatus st = e->prime();
+    if (e->batched()) {
+        if (st.return_code == GRAV_SUCCESS) st = e->run_batch(num_steps, e->dt);
+        num_steps = 0;
+    }
     for (int64_t k = 0; k < num_steps && st.return_code == GRAV_SUCCESS; ++k)
         st = e->step_graph(e->dt);
     if (st.return_code != GRAV_SUCCESS) {

@@ -235,3 +235,56 @@ def test_whfast_many_massive_bodies_match_oracle(g, lib, wl, orc, pairwise):
         assert np.array_equal(i_s, ri), s
         assert np.array_equal(x_s, rx) and np.array_equal(v_s, rv), s
     ens.close()
+
+
+@pytest.mark.parametrize("pairwise", [False, True])
+@pytest.mark.parametrize("planar", [False, True])
+def test_whfast_small_systems_match_oracle(g, lib, wl, orc, pairwise, planar):
+    """Systems of 1 to 48 bodies (16 massive ones at most), which run many steps per launch:
+    counts next to the eight-lane groups and the limits, a dt at which the Kepler solves
+    quarter their arguments and the order by distance changes, escapers that are removed,
+    and planar systems with signed zeros.  Bit for bit against the oracle."""
+    G = wl.G_AU_MSUN_DAY
+    base = [s for s in wl.planetary_ensemble(80, 41, max_test=300) if s[2].size >= 48]
+    systems = []
+    for k, n in enumerate([1, 2, 3, 9, 16] + ([] if pairwise else [17, 25, 40, 47, 48])):
+        x, v, m = (a[:n].copy() for a in base[k])
+        if n > 9:
+            x[n - 1], v[n - 1] = [1.0, 0.2, 0.0], [90.0, 0.0, 0.0]   # leaves, and is removed
+            m[n - 2] = 1e-9   # a massive body among the massless ones
+        if planar:
+            x[:, 2] = v[:, 2] = 0.0
+            x[::2, 2] = v[1::3, 2] = -0.0
+        systems.append((x, v, m))
+    counts0, ids, x, v, m = _concat(systems)
+    dt, tf = 11.0, 700.0
+    ens = g.Ensemble(lib, counts0, G, integrator=WHFAST,
+                     method=GPU_PAIRWISE_FP64 if pairwise else GPU_MASSLESS, dt=dt)
+    ens.upload(ids, x, v, m)
+    ens.run_until(tf)
+    assert ens.kernels_per_step() == 1
+    counts, ido, xo, vo, mo = ens.download()
+    for s, (i_s, x_s, v_s, m_s) in enumerate(_blocks(counts0, counts, ido, xo, vo, mo)):
+        ri, rx, rv, rm = orc.whfast_run(*systems[s], G, 0.0, dt, tf, pairwise=pairwise)
+        assert np.array_equal(i_s, ri), s
+        assert x_s.tobytes() == rx.tobytes() and v_s.tobytes() == rv.tobytes(), s
+        assert np.array_equal(m_s, rm), s
+    ens.close()
+
+
+def test_whfast_small_and_general_paths_agree(g, lib, wl):
+    """The same system by the many-steps-per-launch kernel, and in the kernel-timing mode,
+    which launches every phase of a step."""
+    G = wl.G_AU_MSUN_DAY
+    systems = [s for s in wl.planetary_ensemble(40, 8, max_test=40) if s[2].size <= 48][:6]
+    counts0, ids, x, v, m = _concat(systems)
+    out = []
+    for timing in (False, True):
+        ens = g.Ensemble(lib, counts0, G, integrator=WHFAST, method=GPU_MASSLESS, dt=3.0)
+        ens.upload(ids, x, v, m)
+        ens.set_kernel_timing(timing)
+        ens.run(70)
+        out.append(ens.download())
+        ens.close()
+    for a, b in zip(*out):
+        assert a.tobytes() == b.tobytes()
