@@ -220,6 +220,7 @@ void launch_error_sum(const double *terms, long long count, double *scratch, cud
 
 // ---- IAS15 (k_ias15.cu) ------------------------------------------------
 extern const double kIas15H[8];   // Gauss-Radau spacings
+void ias15_tables(double r[8][8], double c[7][7]);   // 1 / (h_i - h_j), b from g
 void launch_ias_predict(int L, double *x1, double *v1, const double *x0, const double *v0,
                         const double *a0, double h, const double *b, double dt, const double *xe,
                         const double *ve, cudaStream_t s);
@@ -234,6 +235,32 @@ void launch_ias_refine(int L, double *b, double *e, const double q[7], int refin
 void launch_ias_axpy(int L, double *out, const double *x, double c, const double *v,
                      cudaStream_t s);
 void launch_ias_sub(int L, double *out, const double *u, const double *w, cudaStream_t s);
+
+// ---- small systems (k_small.cu) ------------------------------------------
+constexpr int kTinyMax = 48;   // bodies of a system one CTA steps
+struct TinySystem {
+    int n;
+    bool massless;             // GRAV_GPU_MASSLESS, else GRAV_GPU_PAIRWISE_FP64
+    double G, eps;
+    double *x, *v, *xe, *ve, *a;
+    const double *m;
+    double *x1, *v1, *txe, *tve;   // the result of an adaptive step, not yet accepted
+};
+struct TinyRk {
+    int stages;
+    double a[13][12], b[13], dtdw[13];
+};
+struct TinyIas {
+    double spacing[8], r[8][8], c[7][7];
+    double q[7];                      // powers of the step ratio (acceptance)
+    double *b, *g, *e, *b6_old, *a1;  // [7][3n] each, [3n], [3n]
+};
+ErrorStatus tiny_setup();
+void launch_tiny_fixed(const TinySystem &S, int integrator, int steps, double h, cudaStream_t s);
+void launch_tiny_rk(const TinySystem &S, const TinyRk &R, bool accept, bool attempt, double h,
+                    double tol, double *terms, cudaStream_t s);
+void launch_tiny_ias15(const TinySystem &S, const TinyIas &I, bool accept, bool refine, bool step,
+                       double h, unsigned long long *out, cudaStream_t s);
 
 // ---- embedded Runge-Kutta tableaus (host_rk.cpp) -------------------------
 struct RkTableau {

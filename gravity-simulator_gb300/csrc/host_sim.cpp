@@ -10,6 +10,7 @@
 // graph and replayed; a clamped last step is launched directly.
 #include "gs_internal.h"
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -168,6 +169,46 @@ struct gsgpu_sim {
     double *h_terms = nullptr;   // pinned host copy of the 6N error terms
     DBuf i_b0, i_b, i_g, i_e, i_F, i_a1, i_d7, i_max;
     unsigned long long *h_max = nullptr;   // pinned: two maxima
+    // Pairs of a small system under an FP64 force, 0 for any other (set by upload,
+    // which sees the masses).  One CTA forms 128 pairs at a time: with at most
+    // kTinyPairs of them a fixed step by k_tiny_fixed beats the step's launches
+    // (2.5 against 11 us for nine bodies; even at about 600 pairs), and the adaptive
+    // integrators, tens of launches a step, take every system that fits.
+    int tiny_pairs = 0;
+    static constexpr int kTinyPairs = 512;
+    bool tiny_fixed() const { return tiny_pairs > 0 && tiny_pairs <= kTinyPairs && !timer.enabled; }
+    bool tiny_adaptive() const { return tiny_pairs > 0 && !timer.enabled; }
+
+    TinySystem tiny() const
+    {
+        TinySystem t{};
+        t.n = n;
+        t.massless = p.method == GRAV_GPU_MASSLESS;
+        t.G = G;
+        t.eps = p.softening_length;
+        t.x = x.as<double>();
+        t.v = v.as<double>();
+        t.xe = xe.as<double>();
+        t.ve = ve.as<double>();
+        t.a = a.as<double>();
+        t.m = m.as<double>();
+        t.x1 = e_x1.as<double>();
+        t.v1 = e_v1.as<double>();
+        t.txe = e_txe.as<double>();
+        t.tve = e_tve.as<double>();
+        return t;
+    }
+
+    // Enqueue `steps` fixed steps of h of a small system.
+    ErrorStatus run_tiny(int64_t steps, double h)
+    {
+        constexpr int64_t kPerLaunch = 256;   // about a millisecond
+        for (; steps > 0; steps -= kPerLaunch)
+            launch_tiny_fixed(tiny(), integrator, (int)std::min(steps, kPerLaunch), h, stream);
+        GS_CUDA(cudaGetLastError());
+        last_dt = h;
+        return ok();
+    }
 
     ~gsgpu_sim()
     {
@@ -298,31 +339,53 @@ struct gsgpu_sim {
             status->dt = h;
             status->num_steps = 0;
         }
+        const bool tiny_run = tiny_adaptive();
+        TinyIas I{};
+        bool accept = false, refine_next = false;
+        if (tiny_run) {
+            std::copy(kIas15H, kIas15H + 8, I.spacing);
+            ias15_tables(I.r, I.c);
+            I.b = b;
+            I.g = g;
+            I.e = e;
+            I.b6_old = b0 + 6 * SL;
+            I.a1 = a1;
+        }
         while (t < tf) {
-            for (int it = 0; it < 12; ++it) {
-                for (int i = 0; i < 8; ++i) {
-                    launch_ias_predict(L, x1, v1, x.as<double>(), v.as<double>(), a.as<double>(),
-                                       kIas15H[i], b, h, xe.as<double>(), ve.as<double>(), stream);
-                    GS_CUDA(cudaGetLastError());
-                    GS_TRY(engine->compute(x1, m.as<double>(), F + (size_t)i * SL, stream,
-                                           timer.enabled ? &timer : nullptr));
-                    launch_ias_update_gb(L, g, b, F, i, stream);
-                    GS_CUDA(cudaGetLastError());
-                }
-                launch_ias_delta(L, b, b0, d7, stream);
-                GS_CUDA(cudaGetLastError());
-                double md = 0.0, mf = 0.0;
-                GS_TRY(absmax2(d7, F + 7 * SL, &md, &mf));
-                if ((md / mf) < 1e-16) break;
-            }
-            GS_CUDA(cudaMemcpyAsync(txe, xe.p, bytes3(), cudaMemcpyDeviceToDevice, stream));
-            GS_CUDA(cudaMemcpyAsync(tve, ve.p, bytes3(), cudaMemcpyDeviceToDevice, stream));
-            launch_ias_advance(L, x1, v1, txe, tve, x.as<double>(), v.as<double>(), a.as<double>(),
-                               b, h, stream);
-            GS_CUDA(cudaGetLastError());
-            GS_TRY(engine->compute(x1, m.as<double>(), a1, stream, nullptr));
             double mb = 0.0, ma = 0.0;
-            GS_TRY(absmax2(b + 6 * SL, a1, &mb, &ma));
+            if (tiny_run) {
+                launch_tiny_ias15(tiny(), I, accept, refine_next, true, h, h_max, stream);
+                GS_CUDA(cudaGetLastError());
+                GS_CUDA(cudaStreamSynchronize(stream));
+                refine_next = refine_next || accept;
+                accept = false;
+                std::memcpy(&mb, &h_max[0], sizeof(double));
+                std::memcpy(&ma, &h_max[1], sizeof(double));
+            } else {
+                for (int it = 0; it < 12; ++it) {
+                    for (int i = 0; i < 8; ++i) {
+                        launch_ias_predict(L, x1, v1, x.as<double>(), v.as<double>(), a.as<double>(),
+                                           kIas15H[i], b, h, xe.as<double>(), ve.as<double>(), stream);
+                        GS_CUDA(cudaGetLastError());
+                        GS_TRY(engine->compute(x1, m.as<double>(), F + (size_t)i * SL, stream,
+                                               timer.enabled ? &timer : nullptr));
+                        launch_ias_update_gb(L, g, b, F, i, stream);
+                        GS_CUDA(cudaGetLastError());
+                    }
+                    launch_ias_delta(L, b, b0, d7, stream);
+                    GS_CUDA(cudaGetLastError());
+                    double md = 0.0, mf = 0.0;
+                    GS_TRY(absmax2(d7, F + 7 * SL, &md, &mf));
+                    if ((md / mf) < 1e-16) break;
+                }
+                GS_CUDA(cudaMemcpyAsync(txe, xe.p, bytes3(), cudaMemcpyDeviceToDevice, stream));
+                GS_CUDA(cudaMemcpyAsync(tve, ve.p, bytes3(), cudaMemcpyDeviceToDevice, stream));
+                launch_ias_advance(L, x1, v1, txe, tve, x.as<double>(), v.as<double>(),
+                                   a.as<double>(), b, h, stream);
+                GS_CUDA(cudaGetLastError());
+                GS_TRY(engine->compute(x1, m.as<double>(), a1, stream, nullptr));
+                GS_TRY(absmax2(b + 6 * SL, a1, &mb, &ma));
+            }
             const double eb7 = mb / ma;
             double error = std::pow((eb7 / tolerance), 1.0 / 7.0);
             // With every acceleration zero (a single particle, or no mass) the
@@ -341,14 +404,21 @@ struct gsgpu_sim {
                 double qs[7];
                 qs[0] = q;
                 for (int r = 1; r < 7; ++r) qs[r] = qs[r - 1] * q;
-                launch_ias_refine(L, b, e, qs, refine ? 1 : 0, stream);
-                GS_CUDA(cudaGetLastError());
-                refine = true;
-                GS_CUDA(cudaMemcpyAsync(xe.p, txe, bytes3(), cudaMemcpyDeviceToDevice, stream));
-                GS_CUDA(cudaMemcpyAsync(ve.p, tve, bytes3(), cudaMemcpyDeviceToDevice, stream));
-                GS_CUDA(cudaMemcpyAsync(x.p, x1, bytes3(), cudaMemcpyDeviceToDevice, stream));
-                GS_CUDA(cudaMemcpyAsync(v.p, v1, bytes3(), cudaMemcpyDeviceToDevice, stream));
-                GS_CUDA(cudaMemcpyAsync(a.p, a1, bytes3(), cudaMemcpyDeviceToDevice, stream));
+                if (tiny_run) {
+                    // the next launch makes the result the state
+                    std::copy(qs, qs + 7, I.q);
+                    accept = true;
+                    if (oc && oc->due(t)) GS_TRY(tiny_ias_accept(I, accept, refine_next));
+                } else {
+                    launch_ias_refine(L, b, e, qs, refine ? 1 : 0, stream);
+                    GS_CUDA(cudaGetLastError());
+                    refine = true;
+                    GS_CUDA(cudaMemcpyAsync(xe.p, txe, bytes3(), cudaMemcpyDeviceToDevice, stream));
+                    GS_CUDA(cudaMemcpyAsync(ve.p, tve, bytes3(), cudaMemcpyDeviceToDevice, stream));
+                    GS_CUDA(cudaMemcpyAsync(x.p, x1, bytes3(), cudaMemcpyDeviceToDevice, stream));
+                    GS_CUDA(cudaMemcpyAsync(v.p, v1, bytes3(), cudaMemcpyDeviceToDevice, stream));
+                    GS_CUDA(cudaMemcpyAsync(a.p, a1, bytes3(), cudaMemcpyDeviceToDevice, stream));
+                }
                 if (oc && oc->due(t)) GS_TRY(snapshot(oc, v.as<double>(), t, h));
             }
             if (dt_new > (h / 0.25))
@@ -366,8 +436,21 @@ struct gsgpu_sim {
             }
             if (is_exit && *is_exit) break;
         }
+        GS_TRY(tiny_ias_accept(I, accept, refine_next));
         GS_CUDA(cudaStreamSynchronize(stream));
         if (oc) GS_TRY(oc->finish());
+        return ok();
+    }
+
+    // Make the last step's result the state (small systems), if it was accepted
+    // and no launch has done so.
+    ErrorStatus tiny_ias_accept(const TinyIas &I, bool &accept, bool &refine_next)
+    {
+        if (!accept) return ok();
+        launch_tiny_ias15(tiny(), I, true, refine_next, false, 0.0, h_max, stream);
+        GS_CUDA(cudaGetLastError());
+        accept = false;
+        refine_next = true;
         return ok();
     }
 
@@ -406,50 +489,77 @@ struct gsgpu_sim {
         }
         double *vk = e_vk.as<double>(), *xk = e_xk.as<double>();
         const bool device_sum = g_rk_error_sum.load(std::memory_order_relaxed) == 1;
-        while (t < tf) {
-            GS_TRY(force(vk));
-            GS_CUDA(cudaMemcpyAsync(xk, v.p, bytes3(), cudaMemcpyDeviceToDevice, stream));
-            for (int s = 1; s < S; ++s) {
-                launch_rk_emb_stage(x.as<double>(), v.as<double>(), xe.as<double>(),
-                                    ve.as<double>(), vk, xk, e_xs.as<double>(), T->a[s], s, h, L,
-                                    stream);
-                GS_CUDA(cudaGetLastError());
-                GS_TRY(engine->compute(e_xs.as<double>(), m.as<double>(), vk + (size_t)s * L,
-                                       stream, timer.enabled ? &timer : nullptr));
+        // small systems: the host adds their few terms in the reference's order
+        // whatever the mode
+        const bool tiny_run = tiny_adaptive();
+        TinyRk R{};
+        bool accept = false;
+        if (tiny_run) {
+            R.stages = S;
+            for (int s = 0; s < S; ++s) {
+                for (int i = 0; i < 12; ++i) R.a[s][i] = T->a[s][i];
+                R.b[s] = T->b[s];
             }
+        }
+        while (t < tf) {
             double dtdw[13];
             for (int s = 0; s < S; ++s) dtdw[s] = h * dw[s];
-            launch_rk_emb_combine(x.as<double>(), v.as<double>(), xe.as<double>(),
-                                  ve.as<double>(), vk, xk, e_x1.as<double>(), e_v1.as<double>(),
-                                  e_txe.as<double>(), e_tve.as<double>(), e_terms.as<double>(),
-                                  T->b, dtdw, S, h, tolerance, tolerance, L, stream);
-            GS_CUDA(cudaGetLastError());
             double sum = 0.0;
-            if (device_sum) {
-                // one double comes back instead of the 6N terms; not the
-                // reference's order, so the step control is not bit-exact
-                launch_error_sum(e_terms.as<double>(), 2LL * L, e_esum.as<double>(), stream);
+            if (tiny_run) {
+                std::copy(dtdw, dtdw + S, R.dtdw);
+                launch_tiny_rk(tiny(), R, accept, true, h, tolerance, h_terms, stream);
+                accept = false;
                 GS_CUDA(cudaGetLastError());
-                GS_CUDA(cudaMemcpyAsync(h_terms, e_esum.as<double>() + kErrorSumScratch - 1,
-                                        sizeof(double), cudaMemcpyDeviceToHost, stream));
                 GS_CUDA(cudaStreamSynchronize(stream));
-                GS_TRY(engine->check_status(stream));
-                sum = h_terms[0];
-            } else {
-                GS_CUDA(cudaMemcpyAsync(h_terms, e_terms.p, (size_t)2 * L * sizeof(double),
-                                        cudaMemcpyDeviceToHost, stream));
-                GS_CUDA(cudaStreamSynchronize(stream));
-                GS_TRY(engine->check_status(stream));
                 for (int k = 0; k < 2 * L; ++k) sum += h_terms[k];
+            } else {
+                GS_TRY(force(vk));
+                GS_CUDA(cudaMemcpyAsync(xk, v.p, bytes3(), cudaMemcpyDeviceToDevice, stream));
+                for (int s = 1; s < S; ++s) {
+                    launch_rk_emb_stage(x.as<double>(), v.as<double>(), xe.as<double>(),
+                                        ve.as<double>(), vk, xk, e_xs.as<double>(), T->a[s], s, h, L,
+                                        stream);
+                    GS_CUDA(cudaGetLastError());
+                    GS_TRY(engine->compute(e_xs.as<double>(), m.as<double>(), vk + (size_t)s * L,
+                                           stream, timer.enabled ? &timer : nullptr));
+                }
+                launch_rk_emb_combine(x.as<double>(), v.as<double>(), xe.as<double>(),
+                                      ve.as<double>(), vk, xk, e_x1.as<double>(), e_v1.as<double>(),
+                                      e_txe.as<double>(), e_tve.as<double>(), e_terms.as<double>(),
+                                      T->b, dtdw, S, h, tolerance, tolerance, L, stream);
+                GS_CUDA(cudaGetLastError());
+                if (device_sum) {
+                    // one double comes back instead of the 6N terms; not the
+                    // reference's order, so the step control is not bit-exact
+                    launch_error_sum(e_terms.as<double>(), 2LL * L, e_esum.as<double>(), stream);
+                    GS_CUDA(cudaGetLastError());
+                    GS_CUDA(cudaMemcpyAsync(h_terms, e_esum.as<double>() + kErrorSumScratch - 1,
+                                            sizeof(double), cudaMemcpyDeviceToHost, stream));
+                    GS_CUDA(cudaStreamSynchronize(stream));
+                    GS_TRY(engine->check_status(stream));
+                    sum = h_terms[0];
+                } else {
+                    GS_CUDA(cudaMemcpyAsync(h_terms, e_terms.p, (size_t)2 * L * sizeof(double),
+                                            cudaMemcpyDeviceToHost, stream));
+                    GS_CUDA(cudaStreamSynchronize(stream));
+                    GS_TRY(engine->check_status(stream));
+                    for (int k = 0; k < 2 * L; ++k) sum += h_terms[k];
+                }
             }
             double error = std::sqrt(sum / (n * 3 * 2));
             if (error <= 1 || h <= tf * 1e-12) {
                 ++steps;
                 t += h;
-                GS_CUDA(cudaMemcpyAsync(x.p, e_x1.p, bytes3(), cudaMemcpyDeviceToDevice, stream));
-                GS_CUDA(cudaMemcpyAsync(v.p, e_v1.p, bytes3(), cudaMemcpyDeviceToDevice, stream));
-                GS_CUDA(cudaMemcpyAsync(xe.p, e_txe.p, bytes3(), cudaMemcpyDeviceToDevice, stream));
-                GS_CUDA(cudaMemcpyAsync(ve.p, e_tve.p, bytes3(), cudaMemcpyDeviceToDevice, stream));
+                if (tiny_run) {
+                    // the next launch makes the result the state
+                    accept = true;
+                    if (oc && oc->due(t)) GS_TRY(tiny_rk_accept(R, accept));
+                } else {
+                    GS_CUDA(cudaMemcpyAsync(x.p, e_x1.p, bytes3(), cudaMemcpyDeviceToDevice, stream));
+                    GS_CUDA(cudaMemcpyAsync(v.p, e_v1.p, bytes3(), cudaMemcpyDeviceToDevice, stream));
+                    GS_CUDA(cudaMemcpyAsync(xe.p, e_txe.p, bytes3(), cudaMemcpyDeviceToDevice, stream));
+                    GS_CUDA(cudaMemcpyAsync(ve.p, e_tve.p, bytes3(), cudaMemcpyDeviceToDevice, stream));
+                }
                 if (oc && oc->due(t)) GS_TRY(snapshot(oc, v.as<double>(), t, h));
             }
             if (error < 1e-10) error = 1e-10;
@@ -469,8 +579,20 @@ struct gsgpu_sim {
             }
             if (is_exit && *is_exit) break;
         }
+        GS_TRY(tiny_rk_accept(R, accept));
         GS_CUDA(cudaStreamSynchronize(stream));
         if (oc) GS_TRY(oc->finish());
+        return ok();
+    }
+
+    // Make the last attempt's result the state (small systems), if it was
+    // accepted and no launch has done so.
+    ErrorStatus tiny_rk_accept(const TinyRk &R, bool &accept)
+    {
+        if (!accept) return ok();
+        launch_tiny_rk(tiny(), R, true, false, 0.0, 0.0, h_terms, stream);
+        GS_CUDA(cudaGetLastError());
+        accept = false;
         return ok();
     }
 
@@ -570,6 +692,7 @@ struct gsgpu_sim {
 
     int kernels_per_step() const
     {
+        if (tiny_fixed()) return 1;   // at most: a launch takes several steps
         const int f = engine->kernels_per_eval();
         switch (integrator) {
         case INTEGRATOR_EULER: return f + 1;
@@ -697,6 +820,15 @@ ErrorStatus sim_upload(gsgpu_sim *s, const double *x, const double *v, const dou
     GS_CUDA(cudaMemsetAsync(s->xe.p, 0, s->bytes3(), s->stream));
     GS_CUDA(cudaMemsetAsync(s->ve.p, 0, s->bytes3(), s->stream));
     GS_CUDA(cudaMemsetAsync(s->a.p, 0, s->bytes3(), s->stream));
+    s->tiny_pairs = 0;
+    if (s->n <= kTinyMax &&
+        (s->p.method == GRAV_GPU_PAIRWISE_FP64 || s->p.method == GRAV_GPU_MASSLESS)) {
+        int heavy = 0;
+        for (int i = 0; i < s->n; ++i)
+            heavy += s->p.method == GRAV_GPU_PAIRWISE_FP64 || m[i] != 0.0;
+        s->tiny_pairs = std::max(1, heavy * (heavy - 1) / 2 + (s->n - heavy) * heavy);
+        GS_TRY(tiny_setup());
+    }
     s->primed = false;
     s->last_dt = s->dt;
     if (s->graph) {
@@ -751,8 +883,19 @@ ErrorStatus sim_run_until(gsgpu_sim *s, double tf, SimulationStatus *status, con
     while (steps < total) {
         if (clamp && t + dt > tf) dt = tf - t;
         if (status) status->dt = dt;
-        GS_TRY(s->step_graph(dt));
-        ++steps;
+        int64_t batch = 1;
+        if (s->tiny_fixed()) {
+            // Up to 32 steps (a tenth of a millisecond) at once, not past a step
+            // that is clamped or takes a snapshot; one when the run is to end.
+            while (batch < 32 && steps + batch < total && !(is_exit && *is_exit) &&
+                   !(oc && oc->due((double)(steps + batch) * dt)) &&
+                   !(clamp && (double)(steps + batch) * dt + dt > tf))
+                ++batch;
+            GS_TRY(s->run_tiny(batch, dt));
+        } else {
+            GS_TRY(s->step_graph(dt));
+        }
+        steps += batch;
         t = (double)steps * dt;
         if (oc && oc->due(t)) {
             // A force that failed on the device (node-capacity overflow, a
@@ -771,7 +914,7 @@ ErrorStatus sim_run_until(gsgpu_sim *s, double tf, SimulationStatus *status, con
             }
             GS_TRY(s->snapshot(oc, dv, t, dt));
         }
-        if ((steps & 31) == 0) {
+        if ((steps & 31) == 0 || batch > 1) {
             GS_CUDA(cudaStreamSynchronize(s->stream));
             GS_TRY(s->engine->check_status(s->stream));
         }
@@ -825,8 +968,13 @@ int gsgpu_sim_run(gsgpu_sim *sim, int64_t num_steps)
 {
     if (!sim) return GRAV_POINTER_ERROR;
     ErrorStatus st = sim->prime();
-    for (int64_t k = 0; k < num_steps && st.return_code == GRAV_SUCCESS; ++k)
-        st = sim->step_graph(sim->dt);
+    const bool fixed = sim->integrator >= INTEGRATOR_EULER && sim->integrator <= INTEGRATOR_LEAPFROG;
+    int64_t k = 0;
+    if (fixed && sim->tiny_fixed() && st.return_code == GRAV_SUCCESS) {
+        st = sim->run_tiny(num_steps, sim->dt);
+        k = num_steps;
+    }
+    for (; k < num_steps && st.return_code == GRAV_SUCCESS; ++k) st = sim->step_graph(sim->dt);
     if (st.return_code != GRAV_SUCCESS) {
         print_and_free_traceback(&st);
         return st.return_code;

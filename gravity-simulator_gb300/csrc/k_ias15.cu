@@ -16,25 +16,35 @@ namespace gs {
 
 /* Gauss-Radau spacings h_0..h_7 (host: the predictor node is a kernel argument) */
 const double kIas15H[8] = {0.0, 0x1.cce7242fd9812p-5, 0x1.7122082358d27p-3, 0x1.6916742f0c9c5p-2, 0x1.18248525f4802p-1, 0x1.77ea65770fa49p-1, 0x1.c548c982467cdp-1, 0x1.f47d94f4d2bb2p-1};
-/* c[i][j] (j <= i): b from g */
-__constant__ double kRadauC[7][7] = {
-    {0x1.0000000000000p+0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0},
-    {-0x1.cce7242fd9812p-5, 0x1.0000000000000p+0, 0.0, 0.0, 0.0, 0.0, 0.0},
-    {0x1.4c4b384151c1ep-7, -0x1.e45bd12f4f32cp-3, 0x1.0000000000000p+0, 0.0, 0.0, 0.0, 0.0},
-    {-0x1.d4b3379a1992dp-9, 0x1.7f2161e152586p-4, -0x1.2da22e635a1aep-1, 0x1.0000000000000p+0, 0.0, 0.0, 0.0},
-    {0x1.007370e57b89dp-9, -0x1.c08e5e7efcf23p-5, 0x1.a9dcc2e57fbbfp-2, -0x1.22e359c4a74d8p+0, 0x1.0000000000000p+0, 0.0, 0.0},
-    {-0x1.7893e98a2a997p-10, 0x1.595cd739ee74fp-5, -0x1.70bdf2d91dd44p-2, 0x1.4009e0866d488p+0, -0x1.ded88c802f1fcp+0, 0x1.0000000000000p+0, 0.0},
-    {0x1.4d64672378b3dp-10, -0x1.3d865cb429919p-5, 0x1.71a0161ae20fep-2, -0x1.7785b93619434p+0, 0x1.73fc45dfb9889p+1, -0x1.60be78a0a92f1p+1, 0x1.0000000000000p+0}};
-/* r[i][j] = 1 / (h_i - h_j) (j < i): g from the accelerations */
-__constant__ double kRadauR[8][8] = {
-    {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0},
-    {0x1.1c618574b517bp+4, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0},
-    {0x1.6314ac07f6a9ap+2, 0x1.021c2b5e4af6fp+3, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0},
-    {0x1.6afdfcc2a4aefp+1, 0x1.afe76c59caa8ap+1, 0x1.73439c0b4562bp+2, 0.0, 0.0, 0.0, 0.0, 0.0},
-    {0x1.d3e03b89d73cfp+0, 0x1.04c014a3946fbp+1, 0x1.5cdb4a576d57ap+1, 0x1.48fffc3fdf2e6p+2, 0.0, 0.0, 0.0, 0.0},
-    {0x1.5cac8b52e27b1p+0, 0x1.799c3c56b4e9dp+0, 0x1.ce1e8b86f5ae8p+0, 0x1.4f714afea15ccp+1, 0x1.56247c4b878b4p+2, 0.0, 0.0, 0.0},
-    {0x1.212921ce4baffp+0, 0x1.34c8b7028f418p+0, 0x1.6b1448c75e4d5p+0, 0x1.e092f6d7c8a42p+0, 0x1.7a82c7145ec17p+1, 0x1.a787c6413556bp+2, 0.0, 0.0},
-    {0x1.05e3166485188p+0, 0x1.15e18175af101p+0, 0x1.41177c7d3aff5p+0, 0x1.99ab118ef2216p+0, 0x1.296bab4a3e0d2p+1, 0x1.0709d7d8d5e3cp+2, 0x1.5b12a584540e2p+3, 0.0}};
+/* c[i][j] (j <= i): b from g; r[i][j] = 1 / (h_i - h_j) (j < i): g from the
+ * accelerations.  Once for the kernels below, once on the host. */
+#define GS_RADAU_C {                                                                    \
+    {0x1.0000000000000p+0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, \
+    {-0x1.cce7242fd9812p-5, 0x1.0000000000000p+0, 0.0, 0.0, 0.0, 0.0, 0.0}, \
+    {0x1.4c4b384151c1ep-7, -0x1.e45bd12f4f32cp-3, 0x1.0000000000000p+0, 0.0, 0.0, 0.0, 0.0}, \
+    {-0x1.d4b3379a1992dp-9, 0x1.7f2161e152586p-4, -0x1.2da22e635a1aep-1, 0x1.0000000000000p+0, 0.0, 0.0, 0.0}, \
+    {0x1.007370e57b89dp-9, -0x1.c08e5e7efcf23p-5, 0x1.a9dcc2e57fbbfp-2, -0x1.22e359c4a74d8p+0, 0x1.0000000000000p+0, 0.0, 0.0}, \
+    {-0x1.7893e98a2a997p-10, 0x1.595cd739ee74fp-5, -0x1.70bdf2d91dd44p-2, 0x1.4009e0866d488p+0, -0x1.ded88c802f1fcp+0, 0x1.0000000000000p+0, 0.0}, \
+    {0x1.4d64672378b3dp-10, -0x1.3d865cb429919p-5, 0x1.71a0161ae20fep-2, -0x1.7785b93619434p+0, 0x1.73fc45dfb9889p+1, -0x1.60be78a0a92f1p+1, 0x1.0000000000000p+0}}
+#define GS_RADAU_R {                                                                    \
+    {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, \
+    {0x1.1c618574b517bp+4, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, \
+    {0x1.6314ac07f6a9ap+2, 0x1.021c2b5e4af6fp+3, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, \
+    {0x1.6afdfcc2a4aefp+1, 0x1.afe76c59caa8ap+1, 0x1.73439c0b4562bp+2, 0.0, 0.0, 0.0, 0.0, 0.0}, \
+    {0x1.d3e03b89d73cfp+0, 0x1.04c014a3946fbp+1, 0x1.5cdb4a576d57ap+1, 0x1.48fffc3fdf2e6p+2, 0.0, 0.0, 0.0, 0.0}, \
+    {0x1.5cac8b52e27b1p+0, 0x1.799c3c56b4e9dp+0, 0x1.ce1e8b86f5ae8p+0, 0x1.4f714afea15ccp+1, 0x1.56247c4b878b4p+2, 0.0, 0.0, 0.0}, \
+    {0x1.212921ce4baffp+0, 0x1.34c8b7028f418p+0, 0x1.6b1448c75e4d5p+0, 0x1.e092f6d7c8a42p+0, 0x1.7a82c7145ec17p+1, 0x1.a787c6413556bp+2, 0.0, 0.0}, \
+    {0x1.05e3166485188p+0, 0x1.15e18175af101p+0, 0x1.41177c7d3aff5p+0, 0x1.99ab118ef2216p+0, 0x1.296bab4a3e0d2p+1, 0x1.0709d7d8d5e3cp+2, 0x1.5b12a584540e2p+3, 0.0}}
+__constant__ double kRadauC[7][7] = GS_RADAU_C;
+__constant__ double kRadauR[8][8] = GS_RADAU_R;
+
+void ias15_tables(double r[8][8], double c[7][7])
+{
+    static const double R[8][8] = GS_RADAU_R, C[7][7] = GS_RADAU_C;
+    std::copy(&R[0][0], &R[0][0] + 64, &r[0][0]);
+    std::copy(&C[0][0], &C[0][0] + 49, &c[0][0]);
+}
+
 
 
 namespace {

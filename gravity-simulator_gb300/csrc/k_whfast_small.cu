@@ -19,6 +19,7 @@
 // Every value is formed by the operations, and every sum in the order, of
 // k_whfast.cu, so the results are the same bit for bit.  16 us a step for the Sun
 // and eight planets.
+#include "gs_fp64.cuh"
 #include "gs_internal.h"
 #include "gs_whfast.cuh"
 
@@ -50,45 +51,10 @@ __device__ __forceinline__ double bcast8(double v, int src)
     return __shfl_sync(WS_ALL, v, src, 8);
 }
 
-// |x| as an integer that orders like it (NaN last): comparisons of FP64 values
-// take the FP64 pipe, comparisons of their bits do not.
-__device__ __forceinline__ long long abs_bits(double x)
-{
-    return __double_as_longlong(x) & 0x7fffffffffffffffll;
-}
-
-__device__ __forceinline__ bool finite_bits(double x)
-{
-    return abs_bits(x) < 0x7ff0000000000000ll;
-}
-
-// Exponent of |x| between those of 2^-e and 2^e.
-__device__ __forceinline__ bool exponent_within(double x, int e)
-{
-    const int ex = (__double2hiint(x) >> 20) & 0x7ff;
-    return ex >= 1023 - e && ex < 1023 + e;
-}
-
-__device__ __forceinline__ bool is_zero(double x)
-{
-    return abs_bits(x) == 0;
-}
-
-// RN(x / d) from the double-word reciprocal (zh, zl) of d, as sdiv in
-// k_whfast.cu (Brisebarre, Muller and Raina 2004; Markstein 1990).
-__device__ __forceinline__ double div_known(double x, double d, double zh, double zl, bool ok,
-                                            int range)
-{
-    if (!ok || !exponent_within(x, range)) return __ddiv_rn(x, d);
-    const double q = __fma_rn(x, zh, __dmul_rn(x, zl));
-    const double r = __fma_rn(-q, d, x);
-    return __fma_rn(r, zh, q);
-}
-
 __device__ __forceinline__ double div_eta(const SmallSystem &w, double x, int i)
 {
     if (w.eta_ok[i] && is_zero(x)) return x;   // +-0 over a positive divisor
-    return div_known(x, w.eta[i], w.zh[i], w.zl[i], w.eta_ok[i] != 0, 900);
+    return div_known(x, w.eta[i], w.zh[i], w.zl[i], w.eta_ok[i] != 0);
 }
 
 // What depends on the order and the masses alone: eta and its reciprocals
@@ -124,9 +90,7 @@ __device__ void small_order(SmallSystem &w, double G, bool pairwise, bool form_e
     __syncthreads();
     if (t < w.n) {
         const double e = w.eta[t];
-        const double zh = __ddiv_rn(1.0, e);
-        w.zh[t] = zh;
-        w.zl[t] = __ddiv_rn(__fma_rn(-zh, e, 1.0), e);
+        reciprocal2(e, w.zh[t], w.zl[t]);
         w.eta_ok[t] = e > 0.0 && exponent_within(e, 100);
         if (t > 0) w.gm[t] = __ddiv_rn(__dmul_rn(__dmul_rn(G, w.m[0]), e), w.eta[t - 1]);
     }
@@ -238,8 +202,8 @@ __device__ void small_drift(SmallSystem &w, double dt, const StumpffDiv dA, cons
                 z = __dmul_rn(z, 0.25);
                 ++quarter;
             }
-            const double qa = div_known(z, dA.d, dA.zh, dA.zl, true, 900);
-            const double qb = div_known(z, dB.d, dB.zh, dB.zl, true, 900);
+            const double qa = div_known(z, dA.d, dA.zh, dA.zl, true);
+            const double qb = div_known(z, dB.d, dB.zh, dB.zl, true);
             double t = 1.0;
 #pragma unroll
             for (int k = 0; k < 6; ++k) {
@@ -248,7 +212,7 @@ __device__ void small_drift(SmallSystem &w, double dt, const StumpffDiv dA, cons
                 t = __dsub_rn(1.0, k == 0 ? f : __dmul_rn(f, t));
             }
             // lane 0: t / 6, lane 1: t / 2
-            const double head = div_known(t, dC.d, dC.zh, dC.zl, true, 900);
+            const double head = div_known(t, dC.d, dC.zh, dC.zl, true);
             double u3 = bcast8(head, 0), u2 = bcast8(head, 1);
             const double one = __dsub_rn(1.0, __dmul_rn(z, l == 1 ? u2 : u3));
             double u1 = bcast8(one, 0), u0 = bcast8(one, 1);

@@ -232,3 +232,44 @@ def test_energy_drift_against_reference_barnes_hut(lib, g, orc, wl):
     print(f"relative energy drift over 200 steps: GPU group walk {drift_gpu:.3g}, "
           f"reference Barnes-Hut {drift_ref:.3g}")
     assert drift_gpu <= max(drift_ref, 1e-7)
+
+
+@pytest.mark.parametrize("massless", [False, True])
+@pytest.mark.parametrize("n", [2, 3, 9, 32, 33, 43, 48, 49])
+@pytest.mark.parametrize("integ", [1, 2, 3, 4, 5, 8, 9])
+def test_small_systems_bitexact(lib, g, orc, wl, integ, n, massless):
+    """Systems of at most 48 bodies, which one block steps (up to 512 pairs for the fixed steps:
+    32 and 33 bodies under the pairwise force are on either side), with massive and massless
+    bodies interleaved, more than a batch of 32 steps and a clamped last one.  Bit for bit
+    against the oracle."""
+    x, v, m = wl.plummer(n, 60 + n)
+    if massless:
+        m = np.where(np.arange(n) % 3 == 1, 0.0, m)
+    method, code = (g.METHOD_GPU_MASSLESS, 2) if massless else (g.METHOD_GPU_PAIRWISE_FP64, 1)
+    kw = dict(method=method, softening_length=0.05)
+    if integ <= 4:
+        ref = orc.fixed_step_run(integ, code, x, v, m, 1.0, 0.05, 4e-3, 0.2791)
+        kw.update(dt=4e-3, tf=0.2791)
+    elif integ <= 8:
+        ref = orc.rk_embedded_run(integ, code, x, v, m, 1.0, 0.05, 1e-9, 0.4)
+        kw.update(dt=1e-3, tf=0.4, tolerance=1e-9)
+    else:
+        ref = orc.ias15_run(code, x, v, m, 1.0, 0.05, 1e-9, 0.4)
+        kw.update(dt=1e-3, tf=0.4, tolerance=1e-9)
+    _, xo, vo, _ = g.launch_simulation(lib, x.copy(), v.copy(), m, 1.0, integrator=integ, **kw)
+    assert xo.tobytes() == ref[0].tobytes() and vo.tobytes() == ref[1].tobytes()
+
+
+def test_small_system_is_exit_and_single_body(lib, g, orc, wl):
+    """A set exit flag ends a small system's run after one step; one body alone drifts."""
+    x, v, m = wl.plummer(12, 5)
+    _, xo, vo, _ = g.launch_simulation(lib, x.copy(), v.copy(), m, 1.0, integrator=4, dt=1e-3,
+                                       tf=1.0, method=g.METHOD_GPU_PAIRWISE_FP64,
+                                       softening_length=0.01, is_exit=ctypes.c_bool(True))
+    xr, vr = orc.fixed_step_run(4, 1, x, v, m, 1.0, 0.01, 1e-3, 1e-3)
+    assert np.array_equal(xo, xr) and np.array_equal(vo, vr)
+    x1, v1, m1 = x[:1].copy(), v[:1].copy(), m[:1].copy()
+    xr, vr = orc.fixed_step_run(4, 1, x1, v1, m1, 1.0, 0.0, 1e-3, 0.05)
+    _, xo, vo, _ = g.launch_simulation(lib, x1, v1, m1, 1.0, integrator=4, dt=1e-3, tf=0.05,
+                                       method=g.METHOD_GPU_PAIRWISE_FP64)
+    assert np.array_equal(xo, xr) and np.array_equal(vo, vr)
