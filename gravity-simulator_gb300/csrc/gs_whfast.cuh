@@ -2,6 +2,7 @@
 // k_whfast_small.cu: small systems, many steps per launch).
 #pragma once
 
+#include "gs_fp64.cuh"
 #include "gs_internal.h"
 
 namespace gs {
@@ -57,7 +58,8 @@ __device__ __forceinline__ double norm3d(const double *a) { return __dsqrt_rn(do
 // live slot receives a live index.
 __device__ __forceinline__ unsigned long long dist_key(double d)
 {
-    return isnan(d) ? 0x7ff8000000000000ull : (unsigned long long)__double_as_longlong(fabs(d));
+    const unsigned long long k = (unsigned long long)abs_bits(d);
+    return k > 0x7ff0000000000000ull ? 0x7ff8000000000000ull : k;
 }
 
 __device__ __forceinline__ bool neg_zero(double v)
@@ -73,10 +75,12 @@ __device__ __forceinline__ bool neg_zero(double v)
 // Trans. Computers 53(8), 2004), and one correction with the exact remainder
 // r = x - q d gives RN(q + r zh) = RN(x/d) (Markstein, IBM J. Res. Dev.
 // 34(1), 1990: a faithful quotient and a correctly rounded reciprocal).
+// Where |zl| <= 2^-54 zh, RN(x zh) is itself within an ulp (x zh is within half
+// an ulp of x/d), which saves the product with zl: all divisors but 182 and 210.
 // The remainder is exact while its last bit stays above the subnormal
-// range, so |x| outside [2^-960, 2^960] (zeros, subnormals, infinities,
-// NaN) takes the division itself.  Checked against __ddiv_rn bit for bit
-// by gsgpu_stumpff_division_selftest.
+// range, so |x| with an exponent outside [-960, 960) (zeros, subnormals,
+// infinities, NaN) takes the division itself.  Checked against __ddiv_rn bit for
+// bit by gsgpu_stumpff_division_selftest.
 struct StumpffDiv {
     double d, zh, zl;
 };

@@ -34,6 +34,7 @@
 // is graph-capturable.  Node-capacity overflow sets ST_TREE_OVERFLOW, which
 // stays set until the host reports it; the kernels after the expansion then do
 // no work (tree_failed / tree_nodes).
+#include "gs_fp64.cuh"
 #include "gs_octree.h"
 #include "gs_ptx.cuh"
 
@@ -148,13 +149,13 @@ k_bbox_final(const double *__restrict__ part, int blocks, double ocx, double ocy
 // r = x - q w corrects it to RN(q + r zh) = RN(x / w) (Markstein, IBM J.
 // Res. Dev. 34(1), 1990).  The remainder is exact while its last bit stays
 // above the subnormal range: |w| in [2^-100, 2^100] (frame[7]) and |x| in
-// [2^-900, 2^900]; other operands (zeros, subnormals, infinities, NaN)
+// [2^-900, 2^900), tested on its exponent bits (an FP64 comparison costs the FP64
+// pipe as much as an add); other operands (zeros, subnormals, infinities, NaN)
 // take the division itself.  Checked against __ddiv_rn bit for bit by
 // gsgpu_width_division_selftest.
 __device__ __forceinline__ double div_by_width(double x, const double *__restrict__ frame)
 {
-    const double ax = fabs(x);
-    if (frame[7] == 0.0 || !(ax >= 0x1p-900 && ax <= 0x1p+900)) return __ddiv_rn(x, frame[3]);
+    if (is_zero(frame[7]) || !exponent_within(x, 900)) return __ddiv_rn(x, frame[3]);
     const double q = __fma_rn(x, frame[5], __dmul_rn(x, frame[6]));
     const double r = __fma_rn(-q, frame[3], x);
     return __fma_rn(r, frame[5], q);

@@ -412,14 +412,11 @@ __global__ void __launch_bounds__(32 * SEQ_WARPS) k_wh_seq_init(EnsDev E)
 //                   finite Jacobi coordinates and the massive particles'
 //                   slots in order (the massive-body list, and at most
 //                   kSeqMassMax of them for the chain);
-//   k_wh_seq_chain  one thread per system: the sequential steps (massive
+//   k_wh_seq_chain  eight lanes per system: the sequential steps (massive
 //                   particles, and the first steps of each massless run until
 //                   the fixed point), recording each run's offsets; the whole
 //                   chain where the run path does not apply;
 //   k_wh_seq_fill   one thread per slot: the runs (x = jx + offset).
-// The chain is a lane's own work: FP64 instructions of a lane-0-only warp
-// cost the FP64 pipe as much as a full warp's, so a warp of 32 systems'
-// chains does 32 times the work of one system's chain in the same time.
 constexpr int SCAN_THREADS = 128;
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_wh_seq_scan(EnsDev E)
@@ -470,38 +467,58 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_wh_seq_scan(EnsDev E)
         n = E.cnt[s];
     }
     // finite Jacobi coordinates (the run path needs them)
+    // (every load is issued whatever the earlier ones gave: stopping at the first
+    // non-finite value would wait for each in turn)
     bool f = true;
-    for (int i = threadIdx.x; i < n; i += SCAN_THREADS)
-        for (int k = 0; k < 3; ++k) f = f && isfinite(jx[3 * i + k]) && isfinite(jv[3 * i + k]);
+#pragma unroll 8
+    for (int k = threadIdx.x; k < 3 * n; k += SCAN_THREADS)
+        f &= finite_bits(jx[k]) & finite_bits(jv[k]);
     const bool finite = __syncthreads_and(f);
-    // the slots with m != 0 in order: counts over contiguous ranges, an
-    // exclusive scan over the block, then the writes
-    const int per = (n + SCAN_THREADS - 1) / SCAN_THREADS;
-    const int lo = min(n, (int)threadIdx.x * per), hi = min(n, lo + per);
-    int c = 0;
-    for (int i = lo; i < hi; ++i) c += m[i] != 0.0 ? 1 : 0;
+    // the slots with m != 0 in order: each warp counts those of a contiguous
+    // share, 32 slots at a time (coalesced), then writes them behind the others'
+    constexpr int WARPS = SCAN_THREADS / 32;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int incl = c;
-    for (int d = 1; d < 32; d <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += t;
-    }
-    __shared__ int warp_tot[SCAN_THREADS / 32];
-    if (lane == 31) warp_tot[wid] = incl;
+    const int per = ((n + SCAN_THREADS - 1) / SCAN_THREADS) * 32;
+    const int lo = min(n, wid * per), hi = min(n, lo + per);
+    // the massive flags of 32 x 32 slots at a time, one word per lane's 32 slots
+    auto flags = [&](int i0) {
+        unsigned mine = 0;
+#pragma unroll 8
+        for (int k = 0; k < 32; ++k) {
+            const int i = i0 + 32 * k + lane;
+            const unsigned b = __ballot_sync(0xffffffffu, i < hi && !is_zero(m[i]));
+            mine = lane == k ? b : mine;
+        }
+        return mine;
+    };
+    int c = 0;
+    for (int i0 = lo; i0 < hi; i0 += 1024) c += __popc(flags(i0));
+    c = __reduce_add_sync(0xffffffffu, c);
+    __shared__ int warp_tot[WARPS];
+    if (lane == 0) warp_tot[wid] = c;
     __syncthreads();
-    int at = incl - c, total = 0;
-    for (int w = 0; w < SCAN_THREADS / 32; ++w) {
+    int at = 0, total = 0;
+    for (int w = 0; w < WARPS; ++w) {
         if (w < wid) at += warp_tot[w];
         total += warp_tot[w];
     }
     int *mass_idx = E.t_ids + base;
     int *hv = E.hv + base;
     const bool massless = E.variant != WH_PAIRWISE;
-    for (int i = lo; i < hi; ++i) {
-        if (m[i] == 0.0) continue;
-        if (at < kSeqMassMax) mass_idx[at] = i;
-        if (massless) hv[at] = i;   // the massive-body list
-        ++at;
+    for (int i0 = lo; i0 < hi && c > 0; i0 += 1024) {
+        unsigned word = flags(i0);
+        int incl = __popc(word);
+        for (int d = 1; d < 32; d <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += t;
+        }
+        int mine = at + incl - __popc(word);
+        for (; word; word &= word - 1, ++mine) {
+            const int i = i0 + 32 * lane + __ffs(word) - 1;
+            if (mine < kSeqMassMax) mass_idx[mine] = i;
+            if (massless) hv[mine] = i;   // the massive-body list
+        }
+        at += __shfl_sync(0xffffffffu, incl, 31);
     }
     if (!massless)
         for (int i = threadIdx.x; i < n; i += SCAN_THREADS) hv[i] = i;
@@ -511,71 +528,89 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_wh_seq_scan(EnsDev E)
     }
 }
 
-__global__ void k_wh_seq_chain(EnsDev E)
+// Eight lanes per system, one per component of x and v (two idle): a chain step
+// is one subtraction, division and two products for all six, where one thread
+// per system took six of each (59 -> 15 us for 512 systems).  The warp's four
+// systems take their steps together until the last is done.
+constexpr int CHAIN_THREADS = 64;
+__global__ void __launch_bounds__(CHAIN_THREADS) k_wh_seq_chain(EnsDev E)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= E.S) return;
-    const int nmass = E.seq_nmass[s];
-    if (nmass == -2) return;   // empty system
+    const int s0 = (blockIdx.x * CHAIN_THREADS + threadIdx.x) >> 3;
+    const int c = min((int)(threadIdx.x & 7), 5);
+    const bool on = (threadIdx.x & 7) < 6;
+    const int nmass = s0 < E.S ? E.seq_nmass[s0] : -2;
+    const bool live = nmass != -2;   // not an empty system
+    const int s = live ? s0 : 0;
     const int base = E.off[s];
-    const int n = E.cnt[s];
+    const int n = live ? E.cnt[s] : 0;
     const double *m = E.m + base, *eta = E.eta + base;
-    double *x = E.x + 3 * base, *v = E.v + 3 * base;
-    const double *jx = E.jx + 3 * base, *jv = E.jv + 3 * base;
-    double xc[3], vc[3], y[6];
-    for (int k = 0; k < 3; ++k) {
-        xc[k] = __dmul_rn(eta[n - 1], jx[k]);
-        vc[k] = __dmul_rn(eta[n - 1], jv[k]);
-    }
+    double *out = (c < 3 ? E.x : E.v) + 3 * (size_t)base + c % 3;
+    const double *j = (c < 3 ? E.jx : E.jv) + 3 * (size_t)base + c % 3;
+    const int *mass_idx = E.t_ids + base;
     const size_t rb = (size_t)s * (kSeqMassMax + 1);
+    double xc = live ? __dmul_rn(eta[n - 1], j[0]) : 0.0;
     int nr = 0;
-    if (nmass >= 0) {
-        const int *mass_idx = E.t_ids + base;
-        int q = nmass - 1;   // highest massive particle not yet passed
-        int i = n - 1;
-        while (i >= 1) {
-            while (q >= 0 && mass_idx[q] > i) --q;
-            const int mtop = q >= 0 ? mass_idx[q] : -1;
-            if (mtop == i) {
-                jac_step(xc, vc, m[i], eta[i], eta[i - 1], jx + 3 * i, jv + 3 * i, x + 3 * i,
-                         v + 3 * i, y);
-                --i;
-                continue;
-            }
-            const int lo = mtop + 1 > 1 ? mtop + 1 : 1;
-            int j = i;
-            bool fixed = false;
-            while (j >= lo && !fixed) {
-                const double ox[3] = {xc[0], xc[1], xc[2]}, ov[3] = {vc[0], vc[1], vc[2]};
-                jac_step(xc, vc, m[j], eta[j], eta[j - 1], jx + 3 * j, jv + 3 * j, x + 3 * j,
-                         v + 3 * j, y);
-                fixed = true;
-                for (int k = 0; k < 3; ++k)
-                    fixed = fixed && __double_as_longlong(xc[k]) == __double_as_longlong(ox[k]) &&
-                            __double_as_longlong(vc[k]) == __double_as_longlong(ov[k]) &&
-                            isfinite(xc[k]) && isfinite(vc[k]) && !neg_zero(xc[k]) &&
-                            !neg_zero(vc[k]);
-                --j;
-            }
-            if (j >= lo) {
-                E.run_lo[rb + nr] = lo;
-                E.run_hi[rb + nr] = j;
-                for (int k = 0; k < 6; ++k) E.run_y[(rb + nr) * 6 + k] = y[k];
-                ++nr;
-            }
-            i = lo - 1;
+    int q = nmass - 1;   // highest massive particle not yet passed
+    int i = n - 1;
+    int mtop = q >= 0 && i >= 1 ? mass_idx[q] : -1;
+    // the next step's operands, fetched a step ahead where it is the next slot
+    double mi = 0.0, ei = 1.0, ep = 1.0, ji = 0.0;
+    if (i >= 1) {
+        mi = m[i];
+        ei = eta[i];
+        ep = eta[i - 1];
+        ji = j[3 * i];
+    }
+    while (__any_sync(0xffffffffu, i >= 1)) {
+        const bool act = i >= 1;
+        double mi1 = 0.0, ep1 = 1.0, ji1 = 0.0;
+        if (i >= 2) {
+            mi1 = m[i - 1];
+            ep1 = eta[i - 2];
+            ji1 = j[3 * (i - 1)];
         }
-    } else {
-        // the whole chain, particle by particle
-        for (int i = n - 1; i >= 1; --i)
-            jac_step(xc, vc, m[i], eta[i], eta[i - 1], jx + 3 * i, jv + 3 * i, x + 3 * i, v + 3 * i,
-                     y);
+        if (act && nmass >= 0)
+            while (mtop > i) mtop = --q >= 0 ? mass_idx[q] : -1;
+        const double old = xc;
+        const double y = __ddiv_rn(__dsub_rn(xc, __dmul_rn(mi, ji)), ei);
+        const double xi = __dadd_rn(ji, y);
+        const double next = __dmul_rn(ep, y);
+        const bool same = __double_as_longlong(next) == __double_as_longlong(old) &&
+                          finite_bits(next) && !neg_zero(next);
+        const unsigned all = __ballot_sync(0xffffffffu, same);
+        if (!act) continue;
+        xc = next;
+        if (on) out[3 * i] = xi;
+        int to = i - 1;
+        if (nmass >= 0 && mtop != i && ((all >> (threadIdx.x & 24)) & 0xffu) == 0xffu) {
+            // a fixed point: the rest of the massless run takes this offset
+            const int lo = max(mtop + 1, 1);
+            if (to >= lo) {
+                if ((threadIdx.x & 7) == 0) {
+                    E.run_lo[rb + nr] = lo;
+                    E.run_hi[rb + nr] = to;
+                }
+                if (on) E.run_y[(rb + nr) * 6 + c] = y;
+                ++nr;
+                to = lo - 1;
+            }
+        }
+        if (to == i - 1) {
+            ei = ep;
+            mi = mi1;
+            ep = ep1;
+            ji = ji1;
+        } else if (to >= 1) {
+            mi = m[to];
+            ei = eta[to];
+            ep = eta[to - 1];
+            ji = j[3 * to];
+        }
+        i = to;
     }
-    E.seq_runs[s] = nr;
-    for (int k = 0; k < 3; ++k) {
-        x[k] = __ddiv_rn(xc[k], m[0]);
-        v[k] = __ddiv_rn(vc[k], m[0]);
-    }
+    if (!live) return;
+    if ((threadIdx.x & 7) == 0) E.seq_runs[s] = nr;
+    if (on) out[0] = __ddiv_rn(xc, m[0]);
 }
 
 // One thread per slot: a slot of a massless run takes the run's offsets.
@@ -675,9 +710,9 @@ __global__ void __launch_bounds__(32 * PAIR_WARPS) k_wh_pairs(EnsDev E)
 template <int K> __device__ __forceinline__ double sdiv(double x)
 {
     const double d = kStumpffDiv[K].d, zh = kStumpffDiv[K].zh, zl = kStumpffDiv[K].zl;
-    const double ax = fabs(x);
-    if (!(ax >= 0x1p-960 && ax <= 0x1p+960)) return __ddiv_rn(x, d);
-    const double q = __fma_rn(x, zh, __dmul_rn(x, zl));
+    if (!exponent_within(x, 960)) return __ddiv_rn(x, d);
+    constexpr bool two_words = K == SD182 || K == SD210;
+    const double q = two_words ? __fma_rn(x, zh, __dmul_rn(x, zl)) : __dmul_rn(x, zh);
     const double r = __fma_rn(-q, d, x);
     return __fma_rn(r, zh, q);
 }
@@ -685,8 +720,8 @@ template <int K> __device__ __forceinline__ double sdiv(double x)
 __device__ __forceinline__ void stumpff(double z, double &c0, double &c1, double &c2, double &c3)
 {
     int q = 0;
-    while (fabs(z) > 0.1) {
-        z = __ddiv_rn(z, 4.0);
+    while (abs_bits(z) > __double_as_longlong(0.1)) {   // |z| > 0.1
+        z = __dmul_rn(z, 0.25);   // exact scaling, as the other powers of two below
         ++q;
     }
     double t = __dsub_rn(1.0, sdiv<SD210>(z));
@@ -706,8 +741,8 @@ __device__ __forceinline__ void stumpff(double z, double &c0, double &c1, double
     double s1 = __dsub_rn(1.0, __dmul_rn(z, s3));
     double s0 = __dsub_rn(1.0, __dmul_rn(z, s2));
     while (q > 0) {
-        s3 = __ddiv_rn(__dadd_rn(s2, __dmul_rn(s0, s3)), 4.0);
-        s2 = __ddiv_rn(__dmul_rn(s1, s1), 2.0);
+        s3 = __dmul_rn(__dadd_rn(s2, __dmul_rn(s0, s3)), 0.25);
+        s2 = __dmul_rn(__dmul_rn(s1, s1), 0.5);
         s1 = __dmul_rn(s0, s1);
         s0 = __dsub_rn(__dmul_rn(__dmul_rn(2.0, s0), s0), 1.0);
         --q;
@@ -735,7 +770,7 @@ __device__ bool kepler_drift(double *jx, double *jv, double gm, double dt)
     for (int it = 0; it < 500; ++it) {
         const double ss = __dmul_rn(s, s);
         const double z = __dmul_rn(alpha, ss);
-        if (!isfinite(z)) {
+        if (!finite_bits(z)) {
             bad_z = true;
             break;
         }
@@ -749,7 +784,7 @@ __device__ bool kepler_drift(double *jx, double *jv, double gm, double dt)
                                     __dmul_rn(__dmul_rn(gm, ss), c2));
         const double ds = __ddiv_rn(-F, dF);
         s = __dadd_rn(s, ds);
-        if (fabs(ds) < 1e-12) {
+        if (abs_bits(ds) < __double_as_longlong(1e-12)) {
             conv = true;
             break;
         }
@@ -817,7 +852,7 @@ __global__ void k_wh_accel(EnsDev E, int P)
     const int nh = E.nh[s];
     const double e3 = __dmul_rn(__dmul_rn(E.eps, E.eps), E.eps);
     const double G = E.G;
-    const bool massive = (E.variant == WH_PAIRWISE) || m[i] != 0.0;
+    const bool massive = (E.variant == WH_PAIRWISE) || !is_zero(m[i]);
     const double xi[3] = {x[3 * i], x[3 * i + 1], x[3 * i + 2]};
     const double tv[3] = {__dsub_rn(xi[0], x[0]), __dsub_rn(xi[1], x[1]), __dsub_rn(xi[2], x[2])};
     const double tn = norm3d(tv);
@@ -917,7 +952,7 @@ __global__ void k_ens_massless_accel(EnsDev E, int P)
     double a0 = 0.0, a1 = 0.0, a2 = 0.0;
     // the pairwise variant lists every particle and is the symmetric sum of
     // src/acceleration.c:177-234 seen from particle i (same term order)
-    if (E.variant == WH_PAIRWISE || m[i] != 0.0) {
+    if (E.variant == WH_PAIRWISE || !is_zero(m[i])) {
         for (int q = 0; q < nh; ++q) {
             const int j = hv[q];
             if (j == i) continue;
@@ -1081,8 +1116,15 @@ struct gsgpu_ensemble {
     ~gsgpu_ensemble()
     {
         if (graph) cudaGraphExecDestroy(graph);
+        for (int c = 0; c < kSortClasses; ++c) {
+            if (side[c]) cudaStreamDestroy(side[c]);
+            if (ev_join[c]) cudaEventDestroy(ev_join[c]);
+        }
+        if (ev_fork) cudaEventDestroy(ev_fork);
         if (own_stream && stream) cudaStreamDestroy(stream);
     }
+    cudaStream_t side[kSortClasses] = {};
+    cudaEvent_t ev_fork = nullptr, ev_join[kSortClasses] = {};
 
     int pgrid() const { return (P + 127) / 128; }
     int tpb_accel = 128, tpb_drift = 128;   // chosen by autotune()
@@ -1181,20 +1223,41 @@ struct gsgpu_ensemble {
         return st;
     }
 
+    // The classes' launches are independent: all but the first present one run
+    // on side streams, forked from and joined to the ensemble's.  A launch of
+    // few large systems leaves most of the GPU idle: for 512 systems the three
+    // take 76, 25 and 15 us one after the other.
     ErrorStatus sort(double *vec, double *vel)
     {
-        for (int c = 0; c < kSortClasses; ++c) {
+        const bool fork = sort_launches() > 1;
+        if (fork && !ev_fork) {
+            GS_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
+            for (int c = 0; c < kSortClasses; ++c) {
+                GS_CUDA(cudaStreamCreateWithFlags(&side[c], cudaStreamNonBlocking));
+                GS_CUDA(cudaEventCreateWithFlags(&ev_join[c], cudaEventDisableTiming));
+            }
+        }
+        if (fork) GS_CUDA(cudaEventRecord(ev_fork, stream));
+        bool first = true;
+        for (int c = kSortClasses - 1; c >= 0; --c) {   // the largest systems first
             const int count = sort_first[c + 1] - sort_first[c];
             if (count == 0) continue;
+            cudaStream_t on = first ? stream : side[c];
+            if (!first) GS_CUDA(cudaStreamWaitEvent(on, ev_fork, 0));
             const int p2 = sort_pow2[c];
             const size_t smem = (size_t)p2 * 12;
             // one thread per pair of slots for the odd-even passes, 32..1024,
             // unless the autotuner chose fewer
             const int threads = sort_tpb[c] > 0 ? sort_tpb[c] : std::min(1024, std::max(32, p2 / 2));
-            k_wh_sort<<<count, threads, smem, stream>>>(E, vec, vel, p2, vec == E.x ? 1 : 0,
-                                                        sort_list.as<int>() + sort_first[c]);
+            k_wh_sort<<<count, threads, smem, on>>>(E, vec, vel, p2, vec == E.x ? 1 : 0,
+                                                    sort_list.as<int>() + sort_first[c]);
+            GS_CUDA(cudaGetLastError());
+            if (!first) {
+                GS_CUDA(cudaEventRecord(ev_join[c], on));
+                GS_CUDA(cudaStreamWaitEvent(stream, ev_join[c], 0));
+            }
+            first = false;
         }
-        GS_CUDA(cudaGetLastError());
         return ok();
     }
 
@@ -1204,7 +1267,7 @@ struct gsgpu_ensemble {
     ErrorStatus to_cartesian(const EnsDev &D)
     {
         k_wh_seq_scan<<<S, SCAN_THREADS, 0, stream>>>(D);
-        k_wh_seq_chain<<<(S + 63) / 64, 64, 0, stream>>>(D);
+        k_wh_seq_chain<<<(8 * S + CHAIN_THREADS - 1) / CHAIN_THREADS, CHAIN_THREADS, 0, stream>>>(D);
         k_wh_seq_fill<<<pgrid(), 128, 0, stream>>>(D, P);
         GS_CUDA(cudaGetLastError());
         return ok();
