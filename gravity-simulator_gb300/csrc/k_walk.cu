@@ -4,22 +4,32 @@
 // and acceleration_barnes_hut (:33-76).
 //
 // Warp-cooperative walk.  A warp owns 32 consecutive particles in Morton
-// order and walks the union of their traversals: a warp-uniform stack holds,
-// per depth, the node being scanned, the next child to scan and the mask of
-// lanes still inside that subtree.  At each child every lane in the mask
-// makes the reference's own decision for its particle --
-//   cell-membership test on Morton prefixes (compat: the reference's
-//   sorted-keys-by-particle-id read, :120/:145), then the opening test
+// order and walks the union of their traversals.  A shared stack holds nodes
+// with the mask of the lanes whose walk reaches them; each step pops up to 32
+// nodes, every lane loads the records of one into shared memory, and then all
+// lanes go through the batch, each making the reference's own decision for its
+// particle --
+//   cell-membership test (compat: the reference's Morton prefixes with its
+//   sorted-keys-by-particle-id read, src/acceleration_barnes_hut.c:120/:145;
+//   otherwise the sorted index in the cell's range, which is the same test on the
+//   particle's own key), then the opening test
 //   (w_level)^2 < theta^2 |R|^2 (:157-162) -> monopole (:164-174),
 //   else leaf -> particle terms skipping itself (:181-214), else descend --
-// and the warp descends into the child when any lane needs it.  Each
-// particle therefore sees exactly the nodes, in exactly the order, of the
-// reference's depth-first walk; lanes not in a subtree's mask idle there.
+// and the nodes that some lanes open push their children with those lanes'
+// mask (leaves: their particles are staged and summed the same way).  Each
+// particle sees exactly the nodes of the reference's depth-first walk, in
+// another order.
+//
+// What bounds it is instruction issue.  Walking one child at a time (a stack
+// of node, next child and mask per depth) cost about 220 instructions and a
+// chain of dependent loads per interaction; in a batch the loads of 32 nodes are
+// one, and a node costs about 45 instructions.  Walk of the galaxy pair at
+// N = 150,000, theta 0.5: 2.79 -> 1.13 ms.
 //
 // Precision: positions and centres of mass are double-float pairs (hi, lo)
 // relative to the bounding-box centre, so R = (c_hi - x_hi) + (c_lo - x_lo)
 // keeps FP32 relative accuracy for close pairs; pair terms are FP32 with
-// rsqrt; each child's contribution is added to a Kahan-compensated FP32
+// rsqrt; each term is added to a Kahan-compensated FP32
 // accumulator.  The opening test is made in FP32 unless |w^2 - theta^2|R|^2|
 // is within 1e-5 of w^2, in which case it is recomputed in FP64 exactly as
 // the reference does, so every decision equals the reference's.
@@ -33,7 +43,11 @@ namespace gs {
 
 constexpr int WK_THREADS = 128;
 constexpr int WK_WARPS = WK_THREADS / 32;
-constexpr int WK_STACK = OCT_MAX_LEVEL + 2;
+constexpr int WK_STACK = 512;    // stack entries per warp
+// Entries kept free for a depth-first descent: popping one node and pushing its
+// (at most 8) children grows the stack by 7 per level.  Batches shrink so that the
+// stack never passes WK_STACK - WK_RESERVE before such a descent starts.
+constexpr int WK_RESERVE = 8 * (OCT_MAX_LEVEL + 1);
 
 struct WalkArgs {
     const float4 *na;
@@ -42,6 +56,7 @@ struct WalkArgs {
     const int4 *nc;
     const uint64_t *nkey;
     const double *ncom;     // FP64 centre of mass [3*nodes] (exact opening test)
+    const int *depth;
     const float4 *pa;
     const float4 *pb;
     const int *sidx;
@@ -49,7 +64,6 @@ struct WalkArgs {
     const double *x;        // FP64 positions by particle id
     const double *frame;    // cx, cy, cz, width, box_length
     int n;
-    int compat;
     float eps2;
     double theta2;
     double G;
@@ -59,193 +73,251 @@ struct WalkArgs {
     const int *gate;                // when set, the launch runs only if *gate != 0
 };
 
-__device__ __forceinline__ void add3(float &sx, float &cx, float &sy, float &cy, float &sz, float &cz,
-                                     float px, float py, float pz)
+// Kahan-compensated sums of x, y (as a pair, through the paired FP32 operations)
+// and z; n* hold the negated compensations.
+struct Acc3 {
+    float2 s, n;
+    float sz, nz;
+};
+
+__device__ __forceinline__ void add3(Acc3 &a, float2 pxy, float pz)
 {
-    kahan_add(sx, cx, px);
-    kahan_add(sy, cy, py);
-    kahan_add(sz, cz, pz);
+    const float2 minus = make_float2(-1.0f, -1.0f);
+    const float2 y = __fadd2_rn(pxy, a.n);
+    const float2 t = __fadd2_rn(a.s, y);
+    a.n = __ffma2_rn(__ffma2_rn(a.s, minus, t), minus, y);   // y - (t - s)
+    a.s = t;
+    const float yz = __fadd_rn(pz, a.nz);
+    const float tz = __fadd_rn(a.sz, yz);
+    a.nz = __fsub_rn(yz, __fsub_rn(tz, a.sz));
+    a.sz = tz;
 }
 
-template <bool QUAD>
+// One batch of nodes or of leaf particles in shared memory.
+template <bool QUAD, bool COMPAT>
+struct WalkShared {
+    int2 stack[WK_STACK];    // (node, lanes that reach it)
+    float4 a[32], b[32];     // com or position: (hi, mass), (lo, cell side^2)
+    int4 c[32];              // (first child, children, first particle, particles)
+    unsigned mask[32];
+    float4 q[QUAD ? 64 : 1];
+    uint64_t key[COMPAT ? 32 : 1];
+    int level[COMPAT ? 32 : 1];
+};
+
+template <bool QUAD, bool COMPAT>
 __global__ void __launch_bounds__(WK_THREADS)
 k_bh_walk(WalkArgs A)
 {
-    __shared__ int s_node[WK_WARPS][WK_STACK];
-    __shared__ int s_next[WK_WARPS][WK_STACK];
-    __shared__ unsigned s_mask[WK_WARPS][WK_STACK];
-    __shared__ float s_w2[WK_STACK];     // (cell width at depth)^2, FP32
-    __shared__ double s_w[WK_STACK];     // cell width at depth, FP64 (reference formula)
+    __shared__ WalkShared<QUAD, COMPAT> shared_all[WK_WARPS];
 
     if (A.gate && *A.gate == 0) return;   // block-uniform
     if (*A.status & ST_TREE_OVERFLOW) return;   // the build overflowed: no tree to walk
-    const int warp = threadIdx.x >> 5;
+    WalkShared<QUAD, COMPAT> &w = shared_all[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
-    if (threadIdx.x < WK_STACK) {
-        const int lv = threadIdx.x;
-        // box_length / (2 << level)  (src/acceleration_barnes_hut.c:157)
-        const double w = lv >= 1 && lv <= OCT_MAX_LEVEL ? __ddiv_rn(A.frame[4], (double)(2 << lv)) : 0.0;
-        s_w[lv] = w;
-        s_w2[lv] = __double2float_rn(__dmul_rn(w, w));
-    }
-    __syncthreads();
+    const unsigned lt = (1u << lane) - 1u;
 
     const int s = blockIdx.x * WK_THREADS + threadIdx.x;
     const bool valid = s < A.n;
     const int id = valid ? A.sidx[s] : -1;
     uint64_t key_i = 0;
-    float xh = 0.f, yh = 0.f, zh = 0.f, xl = 0.f, yl = 0.f, zl = 0.f;
-    double x0 = 0.0, x1 = 0.0, x2 = 0.0;
+    // negated particle position
+    float2 nxyh = make_float2(0.f, 0.f), nxyl = nxyh;
+    float nzh = 0.f, nzl = 0.f;
     if (valid) {
-        key_i = A.compat ? A.skeys[id] : A.skeys[s];
-        const float4 ph = A.pa[s];
-        const float4 pl = A.pb[s];
-        xh = ph.x; yh = ph.y; zh = ph.z;
-        xl = pl.x; yl = pl.y; zl = pl.z;
-        x0 = A.x[3 * id + 0];
-        x1 = A.x[3 * id + 1];
-        x2 = A.x[3 * id + 2];
+        if (COMPAT) key_i = A.skeys[id];
+        const float4 ph = A.pa[s], pl = A.pb[s];
+        nxyh = make_float2(-ph.x, -ph.y);
+        nxyl = make_float2(-pl.x, -pl.y);
+        nzh = -ph.z;
+        nzl = -pl.z;
     }
     const float th2f = (float)A.theta2;
-    float sx = 0.f, sy = 0.f, sz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
-    unsigned long long n_cell = 0, n_pp = 0;
+    Acc3 acc = {};
+    int n_cell = 0, n_pp = 0;
 
     const unsigned valid_mask = __ballot_sync(0xffffffffu, valid);
-    if (valid_mask == 0) return;
-    if (lane == 0) {
-        s_node[warp][0] = 0;
-        s_next[warp][0] = 0;
-        s_mask[warp][0] = valid_mask;
-    }
+    if (valid_mask == 0) return;   // warp-uniform
+    // the root is opened by every lane without a test: its children start the walk
+    const int4 root = A.nc[0];
+    if (lane < root.y) w.stack[lane] = make_int2(root.x + lane, (int)valid_mask);
+    int top = root.y;
     __syncwarp();
-    int top = 0;
-    int level = 1;   // depth of the children being scanned
-    for (;;) {
-        const int node = s_node[warp][top];
-        const int nxt = s_next[warp][top];
-        const int4 pinfo = A.nc[node];
-        if (nxt >= pinfo.y) {
-            if (top == 0) break;
-            --top;
-            --level;
-            continue;
+    while (top > 0) {
+        int k = min(32, top);
+        const int room = (WK_STACK - WK_RESERVE - top) / 7;
+        if (room < k) k = max(1, room);
+        // load: one node per lane
+        int4 ci = make_int4(0, 0, 0, 0);
+        if (lane < k) {
+            const int2 e = w.stack[top - k + lane];
+            ci = A.nc[e.x];
+            w.a[lane] = A.na[e.x];
+            w.b[lane] = A.nb[e.x];
+            // what the loop needs of the node: (node, -, first particle, particles)
+            w.c[lane] = make_int4(e.x, ci.y, ci.z, ci.w);
+            w.mask[lane] = (unsigned)e.y;
+            if (QUAD) {
+                w.q[2 * lane] = A.nq[2 * (size_t)e.x];
+                w.q[2 * lane + 1] = A.nq[2 * (size_t)e.x + 1];
+            }
+            if (COMPAT) {
+                w.key[lane] = A.nkey[e.x];
+                w.level[lane] = A.depth[e.x];
+            }
+        }
+        top -= k;
+        __syncwarp();
+        unsigned opened = 0;   // lanes that open this lane's node
+#pragma unroll 2
+        for (int j = 0; j < k; ++j) {
+            const float4 ca = w.a[j], cb = w.b[j];
+            const bool act = (w.mask[j] >> lane) & 1u;
+            const float2 dxy = __fadd2_rn(__fadd2_rn(make_float2(ca.x, ca.y), nxyh),
+                                          __fadd2_rn(make_float2(cb.x, cb.y), nxyl));
+            const float dz = (ca.z + nzh) + (cb.z + nzl);
+            const float ns = fmaf(dxy.x, dxy.x, fmaf(dxy.y, dxy.y, dz * dz));
+            const float t = th2f * ns;
+            bool accept = act && cb.w < t;
+            bool inside;
+            if (COMPAT) {
+                const int sh = 3 * (OCT_MAX_LEVEL - w.level[j]);
+                inside = (key_i >> sh) == (w.key[j] >> sh);
+            } else {
+                const int4 cj = w.c[j];
+                inside = (unsigned)(s - cj.z) < (unsigned)cj.w;
+            }
+            if (act && !inside && fabsf(cb.w - t) <= 1e-5f * cb.w) {
+                // exact FP64 test, reference operation order
+                const int c = w.c[j].x;
+                const double r0 = __dsub_rn(A.x[3 * (size_t)id + 0], A.ncom[3 * (size_t)c + 0]);
+                const double r1 = __dsub_rn(A.x[3 * (size_t)id + 1], A.ncom[3 * (size_t)c + 1]);
+                const double r2 = __dsub_rn(A.x[3 * (size_t)id + 2], A.ncom[3 * (size_t)c + 2]);
+                const double nsd = __dadd_rn(__dadd_rn(__dmul_rn(r0, r0), __dmul_rn(r1, r1)),
+                                             __dmul_rn(r2, r2));
+                // box_length / (2 << level)  (src/acceleration_barnes_hut.c:157)
+                const double wd = __ddiv_rn(A.frame[4], (double)(2 << A.depth[c]));
+                accept = __dmul_rn(wd, wd) < __dmul_rn(A.theta2, nsd);
+            }
+            accept = accept && !inside;
+            const unsigned om = __ballot_sync(0xffffffffu, act && !accept);
+            if (lane == j) opened = om;
+            if (!__any_sync(0xffffffffu, accept)) continue;
+            // lanes that do not accept add zeros
+            const float ri = accept ? rsqrt_approx(ns + A.eps2) : 0.0f;
+            const float ri2 = ri * ri;
+            const float ri3 = ri2 * ri;
+            const float sc = ca.w * ri3;
+            float2 pxy = __fmul2_rn(dxy, make_float2(sc, sc));
+            float pz = dz * sc;
+            if (QUAD) {
+                // d = com - x = -R:  G [-Q d / r^5 + 2.5 (d.Q.d) d / r^7]
+                const float4 q0 = w.q[2 * j], q1 = w.q[2 * j + 1];
+                const float qx = q0.x * dxy.x + q0.y * dxy.y + q0.z * dz;
+                const float qy = q0.y * dxy.x + q0.w * dxy.y + q1.x * dz;
+                const float qz = q0.z * dxy.x + q1.x * dxy.y + q1.y * dz;
+                const float dqd = dxy.x * qx + dxy.y * qy + dz * qz;
+                const float ri5 = ri3 * ri2;
+                const float f = 2.5f * dqd * ri5 * ri2;
+                pxy.x += f * dxy.x - qx * ri5;
+                pxy.y += f * dxy.y - qy * ri5;
+                pz += f * dz - qz * ri5;
+            }
+            add3(acc, pxy, pz);
+            n_cell += accept ? 1 : 0;
+        }
+        __syncwarp();   // the batch is read
+        // children of opened nodes, with the opening lanes
+        const int ch = opened ? ci.y : 0;
+        int cin = ch;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, cin, o);
+            if (lane >= o) cin += t;
+        }
+        const int pushes = __shfl_sync(0xffffffffu, cin, 31);
+        if (top + pushes > WK_STACK) {
+            if (lane == 0) atomicOr(A.status, ST_STACK_OVERFLOW);
+            break;
+        }
+        for (int q = 0; q < ch; ++q) w.stack[top + cin - ch + q] = make_int2(ci.x + q, (int)opened);
+        top += pushes;
+        // particles of opened leaves, 32 at a time
+        const int cnt = (opened && ci.y <= 0) ? ci.w : 0;
+        unsigned leaves = __ballot_sync(0xffffffffu, cnt > 0);
+        int skip = 0;   // particles of the first remaining leaf already taken
+        while (leaves) {
+            // lanes take the particles of the remaining leaves in turn
+            int have = 0;
+            int mine = -1;
+            unsigned open_m = 0;
+            while (leaves && have < 32) {
+                const int src = __ffs(leaves) - 1;
+                const int first = __shfl_sync(0xffffffffu, ci.z, src) + skip;
+                const int left = __shfl_sync(0xffffffffu, cnt, src) - skip;
+                const unsigned om = __shfl_sync(0xffffffffu, opened, src);
+                const int take = min(left, 32 - have);
+                if (lane >= have && lane < have + take) {
+                    mine = first + lane - have;
+                    open_m = om;
+                }
+                have += take;
+                skip += take;
+                if (take == left) {
+                    leaves &= leaves - 1;
+                    skip = 0;
+                }
+            }
+            __syncwarp();
+            if (mine >= 0) {
+                w.a[lane] = A.pa[mine];
+                w.b[lane] = A.pb[mine];
+                w.mask[lane] = open_m;
+                w.c[lane].x = mine;
+            }
+            __syncwarp();
+#pragma unroll 2
+            for (int j = 0; j < have; ++j) {
+                const float4 qa = w.a[j], qb = w.b[j];
+                const bool act = ((w.mask[j] >> lane) & 1u) && w.c[j].x != s;
+                const float2 dxy = __fadd2_rn(__fadd2_rn(make_float2(qa.x, qa.y), nxyh),
+                                              __fadd2_rn(make_float2(qb.x, qb.y), nxyl));
+                const float dz = (qa.z + nzh) + (qb.z + nzl);
+                const float r2 = fmaf(dxy.x, dxy.x, fmaf(dxy.y, dxy.y, fmaf(dz, dz, A.eps2)));
+                const float ri = rsqrt_approx(r2);
+                const float sc = act ? qa.w * ri * ri * ri : 0.0f;
+                add3(acc, __fmul2_rn(dxy, make_float2(sc, sc)), dz * sc);
+                n_pp += act ? 1 : 0;
+            }
+            __syncwarp();
         }
         __syncwarp();
-        if (lane == 0) s_next[warp][top] = nxt + 1;
-        const unsigned mask = s_mask[warp][top];
-        __syncwarp();
-        const int c = pinfo.x + nxt;
-        const bool act = (mask >> lane) & 1u;
-        const float4 ca = A.na[c];
-        const float4 cb = A.nb[c];
-        const int4 ci = A.nc[c];
-        const uint64_t ck = A.nkey[c];
-        int dec = 0;   // 1 accepted, 2 leaf, 3 open
-        if (act) {
-            const int sh = 3 * (OCT_MAX_LEVEL - level);
-            const bool inside = (key_i >> sh) == (ck >> sh);
-            if (!inside) {
-                const float dx = (ca.x - xh) + (cb.x - xl);
-                const float dy = (ca.y - yh) + (cb.y - yl);
-                const float dz = (ca.z - zh) + (cb.z - zl);
-                const float ns = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                const float w2 = s_w2[level];
-                const float t = th2f * ns;
-                bool accept;
-                if (fabsf(w2 - t) <= 1e-5f * w2) {
-                    // exact FP64 test, reference operation order
-                    const double r0 = __dsub_rn(x0, A.ncom[3 * c + 0]);
-                    const double r1 = __dsub_rn(x1, A.ncom[3 * c + 1]);
-                    const double r2 = __dsub_rn(x2, A.ncom[3 * c + 2]);
-                    const double nsd = __dadd_rn(__dadd_rn(__dmul_rn(r0, r0), __dmul_rn(r1, r1)),
-                                                 __dmul_rn(r2, r2));
-                    const double wd = s_w[level];
-                    accept = __dmul_rn(wd, wd) < __dmul_rn(A.theta2, nsd);
-                } else {
-                    accept = w2 < t;
-                }
-                if (accept) {
-                    const float r2 = ns + A.eps2;
-                    const float ri = rsqrt_approx(r2);
-                    const float ri2 = ri * ri;
-                    const float ri3 = ri2 * ri;
-                    const float sc = ca.w * ri3;
-                    float px = dx * sc, py = dy * sc, pz = dz * sc;
-                    if (QUAD) {
-                        // d = com - x = -R:  G [-Q d / r^5 + 2.5 (d.Q.d) d / r^7]
-                        const float4 q0 = A.nq[2 * c];
-                        const float4 q1 = A.nq[2 * c + 1];
-                        const float qx = q0.x * dx + q0.y * dy + q0.z * dz;
-                        const float qy = q0.y * dx + q0.w * dy + q1.x * dz;
-                        const float qz = q0.z * dx + q1.x * dy + q1.y * dz;
-                        const float dqd = dx * qx + dy * qy + dz * qz;
-                        const float ri5 = ri3 * ri2;
-                        const float f = 2.5f * dqd * ri5 * ri2;
-                        px += f * dx - qx * ri5;
-                        py += f * dy - qy * ri5;
-                        pz += f * dz - qz * ri5;
-                    }
-                    add3(sx, cx, sy, cy, sz, cz, px, py, pz);
-                    ++n_cell;
-                    dec = 1;
-                }
-            }
-            if (dec == 0) dec = (ci.y <= 0) ? 2 : 3;
-        }
-        const unsigned leaf_mask = __ballot_sync(0xffffffffu, dec == 2);
-        const unsigned open_mask = __ballot_sync(0xffffffffu, dec == 3);
-        if (leaf_mask) {
-            float px = 0.f, py = 0.f, pz = 0.f;
-            for (int k = 0; k < ci.w; ++k) {
-                const int p = ci.z + k;
-                const float4 qa = A.pa[p];
-                const float4 qb = A.pb[p];
-                const int pid = A.sidx[p];
-                if (dec == 2 && pid != id) {
-                    const float dx = (qa.x - xh) + (qb.x - xl);
-                    const float dy = (qa.y - yh) + (qb.y - yl);
-                    const float dz = (qa.z - zh) + (qb.z - zl);
-                    const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, A.eps2)));
-                    const float ri = rsqrt_approx(r2);
-                    const float sc = qa.w * ri * ri * ri;
-                    px = fmaf(dx, sc, px);
-                    py = fmaf(dy, sc, py);
-                    pz = fmaf(dz, sc, pz);
-                    ++n_pp;
-                }
-            }
-            if (dec == 2) add3(sx, cx, sy, cy, sz, cz, px, py, pz);
-        }
-        if (open_mask) {
-            if (top + 1 >= WK_STACK) {
-                if (lane == 0) atomicOr(A.status, ST_STACK_OVERFLOW);
-                break;
-            }
-            ++top;
-            ++level;
-            __syncwarp();
-            if (lane == 0) {
-                s_node[warp][top] = c;
-                s_next[warp][top] = 0;
-                s_mask[warp][top] = open_mask;
-            }
-            __syncwarp();
-        }
     }
     if (valid) {
-        A.a[3 * id + 0] = A.G * ((double)sx - (double)cx);
-        A.a[3 * id + 1] = A.G * ((double)sy - (double)cy);
-        A.a[3 * id + 2] = A.G * ((double)sz - (double)cz);
+        A.a[3 * (size_t)id + 0] = A.G * ((double)acc.s.x + (double)acc.n.x);
+        A.a[3 * (size_t)id + 1] = A.G * ((double)acc.s.y + (double)acc.n.y);
+        A.a[3 * (size_t)id + 2] = A.G * ((double)acc.sz + (double)acc.nz);
     }
     // interaction counts (warp sums, one atomic per warp)
+    unsigned long long tc = n_cell, tp = n_pp;
     for (int o = 16; o > 0; o >>= 1) {
-        n_cell += __shfl_down_sync(0xffffffffu, n_cell, o);
-        n_pp += __shfl_down_sync(0xffffffffu, n_pp, o);
+        tc += __shfl_down_sync(0xffffffffu, tc, o);
+        tp += __shfl_down_sync(0xffffffffu, tp, o);
     }
     if (lane == 0) {
-        atomicAdd(&A.counters[0], n_cell);
-        atomicAdd(&A.counters[1], n_pp);
+        atomicAdd(&A.counters[0], tc);
+        atomicAdd(&A.counters[1], tp);
     }
+}
+
+static void launch_walk_kernel(const WalkArgs &w, bool quad, bool compat, cudaStream_t s)
+{
+    const int grid = (w.n + WK_THREADS - 1) / WK_THREADS;
+    if (compat)
+        k_bh_walk<false, true><<<grid, WK_THREADS, 0, s>>>(w);
+    else if (quad)
+        k_bh_walk<true, false><<<grid, WK_THREADS, 0, s>>>(w);
+    else
+        k_bh_walk<false, false><<<grid, WK_THREADS, 0, s>>>(w);
 }
 
 // ------------------------------------------------------------------------
@@ -281,6 +353,7 @@ class BarnesHutEngine final : public Engine {
         w.nc = tree_.w_nc.as<int4>();
         w.nkey = tree_.w_nkey.as<uint64_t>();
         w.ncom = tree_.t_com.as<double>();
+        w.depth = tree_.t_depth.as<int>();
         w.pa = tree_.w_pa.as<float4>();
         w.pb = tree_.w_pb.as<float4>();
         w.sidx = tree_.sidx.as<int>();
@@ -288,7 +361,6 @@ class BarnesHutEngine final : public Engine {
         w.x = d_x;
         w.frame = tree_.frame.as<double>();
         w.n = n_;
-        w.compat = compat_ ? 1 : 0;
         w.eps2 = (float)(eps_ * eps_);
         w.theta2 = theta_ * theta_;
         w.G = G_;
@@ -304,11 +376,7 @@ class BarnesHutEngine final : public Engine {
             return ok();
         }
         if (timer) GS_TRY(timer->begin(s));
-        const int grid = (n_ + WK_THREADS - 1) / WK_THREADS;
-        if (quad_)
-            k_bh_walk<true><<<grid, WK_THREADS, 0, s>>>(w);
-        else
-            k_bh_walk<false><<<grid, WK_THREADS, 0, s>>>(w);
+        launch_walk_kernel(w, quad_, compat_, s);
         GS_CUDA(cudaGetLastError());
         if (timer) GS_TRY(timer->end(s));
         return ok();
@@ -376,6 +444,7 @@ ErrorStatus launch_bh_walk(const OctreeDevice &t, const double *d_x, double thet
     w.nc = t.w_nc.as<int4>();
     w.nkey = t.w_nkey.as<uint64_t>();
     w.ncom = t.t_com.as<double>();
+    w.depth = t.t_depth.as<int>();
     w.pa = t.w_pa.as<float4>();
     w.pb = t.w_pb.as<float4>();
     w.sidx = t.sidx.as<int>();
@@ -383,7 +452,6 @@ ErrorStatus launch_bh_walk(const OctreeDevice &t, const double *d_x, double thet
     w.x = d_x;
     w.frame = t.frame.as<double>();
     w.n = t.n;
-    w.compat = t.compat ? 1 : 0;
     w.eps2 = (float)(eps * eps);
     w.theta2 = theta * theta;
     w.G = G;
@@ -391,11 +459,7 @@ ErrorStatus launch_bh_walk(const OctreeDevice &t, const double *d_x, double thet
     w.counters = counters;
     w.status = reinterpret_cast<unsigned *>(t.ctr.as<int>() + CTR_STATUS);
     w.gate = gate;
-    const int grid = (t.n + WK_THREADS - 1) / WK_THREADS;
-    if (t.quad)
-        k_bh_walk<true><<<grid, WK_THREADS, 0, s>>>(w);
-    else
-        k_bh_walk<false><<<grid, WK_THREADS, 0, s>>>(w);
+    launch_walk_kernel(w, t.quad, t.compat, s);
     GS_CUDA(cudaGetLastError());
     return ok();
 }
