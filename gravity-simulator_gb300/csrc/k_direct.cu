@@ -24,8 +24,8 @@
 //   Measured at N = 100,000: 3.76 -> 3.51 ms (57 TFLOP/s at 20 per pair term, 0.74
 //   of the FP32 FMA peak; the pair term's own ceiling is 20/24 of it).
 //
-// GRAV_GPU_PAIRWISE_FP64 (reference order): a warp per ten particles forms
-// the pair terms of all other particles, 32 at a time, and sums them in index
+// GRAV_GPU_PAIRWISE_FP64 (reference order): a CTA of a few particles forms
+// the pair terms of all other particles, 128 at a time, and sums them in index
 // order with every FP64 product, sum, sqrt and quotient rounded separately --
 // the same operations as the reference's symmetric loop applies to that
 // particle, so the result equals the reference's bit for bit where the
@@ -383,47 +383,72 @@ __global__ void k_reduce_splits(const float2 *__restrict__ partial, int splits, 
     if (i < n) a[3 * (size_t)i + k] = G * reduce_row(partial, splits, n_pad, k, i);
 }
 
-// FP64, reference operation order (see file comment).  One warp per PER
-// particles: for 32 consecutive j the lanes form the pair terms of the PER
-// particles (each term is independent), then lane 3p + c subtracts the
-// component-c terms of particle p from its accumulator one by one in j
-// order, which is the order the reference's loop adds them to a_i.  With
-// PER = 10, ten particles share each in-order accumulation instruction (30
-// of 32 lanes); with PER = 1 there are ten times as many warps, which small
-// systems need to fill the GPU.
-constexpr int RF_WARPS = 4;
-constexpr int RF_PER_WARP_LARGE = 10;
-constexpr int RF_LARGE_N = 32768;   // from here on, ten particles per warp
+// FP64, reference operation order (see file comment).  A CTA of eight warps,
+// two per SM sub-partition, owns P particles.  For 128 consecutive j the warps
+// form the pair terms of the P particles (each term is independent; a warp takes
+// 32 j of one particle at a time); then lane 3p + c of warp 0 subtracts the
+// component-c terms of particle p from its accumulator one by one in j order,
+// which is the order the reference's loop adds them to a_i, while the other warps
+// form the next 128.  (The own term and those past the end are +0, which leave
+// the accumulator as it is.)
+//
+// An FP64 instruction holds its sub-partition for 64 cycles whatever its lanes
+// do, so the time is the instructions of the busiest one: 32 per 32 terms and one
+// per j for the ordered sums of all P particles.  With a warp per particle the
+// ordered sums, three lanes wide, took as many instructions as the terms; the
+// shares below make the four sub-partitions' counts equal, 32 (P + 1) per round.
+// Leapfrog step: N = 1,024 163 -> 91 us, 4,096 2.13 -> 1.15 ms, 33,000 81 -> 74 ms.
+constexpr int RF_THREADS = 256;             // two warps per sub-partition
+constexpr int RF_CHUNK = 128;              // j per round
+constexpr int RF_ROW = RF_CHUNK + 1;       // stride of a component's terms (bank spread)
+constexpr int RF_MAX_P = 10;               // 30 lanes of ordered sums
 
-template <int RF_PER_WARP>
-__global__ void __launch_bounds__(32 * RF_WARPS)
-k_direct_fp64_reference_order(const double *__restrict__ x, const double *__restrict__ m,
-                              int n, double G, double eps2, double *__restrict__ a)
+__host__ __device__ constexpr size_t rf_smem(int P)
 {
-    __shared__ double terms[RF_WARPS][RF_PER_WARP * 3][32];
-    __shared__ double xi_s[RF_WARPS][RF_PER_WARP * 3];
+    return ((size_t)2 * 3 * P * RF_ROW + 3 * RF_MAX_P) * sizeof(double);
+}
+
+__global__ void __launch_bounds__(RF_THREADS)
+k_direct_fp64_reference_order(const double *__restrict__ x, const double *__restrict__ m,
+                              int n, int P, double G, double eps2, double *__restrict__ a)
+{
+    extern __shared__ __align__(16) double rf_terms[];   // [2][3 P][RF_ROW], then x_i
+    double *xi = rf_terms + 2 * 3 * P * RF_ROW;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int i0 = (blockIdx.x * RF_WARPS + w) * RF_PER_WARP;
-    if (i0 >= n) return;   // warp-uniform
-    const int np = min(RF_PER_WARP, n - i0);
-    if (lane < 3 * np) xi_s[w][lane] = x[3 * i0 + lane];
-    __syncwarp();
-    double acc = 0.0;   // lane 3p + c < 3 np: component c of a_(i0 + p)
-    for (int base = 0; base < n; base += 32) {
-        const int j = base + lane;
+    const int i0 = blockIdx.x * P;
+    const int np = min(P, n - i0);
+    if (threadIdx.x < 3 * np) xi[threadIdx.x] = x[3 * (size_t)i0 + threadIdx.x];
+    __syncthreads();
+    // items of a round: (32 j, particle), particles fastest; the sub-partition of
+    // warp 0, which adds, takes np - 3 of the 4 np (warp 4), the others np + 1 each
+    const int own = max(0, np - 3);
+    const int per = (4 * np - own + 2) / 3;
+    const int sub = w & 3;
+    int e0 = sub == 0 ? 0 : min(4 * np, own + (sub - 1) * per);
+    int e1 = sub == 0 ? own : min(4 * np, e0 + per);
+    const int half = sub == 0 ? e0 : e0 + (e1 - e0 + 1) / 2;
+    (w < 4 ? e1 : e0) = half;
+    auto produce = [&](int chunk) {
+        double *buf = rf_terms + (chunk & 1) * 3 * P * RF_ROW;
+        int quarter = -1, j = 0;
         double xj0 = 0.0, xj1 = 0.0, xj2 = 0.0, mj = 0.0;
-        if (j < n) {
-            xj0 = x[3 * j + 0];
-            xj1 = x[3 * j + 1];
-            xj2 = x[3 * j + 2];
-            mj = m[j];
-        }
-        for (int p = 0; p < np; ++p) {
+        for (int e = e0; e < e1; ++e) {
+            const int q = e / np, p = e - q * np;
+            if (q != quarter) {
+                quarter = q;
+                j = chunk * RF_CHUNK + q * 32 + lane;
+                if (j < n) {
+                    xj0 = x[3 * (size_t)j + 0];
+                    xj1 = x[3 * (size_t)j + 1];
+                    xj2 = x[3 * (size_t)j + 2];
+                    mj = m[j];
+                }
+            }
             double t0 = 0.0, t1 = 0.0, t2 = 0.0;
             if (j < n && j != i0 + p) {
-                const double r0 = __dsub_rn(xi_s[w][3 * p + 0], xj0);
-                const double r1 = __dsub_rn(xi_s[w][3 * p + 1], xj1);
-                const double r2 = __dsub_rn(xi_s[w][3 * p + 2], xj2);
+                const double r0 = __dsub_rn(xi[3 * p + 0], xj0);
+                const double r1 = __dsub_rn(xi[3 * p + 1], xj1);
+                const double r2 = __dsub_rn(xi[3 * p + 2], xj2);
                 const double s = __dadd_rn(
                     __dadd_rn(__dadd_rn(__dmul_rn(r0, r0), __dmul_rn(r1, r1)), __dmul_rn(r2, r2)),
                     eps2);
@@ -433,21 +458,28 @@ k_direct_fp64_reference_order(const double *__restrict__ x, const double *__rest
                 t1 = __dmul_rn(__dmul_rn(t, r1), mj);
                 t2 = __dmul_rn(__dmul_rn(t, r2), mj);
             }
-            terms[w][3 * p + 0][lane] = t0;
-            terms[w][3 * p + 1][lane] = t1;
-            terms[w][3 * p + 2][lane] = t2;
+            double *out = buf + 3 * p * RF_ROW + q * 32 + lane;
+            out[0] = t0;
+            out[RF_ROW] = t1;
+            out[2 * RF_ROW] = t2;
+        }
+    };
+    const int chunks = (n + RF_CHUNK - 1) / RF_CHUNK;
+    double acc = 0.0;   // lane 3p + c < 3 np of warp 0: component c of a_(i0 + p)
+    produce(0);
+    __syncthreads();
+    for (int c = 0; c < chunks; ++c) {
+        if (w == 0 && lane < 3 * np) {
+            const double *tc = rf_terms + ((c & 1) * 3 * P + lane) * RF_ROW;
+            const int cnt = min(RF_CHUNK, n - c * RF_CHUNK);
+#pragma unroll 16
+            for (int q = 0; q < cnt; ++q) acc = __dsub_rn(acc, tc[q]);
         }
         __syncwarp();
-        if (lane < 3 * np) {
-            const int cnt = min(32, n - base);
-            const int self = i0 + lane / 3 - base;   // this particle's own slot, if in the chunk
-            const double *tc = terms[w][lane];
-            for (int q = 0; q < cnt; ++q)
-                if (q != self) acc = __dsub_rn(acc, tc[q]);
-        }
-        __syncwarp();
+        if (c + 1 < chunks) produce(c + 1);
+        __syncthreads();
     }
-    if (lane < 3 * np) a[3 * i0 + lane] = acc;
+    if (w == 0 && lane < 3 * np) a[3 * (size_t)i0 + lane] = acc;
 }
 
 // ------------------------------------------------------------------------
@@ -518,9 +550,29 @@ class DirectEngine final : public Engine {
         n_ = n;
         G_ = G;
         eps_ = p.softening_length;
-        if (fp64_) return ok();
         const DeviceInfo *dev = nullptr;
         GS_TRY(device_info(&dev));
+        if (fp64_) {
+            // particles per CTA: the fewest instructions of the busiest SM.  Per round
+            // of 128 j and CTA, in units of 32: P + 1 (four at least, the ordered sums
+            // alone), and once the first round's terms, on three warps.
+            const long rounds = (n + RF_CHUNK - 1) / RF_CHUNK;
+            long best = 0;
+            for (int P = 1; P <= RF_MAX_P; ++P) {
+                const long ctas = (n + P - 1) / P;
+                const long first = (4 * P - std::max(0, P - 3) + 2) / 3;
+                const long cost = (ctas + dev->sm_count - 1) / dev->sm_count *
+                                  (rounds * std::max(4, P + 1) + first);
+                if (best == 0 || cost <= best) {
+                    best = cost;
+                    p_ = P;
+                }
+            }
+            GS_CUDA(cudaFuncSetAttribute(k_direct_fp64_reference_order,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)rf_smem(RF_MAX_P)));
+            return ok();
+        }
         n_pad_ = ((n + DS_ITILE - 1) / DS_ITILE) * DS_ITILE;
         granules_ = (n + DS_GRANULE - 1) / DS_GRANULE;
         if (n <= DS_RUN_N) {
@@ -553,14 +605,9 @@ class DirectEngine final : public Engine {
                         ForceTimer *timer) override
     {
         if (fp64_) {
-            const bool large = n_ >= RF_LARGE_N;
-            const int per_cta = RF_WARPS * (large ? RF_PER_WARP_LARGE : 1);
-            const int grid = (n_ + per_cta - 1) / per_cta;
             if (timer) GS_TRY(timer->begin(s));
-            auto kernel = large ? k_direct_fp64_reference_order<RF_PER_WARP_LARGE>
-                                : k_direct_fp64_reference_order<1>;
-            kernel<<<grid, 32 * RF_WARPS, 0, s>>>(d_x, d_m, n_, G_, eps_ * eps_,
-                                                                      d_a);
+            k_direct_fp64_reference_order<<<(n_ + p_ - 1) / p_, RF_THREADS, rf_smem(p_), s>>>(
+                d_x, d_m, n_, p_, G_, eps_ * eps_, d_a);
             GS_CUDA(cudaGetLastError());
             if (timer) GS_TRY(timer->end(s));
             return ok();
@@ -605,6 +652,7 @@ class DirectEngine final : public Engine {
 
   private:
     bool fp64_;
+    int p_ = 1;   // particles per CTA of the FP64 kernel
     int n_ = 0, n_pad_ = 0, i_tiles_ = 0, granules_ = 1, per_ = 1, splits_ = 1;
     double G_ = 1.0, eps_ = 0.0;
     double c_[3] = {0.0, 0.0, 0.0};

@@ -116,6 +116,15 @@ def test_cpu_method_code_rejected(lib, g, wl):
     assert e.value.code == g.GRAV_VALUE_ERROR
 
 
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 127, 128, 129, 456, 457, 700, 1064, 1065, 1500, 4097])
+def test_fp64_reference_order_bitexact_sizes(lib, g, orc, wl, n):
+    """Counts next to the 128-term rounds, and counts whose blocks own 1 to 10 particles, the
+    last of them fewer."""
+    x, v, m = wl.plummer(n, 40 + n)
+    a = g.acceleration(lib, x, m, 1.0, g.METHOD_GPU_PAIRWISE_FP64, 1.0, 0.01, -1)
+    assert a.tobytes() == orc.pairwise(x, m, 1.0, 0.01).tobytes()
+
+
 def test_fp64_reference_order_bitexact_large(lib, g, orc, wl):
     """Above 32,768 particles the FP64 reference-order sum runs ten particles
     per warp; still the reference's operations in the reference's order."""
