@@ -107,6 +107,14 @@ class Engine {
     virtual ErrorStatus setup(int n, double G, const AccelerationParam &p) = 0;
     virtual ErrorStatus compute(const double *d_x, const double *d_m, double *d_a,
                                 cudaStream_t s, ForceTimer *timer) = 0;
+    // The masses of the following compute() calls, on the device: called before
+    // the first of them, and again whenever the masses change.
+    virtual ErrorStatus set_masses(const double *d_m, cudaStream_t s)
+    {
+        (void)d_m;
+        (void)s;
+        return ok();
+    }
     // kernels launched by one compute()
     virtual int kernels_per_eval() const = 0;
     // true when compute() never synchronises with the host (graph-capturable)

@@ -128,6 +128,7 @@ ErrorStatus accel_host(double *a, const System *system, const AccelerationParam 
                             cudaMemcpyHostToDevice, c->stream));
     GS_CUDA(cudaMemcpyAsync(c->m.p, system->m, (size_t)n * sizeof(double), cudaMemcpyHostToDevice,
                             c->stream));
+    GS_TRY(c->engine->set_masses(c->m.as<double>(), c->stream));
     GS_TRY(c->engine->compute(c->x.as<double>(), c->m.as<double>(), c->a.as<double>(), c->stream,
                               nullptr));
     GS_CUDA(cudaMemcpyAsync(a, c->a.p, (size_t)n * 3 * sizeof(double), cudaMemcpyDeviceToHost,
@@ -817,6 +818,7 @@ ErrorStatus sim_upload(gsgpu_sim *s, const double *x, const double *v, const dou
     GS_CUDA(cudaMemcpyAsync(s->v.p, v, s->bytes3(), cudaMemcpyHostToDevice, s->stream));
     GS_CUDA(cudaMemcpyAsync(s->m.p, m, (size_t)s->n * sizeof(double), cudaMemcpyHostToDevice,
                             s->stream));
+    GS_TRY(s->engine->set_masses(s->m.as<double>(), s->stream));
     GS_CUDA(cudaMemsetAsync(s->xe.p, 0, s->bytes3(), s->stream));
     GS_CUDA(cudaMemsetAsync(s->ve.p, 0, s->bytes3(), s->stream));
     GS_CUDA(cudaMemsetAsync(s->a.p, 0, s->bytes3(), s->stream));
