@@ -18,7 +18,6 @@ from __future__ import annotations
 import ctypes
 import os
 import threading
-import time
 from pathlib import Path
 from queue import Queue
 from typing import Optional
@@ -443,9 +442,8 @@ def launch_simulation(lib: ctypes.CDLL, x: np.ndarray, v: np.ndarray,
     )
     th = threading.Thread(target=run, args=args)
     th.start()
-    while th.is_alive():
-        time.sleep(0.002)
-    th.join()
+    while th.is_alive():   # returns as soon as the run ends; interruptible in between
+        th.join(0.05)
     ret = q.get()
     if ret != 0:
         raise RuntimeError("Simulation failed. Please check the C library traceback.")
