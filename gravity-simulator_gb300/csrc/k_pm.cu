@@ -2,23 +2,31 @@
 // cosmological leapfrog (src/integrator_cosmology_leapfrog.c:24-255).
 //
 // One evaluation on a g^3 periodic mesh:
-//   k_pm_deposit   cloud-in-cell mass deposit, one thread per particle,
-//                  eight FP64 atomic adds (the reference's OpenMP loop has
-//                  unsynchronised += here);
-//   k_pm_contrast  delta = rho / (V_cell rho_mean) - 1;
+//   k_pm_fill      the mesh at -1;
+//   deposit        cloud-in-cell deposit of m / (V_cell rho_mean), eight FP64
+//                  atomic adds per particle (the reference's OpenMP loop has
+//                  unsynchronised += here), which makes the mesh the density
+//                  contrast rho / (V_cell rho_mean) - 1;
 //   cuFFT D2Z      the r2c transform (FFTW's layout: g x g x (g/2+1));
-//   k_pm_green     multiply by -1/k^2 (0 at k = 0);
+//   k_pm_green     multiply by -1/k^2 (0 at k = 0), from a table by the integer
+//                  |n|^2;
 //   cuFFT Z2D      the unnormalised c2r transform;
-//   k_pm_gradient  fourth-order central differences of phi * factor into the
-//                  acceleration mesh (the reference scales phi in place
-//                  first; the product is formed on load here, same bits);
-//   k_pm_interp    cloud-in-cell interpolation back to the particles.
+//   k_pm_gradient  fourth-order central differences of phi into the
+//                  acceleration mesh, without their constant factor;
+//   interpolation  cloud-in-cell, back to the particles; the caller's multiplier
+//                  carries the factor.
+// A step of the cosmological leapfrog is one particle kernel between two
+// evaluations (k_pm_particles): interpolation, the kick that ends a step, the kick
+// and the drift that begin the next, the periodic wrap, and the deposit at the
+// new positions.  As five kernels these took 463 us a step at 128^3 particles, with
+// the accelerations and momenta written and read in between; fused, 409 us.
 // Every kernel computes the reference's quantity in FP64.  The FP64 pipe of
 // this GPU runs at 1/64 of the FP32 rate and bounds the particle kernels, so
 // they use algebraically equal forms with fewer FP64 operations than the
 // reference's expressions: weight products shared between the eight
-// corners, fused multiply-adds, the constant divisions of the kicks, the
-// drift and the gradient folded into one multiplier each.  These round
+// corners, fused multiply-adds, the cell index by a directed addition of 2^52,
+// constant factors folded into one multiplier, comparisons on the bits (an FP64
+// comparison costs as much as an add).  These round
 // differently from the reference's order by a few ulps, far below the
 // differences of the transforms (cuFFT against FFTW) and of the atomic
 // deposit order.  The file is compiled with --fmad=false; the fused
@@ -26,6 +34,7 @@
 //
 // Memory: delta / phi g^3 doubles, the spectrum g^2 (g/2+1) complex, the
 // acceleration mesh 3 g^3 doubles: 56 g^3 bytes, 940 MB at g = 256.
+#include "gs_fp64.cuh"
 #include "gs_internal.h"
 
 #include <cufft.h>
@@ -68,6 +77,7 @@ struct PmGeom {
     double cx, cy, cz;   // box centre
     double half;         // box_length / 2
     double inv_cell;     // 1 / (box_length / g)
+    double shift[3];     // half - centre
     int g;
 };
 
@@ -79,20 +89,32 @@ __device__ __forceinline__ int wrap_index(int n, int g)
     return r < 0 ? r + g : r;
 }
 
-// Cell indices and weights of one particle (src/acceleration_PM.c:44-58).
-__device__ __forceinline__ void cic_cell(const double *xi, const PmGeom &G, int idx[2][3],
+// Cell indices and weights of one particle (src/acceleration_PM.c:44-58).  Inside
+// the box the cell is the integer part of u = (x - c + half) / cell, taken by
+// adding 2^52 rounded down: six FP64 operations a dimension.
+__device__ __forceinline__ void cic_cell(const double xi[3], const PmGeom &G, int idx[2][3],
                                          double w[2][3])
 {
     const double c[3] = {G.cx, G.cy, G.cz};
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        const double normalized = (xi[d] - c[d] + G.half) * G.inv_cell;
-        const int nd = (int)normalized;
-        const double weight = normalized - nd;
-        w[1][d] = weight;
-        w[0][d] = 1.0 - weight;
-        idx[0][d] = wrap_index(nd, G.g);
-        idx[1][d] = wrap_index(nd + 1, G.g);
+        const double u = (xi[d] + G.shift[d]) * G.inv_cell;
+        if ((unsigned)__double2hiint(u) < 0x41d00000u) {   // 0 <= u < 2^30
+            const double t = __dadd_rd(u, 0x1p52);
+            const int nd = __double2loint(t);
+            w[1][d] = u - (t - 0x1p52);
+            w[0][d] = 1.0 - w[1][d];
+            idx[0][d] = nd < G.g ? nd : nd % G.g;
+            idx[1][d] = idx[0][d] + 1 < G.g ? idx[0][d] + 1 : 0;
+        } else {
+            const double normalized = (xi[d] - c[d] + G.half) * G.inv_cell;
+            const int nd = (int)normalized;
+            const double weight = normalized - nd;
+            w[1][d] = weight;
+            w[0][d] = 1.0 - weight;
+            idx[0][d] = wrap_index(nd, G.g);
+            idx[1][d] = wrap_index(nd + 1, G.g);
+        }
     }
 }
 
@@ -103,16 +125,13 @@ __host__ __device__ constexpr int corner_bits(int c)
     return c == 3 ? 4 : (c == 4 ? 3 : c);
 }
 
-__global__ void k_pm_deposit(const double *__restrict__ x, const double *__restrict__ m, int n,
-                             PmGeom G, double *__restrict__ delta)
+__device__ __forceinline__ void deposit_one(const double xi[3], double mi, const PmGeom &G,
+                                            double *__restrict__ delta)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
     int idx[2][3];
     double w[2][3];
-    cic_cell(x + 3 * (size_t)i, G, idx, w);
+    cic_cell(xi, G, idx, w);
     const long long g = G.g, g2 = g * g;
-    const double mi = m[i];
     double mx[2], mxy[2][2];
 #pragma unroll
     for (int bx = 0; bx < 2; ++bx) {
@@ -129,76 +148,20 @@ __global__ void k_pm_deposit(const double *__restrict__ x, const double *__restr
     }
 }
 
-// delta = rho / (V_cell rho_mean) - 1 with inv = 1 / (V_cell rho_mean)
-__global__ void k_pm_contrast(double *__restrict__ delta, long long cells, double inv)
+// src/acceleration_PM.c:112-210, in units of the gradient mesh
+__device__ __forceinline__ void interp_one(const double xi[3], const PmGeom &G,
+                                           const double *__restrict__ acc, double s[3])
 {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= cells) return;
-    delta[i] = fma(delta[i], inv, -1.0);
-}
-
-// src/acceleration_PM.c:321-345
-__global__ void k_pm_green(double2 *__restrict__ spec, int g, double two_pi_over_l2)
-{
-    const int h = g / 2 + 1;
-    const long long total = (long long)g * g * h;
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= total) return;
-    const int k = (int)(e % h);
-    const long long ij = e / h;
-    const int j = (int)(ij % g), i = (int)(ij / g);
-    const int kx = (i < h) ? i : i - g;
-    const int ky = (j < h) ? j : j - g;
-    const int kz = k;
-    const double k_sq = (double)(kx * kx + ky * ky + kz * kz) * two_pi_over_l2;
-    const double kernel = k_sq == 0.0 ? 0.0 : -1.0 / k_sq;
-    double2 v = spec[e];
-    v.x *= kernel;
-    v.y *= kernel;
-    spec[e] = v;
-}
-
-// src/acceleration_PM.c:212-272: (phi[-2] - 8 phi[-1] + 8 phi[+1] - phi[+2])
-// * factor / (12 cell_length), as ((phi[-2] - phi[+2]) + 8 (phi[+1] - phi[-1]))
-// * scale with scale = factor / (12 cell_length).
-__global__ void k_pm_gradient(const double *__restrict__ phi, int g, double scale,
-                              double *__restrict__ acc)
-{
-    const long long g2 = (long long)g * g, cells = g2 * g;
-    const long long index = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (index >= cells) return;
-    const int k = (int)(index % g);
-    const int j = (int)((index / g) % g);
-    const int i = (int)(index / g2);
-    const int c[3] = {i, j, k};
-    const long long st[3] = {g2, g, 1};
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const long long b = index - c[d] * st[d];
-        const double pm2 = phi[b + (long long)((c[d] - 2 + g) % g) * st[d]];
-        const double pm1 = phi[b + (long long)((c[d] - 1 + g) % g) * st[d]];
-        const double pp1 = phi[b + (long long)((c[d] + 1) % g) * st[d]];
-        const double pp2 = phi[b + (long long)((c[d] + 2) % g) * st[d]];
-        acc[index * 3 + d] = fma(8.0, pp1 - pm1, pm2 - pp2) * scale;
-    }
-}
-
-// src/acceleration_PM.c:112-210
-__global__ void k_pm_interp(const double *__restrict__ x, int n, PmGeom G,
-                            const double *__restrict__ acc, double *__restrict__ a)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
     int idx[2][3];
     double w[2][3];
-    cic_cell(x + 3 * (size_t)i, G, idx, w);
+    cic_cell(xi, G, idx, w);
     const long long g = G.g, g2 = g * g;
     double wxy[2][2];
 #pragma unroll
     for (int bx = 0; bx < 2; ++bx)
 #pragma unroll
         for (int by = 0; by < 2; ++by) wxy[bx][by] = w[bx][0] * w[by][1];
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+    s[0] = s[1] = s[2] = 0.0;
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
         const int bx = corner_bits(c) & 1, by = (corner_bits(c) >> 1) & 1,
@@ -206,13 +169,145 @@ __global__ void k_pm_interp(const double *__restrict__ x, int n, PmGeom G,
         const long long cell = idx[bx][0] * g2 + idx[by][1] * g + idx[bz][2];
         const double wc = wxy[bx][by] * w[bz][2];
         const double *ac = acc + cell * 3;
-        s0 = fma(ac[0], wc, s0);
-        s1 = fma(ac[1], wc, s1);
-        s2 = fma(ac[2], wc, s2);
+        s[0] = fma(ac[0], wc, s[0]);
+        s[1] = fma(ac[1], wc, s[1]);
+        s[2] = fma(ac[2], wc, s[2]);
     }
-    a[3 * (size_t)i + 0] = s0;
-    a[3 * (size_t)i + 1] = s1;
-    a[3 * (size_t)i + 2] = s2;
+}
+
+__global__ void k_pm_fill(double *__restrict__ mesh, long long cells, double value)
+{
+    const long long i = 2 * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
+    if (i + 1 < cells)
+        *reinterpret_cast<double2 *>(mesh + i) = make_double2(value, value);
+    else if (i < cells)
+        mesh[i] = value;
+}
+
+__global__ void k_pm_deposit(const double *__restrict__ x, const double *__restrict__ mn, int n,
+                             PmGeom G, double *__restrict__ delta)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double xi[3] = {x[3 * (size_t)i], x[3 * (size_t)i + 1], x[3 * (size_t)i + 2]};
+    deposit_one(xi, mn[i], G, delta);
+}
+
+// -1 / (|n|^2 (2 pi / L)^2) by the integer |n|^2 of a mode (src/acceleration_PM.c:
+// 321-345), 0 for the mean; the division is made once per value instead of once
+// per mode (25 us a transform at 128^3).
+__global__ void k_pm_green_table(double *__restrict__ table, int len, double two_pi_over_l2)
+{
+    const int k2 = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k2 < len) table[k2] = k2 == 0 ? 0.0 : -1.0 / ((double)k2 * two_pi_over_l2);
+}
+
+__global__ void k_pm_green(double2 *__restrict__ spec, int g, const double *__restrict__ table)
+{
+    // fewer than 2^31 modes: 32-bit index arithmetic
+    const unsigned h = g / 2 + 1, ug = g;
+    const unsigned e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= ug * ug * h) return;
+    const unsigned ij = e / h;
+    const int k = (int)(e - ij * h);
+    const int i = (int)(ij / ug), j = (int)(ij - (unsigned)i * ug);
+    const int kx = (i < (int)h) ? i : i - g;
+    const int ky = (j < (int)h) ? j : j - g;
+    const double kernel = __ldg(table + kx * kx + ky * ky + k * k);
+    double2 v = spec[e];
+    v.x *= kernel;
+    v.y *= kernel;
+    spec[e] = v;
+}
+
+// src/acceleration_PM.c:212-272 without the constant factor / (12 cell_length):
+// phi[-2] - 8 phi[-1] + 8 phi[+1] - phi[+2] as (phi[-2] - phi[+2]) +
+// 8 (phi[+1] - phi[-1]).
+__global__ void k_pm_gradient(const double *__restrict__ phi, int g, double *__restrict__ acc)
+{
+    // at most 2^31 cells: 32-bit index arithmetic
+    const unsigned ug = g, g2 = ug * ug;
+    const unsigned index = blockIdx.x * blockDim.x + threadIdx.x;
+    if (index >= g2 * ug) return;
+    const unsigned ij = index / ug;
+    const int k = (int)(index - ij * ug), i = (int)(ij / ug), j = (int)(ij - (unsigned)i * ug);
+    const int c[3] = {i, j, k};
+    const unsigned st[3] = {g2, ug, 1u};
+    // c + o on the periodic axis, o in [-2, 2] (twice for g = 1)
+    auto at = [&](int cd, int o) {
+        int q = cd + o;
+        q += q < 0 ? g : 0;
+        q += q < 0 ? g : 0;
+        q -= q >= g ? g : 0;
+        q -= q >= g ? g : 0;
+        return (unsigned)q;
+    };
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const unsigned b = index - (unsigned)c[d] * st[d];
+        const double pm2 = phi[b + at(c[d], -2) * st[d]], pm1 = phi[b + at(c[d], -1) * st[d]];
+        const double pp1 = phi[b + at(c[d], 1) * st[d]], pp2 = phi[b + at(c[d], 2) * st[d]];
+        acc[3 * (size_t)index + d] = fma(8.0, pp1 - pm1, pm2 - pp2);
+    }
+}
+
+__global__ void k_pm_interp(const double *__restrict__ x, int n, PmGeom G,
+                            const double *__restrict__ acc, double scale, double *__restrict__ a)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double xi[3] = {x[3 * (size_t)i], x[3 * (size_t)i + 1], x[3 * (size_t)i + 2]};
+    double s[3];
+    interp_one(xi, G, acc, s);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) a[3 * (size_t)i + d] = s[d] * scale;
+}
+
+// Total mass, by a fixed tree (the host's one-by-one sum of 2 million masses took
+// 2 ms of a run), then 1 / (V_cell rho_mean) into *inv, rho_mean = mass / volume
+// (src/integrator_cosmology_leapfrog.c:66-70).
+constexpr int MS_BLOCKS = 256, MS_THREADS = 256;
+__device__ __forceinline__ double block_sum(double v, double *sh)
+{
+    sh[threadIdx.x] = v;
+    __syncthreads();
+    for (int w = MS_THREADS / 2; w > 0; w >>= 1) {
+        if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
+        __syncthreads();
+    }
+    return sh[0];
+}
+
+__global__ void __launch_bounds__(MS_THREADS)
+k_pm_mass_parts(const double *__restrict__ m, int n, double *__restrict__ part)
+{
+    __shared__ double sh[MS_THREADS];
+    double v = 0.0;
+    for (long long i = (long long)blockIdx.x * MS_THREADS + threadIdx.x; i < n;
+         i += (long long)MS_BLOCKS * MS_THREADS)
+        v += m[i];
+    v = block_sum(v, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = v;
+}
+
+// *inv = 1 / (V_cell rho_mean) from the mass parts
+__global__ void __launch_bounds__(MS_THREADS)
+k_pm_mass_inv(const double *__restrict__ part, double volume, double cell_volume,
+              double *__restrict__ inv)
+{
+    static_assert(MS_BLOCKS == MS_THREADS, "a part per thread");
+    __shared__ double sh[MS_THREADS];
+    const double total = block_sum(part[threadIdx.x], sh);
+    if (threadIdx.x == 0) *inv = 1.0 / (cell_volume * (total / volume));
+}
+
+// mn = m * inv, inv given or read from *d_inv
+__global__ void k_pm_mass_scale(const double *__restrict__ m, int n,
+                                const double *__restrict__ d_inv, double inv,
+                                double *__restrict__ mn)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) mn[i] = m[i] * (d_inv ? *d_inv : inv);
 }
 
 // ---- cosmological leapfrog (src/integrator_cosmology_leapfrog.c) -----------
@@ -220,6 +315,8 @@ __global__ void k_pm_interp(const double *__restrict__ x, int n, PmGeom G,
 __device__ __forceinline__ double periodic(double xv, double c, double bw)
 {
     const double p = xv - c;
+    // inside, tested on the bits (NaN goes on and fails both comparisons)
+    if (abs_bits(p) <= __double_as_longlong(bw)) return xv;
     if (p < -bw) {
         xv = ((int)(p / bw) % 2 != 0) ? fmod(p, bw) + bw : fmod(p, bw);
         xv += c;
@@ -257,24 +354,43 @@ __global__ void k_cosmo_velocity(double *__restrict__ v, const double *__restric
     v[k] = p[k] / (t * t);
 }
 
-// momentum -= (0.5 dt) a / da (:142-149, :176-183); c = 0.5 dt / da
-__global__ void k_cosmo_kick(double *__restrict__ p, const double *__restrict__ a, int len,
-                             double c)
+// The particles between two evaluations: accelerations interpolated from the
+// gradient mesh (GATHER) or read from `a`, the kick that ends a step,
+// p -= k1 a (:176-183), and with MOVE the kick and the drift that begin the next,
+// p -= k2 a (:142-149), x += c p (:152-160), wrapped (:163), and its deposit.
+// k1 and k2 carry 0.5 dt / da and the acceleration's constant factor,
+// c = dt / (a^2 da).  Without MOVE the accelerations are kept in `a`.
+template <bool GATHER, bool MOVE>
+__global__ void k_pm_particles(double *__restrict__ x, double *__restrict__ p,
+                               const double *__restrict__ mn, double *__restrict__ a, int n,
+                               PmGeom G, const double *__restrict__ acc, double k1, double k2,
+                               double c, double bw, double *__restrict__ delta)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= len) return;
-    p[k] = fma(-c, a[k], p[k]);
-}
-
-// x += dt p / (a^2 da) (:152-160), then the periodic wrap (:163); c = dt / (a^2 da)
-__global__ void k_cosmo_drift(double *__restrict__ x, const double *__restrict__ p, int len,
-                              double c, double cx, double cy, double cz, double bw)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= len) return;
-    const int d = k % 3;
-    const double xv = fma(c, p[k], x[k]);
-    x[k] = periodic(xv, d == 0 ? cx : (d == 1 ? cy : cz), bw);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const size_t q = 3 * (size_t)i;
+    double xi[3] = {x[q], x[q + 1], x[q + 2]};
+    double s[3];
+    if (GATHER) {
+        interp_one(xi, G, acc, s);
+    } else {
+        for (int d = 0; d < 3; ++d) s[d] = a[q + d];
+    }
+    const double centre[3] = {G.cx, G.cy, G.cz};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        double pd = p[q + d];
+        if (GATHER) pd = fma(-k1, s[d], pd);
+        if (MOVE) {
+            pd = fma(-k2, s[d], pd);
+            xi[d] = periodic(fma(c, pd, xi[d]), centre[d], bw);
+            x[q + d] = xi[d];
+        } else {
+            a[q + d] = s[d];
+        }
+        p[q + d] = pd;
+    }
+    if (MOVE) deposit_one(xi, mn[i], G, delta);
 }
 
 }  // namespace
@@ -306,49 +422,94 @@ class PmSolver {
         return ok();
     }
 
-    // src/acceleration_PM.c:274-391 on device arrays.
-    ErrorStatus compute(double *d_a, int n, const double *d_x, const double *d_m,
-                        const double *box_center, double box_width, double H0, double omega_m,
-                        double mean_bkg_density, int g, double scale_factor, cudaStream_t s)
+    // A run's constants: geometry and the Green's function table.
+    ErrorStatus prepare(const double *box_center, double box_width, int g, cudaStream_t s)
     {
         GS_TRY(setup(g));
         const double box_length = box_width * 2.0;
-        const long long cells = (long long)g * g * g;
-        PmGeom G;
-        G.cx = box_center[0];
-        G.cy = box_center[1];
-        G.cz = box_center[2];
-        G.half = box_length / 2.0;
-        const double cell_length = box_length / g;
-        G.inv_cell = 1.0 / cell_length;
-        G.g = g;
-        double *mesh = mesh_.as<double>();
-        GS_CUDA(cudaMemsetAsync(mesh, 0, (size_t)cells * sizeof(double), s));
-        k_pm_deposit<<<blocks(n), TPB, 0, s>>>(d_x, d_m, n, G, mesh);
-        const double cell_volume = cell_length * cell_length * cell_length;
-        k_pm_contrast<<<blocks(cells), TPB, 0, s>>>(mesh, cells,
-                                                    1.0 / (cell_volume * mean_bkg_density));
-        GS_CUDA(cudaGetLastError());
-        GS_CUFFT(cufftSetStream(fwd_, s));
-        GS_CUFFT(cufftExecD2Z(fwd_, mesh, spec_.as<cufftDoubleComplex>()));
-        const double two_pi_over_l2 = 4.0 * M_PI * M_PI / (box_length * box_length);
-        const long long half = (long long)g * g * (g / 2 + 1);
-        k_pm_green<<<blocks(half), TPB, 0, s>>>(spec_.as<double2>(), g, two_pi_over_l2);
-        GS_CUDA(cudaGetLastError());
-        GS_CUFFT(cufftSetStream(inv_, s));
-        GS_CUFFT(cufftExecZ2D(inv_, spec_.as<cufftDoubleComplex>(), mesh));
-        const double factor = ((3.0 / 2.0) * omega_m * H0 * H0) / (scale_factor * (double)cells);
-        k_pm_gradient<<<blocks(cells), TPB, 0, s>>>(mesh, g, factor / (12.0 * cell_length),
-                                                    acc_.as<double>());
-        k_pm_interp<<<blocks(n), TPB, 0, s>>>(d_x, n, G, acc_.as<double>(), d_a);
+        cell_length_ = box_length / g;
+        geom_.cx = box_center[0];
+        geom_.cy = box_center[1];
+        geom_.cz = box_center[2];
+        geom_.half = box_length / 2.0;
+        geom_.inv_cell = 1.0 / cell_length_;
+        for (int d = 0; d < 3; ++d) geom_.shift[d] = geom_.half - box_center[d];
+        geom_.g = g;
+        const int top = g / 2;
+        const int len = 3 * top * top + 1;
+        GS_TRY(green_.reserve((size_t)len * sizeof(double)));
+        k_pm_green_table<<<blocks(len), TPB, 0, s>>>(green_.as<double>(), len,
+                                                     4.0 * M_PI * M_PI / (box_length * box_length));
         GS_CUDA(cudaGetLastError());
         return ok();
     }
 
+    // Masses as the deposit takes them: m / (V_cell rho_mean), with rho_mean given
+    // or the total mass over the box's volume.
+    ErrorStatus scale_masses(const double *d_m, int n, double box_width, bool given, double rho_mean,
+                             cudaStream_t s)
+    {
+        GS_TRY(mn_.reserve((size_t)n * sizeof(double)));
+        const double cell_volume = cell_length_ * cell_length_ * cell_length_;
+        double *inv = nullptr;
+        if (!given) {
+            GS_TRY(part_.reserve((MS_BLOCKS + 1) * sizeof(double)));
+            inv = part_.as<double>() + MS_BLOCKS;
+            k_pm_mass_parts<<<MS_BLOCKS, MS_THREADS, 0, s>>>(d_m, n, part_.as<double>());
+            k_pm_mass_inv<<<1, MS_THREADS, 0, s>>>(
+                part_.as<double>(), (box_width * 2) * (box_width * 2) * (box_width * 2), cell_volume,
+                inv);
+        }
+        k_pm_mass_scale<<<blocks(n), TPB, 0, s>>>(d_m, n, inv, given ? 1.0 / (cell_volume * rho_mean)
+                                                                     : 0.0, mn_.as<double>());
+        GS_CUDA(cudaGetLastError());
+        return ok();
+    }
+
+    // The mesh ready for a deposit.
+    ErrorStatus clear(cudaStream_t s)
+    {
+        const long long cells = (long long)g_ * g_ * g_;
+        k_pm_fill<<<blocks((cells + 1) / 2), TPB, 0, s>>>(mesh_.as<double>(), cells, -1.0);
+        GS_CUDA(cudaGetLastError());
+        return ok();
+    }
+
+    // src/acceleration_PM.c:311-380 from the deposited mesh to the gradient mesh.
+    ErrorStatus solve(cudaStream_t s)
+    {
+        double *mesh = mesh_.as<double>();
+        GS_CUFFT(cufftSetStream(fwd_, s));
+        GS_CUFFT(cufftExecD2Z(fwd_, mesh, spec_.as<cufftDoubleComplex>()));
+        const long long half = (long long)g_ * g_ * (g_ / 2 + 1);
+        k_pm_green<<<blocks(half), TPB, 0, s>>>(spec_.as<double2>(), g_, green_.as<double>());
+        GS_CUDA(cudaGetLastError());
+        GS_CUFFT(cufftSetStream(inv_, s));
+        GS_CUFFT(cufftExecZ2D(inv_, spec_.as<cufftDoubleComplex>(), mesh));
+        const long long cells = (long long)g_ * g_ * g_;
+        k_pm_gradient<<<blocks(cells), TPB, 0, s>>>(mesh, g_, acc_.as<double>());
+        GS_CUDA(cudaGetLastError());
+        return ok();
+    }
+
+    // The gradient mesh's constant factor.
+    double scale(double H0, double omega_m, double scale_factor) const
+    {
+        const double cells = (double)((long long)g_ * g_ * g_);
+        return ((3.0 / 2.0) * omega_m * H0 * H0) / (scale_factor * cells) / (12.0 * cell_length_);
+    }
+
+    const PmGeom &geom() const { return geom_; }
+    double *mesh() const { return mesh_.as<double>(); }
+    const double *acc() const { return acc_.as<double>(); }
+    const double *masses() const { return mn_.as<double>(); }
+
   private:
     int g_ = 0;
+    double cell_length_ = 1.0;
+    PmGeom geom_{};
     cufftHandle fwd_ = 0, inv_ = 0;
-    DBuf mesh_, spec_, acc_;
+    DBuf mesh_, spec_, acc_, green_, mn_, part_;
 };
 
 namespace {
@@ -415,9 +576,18 @@ ErrorStatus pm_acceleration_host(double *a, int n, const double *x, const double
     GS_CUDA(cudaMemcpyAsync(c->x.p, x, b3, cudaMemcpyHostToDevice, c->stream));
     GS_CUDA(cudaMemcpyAsync(c->m.p, m, (size_t)n * sizeof(double), cudaMemcpyHostToDevice,
                             c->stream));
-    GS_TRY(c->solver.compute(c->a.as<double>(), n, c->x.as<double>(), c->m.as<double>(),
-                             box_center, box_width, H0, omega_m, mean_bkg_density, g,
-                             scale_factor, c->stream));
+    PmSolver &pm = c->solver;
+    GS_TRY(pm.prepare(box_center, box_width, g, c->stream));
+    GS_TRY(pm.scale_masses(c->m.as<double>(), n, box_width, true, mean_bkg_density, c->stream));
+    GS_TRY(pm.clear(c->stream));
+    k_pm_deposit<<<blocks(n), TPB, 0, c->stream>>>(c->x.as<double>(), pm.masses(), n, pm.geom(),
+                                                   pm.mesh());
+    GS_CUDA(cudaGetLastError());
+    GS_TRY(pm.solve(c->stream));
+    k_pm_interp<<<blocks(n), TPB, 0, c->stream>>>(c->x.as<double>(), n, pm.geom(), pm.acc(),
+                                                  pm.scale(H0, omega_m, scale_factor),
+                                                  c->a.as<double>());
+    GS_CUDA(cudaGetLastError());
     GS_CUDA(cudaMemcpyAsync(a, c->a.p, b3, cudaMemcpyDeviceToHost, c->stream));
     GS_CUDA(cudaStreamSynchronize(c->stream));
     return ok();
@@ -457,15 +627,17 @@ ErrorStatus pm_leapfrog_cosmology(CosmologicalSystem *system, SimulationStatus *
     const bool is_output = op && op->method != OUTPUT_METHOD_DISABLED;
     double next_output_time = is_output ? op->output_interval : 0.0;
     if (is_output && op->output_initial) GS_TRY(output_snapshot_cosmology(op, system, t));
-    double msum = 0.0;   // vec_sum (src/math_functions.c:13-21), in order
-    for (int i = 0; i < n; ++i) msum += system->m[i];
-    const double mean_bkg_density = msum / ((bw * 2) * (bw * 2) * (bw * 2));
-
+    PmSolver &pm = pc->solver;
+    GS_TRY(pm.prepare(c, bw, g, s));
+    GS_TRY(pm.scale_masses(m.as<double>(), n, bw, false, 0.0, s));
     k_cosmo_wrap<<<blocks(L), TPB, 0, s>>>(x.as<double>(), L, c[0], c[1], c[2], bw);
     k_cosmo_momentum<<<blocks(L), TPB, 0, s>>>(p.as<double>(), v.as<double>(), L, t);
     GS_CUDA(cudaGetLastError());
-    GS_TRY(pc->solver.compute(a.as<double>(), n, x.as<double>(), m.as<double>(), c, bw, H0,
-                              omega_m, mean_bkg_density, g, t, s));
+    GS_TRY(pm.clear(s));
+    k_pm_deposit<<<blocks(n), TPB, 0, s>>>(x.as<double>(), pm.masses(), n, pm.geom(), pm.mesh());
+    GS_CUDA(cudaGetLastError());
+    GS_TRY(pm.solve(s));
+    double factor = pm.scale(H0, omega_m, t);   // of the accelerations now in the mesh
     // ceil((a_final - a_begin) / dt) steps; dt = 0 (allowed by the checks)
     // gives no finite count, and no steps are taken
     const double q = (a_final - a_begin) / dt;
@@ -473,27 +645,43 @@ ErrorStatus pm_leapfrog_cosmology(CosmologicalSystem *system, SimulationStatus *
     if (status) status->dt = dt;
     int64_t steps = 0;
     GS_CUDA(cudaEventRecord(pc->ev[0], s));
+    double k1 = 0.0;        // the pending kick of the step before
+    bool gather = true;     // whether it is pending: the accelerations are in the mesh alone
     while (steps < total) {
         if (t + dt > a_final) dt = a_final - t;
         if (status) status->dt = dt;
+        // end of the step before, this step's first kick and its drift
         double da = compute_da(t, H0, omega_m, omega_lambda);
-        k_cosmo_kick<<<blocks(L), TPB, 0, s>>>(p.as<double>(), a.as<double>(), L, 0.5 * dt / da);
+        const double k2 = 0.5 * dt / da * factor;
         t += 0.5 * dt;
         da = compute_da(t, H0, omega_m, omega_lambda);
-        k_cosmo_drift<<<blocks(L), TPB, 0, s>>>(x.as<double>(), p.as<double>(), L,
-                                                dt / (t * t * da), c[0], c[1], c[2], bw);
+        GS_TRY(pm.clear(s));
+        auto move = gather ? k_pm_particles<true, true> : k_pm_particles<false, true>;
+        move<<<blocks(n), TPB, 0, s>>>(x.as<double>(), p.as<double>(), pm.masses(), a.as<double>(),
+                                       n, pm.geom(), pm.acc(), k1, k2, dt / (t * t * da), bw,
+                                       pm.mesh());
         GS_CUDA(cudaGetLastError());
-        GS_TRY(pc->solver.compute(a.as<double>(), n, x.as<double>(), m.as<double>(), c, bw, H0,
-                                  omega_m, mean_bkg_density, g, t, s));
-        k_cosmo_kick<<<blocks(L), TPB, 0, s>>>(p.as<double>(), a.as<double>(), L, 0.5 * dt / da);
-        GS_CUDA(cudaGetLastError());
+        GS_TRY(pm.solve(s));
+        factor = pm.scale(H0, omega_m, t);
+        k1 = 0.5 * dt / da * factor;
         ++steps;
         t = a_begin + steps * dt;
         if (status) {
             status->t = t;
             status->num_steps = steps;
         }
-        if (is_output && t >= next_output_time) {
+        const bool stop = steps >= total || (is_exit && *is_exit);
+        const bool snap = is_output && t >= next_output_time;
+        gather = !(stop || snap);
+        if (!gather) {
+            // the step's last kick by itself; the next step's takes the stored
+            // accelerations
+            k_pm_particles<true, false><<<blocks(n), TPB, 0, s>>>(
+                x.as<double>(), p.as<double>(), pm.masses(), a.as<double>(), n, pm.geom(), pm.acc(),
+                k1, 0.0, 0.0, bw, pm.mesh());
+            GS_CUDA(cudaGetLastError());
+        }
+        if (snap) {
             // the host arrays get x and v = p / a^2, then the snapshot (:198-221)
             k_cosmo_velocity<<<blocks(L), TPB, 0, s>>>(v.as<double>(), p.as<double>(), L, t);
             GS_CUDA(cudaGetLastError());
@@ -503,7 +691,7 @@ ErrorStatus pm_leapfrog_cosmology(CosmologicalSystem *system, SimulationStatus *
             GS_TRY(output_snapshot_cosmology(op, system, t));
             next_output_time = op->output_count_ * op->output_interval;
         }
-        if (is_exit && *is_exit) break;
+        if (stop) break;
     }
     GS_CUDA(cudaEventRecord(pc->ev[1], s));
     GS_CUDA(cudaMemcpyAsync(system->x, x.p, b3, cudaMemcpyDeviceToHost, s));
