@@ -207,6 +207,92 @@ def test_group_walk_accuracy(lib, g, orc, wl, theta, leaf):
     assert cells > 0 and pairs > 0
 
 
+def group_origins(orc, x, m, leaf=16, size=32):
+    """First particle of the group that each particle is walked with: runs of
+    consecutive children of at most `size` particles in a larger cell, cut into
+    pieces of `size`; a piece that does not fit its cell (it holds a particle at
+    the box maximum, whose key wraps) is walked particle by particle."""
+    t = orc.build_tree(x, m, leaf, False)
+    num, kids, p0, c0 = (np.asarray(t[k]) for k in ("num_particles", "num_children",
+                                                    "first_particle", "first_child"))
+    ids = np.asarray(t["sorted_indices"])
+    first = np.empty(len(x), int)
+
+    def cut(begin, count, cell):
+        for b in range(begin, begin + count, size):
+            own = ids[b:min(b + size, begin + count)]
+            fits = np.ptp(x[own], axis=0).max() <= t["box_width"] / 2.0 ** t["depth"][cell]
+            first[own] = own[0] if fits else own
+
+    if num[0] <= size or kids[0] == 0:
+        cut(0, len(x), 0)
+    for q in np.where((num > size) & (kids > 0))[0]:
+        begin = p0[q]
+        for c in range(c0[q], c0[q] + kids[q]):
+            if num[c] > size:
+                cut(begin, p0[c] - begin, q)
+                begin = p0[c] + num[c]
+                if kids[c] == 0:
+                    cut(p0[c], num[c], c)
+        cut(begin, p0[q] + num[q] - begin, q)
+    return first
+
+
+def fp32_offsets(x, origin):
+    """Positions as the walk forms them: FP32 offsets from a group's first
+    particle, from double-float copies about the frame's centre."""
+    c = x - 0.5 * (x.min(0) + x.max(0))
+    hi = c.astype(np.float32)
+    lo = (c - hi).astype(np.float32)
+    return ((hi - hi[origin]) + (lo - lo[origin])).astype(np.float64)
+
+
+@pytest.mark.parametrize("clusters,size,eps", [
+    (1, 1, 0.0), (1, 2, 0.0), (1, 16, 0.0), (1, 17, 0.0), (2, 33, 0.0), (3, 15, 0.0), (4, 32, 1e-4),
+    (5, 31, 0.0), (31, 16, 0.0), (129, 17, 0.0), (130, 1, 0.0), (131, 33, 1e-4), (257, 20, 0.0),
+    (4096, 33, 0.0), (4096, 33, 1e-4)])
+def test_group_walk_lists_vs_direct_sum(lib, g, orc, clusters, size, eps):
+    """Group walk against the FP64 direct sum of the positions it forms (FP32
+    offsets from the group's first particle), where both are the same: compact
+    clusters on a jittered grid and an angle at which an accepted cell holds one
+    cluster.  Group sizes around one row (16) and a full group (32), cell lists
+    around whole turns and around the list's capacity (128), and both forms of
+    the walk (a CTA per group; 4,096 clusters of 33 make enough groups for a warp
+    each).  Cell side < theta d <= 0.43 h, so its diagonal is below the clusters'
+    separation 0.8 h; a cluster's radius is 0.005 h, so beyond the quadrupole a
+    cell's term is off by at most 4 (0.01 / 0.8)^3 = 8e-6 of itself, and the FP32
+    terms add less than 4e-6 of the sum of magnitudes."""
+    rng = np.random.default_rng(clusters * 64 + size)
+    grid = int(np.ceil(clusters ** (1.0 / 3.0) - 1e-9))
+    h = 1.0 / grid
+    k = np.arange(clusters)
+    c = np.stack([k % grid, k // grid % grid, k // grid // grid], 1) * h
+    c = c + rng.uniform(-0.1 * h, 0.1 * h, c.shape)
+    d = rng.normal(size=(clusters, size, 3))
+    d *= (0.005 * h * rng.uniform(0.2, 1.0, (clusters, size, 1))) / np.linalg.norm(d, axis=2, keepdims=True)
+    x = np.ascontiguousarray((c[:, None, :] + d).reshape(-1, 3))
+    n = len(x)
+    m = rng.uniform(0.5, 1.5, n) / n
+    rows = rng.permutation(n)[:256].astype(np.int32)
+    # a particle on the box maximum sits in a cell on the far side (its key
+    # wraps), whose centre is not near its cluster: those clusters are left out
+    plain = ~np.isin(rows // size, x.argmax(0) // size)
+    rows = rows[plain] if plain.any() else rows
+    first = group_origins(orc, x, m)
+    exact, absum = np.empty((len(rows), 3)), np.empty((len(rows), 1))
+    for i, r in enumerate(rows):
+        off = fp32_offsets(x, first[r])
+        d = off - off[r]
+        r2 = (d * d).sum(1)
+        w = m / np.where(r2 > 0.0, (r2 + eps * eps) ** 1.5, 1.0)
+        exact[i] = (w[:, None] * d).sum(0)
+        absum[i] = (w * np.sqrt(r2)).sum()
+    a = g.acceleration(lib, x, m, 1.0, g.METHOD_GPU_BARNES_HUT_GROUP, opening_angle=0.25 / grid,
+                       softening_length=eps)
+    assert np.isfinite(a).all()
+    assert (np.abs(a[rows] - exact) <= 1.2e-5 * absum).all()
+
+
 def test_group_walk_degenerate_and_unsoftened(lib, g, orc, wl):
     """A 200-particle coincident cluster (one depth-21 leaf with more
     particles than one list round) with softening, and an unsoftened
