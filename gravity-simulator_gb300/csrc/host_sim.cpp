@@ -173,10 +173,11 @@ struct gsgpu_sim {
     // Pairs of a small system under an FP64 force, 0 for any other (set by upload,
     // which sees the masses).  One CTA forms 128 pairs at a time: with at most
     // kTinyPairs of them a fixed step by k_tiny_fixed beats the step's launches
-    // (2.5 against 11 us for nine bodies; even at about 600 pairs), and the adaptive
-    // integrators, tens of launches a step, take every system that fits.
+    // (leapfrog, 5.5 against 8.8 us for nine bodies, 7.8 against 9.0 for 23; from a
+    // third round of pairs on it loses, 11.0 against 9.1 for 24 bodies), and the
+    // adaptive integrators, tens of launches a step, take every system that fits.
     int tiny_pairs = 0;
-    static constexpr int kTinyPairs = 512;
+    static constexpr int kTinyPairs = 256;
     bool tiny_fixed() const { return tiny_pairs > 0 && tiny_pairs <= kTinyPairs && !timer.enabled; }
     bool tiny_adaptive() const { return tiny_pairs > 0 && !timer.enabled; }
 
