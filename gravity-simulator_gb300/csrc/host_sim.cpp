@@ -171,16 +171,24 @@ struct gsgpu_sim {
     DBuf i_b0, i_b, i_g, i_e, i_F, i_a1, i_d7, i_max;
     unsigned long long *h_max = nullptr;   // pinned: two maxima
     // Pairs of a small system under an FP64 force, 0 for any other (set by upload,
-    // which sees the masses).  One CTA forms 128 pairs at a time: with at most
-    // kTinyPairs of them a fixed step by k_tiny_fixed beats the step's launches
-    // (leapfrog, 5.5 against 8.8 us for nine bodies, 7.8 against 9.0 for 23; from a
-    // third round of pairs on it loses, 11.0 against 9.1 for 24 bodies), and the
-    // adaptive integrators, tens of launches a step, take every system that fits.
+    // which sees the masses).  One CTA forms 128 pairs at a time, so a force costs
+    // it about as many rounds of them, and the pairwise force by launches does not
+    // grow below 48 bodies.  Microseconds in one block against by launches: a
+    // leapfrog step 5.5 and 8.8 (9 bodies), 7.8 and 9.0 (23), 11.0 and 9.1 (24, a
+    // third round); a Runge-Kutta run of 300 days 19,100 and 20,700 (32 bodies, 496
+    // pairs), 27,100 and 22,800 (40); IAS15, a dozen forces a step in one launch, 94
+    // and 120 thousand (40 bodies, 780 pairs), 140 and 122 thousand (48).  The
+    // massless force takes several launches: 38 a leapfrog step against 9.8 for the
+    // 243 pairs of 32 bodies, so there the block takes every system that fits.
     int tiny_pairs = 0;
-    static constexpr int kTinyPairs = 256;
-    bool tiny_fixed() const { return tiny_pairs > 0 && tiny_pairs <= kTinyPairs && !timer.enabled; }
-    bool tiny_adaptive() const { return tiny_pairs > 0 && !timer.enabled; }
-
+    bool one_block(int limit) const
+    {
+        return tiny_pairs > 0 && !timer.enabled &&
+               (tiny_pairs <= limit || p.method == GRAV_GPU_MASSLESS);
+    }
+    bool tiny_fixed() const { return one_block(256); }
+    bool tiny_rk() const { return one_block(512); }
+    bool tiny_ias15() const { return one_block(800); }
     TinySystem tiny() const
     {
         TinySystem t{};
@@ -341,7 +349,7 @@ struct gsgpu_sim {
             status->dt = h;
             status->num_steps = 0;
         }
-        const bool tiny_run = tiny_adaptive();
+        const bool tiny_run = tiny_ias15();
         TinyIas I{};
         bool accept = false, refine_next = false;
         if (tiny_run) {
@@ -493,7 +501,7 @@ struct gsgpu_sim {
         const bool device_sum = g_rk_error_sum.load(std::memory_order_relaxed) == 1;
         // small systems: the host adds their few terms in the reference's order
         // whatever the mode
-        const bool tiny_run = tiny_adaptive();
+        const bool tiny_run = tiny_rk();
         TinyRk R{};
         bool accept = false;
         if (tiny_run) {

@@ -235,11 +235,12 @@ def test_energy_drift_against_reference_barnes_hut(lib, g, orc, wl):
 
 
 @pytest.mark.parametrize("massless", [False, True])
-@pytest.mark.parametrize("n", [2, 3, 9, 32, 33, 43, 48, 49])
+@pytest.mark.parametrize("n", [2, 3, 9, 23, 24, 32, 33, 40, 41, 43, 48, 49])
 @pytest.mark.parametrize("integ", [1, 2, 3, 4, 5, 8, 9])
 def test_small_systems_bitexact(lib, g, orc, wl, integ, n, massless):
-    """Systems of at most 48 bodies, which one block steps (up to 512 pairs for the fixed steps:
-    32 and 33 bodies under the pairwise force are on either side), with massive and massless
+    """Systems of at most 48 bodies, which one block steps (under the pairwise force up to 256
+    pairs for the fixed steps, 512 for Runge-Kutta and 800 for IAS15: 23 and 24, 32 and 33, 40 and
+    41 bodies are on either side), with massive and massless
     bodies interleaved, more than a batch of 32 steps and a clamped last one.  Bit for bit
     against the oracle."""
     x, v, m = wl.plummer(n, 60 + n)
