@@ -73,7 +73,7 @@ struct OctreeDevice {
     DBuf w_nc;                // int4[cap]: (first_child, num_children, first_particle, count)
     DBuf w_nkey;              // uint64[cap]: key used by the cell-membership test
     DBuf w_pa, w_pb;          // float4[n] in sorted order: (x_hi, m), (x_lo, 0)
-    DBuf xm;                  // double[4n] in sorted order: x, y, z, m (the multipole sums' input)
+    DBuf mx;                  // double[4n] in sorted order: m, m x, m y, m z (the multipole sums' input)
     DBuf g_list;              // int2[n]: particle groups of the group walk (first, count)
     DBuf g_ctr;               // int[4]: group count, work-queue head
     // Particles whose Morton coordinate left [0, 2^21) and was masked (the

@@ -501,24 +501,46 @@ __global__ void k_tree_links(const int *__restrict__ ctr, const int4 *__restrict
     }
 }
 
-// Running sums of the particles of one leaf, sorted order (reference :667-674).
 // Mass and mass-weighted coordinate sums of sorted particles [first,
-// first + count) in sorted order (the reference's order), read from the
-// sorted (x, y, z, m) copy: contiguous 32-byte records instead of gathers
-// through the sorted ids into the caller's arrays; same values, same sums.
-__device__ __forceinline__ void add_particles(const double *__restrict__ xm, int first, int count,
+// first + count) in sorted order (reference :667-674), from the sorted
+// (m, m x, m y, m z) records: four ordered additions per particle.  The products
+// are the ones the reference forms inside the sum; formed once per particle when
+// the records are written, they need not be formed again for the leaf and for
+// its parent (7 and 2 FP64 instructions per particle before; k_leaf_multipoles
+// 90 and 65 us at N = 1,048,576).
+__device__ __forceinline__ void add_particles(const double *__restrict__ mx, int first, int count,
                                               double &M, double &S0, double &S1, double &S2)
 {
 #pragma unroll 4
     for (int p = first; p < first + count; ++p) {
-        const double2 a = __ldg(reinterpret_cast<const double2 *>(xm + 4 * (size_t)p));
-        const double2 b = __ldg(reinterpret_cast<const double2 *>(xm + 4 * (size_t)p) + 1);
-        const double mp = b.y;
-        M = __dadd_rn(M, mp);
-        S0 = __dadd_rn(S0, __dmul_rn(mp, a.x));
-        S1 = __dadd_rn(S1, __dmul_rn(mp, a.y));
-        S2 = __dadd_rn(S2, __dmul_rn(mp, b.x));
+        const double2 a = __ldg(reinterpret_cast<const double2 *>(mx + 4 * (size_t)p));
+        const double2 b = __ldg(reinterpret_cast<const double2 *>(mx + 4 * (size_t)p) + 1);
+        M = __dadd_rn(M, a.x);
+        S0 = __dadd_rn(S0, a.y);
+        S1 = __dadd_rn(S1, b.x);
+        S2 = __dadd_rn(S2, b.y);
     }
+}
+
+// acc plus the values q[4 p] of p in [p0, p1), in order; eight loads are in
+// flight while eight values are added, so that the chain of additions waits for
+// the first eight only.
+__device__ __forceinline__ double add_run(double acc, const double *__restrict__ q, int p0, int p1)
+{
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = p0 + u < p1 ? __ldg(q + 4 * (size_t)(p0 + u)) : 0.0;
+    for (int p = p0; p < p1; p += 8) {
+        double w[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) w[u] = p + 8 + u < p1 ? __ldg(q + 4 * (size_t)(p + 8 + u)) : 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            if (p + u < p1) acc = __dadd_rn(acc, v[u]);
+            v[u] = w[u];
+        }
+    }
+    return acc;
 }
 
 __device__ __forceinline__ void split_df(double v, float &hi, float &lo)
@@ -579,7 +601,7 @@ __device__ __forceinline__ float df_offset(float ph, float pl, float ch, float c
 }
 
 struct MultipoleArgs {
-    const double *xm;   // sorted (x, y, z, m) records
+    const double *mx;   // sorted (m, m x, m y, m z) records
     const int4 *in_rec; // internal nodes: (first child, children | inner mask << 8, parent, id)
     const int4 *nc;     // nodes: (first child, children, first particle, particles)
     const int *t_depth;
@@ -596,58 +618,76 @@ struct MultipoleArgs {
 // Q = sum_c [Q_c + M_c (3 s s^T - |s|^2 I)], s = com_c - com, in FP32 from the
 // children's walk records (FP64 runs at 1/64 of the FP32 rate here, and the walk
 // uses FP32 quadrupoles).  Children's values written by other threads of the
-// same launch are read through L2 (__ldcg), after the fence that follows the
+// same launch are read through L2 (__ldcg), after the acquire on the
 // arrival counter.
 //
 // A node is computed by the four lanes of a group: lane j keeps one of the
 // four ordered sums (j = 0 the mass, j = 1..3 the sums of m x, m y, m z), so
-// a particle costs one FP64 multiply and one add for all four sums (lane 0
-// multiplies the mass by 1.0, which is exact: its sum is the plain mass sum),
-// and the three quotients are one division.  Each sum sees the same operands in
-// the same order as a one-thread loop would, so the values are the same bit for
-// bit.
+// a particle costs one FP64 addition for all four sums, and the three quotients
+// are one division.  Each sum sees the same operands in the same order as a
+// one-thread loop would, so the values are the same bit for bit.
 //
 // Near the root a single group climbs alone, and what bounds it is the chain of
 // dependent loads of each level.  The record and the sums are laid out so that
 // a level is one round of loads: the record says which children are internal,
-// their sums are indexed by node id, and all of them (and the leaf children's
-// particle ranges) are issued before the first is used; the caller loads the
-// parent's record meanwhile.  With child type, index and sums each behind the
-// other, eight times in a row, a level took about 17 us and the kernel 309 us
-// at N = 60,000 and 311 us at N = 1,048,576.
-__device__ void multipole_node4(const int4 rec, int j, unsigned gmask, const MultipoleArgs &A)
+// their sums are indexed by node id, and all of them, the leaf children's
+// particle ranges and the children's quadrupoles (two children a lane) are
+// issued before the first is used; the caller loads the parent's record
+// meanwhile.  With child type, index and sums each behind the other, eight times
+// in a row, a level took about 17 us and the kernel 309 us at N = 60,000 and
+// 311 us at N = 1,048,576; with the quadrupoles in a round of their own and
+// the particles of leaf children four at a time 103 and 157 us; now 55 and 91.
+template <bool QUAD>
+__device__ __forceinline__ void multipole_node4(const int4 rec, int j, unsigned gmask, const MultipoleArgs &A)
 {
     const int fc = rec.x, nch = rec.y & 255, inner = rec.y >> 8, id = rec.w;
-    const int end = fc + nch;
-    double v[8];
-    int2 leaf[8];
+    // this lane's sum of every internal child, the particles of every leaf child
+    __shared__ double s_sum[8][OT_THREADS];
+    __shared__ int2 s_leaf[8][OT_THREADS];
+    {
+        double v[8];
+        int2 leaf[8];
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        v[r] = 0.0;
-        leaf[r] = make_int2(0, 0);
-        if (r < nch) {
-            if ((inner >> r) & 1)
-                v[r] = __ldcg(A.t_sum + 4 * (size_t)(fc + r) + j);
-            else
-                leaf[r] = reinterpret_cast<const int2 *>(A.nc + fc + r)[1];
-        }
-    }
-    double acc = 0.0;
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        if (r >= nch) break;
-        if ((inner >> r) & 1) {
-            acc = __dadd_rn(acc, v[r]);
-        } else {
-            const int p1 = leaf[r].x + leaf[r].y;
-#pragma unroll 4
-            for (int p = leaf[r].x; p < p1; ++p) {
-                const double *q = A.xm + 4 * (size_t)p;
-                const double mp = __ldg(q + 3);
-                const double xv = j == 0 ? 1.0 : __ldg(q + j - 1);
-                acc = __dadd_rn(acc, __dmul_rn(mp, xv));
+        for (int r = 0; r < 8; ++r) {
+            v[r] = 0.0;
+            leaf[r] = make_int2(0, 0);
+            if (r < nch) {
+                if ((inner >> r) & 1)
+                    v[r] = __ldcg(A.t_sum + 4 * (size_t)(fc + r) + j);
+                else
+                    leaf[r] = reinterpret_cast<const int2 *>(A.nc + fc + r)[1];
             }
         }
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            s_sum[r][threadIdx.x] = v[r];
+            s_leaf[r][threadIdx.x] = leaf[r];
+        }
+    }
+    // quadrupoles of children j and j + 4
+    float4 ca[2], cb[2], qa[2], qb[2];
+    if (QUAD) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            if (j + 4 * k < nch) {
+                const size_t c = fc + j + 4 * k;
+                ca[k] = __ldcg(A.na + c);
+                cb[k] = __ldcg(A.nb + c);
+                qa[k] = __ldcg(A.nq + 2 * c);
+                qb[k] = __ldcg(A.nq + 2 * c + 1);
+            }
+    }
+    // children in order; the particles of consecutive leaf children are one run
+    double acc = 0.0;
+    for (int r = 0; r < nch;) {
+        int p0 = 0, p1 = 0;
+        for (; r < nch && !((inner >> r) & 1); ++r) {
+            const int2 leaf = s_leaf[r][threadIdx.x];
+            if (p1 <= p0) p0 = leaf.x;
+            p1 = leaf.x + leaf.y;
+        }
+        acc = add_run(acc, A.mx + j, p0, p1);
+        for (; r < nch && ((inner >> r) & 1); ++r) acc = __dadd_rn(acc, s_sum[r][threadIdx.x]);
     }
     A.t_sum[4 * (size_t)id + j] = acc;
     const double M = __shfl_sync(gmask, acc, 0, 4);
@@ -669,21 +709,25 @@ __device__ void multipole_node4(const int4 rec, int j, unsigned gmask, const Mul
         A.na[id] = make_float4(h[0], h[1], h[2], (float)M);
         A.nb[id] = make_float4(l[0], l[1], l[2], cell_side2(A.frame, A.t_depth[id]));
     }
-    if (A.nq) {
-        // every lane of the group forms the same sums; lane 0 stores them
+    if (QUAD) {
         float Q[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-        for (int c = fc; c < end; ++c) {
-            const float4 ca = __ldcg(A.na + c), cb = __ldcg(A.nb + c);
-            const float4 qa = __ldcg(A.nq + 2 * (size_t)c), qb = __ldcg(A.nq + 2 * (size_t)c + 1);
-            add_quad(Q, ca.w, df_offset(ca.x, cb.x, h[0], l[0]), df_offset(ca.y, cb.y, h[1], l[1]),
-                     df_offset(ca.z, cb.z, h[2], l[2]));
-            Q[0] += qa.x;
-            Q[1] += qa.y;
-            Q[2] += qa.z;
-            Q[3] += qa.w;
-            Q[4] += qb.x;
-            Q[5] += qb.y;
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            if (j + 4 * k < nch) {
+                add_quad(Q, ca[k].w, df_offset(ca[k].x, cb[k].x, h[0], l[0]),
+                         df_offset(ca[k].y, cb[k].y, h[1], l[1]),
+                         df_offset(ca[k].z, cb[k].z, h[2], l[2]));
+                Q[0] += qa[k].x;
+                Q[1] += qa[k].y;
+                Q[2] += qa[k].z;
+                Q[3] += qa[k].w;
+                Q[4] += qb[k].x;
+                Q[5] += qb[k].y;
+            }
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            Q[q] += __shfl_xor_sync(gmask, Q[q], 1, 4);
+            Q[q] += __shfl_xor_sync(gmask, Q[q], 2, 4);
         }
         if (j == 0) store_quad(A.nq, id, Q);
     }
@@ -697,8 +741,12 @@ __device__ void multipole_node4(const int4 rec, int j, unsigned gmask, const Mul
 // node is computed once, by the same arithmetic in the same child order as a
 // level-by-level pass, so the sums are identical to it.  Every decision below
 // is the same for the four lanes of a group (they share the node), so the
-// group's shuffles and barriers see all four.
-__global__ void __launch_bounds__(OT_THREADS) k_multipole_up(const int *__restrict__ ctr,
+// group's shuffles and barriers see all four.  Two CTAs per SM with quadrupoles
+// (three or four: the registers of the loads in flight spill, 8 to 17 us longer at
+// N = 60,000), four without (95 us at N = 150,000 with one particle per leaf,
+// three and six 109).
+template <bool QUAD>
+__global__ void __launch_bounds__(OT_THREADS, QUAD ? 2 : 4) k_multipole_up(const int *__restrict__ ctr,
                                                              MultipoleArgs A)
 {
     const int ni = ctr[CTR_SAFE_INTERNAL];
@@ -711,16 +759,21 @@ __global__ void __launch_bounds__(OT_THREADS) k_multipole_up(const int *__restri
         for (;;) {
             const int p = rec.z;
             const int4 up = p >= 0 ? A.in_rec[p] : make_int4(0, 0, 0, 0);
-            multipole_node4(rec, j, gmask, A);
+            multipole_node4<QUAD>(rec, j, gmask, A);
             if (p < 0) break;
-            // each lane's writes are visible before lane 0 counts the group in
-            __threadfence();
+            // The lanes' writes happen before the barrier, and lane 0's release
+            // makes them visible with its own; its acquire orders the other
+            // groups' writes before the reads below.
             __syncwarp(gmask);
             int arrived = 0;
-            if (j == 0) arrived = atomicAdd(&A.in_arrive[p], 1);
+            if (j == 0)
+                asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;"
+                             : "=r"(arrived)
+                             : "l"(A.in_arrive + p)
+                             : "memory");
             arrived = __shfl_sync(gmask, arrived, 0, 4);
             if (arrived != __popc(up.y >> 8) - 1) break;
-            __threadfence();
+            __syncwarp(gmask);
             rec = up;
         }
     }
@@ -754,7 +807,7 @@ __global__ void k_leaf_multipoles(const int *__restrict__ ctr, int compat, Multi
         double M = 0.0, c0 = 0.0, c1 = 0.0, c2 = 0.0;
         if (!compat) {
             double S0 = 0.0, S1 = 0.0, S2 = 0.0;
-            add_particles(A.xm, fp, np, M, S0, S1, S2);
+            add_particles(A.mx, fp, np, M, S0, S1, S2);
             c0 = __ddiv_rn(S0, M);
             c1 = __ddiv_rn(S1, M);
             c2 = __ddiv_rn(S2, M);
@@ -781,7 +834,7 @@ __global__ void k_leaf_multipoles(const int *__restrict__ ctr, int compat, Multi
 __global__ void k_walk_particles(int n, const double *__restrict__ frame, const double *__restrict__ x,
                                  const double *__restrict__ m, const int *__restrict__ sidx,
                                  float4 *__restrict__ pa, float4 *__restrict__ pb,
-                                 double *__restrict__ xm,
+                                 double *__restrict__ mx,
                                  const unsigned char *__restrict__ misplaced,
                                  int *__restrict__ mlist)
 {
@@ -792,14 +845,15 @@ __global__ void k_walk_particles(int n, const double *__restrict__ frame, const 
         const int at = atomicAdd(&mlist[0], 1);
         if (at < kMisplacedCap) mlist[1 + at] = p;
     }
-    double2 *xo = reinterpret_cast<double2 *>(xm + 4 * (size_t)p);
-    xo[0] = make_double2(x[3 * id + 0], x[3 * id + 1]);
-    xo[1] = make_double2(x[3 * id + 2], m[id]);
+    const double mp = m[id];
+    double2 *out = reinterpret_cast<double2 *>(mx + 4 * (size_t)p);
+    out[0] = make_double2(mp, __dmul_rn(mp, x[3 * id + 0]));
+    out[1] = make_double2(__dmul_rn(mp, x[3 * id + 1]), __dmul_rn(mp, x[3 * id + 2]));
     float h0, l0, h1, l1, h2, l2;
     split_df(__dsub_rn(x[3 * id + 0], frame[0]), h0, l0);
     split_df(__dsub_rn(x[3 * id + 1], frame[1]), h1, l1);
     split_df(__dsub_rn(x[3 * id + 2], frame[2]), h2, l2);
-    pa[p] = make_float4(h0, h1, h2, (float)m[id]);
+    pa[p] = make_float4(h0, h1, h2, (float)mp);
     pb[p] = make_float4(l0, l1, l2, 0.0f);
 }
 
@@ -842,7 +896,7 @@ ErrorStatus OctreeDevice::setup(int n_, int leaf_max_, bool compat_, bool quad_)
     GS_TRY(mlist.reserve((size_t)(1 + kMisplacedCap) * sizeof(int)));
     GS_TRY(w_pa.reserve((size_t)n * sizeof(float4)));
     GS_TRY(w_pb.reserve((size_t)n * sizeof(float4)));
-    GS_TRY(xm.reserve((size_t)n * 4 * sizeof(double)));
+    GS_TRY(mx.reserve((size_t)n * 4 * sizeof(double)));
     GS_TRY(g_list.reserve((size_t)n * sizeof(int2)));
     GS_TRY(g_ctr.reserve(4 * sizeof(int)));
     if (quad) GS_TRY(w_nq.reserve((size_t)cap * 2 * sizeof(float4)));
@@ -906,7 +960,7 @@ ErrorStatus OctreeDevice::build(const double *d_x, const double *d_m, cudaStream
                                                  t_fp.as<int>(), t_int.as<int>(),
                                                  t_parent.as<int>(), leaf_of.as<int>());
     MultipoleArgs A;
-    A.xm = xm.as<double>();
+    A.mx = mx.as<double>();
     A.in_rec = in_rec.as<int4>();
     A.nc = w_nc.as<int4>();
     A.t_depth = t_depth.as<int>();
@@ -922,7 +976,7 @@ ErrorStatus OctreeDevice::build(const double *d_x, const double *d_m, cudaStream
     GS_CUDA(cudaMemsetAsync(mlist.p, 0, sizeof(int), s));
     k_walk_particles<<<pb, OT_THREADS, 0, s>>>(n, frame.as<double>(), d_x, d_m, sidx.as<int>(),
                                                w_pa.as<float4>(), w_pb.as<float4>(),
-                                               xm.as<double>(), misplaced.as<unsigned char>(),
+                                               mx.as<double>(), misplaced.as<unsigned char>(),
                                                mlist.as<int>());
     k_leaf_multipoles<<<grid, OT_THREADS, 0, s>>>(
         ctr.as<int>(), compat ? 1 : 0, A, w_pa.as<float4>(), w_pb.as<float4>(),
@@ -930,7 +984,8 @@ ErrorStatus OctreeDevice::build(const double *d_x, const double *d_m, cudaStream
         t_nc.as<int>(), t_fc.as<int>(), w_nc.as<int4>(), w_nkey.as<uint64_t>());
     // four lanes per internal node: a larger grid, so that every node of a
     // tree of up to about 2^16 internal nodes starts at once
-    k_multipole_up<<<dev->sm_count * 8, OT_THREADS, 0, s>>>(ctr.as<int>(), A);
+    (A.nq ? k_multipole_up<true> : k_multipole_up<false>)<<<dev->sm_count * 8, OT_THREADS, 0, s>>>(
+        ctr.as<int>(), A);
     GS_CUDA(cudaGetLastError());
     return ok();
 }

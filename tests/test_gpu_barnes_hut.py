@@ -92,6 +92,20 @@ def test_octree_bitexact_at_scan_tile_edges(lib, g, orc, wl, n, leaf):
     assert_same_tree(gt, orc.build_tree(x, m, leaf, True))
 
 
+@pytest.mark.parametrize("leaf", [2, 7, 8, 9, 16, 33])
+def test_octree_bitexact_at_run_edges(lib, g, orc, wl, leaf):
+    """The climb adds the particles of consecutive leaf children eight at a time."""
+    x, v, m = wl.galaxy_pair(6000, 40 + leaf)
+    assert_same_tree(gpu_octree(lib, g, x, m, leaf), orc.build_tree(x, m, leaf, True))
+
+
+@pytest.mark.parametrize("n", [1023, 1024, 1025, 200000, 200001, 400000, 400001])
+def test_octree_bitexact_at_sort_tile_edges(lib, g, orc, wl, n):
+    """Sort tiles of 1,024, 2,048 (above 200,000 particles) and 4,096 (above 400,000)."""
+    x, v, m = wl.galaxy_pair(n, 3)
+    assert_same_tree(gpu_octree(lib, g, x, m, 16), orc.build_tree(x, m, 16, True))
+
+
 def test_octree_bitexact_galaxy_collision_2097152(lib, g, orc, wl):
     """Morton keys, order and tree of the galaxy-collision workload at full
     size, bit-exact."""
