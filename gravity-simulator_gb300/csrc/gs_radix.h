@@ -26,7 +26,7 @@ class RadixSorter {
     static int launches(int key_bits) { return 2 + passes_for(key_bits); }
 
   private:
-    int capacity_ = 0, tiles_ = 0, sm_count_ = 1;
+    int capacity_ = 0, items_ = 16, tiles_ = 0, sm_count_ = 1;
     DBuf hist_, lookback_, tmp_keys_, tmp_vals_;
 };
 

@@ -11,10 +11,10 @@
 //                        pass (a digit's count does not depend on the order);
 //   2. k_radix_bases  -- per pass, the exclusive scan over digits: where each
 //                        digit's run starts in the output;
-//   3. k_radix_onesweep, once per pass -- a CTA takes the next tile of 4096
-//      elements (tile order = start order, from an atomic counter), ranks
-//      them stably by warp match (each warp owns 512 consecutive elements,
-//      16 rounds of 32, ranked in index order), publishes its per-digit
+//   3. k_radix_onesweep, once per pass -- a CTA takes the next tile of 1024,
+//      2048 or 4096 elements (tile order = start order, from an atomic counter),
+//      ranks them stably by warp match (each warp owns an eighth of them,
+//      rounds of 32, ranked in index order), publishes its per-digit
 //      counts, then for each digit walks back over the preceding tiles'
 //      published counts / inclusive prefixes until it meets a prefix, and
 //      writes the tile out through shared memory in digit order (coalesced
@@ -35,8 +35,6 @@
 namespace gs {
 
 constexpr int RX_THREADS = 256;
-constexpr int RX_ITEMS = 16;
-constexpr int RX_TILE = RX_THREADS * RX_ITEMS;   // 4096
 constexpr int RX_WARPS = RX_THREADS / 32;
 constexpr int RX_MAX_PASSES = 8;
 constexpr int RX_LOOKBACK = 8;   // predecessor tiles read per look-back round
@@ -96,6 +94,7 @@ __device__ __forceinline__ void st_volatile(unsigned long long *p, unsigned long
     *reinterpret_cast<volatile unsigned long long *>(p) = v;
 }
 
+template <int ITEMS>
 __global__ void __launch_bounds__(RX_THREADS)
 k_radix_onesweep(const uint64_t *__restrict__ keys_in, const int *__restrict__ vals_in,
                  uint64_t *__restrict__ keys_out, int *__restrict__ vals_out,
@@ -103,29 +102,30 @@ k_radix_onesweep(const uint64_t *__restrict__ keys_in, const int *__restrict__ v
                  unsigned long long *__restrict__ lookback, int *__restrict__ tile_ctr,
                  unsigned *__restrict__ status)
 {
+    constexpr int kTile = RX_THREADS * ITEMS;
     __shared__ unsigned whist[RX_WARPS][256];
     __shared__ unsigned tile_off[256];     // output position of the tile's first element of digit d
     __shared__ unsigned local_start[256];  // position of digit d's run within the tile
     __shared__ unsigned wsum[RX_WARPS];
-    __shared__ uint64_t stage[RX_TILE];    // the tile in digit order (keys, then values)
+    __shared__ uint64_t stage[kTile];    // the tile in digit order (keys, then values)
     __shared__ int s_tile;
     if (threadIdx.x == 0) s_tile = atomicAdd(tile_ctr, 1);
     for (int d = threadIdx.x; d < RX_WARPS * 256; d += RX_THREADS) (&whist[0][0])[d] = 0u;
     __syncthreads();
     const int tile = s_tile;
     const int n = *d_n;
-    if (tile * RX_TILE >= n) return;   // block-uniform: no later tile waits on it
+    if (tile * kTile >= n) return;   // block-uniform: no later tile waits on it
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
 
-    const int wbase = tile * RX_TILE + warp * (RX_ITEMS * 32);
-    uint64_t key[RX_ITEMS];
-    int val[RX_ITEMS];
-    unsigned rank[RX_ITEMS];
-    unsigned dig[RX_ITEMS];
+    const int wbase = tile * kTile + warp * (ITEMS * 32);
+    uint64_t key[ITEMS];
+    int val[ITEMS];
+    unsigned rank[ITEMS];
+    unsigned dig[ITEMS];
     const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
-    for (int r = 0; r < RX_ITEMS; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
         const int e = wbase + r * 32 + lane;
         const bool in = e < n;
         key[r] = in ? keys_in[e] : 0ull;
@@ -212,10 +212,10 @@ k_radix_onesweep(const uint64_t *__restrict__ keys_in, const int *__restrict__ v
     // The tile goes through shared memory in digit order, so that
     // consecutive threads write consecutive output slots of a digit's run
     // (coalesced) instead of scattering element by element.
-    const int valid = min(RX_TILE, n - tile * RX_TILE);
-    unsigned lpos[RX_ITEMS];
+    const int valid = min(kTile, n - tile * kTile);
+    unsigned lpos[ITEMS];
 #pragma unroll
-    for (int r = 0; r < RX_ITEMS; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
         const int e = wbase + r * 32 + lane;
         lpos[r] = 0;
         if (e < n) {
@@ -225,9 +225,9 @@ k_radix_onesweep(const uint64_t *__restrict__ keys_in, const int *__restrict__ v
         }
     }
     __syncthreads();
-    unsigned dst[RX_ITEMS];
+    unsigned dst[ITEMS];
 #pragma unroll
-    for (int r = 0; r < RX_ITEMS; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
         const int i = r * RX_THREADS + threadIdx.x;
         dst[r] = 0;
         if (i < valid) {
@@ -240,13 +240,13 @@ k_radix_onesweep(const uint64_t *__restrict__ keys_in, const int *__restrict__ v
     __syncthreads();
     int *vstage = reinterpret_cast<int *>(stage);
 #pragma unroll
-    for (int r = 0; r < RX_ITEMS; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
         const int e = wbase + r * 32 + lane;
         if (e < n) vstage[lpos[r]] = val[r];
     }
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < RX_ITEMS; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
         const int i = r * RX_THREADS + threadIdx.x;
         if (i < valid) vals_out[dst[r]] = vstage[i];
     }
@@ -259,7 +259,13 @@ ErrorStatus RadixSorter::reserve(int cap)
     GS_TRY(device_info(&dev));
     sm_count_ = dev->sm_count;
     capacity_ = cap;
-    tiles_ = (cap + RX_TILE - 1) / RX_TILE;
+    // A small sort is as long as one tile's chain of phases: more and smaller
+    // tiles while they fit the GPU at once.  Step of a galaxy pair (eight passes)
+    // with 4, 8 and 16 elements a thread: 489, 498 and 522 us at 60,000 particles,
+    // 818, 829 and 848 at 150,000, 1357, 1345 and 1373 at 300,000, 2467, 2430 and
+    // 2420 at 600,000.
+    items_ = cap <= 200000 ? 4 : cap <= 400000 ? 8 : 16;
+    tiles_ = (cap + RX_THREADS * items_ - 1) / (RX_THREADS * items_);
     GS_TRY(hist_.reserve((size_t)(RX_MAX_PASSES * 256 + RX_MAX_PASSES) * sizeof(unsigned)));
     GS_TRY(lookback_.reserve((size_t)RX_MAX_PASSES * tiles_ * 256 * sizeof(unsigned long long)));
     GS_TRY(tmp_keys_.reserve((size_t)cap * sizeof(uint64_t)));
@@ -276,7 +282,8 @@ ErrorStatus RadixSorter::sort(uint64_t *keys, int *vals, const int *d_n, int max
     const int passes = passes_for(key_bits);
     if (passes > RX_MAX_PASSES) return GS_RAISE(GRAV_VALUE_ERROR, "radix sort keys wider than 64 bits");
     if (max_n <= 0) return ok();
-    const int tiles = (max_n + RX_TILE - 1) / RX_TILE;
+    const int tile = RX_THREADS * items_, tiles = (max_n + tile - 1) / tile;
+    auto pass = items_ == 4 ? k_radix_onesweep<4> : items_ == 8 ? k_radix_onesweep<8> : k_radix_onesweep<16>;
     unsigned *hist = hist_.as<unsigned>();
     int *tile_ctr = reinterpret_cast<int *>(hist + RX_MAX_PASSES * 256);
     GS_CUDA(cudaMemsetAsync(hist_.p, 0, (size_t)(RX_MAX_PASSES * 256 + RX_MAX_PASSES) * sizeof(unsigned),
@@ -288,7 +295,7 @@ ErrorStatus RadixSorter::sort(uint64_t *keys, int *vals, const int *d_n, int max
     uint64_t *kin = keys, *kout = tmp_keys_.as<uint64_t>();
     int *vin = vals, *vout = tmp_vals_.as<int>();
     for (int p = 0; p < passes; ++p) {
-        k_radix_onesweep<<<tiles, RX_THREADS, 0, s>>>(
+        pass<<<tiles, RX_THREADS, 0, s>>>(
             kin, vin, kout, vout, d_n, 8 * p, hist + 256 * p,
             lookback_.as<unsigned long long>() + (size_t)p * tiles * 256, tile_ctr + p, status);
         std::swap(kin, kout);
