@@ -203,7 +203,19 @@ __global__ void k_morton(const double *__restrict__ x, int n, const double *__re
 // no level-by-level expansion and no sort of the nodes.
 constexpr int TC_ITEMS = 8;
 constexpr int TC_TILE = OT_THREADS * TC_ITEMS;   // particles per scan tile
-constexpr int TN_TILE = OT_THREADS;              // internal nodes per scan tile
+constexpr int TN_ROUND = OT_THREADS / 8;         // internal nodes a CTA works on at once
+constexpr int TN_ROUNDS = 8;                     // rounds per scan tile at most
+constexpr int TN_MANY = 1216;                    // scan tiles from which a tile takes more rounds
+
+// Internal nodes per scan tile of a tree with ni of them.  A round is a chain
+// of dependent loads (the searches of the octants' ends), so a small tree takes
+// one round per tile: eight rounds left 8 of 152 SMs with work at 60,000 particles
+// and 16 per leaf (38 us, now 11).  Tiles grow with the tree so
+// that their scan, by one CTA, stays short.
+__device__ __forceinline__ int node_tile(int ni)
+{
+    return TN_ROUND * min(TN_ROUNDS, 1 + ni / (TN_ROUND * TN_MANY));
+}
 
 // Levels (octant digits) shared by two 63-bit keys.
 __device__ __forceinline__ int shared_levels(uint64_t a, uint64_t b)
@@ -373,11 +385,11 @@ k_tree_children(const uint64_t *__restrict__ keys, int n, int cap, const int2 *_
 {
     const int ni = ctr[CTR_SAFE_INTERNAL];
     const int lane = threadIdx.x & 31, o = lane & 7, g0 = lane & ~7;
-    const int tiles = (ni + TN_TILE - 1) / TN_TILE;
+    const int size = node_tile(ni), tiles = (ni + size - 1) / size;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         unsigned mine = 0;
-        for (int q = 0; q < TN_TILE; q += OT_THREADS / 8) {
-            const int ii = tile * TN_TILE + q + (threadIdx.x >> 3);
+        for (int q = 0; q < size; q += TN_ROUND) {
+            const int ii = tile * size + q + (threadIdx.x >> 3);
             const bool act = ii < ni;
             int s = 0, end = 0;
             if (act) {
@@ -423,19 +435,20 @@ k_tree_nodes(int n, int leaf_max, const unsigned *__restrict__ tile_off,
              int *__restrict__ t_np, int *__restrict__ t_fp, int *__restrict__ t_depth,
              int *__restrict__ t_int)
 {
-    __shared__ int s_fc[TN_TILE];
+    __shared__ int s_fc[TN_ROUND * TN_ROUNDS];
     const int ni = ctr[CTR_SAFE_INTERNAL];
     const int lane = threadIdx.x & 31, o = lane & 7, g0 = lane & ~7;
-    const int tiles = (ni + TN_TILE - 1) / TN_TILE;
+    const int size = node_tile(ni), tiles = (ni + size - 1) / size;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int mine = tile * TN_TILE + (int)threadIdx.x;
+        const int mine = tile * size + (int)threadIdx.x;
         unsigned sum;
-        const unsigned before = block_exclusive(mine < ni ? (unsigned)in_nch[mine] : 0u, sum);
+        const unsigned before = block_exclusive(
+            (int)threadIdx.x < size && mine < ni ? (unsigned)in_nch[mine] : 0u, sum);
         s_fc[threadIdx.x] = 1 + (int)(tile_off[tile] + before);
         __syncthreads();
-        for (int q = 0; q < TN_TILE; q += OT_THREADS / 8) {
+        for (int q = 0; q < size; q += TN_ROUND) {
             const int local = q + (int)(threadIdx.x >> 3);
-            const int ii = tile * TN_TILE + local;
+            const int ii = tile * size + local;
             const bool act = ii < ni;
             int2 sd = make_int2(0, 0);
             int end = 0;
@@ -883,7 +896,9 @@ ErrorStatus OctreeDevice::setup(int n_, int leaf_max_, bool compat_, bool quad_)
     GS_TRY(in_end.reserve((size_t)cap * 8 * sizeof(int)));
     GS_TRY(in_rec.reserve((size_t)cap * sizeof(int4)));
     GS_TRY(scan_tiles.reserve(
-        (size_t)(std::max((n + TC_TILE - 1) / TC_TILE, (cap + TN_TILE - 1) / TN_TILE) + 1) *
+        (size_t)(std::max(std::max((n + TC_TILE - 1) / TC_TILE, TN_MANY + TN_ROUNDS),
+                          cap / (TN_ROUND * TN_ROUNDS) + 1) +
+                 1) *
         sizeof(unsigned)));
     GS_TRY(t_mass.reserve((size_t)cap * sizeof(double)));
     GS_TRY(t_com.reserve((size_t)cap * 3 * sizeof(double)));

@@ -63,25 +63,23 @@ k_radix_hist(const uint64_t *__restrict__ keys, const int *__restrict__ d_n, int
     }
 }
 
-// hist[p][d] <- number of elements of pass p with a digit below d.
-__global__ void __launch_bounds__(256) k_radix_bases(unsigned *__restrict__ hist, int passes)
+// hist[p][d] <- number of elements of pass p with a digit below d; a block per
+// pass.
+__global__ void __launch_bounds__(256) k_radix_bases(unsigned *__restrict__ hist)
 {
     __shared__ unsigned wsum[8];
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    for (int p = 0; p < passes; ++p) {
-        const unsigned c = hist[p * 256 + t];
-        unsigned incl = c;
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned u = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += u;
-        }
-        if (lane == 31) wsum[warp] = incl;
-        __syncthreads();
-        unsigned before = 0;
-        for (int w = 0; w < warp; ++w) before += wsum[w];
-        hist[p * 256 + t] = before + incl - c;
-        __syncthreads();
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, p = blockIdx.x;
+    const unsigned c = hist[p * 256 + t];
+    unsigned incl = c;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
     }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    unsigned before = 0;
+    for (int w = 0; w < warp; ++w) before += wsum[w];
+    hist[p * 256 + t] = before + incl - c;
 }
 
 __device__ __forceinline__ unsigned long long ld_volatile(const unsigned long long *p)
@@ -291,7 +289,7 @@ ErrorStatus RadixSorter::sort(uint64_t *keys, int *vals, const int *d_n, int max
     GS_CUDA(cudaMemsetAsync(lookback_.p, 0,
                             (size_t)passes * tiles * 256 * sizeof(unsigned long long), s));
     k_radix_hist<<<std::min(tiles, sm_count_ * 4), RX_THREADS, 0, s>>>(keys, d_n, passes, hist);
-    k_radix_bases<<<1, 256, 0, s>>>(hist, passes);
+    k_radix_bases<<<passes, 256, 0, s>>>(hist);
     uint64_t *kin = keys, *kout = tmp_keys_.as<uint64_t>();
     int *vin = vals, *vout = tmp_vals_.as<int>();
     for (int p = 0; p < passes; ++p) {

@@ -130,12 +130,21 @@ struct GroupListArgs {
     int *gctr;
 };
 
-// Entries of particles [first, first + count), cut into pieces; written from
-// groups[at] on when at >= 0.  Returns their number.
-__device__ int put_groups(const GroupListArgs &A, int first, int count, int depth, int at)
+// The groups of one cell: pieces (first particle, count), the count negative
+// for particles that go to the list one by one.  A cell of more than GL_PIECES
+// pieces (oversized leaves) is cut again when they are written.
+constexpr int GL_PIECES = 16;
+struct CellGroups {
+    int pieces = 0, entries = 0;
+    int2 piece[GL_PIECES];
+};
+
+// Cuts particles [first, first + count) into pieces; writes them from
+// groups[at] on when at >= 0.
+__device__ __noinline__ void put_groups(const GroupListArgs &A, int first, int count, int depth, int at,
+                                        CellGroups &g)
 {
     const int nmis = A.mlist[0];
-    int entries = 0;
     for (int b = 0; b < count; b += GW_GROUP) {
         const int f = first + b, c = min(GW_GROUP, count - b);
         bool measure = nmis > kMisplacedCap;
@@ -143,37 +152,47 @@ __device__ int put_groups(const GroupListArgs &A, int first, int count, int dept
             const int q = A.mlist[1 + k];
             measure = q >= f && q < f + c;
         }
-        if (!measure || group_extent_fits(f, c, depth, A.pa, A.pb, A.frame[4])) {
-            if (at >= 0) A.groups[at + entries] = make_int2(f, c);
-            ++entries;
-        } else {
-            if (at >= 0)
-                for (int q = 0; q < c; ++q) A.groups[at + entries + q] = make_int2(f + q, 1);
-            entries += c;
+        const bool fits = !measure || group_extent_fits(f, c, depth, A.pa, A.pb, A.frame[4]);
+        if (at >= 0) {
+            if (fits)
+                A.groups[at + g.entries] = make_int2(f, c);
+            else
+                for (int q = 0; q < c; ++q) A.groups[at + g.entries + q] = make_int2(f + q, 1);
+        } else if (g.pieces < GL_PIECES) {
+            g.piece[g.pieces] = make_int2(f, fits ? c : -c);
         }
+        ++g.pieces;
+        g.entries += fits ? 1 : c;
     }
-    return entries;
 }
 
-// Groups of one cell, written from groups[at] on when at >= 0; returns their number.
-__device__ int cell_groups(const GroupListArgs &A, int cell, int at)
+// The groups of one cell, written from groups[at] on when at >= 0.
+__device__ void cell_groups(const GroupListArgs &A, int cell, int at, CellGroups &g)
 {
+    g.pieces = g.entries = 0;
     const int4 ci = A.nc[cell];
     // a smaller cell is grouped by its parent; a leaf (the root) is cut
-    if (ci.w <= GW_GROUP || ci.y <= 0)
-        return cell == 0 && ci.w > 0 ? put_groups(A, ci.z, ci.w, A.depth[cell], at) : 0;
+    if (ci.w <= GW_GROUP || ci.y <= 0) {
+        if (cell == 0 && ci.w > 0) put_groups(A, ci.z, ci.w, A.depth[cell], at, g);
+        return;
+    }
+    int4 child[8];   // all in flight together
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        child[k] = k < ci.y ? A.nc[ci.x + k] : make_int4(0, 1, 0, GW_GROUP + 1);
     // Runs of consecutive children of at most GW_GROUP particles each are
     // contiguous in sorted order and lie in this cell: each run is cut into
     // pieces of GW_GROUP particles (the last one shorter), so that groups
     // fill the warp's lanes (children of 20, 20 and 20 particles make groups
     // of 32 and 28, not three of 20).
-    int first = 0, count = 0, entries = 0;
-    for (int k = 0; k <= ci.y; ++k) {
-        const int4 ch = k < ci.y ? A.nc[ci.x + k] : make_int4(0, 1, 0, GW_GROUP + 1);
+    int first = 0, count = 0;
+#pragma unroll
+    for (int k = 0; k <= 8; ++k) {
+        const int4 ch = k < 8 ? child[k] : make_int4(0, 1, 0, GW_GROUP + 1);
         if (ch.w > GW_GROUP) {   // a child walked as its own cell, or the end
-            entries += put_groups(A, first, count, A.depth[cell], at < 0 ? -1 : at + entries);
+            if (count > 0) put_groups(A, first, count, A.depth[cell], at, g);
             if (ch.y <= 0)       // an oversized leaf (depth limit)
-                entries += put_groups(A, ch.z, ch.w, A.depth[ci.x + k], at < 0 ? -1 : at + entries);
+                put_groups(A, ch.z, ch.w, A.depth[ci.x + k], at, g);
             count = 0;
             continue;
         }
@@ -181,7 +200,6 @@ __device__ int cell_groups(const GroupListArgs &A, int cell, int at)
         if (count == 0) first = ch.z;
         count += ch.w;
     }
-    return entries;
 }
 
 constexpr int GL_THREADS = 256;
@@ -196,7 +214,9 @@ __global__ void __launch_bounds__(GL_THREADS) k_group_list(GroupListArgs A)
     for (int b = blockIdx.x * GL_THREADS; b < cells; b += gridDim.x * GL_THREADS) {   // block-uniform
         const int i = b + threadIdx.x;
         const int cell = i < internal ? A.in_rec[i].w : i == 0 ? 0 : -1;
-        const int entries = cell >= 0 ? cell_groups(A, cell, -1) : 0;
+        CellGroups g;
+        if (cell >= 0) cell_groups(A, cell, -1, g);
+        const int entries = g.entries;
         int incl = entries;
         for (int o = 1; o < 32; o <<= 1) {
             const int t = __shfl_up_sync(0xffffffffu, incl, o);
@@ -211,7 +231,16 @@ __global__ void __launch_bounds__(GL_THREADS) k_group_list(GroupListArgs A)
         }
         if (threadIdx.x == 0) s_base = total > 0 ? atomicAdd(&A.gctr[0], total) : 0;
         __syncthreads();
-        if (entries > 0) cell_groups(A, cell, s_base + before + incl - entries);
+        int at = s_base + before + incl - entries;
+        if (g.pieces > GL_PIECES) {
+            cell_groups(A, cell, at, g);
+        } else {
+            for (int k = 0; k < g.pieces; ++k) {
+                const int2 v = g.piece[k];
+                if (v.y > 0) A.groups[at++] = v;
+                for (int q = 0; q < -v.y; ++q) A.groups[at++] = make_int2(v.x + q, 1);
+            }
+        }
         __syncthreads();   // s_warp and s_base are read
     }
 }
