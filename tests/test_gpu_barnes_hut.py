@@ -157,6 +157,25 @@ def test_walk_vs_oracle(lib, g, orc, wl, compat, theta, leaf):
     check_terms(a, a_o, mag)
 
 
+@pytest.mark.parametrize("compat", [True, False])
+@pytest.mark.parametrize("n,theta,leaf", [(2, 0.5, 1), (31, 0.5, 1), (32, 0.5, 1), (33, 0.9, 2),
+                                          (65, 0.8, 3), (1000, 0.5, 40), (4097, 0.3, 1),
+                                          (62208, 0.7, 1), (62240, 0.7, 1)])
+def test_walk_edges_vs_oracle(lib, g, orc, wl, compat, n, theta, leaf):
+    """Warps that are not full, leaves longer than a warp, lists around their capacity, and both
+    forms of the walk (62,208 particles are 1,944 warps, the last count that a block each walks).
+    Every decision equals the oracle's."""
+    x, v, m = wl.plummer(n, n)
+    if n > 100:
+        x[60:64] = x[70]   # coincident particles
+    method = g.METHOD_GPU_BARNES_HUT_COMPAT if compat else g.METHOD_GPU_BARNES_HUT
+    a = g.acceleration(lib, x, m, 1.0, method, opening_angle=theta, softening_length=0.01,
+                       max_num_particles_per_leaf=leaf)
+    a_o, cnt, mag = orc.bh_counts(x, m, 1.0, 0.01, theta, leaf, compat)
+    assert gpu_counts(lib) == (int(cnt[:, 0].sum()), int(cnt[:, 1].sum()))
+    check_terms(a, a_o, mag)
+
+
 def test_reference_entry_point_acceleration_barnes_hut(lib, g, orc, wl):
     """acceleration_barnes_hut() with the reference's method code 3 runs the
     reference-compatible GPU walk."""
