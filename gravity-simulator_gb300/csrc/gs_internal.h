@@ -101,6 +101,18 @@ struct ForceTimer {
 // ---- force engines -----------------------------------------------------
 // One engine per (method, N); it owns its scratch memory.  compute() reads
 // FP64 positions and masses on the device and writes FP64 accelerations.
+// State of n bodies on the device, 3n values each, with its compensation terms.
+struct StepState {
+    double *x, *xe, *v, *ve;
+    int n;
+};
+
+// A kick v += a h at the end of a force kernel (none when v is null).
+struct Kick {
+    double *v, *ve;
+    double h;
+};
+
 class Engine {
   public:
     virtual ~Engine() {}
@@ -117,6 +129,12 @@ class Engine {
     }
     // kernels launched by one compute()
     virtual int kernels_per_eval() const = 0;
+    // One leapfrog step of h from the state after the half kick: x += v h, the
+    // accelerations at x, v += a h, each update compensated.  An engine that
+    // forms the same updates inside its own kernels saves their launches.
+    virtual ErrorStatus leapfrog(const StepState &q, const double *d_m, double *d_a, double h,
+                                 cudaStream_t s, ForceTimer *timer);
+    virtual int kernels_per_leapfrog() const { return kernels_per_eval() + 2; }
     // true when compute() never synchronises with the host (graph-capturable)
     virtual bool capturable() const { return true; }
     // device status word of the engine (may be null)

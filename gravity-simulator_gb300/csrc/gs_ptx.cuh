@@ -5,6 +5,8 @@
 
 #include <cstdint>
 
+#include "gs_internal.h"
+
 namespace gs {
 
 // Time limit of one bounded wait (ns of %globaltimer).
@@ -106,6 +108,19 @@ __device__ __forceinline__ void comp_update(double &y, double &err, double d, do
     err = __dadd_rn(err, __dmul_rn(d, dt));
     y = __dadd_rn(y0, err);
     err = __dadd_rn(err, __dsub_rn(y0, y));
+}
+
+// Element k of a force kernel's result: a[k], and the kick that follows it.
+__device__ __forceinline__ void store_and_kick(double *__restrict__ a, size_t k, double value,
+                                               const Kick &kick)
+{
+    a[k] = value;
+    if (kick.v) {
+        double v = kick.v[k], e = kick.ve[k];
+        comp_update(v, e, value, kick.h);
+        kick.v[k] = v;
+        kick.ve[k] = e;
+    }
 }
 
 }  // namespace gs

@@ -687,11 +687,12 @@ struct gsgpu_sim {
             GS_CUDA(cudaMemcpyAsync(a.p, vk[3], bytes3(), cudaMemcpyDeviceToDevice, stream));
             break;
         }
-        case INTEGRATOR_LEAPFROG:
-            launch_comp_update(x.as<double>(), xe.as<double>(), v.as<double>(), h, 1.0, L, stream);
-            GS_TRY(force(a.as<double>()));
-            launch_comp_update(v.as<double>(), ve.as<double>(), a.as<double>(), h, 1.0, L, stream);
+        case INTEGRATOR_LEAPFROG: {
+            const StepState q = {x.as<double>(), xe.as<double>(), v.as<double>(), ve.as<double>(), n};
+            GS_TRY(engine->leapfrog(q, m.as<double>(), a.as<double>(), h, stream,
+                                    timer.enabled ? &timer : nullptr));
             break;
+        }
         default:
             return GS_RAISE(GRAV_NOT_IMPLEMENTED_ERROR, "integrator %d is not built", integrator);
         }
@@ -708,7 +709,7 @@ struct gsgpu_sim {
         case INTEGRATOR_EULER: return f + 1;
         case INTEGRATOR_EULER_CROMER: return f + 2;
         case INTEGRATOR_RK4: return 4 * f + 4;
-        case INTEGRATOR_LEAPFROG: return f + 2;
+        case INTEGRATOR_LEAPFROG: return engine->kernels_per_leapfrog();
         default: return f;
         }
     }

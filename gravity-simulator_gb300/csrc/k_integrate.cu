@@ -29,6 +29,16 @@ __global__ void k_comp_update(double *__restrict__ y, double *__restrict__ err,
     err[k] = ee;
 }
 
+ErrorStatus Engine::leapfrog(const StepState &q, const double *d_m, double *d_a, double h,
+                             cudaStream_t s, ForceTimer *timer)
+{
+    launch_comp_update(q.x, q.xe, q.v, h, 1.0, 3 * q.n, s);
+    GS_TRY(compute(q.x, d_m, d_a, s, timer));
+    launch_comp_update(q.v, q.ve, d_a, h, 1.0, 3 * q.n, s);
+    GS_CUDA(cudaGetLastError());
+    return ok();
+}
+
 // Leapfrog initial half kick: err += (0.5 * a) * dt (src/integrator.c:978).
 __global__ void k_comp_update_scaled(double *__restrict__ y, double *__restrict__ err,
                                      const double *__restrict__ d, double coef, double dt,
