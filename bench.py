@@ -981,7 +981,8 @@ def run_cosmo(args, world, rank, local, wk, g, lib):
                                "particle-mesh code (tests/test_gpu_pm.py)"},
         "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak64.value,
                      "unit": "TFLOP/s", "frac": achieved / peak64.value, "traffic": None,
-                     "kernel": "whole step (4 kernels + 2 cuFFT transforms)",
+                     "kernel": f"whole step ({kps.value} kernels"
+                               f"{' + 2 cuFFT transforms' if kps.value == 4 else ''})",
                      "algorithmic_flop_per_step": flop_step,
                      "peak_source": "FP64 FMA probe on this GPU (gsgpu_measure_fma_peak), "
                                     "not in MEASURED_PEAKS.json"},

@@ -1,0 +1,21 @@
+// gs_fft.h -- FP64 convolution of a real periodic mesh (k_fft.cu).
+#pragma once
+
+#include "gs_internal.h"
+
+namespace gs {
+
+// Mesh sizes that convolve_mesh takes.
+bool convolve_supports(int g);
+
+// Twiddle factors exp(-2 pi i k / g), k < g, for convolve_mesh.
+ErrorStatus convolve_table(int g, double2 *tw, cudaStream_t s);
+
+// mesh [g^3] <- g^3 times its convolution with the kernel whose transform is
+// the real table[kx^2 + ky^2 + kz^2] (|k| at most g / 2 on each axis), in place.
+ErrorStatus convolve_mesh(double *mesh, int g, const double *table, const double2 *tw,
+                          cudaStream_t s);
+
+constexpr int kConvolveLaunches = 5;
+
+}  // namespace gs

@@ -144,16 +144,14 @@ ErrorStatus launch_cosmological_simulation(CosmologicalSystem *system, OutputPar
 
 // Device time (CUDA events on the run's stream) of the step loop of the
 // calling thread's last leapfrog_cosmology / launch_cosmological_simulation,
-// and its step count.  Kernels of this library per step: the mesh fill, the
-// particles, the Green's function and the gradient.
+// its step count and this library's kernels per step.
 int gsgpu_cosmology_last_timing(double *loop_ms, int64_t *steps, int *kernels_per_step)
 {
-    ErrorStatus st = gs::pm_last_timing(loop_ms, steps);
+    ErrorStatus st = gs::pm_last_timing(loop_ms, steps, kernels_per_step);
     if (st.return_code != GRAV_SUCCESS) {
         print_and_free_traceback(&st);
         return st.return_code;
     }
-    if (kernels_per_step) *kernels_per_step = 4;
     return 0;
 }
 

@@ -7,10 +7,10 @@
 //                  atomic adds per particle (the reference's OpenMP loop has
 //                  unsynchronised += here), which makes the mesh the density
 //                  contrast rho / (V_cell rho_mean) - 1;
-//   cuFFT D2Z      the r2c transform (FFTW's layout: g x g x (g/2+1));
-//   k_pm_green     multiply by -1/k^2 (0 at k = 0), from a table by the integer
-//                  |n|^2;
-//   cuFFT Z2D      the unnormalised c2r transform;
+//   the potential  the mesh convolved with -1/k^2 (0 at k = 0), from a table by
+//                  the integer |n|^2: for g = 32, 64, 128 and 256 in place by
+//                  k_fft.cu, otherwise cuFFT D2Z (FFTW's layout:
+//                  g x g x (g/2+1)), k_pm_green, and cuFFT Z2D, unnormalised;
 //   k_pm_gradient  fourth-order central differences of phi into the
 //                  acceleration mesh, without their constant factor;
 //   interpolation  cloud-in-cell, back to the particles; the caller's multiplier
@@ -28,12 +28,13 @@
 // constant factors folded into one multiplier, comparisons on the bits (an FP64
 // comparison costs as much as an add).  These round
 // differently from the reference's order by a few ulps, far below the
-// differences of the transforms (cuFFT against FFTW) and of the atomic
+// differences of the transforms (against FFTW's) and of the atomic
 // deposit order.  The file is compiled with --fmad=false; the fused
 // operations are the explicit fma() calls.
 //
-// Memory: delta / phi g^3 doubles, the spectrum g^2 (g/2+1) complex, the
-// acceleration mesh 3 g^3 doubles: 56 g^3 bytes, 940 MB at g = 256.
+// Memory: delta / phi g^3 doubles, the acceleration mesh 3 g^3 doubles: 32 g^3
+// bytes, 537 MB at g = 256; with cuFFT also the spectrum g^2 (g/2+1) complex.
+#include "gs_fft.h"
 #include "gs_fp64.cuh"
 #include "gs_internal.h"
 
@@ -412,12 +413,16 @@ class PmSolver {
         fwd_ = inv_ = 0;
         g_ = 0;
         const long long cells = (long long)g * g * g;
-        const long long half = (long long)g * g * (g / 2 + 1);
         GS_TRY(mesh_.reserve((size_t)cells * sizeof(double)));
-        GS_TRY(spec_.reserve((size_t)half * sizeof(double2)));
         GS_TRY(acc_.reserve((size_t)cells * 3 * sizeof(double)));
-        GS_CUFFT(cufftPlan3d(&fwd_, g, g, g, CUFFT_D2Z));
-        GS_CUFFT(cufftPlan3d(&inv_, g, g, g, CUFFT_Z2D));
+        if (convolve_supports(g)) {
+            GS_TRY(tw_.reserve((size_t)g * sizeof(double2)));
+        } else {
+            const long long half = (long long)g * g * (g / 2 + 1);
+            GS_TRY(spec_.reserve((size_t)half * sizeof(double2)));
+            GS_CUFFT(cufftPlan3d(&fwd_, g, g, g, CUFFT_D2Z));
+            GS_CUFFT(cufftPlan3d(&inv_, g, g, g, CUFFT_Z2D));
+        }
         g_ = g;
         return ok();
     }
@@ -441,6 +446,7 @@ class PmSolver {
         k_pm_green_table<<<blocks(len), TPB, 0, s>>>(green_.as<double>(), len,
                                                      4.0 * M_PI * M_PI / (box_length * box_length));
         GS_CUDA(cudaGetLastError());
+        if (convolve_supports(g)) GS_TRY(convolve_table(g, tw_.as<double2>(), s));
         return ok();
     }
 
@@ -479,18 +485,26 @@ class PmSolver {
     ErrorStatus solve(cudaStream_t s)
     {
         double *mesh = mesh_.as<double>();
-        GS_CUFFT(cufftSetStream(fwd_, s));
-        GS_CUFFT(cufftExecD2Z(fwd_, mesh, spec_.as<cufftDoubleComplex>()));
-        const long long half = (long long)g_ * g_ * (g_ / 2 + 1);
-        k_pm_green<<<blocks(half), TPB, 0, s>>>(spec_.as<double2>(), g_, green_.as<double>());
-        GS_CUDA(cudaGetLastError());
-        GS_CUFFT(cufftSetStream(inv_, s));
-        GS_CUFFT(cufftExecZ2D(inv_, spec_.as<cufftDoubleComplex>(), mesh));
+        if (convolve_supports(g_)) {
+            GS_TRY(convolve_mesh(mesh, g_, green_.as<double>(), tw_.as<double2>(), s));
+        } else {
+            GS_CUFFT(cufftSetStream(fwd_, s));
+            GS_CUFFT(cufftExecD2Z(fwd_, mesh, spec_.as<cufftDoubleComplex>()));
+            const long long half = (long long)g_ * g_ * (g_ / 2 + 1);
+            k_pm_green<<<blocks(half), TPB, 0, s>>>(spec_.as<double2>(), g_, green_.as<double>());
+            GS_CUDA(cudaGetLastError());
+            GS_CUFFT(cufftSetStream(inv_, s));
+            GS_CUFFT(cufftExecZ2D(inv_, spec_.as<cufftDoubleComplex>(), mesh));
+        }
         const long long cells = (long long)g_ * g_ * g_;
         k_pm_gradient<<<blocks(cells), TPB, 0, s>>>(mesh, g_, acc_.as<double>());
         GS_CUDA(cudaGetLastError());
         return ok();
     }
+
+    // Kernels of this library in a step: the fill, the particles, the potential and
+    // the gradient.
+    int kernels_per_step() const { return 3 + (convolve_supports(g_) ? kConvolveLaunches : 1); }
 
     // The gradient mesh's constant factor.
     double scale(double H0, double omega_m, double scale_factor) const
@@ -509,7 +523,7 @@ class PmSolver {
     double cell_length_ = 1.0;
     PmGeom geom_{};
     cufftHandle fwd_ = 0, inv_ = 0;
-    DBuf mesh_, spec_, acc_, green_, mn_, part_;
+    DBuf mesh_, spec_, acc_, green_, tw_, mn_, part_;
 };
 
 namespace {
@@ -703,11 +717,12 @@ ErrorStatus pm_leapfrog_cosmology(CosmologicalSystem *system, SimulationStatus *
     return ok();
 }
 
-ErrorStatus pm_last_timing(double *loop_ms, int64_t *steps)
+ErrorStatus pm_last_timing(double *loop_ms, int64_t *steps, int *kernels)
 {
     if (!tl_pm) return GS_RAISE(GRAV_VALUE_ERROR, "no cosmological run on this thread");
     if (loop_ms) *loop_ms = tl_pm->loop_ms;
     if (steps) *steps = tl_pm->loop_steps;
+    if (kernels) *kernels = tl_pm->solver.kernels_per_step();
     return ok();
 }
 

@@ -52,6 +52,41 @@ def test_acceleration_pm_oracle_g64(lib, g, orc):
     _close(a, a_ref)
 
 
+def mesh_reference(x, m, c, bw, H0, om, rho, grid, sf):
+    """The same quantity with numpy's transforms."""
+    cell = 2.0 * bw / grid
+    u = (x - c + bw) / cell
+    i0 = np.floor(u).astype(int)
+    idx, w = (i0 % grid, (i0 + 1) % grid), (1.0 - (u - i0), u - i0)
+    mesh, flat = np.zeros(grid ** 3), []
+    for e in np.ndindex(2, 2, 2):
+        q = (idx[e[0]][:, 0] * grid + idx[e[1]][:, 1]) * grid + idx[e[2]][:, 2]
+        flat.append((q, w[e[0]][:, 0] * w[e[1]][:, 1] * w[e[2]][:, 2]))
+        mesh += np.bincount(q, m * flat[-1][1], grid ** 3)
+    delta = (mesh / (cell ** 3 * rho) - 1.0).reshape(grid, grid, grid)
+    k = np.minimum(np.arange(grid), grid - np.arange(grid))
+    k2 = (k[:, None, None] ** 2 + k[:, None] ** 2 + k[:grid // 2 + 1] ** 2) * (np.pi / bw) ** 2
+    k2[0, 0, 0] = np.inf
+    phi = np.fft.irfftn(np.fft.rfftn(delta) / -k2, (grid,) * 3, (0, 1, 2)) * 1.5 * om * H0 ** 2 / sf
+    a = np.zeros_like(x)
+    for d in range(3):
+        gr = np.roll(phi, 2, d) - 8 * np.roll(phi, 1, d) + 8 * np.roll(phi, -1, d) - np.roll(phi, -2, d)
+        for q, ww in flat:
+            a[:, d] += (gr / (12.0 * cell)).reshape(-1)[q] * ww
+    return a
+
+
+@pytest.mark.parametrize("grid", [16, 31, 32, 64, 66, 128, 256])
+def test_acceleration_pm_mesh_sizes(lib, g, grid):
+    """Sizes of the mesh's own transforms (32, 64, 128, 256) and, around them, the library's."""
+    rng = np.random.default_rng(grid)
+    c, bw = np.array([1.0, -2.0, 3.0]), 7.0
+    x = c + np.clip(rng.standard_normal((20000, 3)) * 2.0, -0.999 * bw, 0.999 * bw)
+    m = rng.uniform(0.5, 1.5, len(x))
+    args = (c, bw, 70.0, 0.3, m.sum() / (2 * bw) ** 3, grid, 0.25)
+    _close(g.acceleration_pm(lib, x, m, *args), mesh_reference(x, m, *args))
+
+
 def test_acceleration_pm_momentum_and_determinism(lib, g):
     """Size-independent properties at 128^3 and 2M particles: the mesh force
     of a periodic box sums to zero (Newton's third law on the mesh, to the
