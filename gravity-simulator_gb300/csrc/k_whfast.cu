@@ -1133,7 +1133,7 @@ struct gsgpu_ensemble {
     int sort_tpb[kSortClasses] = {0, 0, 0};
     bool tuned = false;
     // WHFast of at most one small system per SM: k_wh_small, a batch of steps per
-    // launch (16 us a step for the Sun and eight planets, 119 us by the launches
+    // launch (19 us a step for the Sun and eight planets, 119 us by the launches
     // below).  With more systems the FP64 pipes are full and the dense lanes of the
     // per-particle kernels win.  Set by upload, which sees the masses.
     bool small = false;

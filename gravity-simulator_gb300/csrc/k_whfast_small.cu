@@ -17,7 +17,7 @@
 //     reciprocals formed when the order of the bodies changes;
 //   * interaction: a lane per pair distance, per quotient and per ordered sum.
 // Every value is formed by the operations, and every sum in the order, of
-// k_whfast.cu, so the results are the same bit for bit.  16 us a step for the Sun
+// k_whfast.cu, so the results are the same bit for bit.  19 us a step for the Sun
 // and eight planets.
 #include "gs_fp64.cuh"
 #include "gs_internal.h"

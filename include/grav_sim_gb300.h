@@ -451,8 +451,9 @@ int gsgpu_sim_set_learned_policy(gsgpu_sim *sim, int policy);
  * control -- and the run -- equal the reference's bit for bit; 1 adds them on
  * the device in a fixed grouping and copies one double back (no 6N-double copy
  * and host loop per attempt; the sum's rounding differs from the reference's
- * in the last bits, so accepted steps and step sizes may differ slightly).
- * GRAV_VALUE_ERROR for other modes. */
+ * in the last bits, so accepted steps and step sizes may differ slightly; a
+ * system of a few dozen bodies, whose attempt is one launch, keeps the order
+ * of mode 0).  GRAV_VALUE_ERROR for other modes. */
 int gsgpu_set_rk_error_sum(int mode);
 /* Learned method: copy up to `count` training samples of one snapshot
  * (features [count][32], targets [count][3]); returns the number copied. */
