@@ -1,5 +1,6 @@
 // k_fft.cu -- FP64 convolution of a real g^3 mesh with a real, even kernel given
-// by its transform, for g = 32, 64, 128 and 256 (the particle-mesh potential).
+// by its transform, for even g of small prime factors from 32 to 256 (the
+// particle-mesh potential).
 //
 // The mesh is read as g x g x g/2 complex numbers, two neighbours on the last
 // axis in one: C = E + i O with E the even and O the odd planes.  Transforms
@@ -14,13 +15,16 @@
 // A line of N = R1 R2 points, n = c + R2 r, k = q + R1 s (Cooley and Tukey, 1965):
 // R2 threads each transform R1 points over r in registers, multiply by
 // exp(-2 pi i c q / N), exchange through shared memory, and transform R2 points
-// over c.  The inverse of the last axis takes the same steps backwards, so its
+// over c (for R1 > R2 several times, and where R2 does not divide R1 with idle
+// threads).  The inverse of the last axis takes the same steps backwards, so its
 // input is where the forward transform left it.
 //
 // Bound: the FP64 pipe (an FP64 warp instruction holds its SM sub-partition for
 // 64 cycles): at g = 128, 1.38e8 operations, 221 us.  The library's transforms
 // took 490 us there and the multiplication 8; these five launches take 312 (51 for
-// each pass of lines, 108 for the pairs).  Accelerations differ from an extended
+// each pass of lines, 108 for the pairs).  A step with 24^3 particles, before and
+// now: g = 32 104 and 60 us, 48 104 and 72, 60 145 and 86, 96 297 and 173, 160 1311
+// and 867, 256 4195 and 2729.  Accelerations differ from an extended
 // precision computation by as much with either (1e-14 at g = 32 to 256).
 #include "gs_fft.h"
 
@@ -30,6 +34,11 @@ namespace {
 constexpr double kSqrtHalf = 0.70710678118654752440;   // cos(pi / 4)
 constexpr double kCos8 = 0.92387953251128675613;       // cos(pi / 8)
 constexpr double kSin8 = 0.38268343236508977173;       // sin(pi / 8)
+constexpr double kSin3 = 0.86602540378443864676;       // sin(2 pi / 3)
+constexpr double kCos5 = 0.30901699437494742410;       // cos(2 pi / 5)
+constexpr double kSin5 = 0.95105651629515357212;       // sin(2 pi / 5)
+constexpr double kCos25 = -0.80901699437494742410;     // cos(4 pi / 5)
+constexpr double kSin25 = 0.58778525229247312917;      // sin(4 pi / 5)
 
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
@@ -60,6 +69,94 @@ __device__ __forceinline__ double2 eighth(double2 a)
 // In place, natural order: v[k] <- sum_n v[n] exp(-+ 2 pi i n k / R).
 template <int R, bool INV>
 struct Dft;
+
+template <bool INV>
+struct Dft<2, INV> {
+    static __device__ __forceinline__ void run(double2 *v)
+    {
+        const double2 a = v[0];
+        v[0] = cadd(a, v[1]);
+        v[1] = csub(a, v[1]);
+    }
+};
+
+template <bool INV>
+struct Dft<3, INV> {
+    static __device__ __forceinline__ void run(double2 *v)
+    {
+        const double2 a = cadd(v[1], v[2]), d = quarter<INV>(csub(v[1], v[2]));
+        const double2 p = make_double2(fma(-0.5, a.x, v[0].x), fma(-0.5, a.y, v[0].y));
+        v[0] = cadd(v[0], a);
+        v[1] = make_double2(fma(kSin3, d.x, p.x), fma(kSin3, d.y, p.y));
+        v[2] = make_double2(fma(-kSin3, d.x, p.x), fma(-kSin3, d.y, p.y));
+    }
+};
+
+template <bool INV>
+struct Dft<5, INV> {
+    static __device__ __forceinline__ void run(double2 *v)
+    {
+        const double2 a = cadd(v[1], v[4]), b = cadd(v[2], v[3]);
+        const double2 c = quarter<INV>(csub(v[1], v[4])), d = quarter<INV>(csub(v[2], v[3]));
+        const double2 p = make_double2(fma(kCos5, a.x, fma(kCos25, b.x, v[0].x)),
+                                       fma(kCos5, a.y, fma(kCos25, b.y, v[0].y)));
+        const double2 q = make_double2(fma(kCos25, a.x, fma(kCos5, b.x, v[0].x)),
+                                       fma(kCos25, a.y, fma(kCos5, b.y, v[0].y)));
+        const double2 r = make_double2(fma(kSin5, c.x, kSin25 * d.x), fma(kSin5, c.y, kSin25 * d.y));
+        const double2 t = make_double2(fma(kSin25, c.x, -(kSin5 * d.x)), fma(kSin25, c.y, -(kSin5 * d.y)));
+        v[0] = cadd(v[0], cadd(a, b));
+        v[1] = cadd(p, r);
+        v[4] = csub(p, r);
+        v[2] = cadd(q, t);
+        v[3] = csub(q, t);
+    }
+};
+
+// R = A B with A and B coprime, without twiddle factors (Good, 1958): with
+// n = B n1 + A n2 mod R and k the number that is k1 mod A and k2 mod B.
+template <int A, int B, bool INV>
+struct Coprime {
+    static constexpr int R = A * B;
+    static constexpr int index(int k1, int k2)
+    {
+        int k = 0;
+        while (k % A != k1 || k % B != k2) ++k;
+        return k;
+    }
+    template <int K1, int K2>
+    static __device__ __forceinline__ void place(double2 *v, const double2 (&t)[A][B])
+    {
+        constexpr int k = index(K1, K2);
+        v[k] = t[K1][K2];
+        if constexpr (K2 + 1 < B)
+            place<K1, K2 + 1>(v, t);
+        else if constexpr (K1 + 1 < A)
+            place<K1 + 1, 0>(v, t);
+    }
+    static __device__ __forceinline__ void run(double2 *v)
+    {
+        double2 t[A][B];
+#pragma unroll
+        for (int n2 = 0; n2 < B; ++n2) {
+            double2 u[A];
+#pragma unroll
+            for (int n1 = 0; n1 < A; ++n1) u[n1] = v[(B * n1 + A * n2) % R];
+            Dft<A, INV>::run(u);
+#pragma unroll
+            for (int k1 = 0; k1 < A; ++k1) t[k1][n2] = u[k1];
+        }
+#pragma unroll
+        for (int k1 = 0; k1 < A; ++k1) Dft<B, INV>::run(t[k1]);
+        place<0, 0>(v, t);
+    }
+};
+
+template <bool INV>
+struct Dft<6, INV> : Coprime<2, 3, INV> {};
+template <bool INV>
+struct Dft<10, INV> : Coprime<2, 5, INV> {};
+template <bool INV>
+struct Dft<12, INV> : Coprime<4, 3, INV> {};
 
 template <bool INV>
 struct Dft<4, INV> {
@@ -119,28 +216,24 @@ struct Dft<16, INV> {
     }
 };
 
-// N = R1 R2 with R2 <= R1 <= 2 R2
+// N = R1 R2.  Where R2 does not divide R1, threads are idle in the second step;
+// the order of the factors is the one with fewer operations in all.
+constexpr int first_radix(int n)
+{
+    switch (n) {
+    case 16: return 4;
+    case 20: return 5;
+    case 24: case 30: case 36: case 48: return 6;
+    case 32: case 40: case 64: return 8;
+    case 50: case 60: case 80: case 100: return 10;
+    case 72: case 96: case 120: case 144: return 12;
+    default: return 16;   // 128, 160, 192, 256
+    }
+}
 template <int N>
-struct Split;
-template <>
-struct Split<16> {
-    static constexpr int R1 = 4, R2 = 4;
-};
-template <>
-struct Split<32> {
-    static constexpr int R1 = 8, R2 = 4;
-};
-template <>
-struct Split<64> {
-    static constexpr int R1 = 8, R2 = 8;
-};
-template <>
-struct Split<128> {
-    static constexpr int R1 = 16, R2 = 8;
-};
-template <>
-struct Split<256> {
-    static constexpr int R1 = 16, R2 = 16;
+struct Split {
+    static constexpr int R1 = first_radix(N), R2 = N / R1;
+    static_assert(R1 * R2 == N, "two radices");
 };
 
 // Lines along one of the first two axes.  A CTA takes LINES neighbouring lines
@@ -153,15 +246,17 @@ __global__ void __launch_bounds__(LINES *Split<N>::R2)
 k_fft_lines(double2 *__restrict__ data, unsigned lines_per_slab, size_t outer, unsigned stride,
             const double2 *__restrict__ tw)
 {
-    constexpr int R1 = Split<N>::R1, R2 = Split<N>::R2, M = R1 / R2;
+    constexpr int R1 = Split<N>::R1, R2 = Split<N>::R2, M = (R1 + R2 - 1) / R2;
     __shared__ double2 s[N * LINES];
-    const unsigned tiles = lines_per_slab / LINES;
+    const unsigned tiles = (lines_per_slab + LINES - 1) / LINES;
     const unsigned slab = blockIdx.x / tiles, tile = blockIdx.x - slab * tiles;
     const int line = threadIdx.x % LINES, t = threadIdx.x / LINES;
+    const bool live = tile * LINES + line < lines_per_slab;
     double2 *base = data + (size_t)slab * outer + tile * LINES + line;
     double2 v[R1];
 #pragma unroll
-    for (int r = 0; r < R1; ++r) v[r] = base[(size_t)(t + R2 * r) * stride];
+    for (int r = 0; r < R1; ++r)
+        v[r] = live ? base[(size_t)(t + R2 * r) * stride] : make_double2(0.0, 0.0);
     Dft<R1, INV>::run(v);
 #pragma unroll
     for (int q = 0; q < R1; ++q) {
@@ -172,12 +267,15 @@ k_fft_lines(double2 *__restrict__ data, unsigned lines_per_slab, size_t outer, u
 #pragma unroll
     for (int u = 0; u < M; ++u) {
         const int q = t + R2 * u;
+        if (R1 % R2 != 0 && q >= R1) break;
         double2 w[R2];
 #pragma unroll
         for (int c = 0; c < R2; ++c) w[c] = s[(c * R1 + q) * LINES + line];
         Dft<R2, INV>::run(w);
+        if (live) {
 #pragma unroll
-        for (int k = 0; k < R2; ++k) base[(size_t)(q + R1 * k) * stride] = w[k];
+            for (int k = 0; k < R2; ++k) base[(size_t)(q + R1 * k) * stride] = w[k];
+        }
     }
 }
 
@@ -196,7 +294,8 @@ __device__ __forceinline__ double2 swapped(double2 a, bool swap)
 // the even lane on P and E, the odd lane on Q and O.
 template <int G>
 struct PairShape {
-    static constexpr int H = G / 2, R1 = Split<H>::R1, R2 = Split<H>::R2, M = R1 / R2;
+    static constexpr int H = G / 2, R1 = Split<H>::R1, R2 = Split<H>::R2;
+    static constexpr int M = (R1 + R2 - 1) / R2;
     static constexpr int PER = 2 * R2;              // threads of a pair
     static constexpr int PAIRS = 128 / PER;         // pairs of a CTA
     static constexpr int ROW = R2 + 1;              // padded row of the exchange
@@ -214,7 +313,8 @@ k_fft_pairs(double2 *__restrict__ data, const double *__restrict__ table,
     __shared__ double2 s[S::PAIRS * 2 * R1 * S::ROW];
     const int odd = threadIdx.x & 1, t = (threadIdx.x % S::PER) >> 1, local = threadIdx.x / S::PER;
     const unsigned pair = blockIdx.x * S::PAIRS + local;
-    const bool live = pair < S::COUNT;
+    const bool held = local < S::PAIRS;   // the block's last threads may have no pair
+    const bool live = held && pair < S::COUNT;
     unsigned i = 0, j = 0;
     if (live) {
         constexpr unsigned kWhole = (unsigned)(H - 1) * G;
@@ -230,7 +330,7 @@ k_fft_pairs(double2 *__restrict__ data, const double *__restrict__ table,
     const unsigned ni = (G - i) % G, nj = (G - j) % G;
     const bool self = ni == i && nj == j;
     double2 *line = data + (size_t)(odd ? ni * G + nj : i * G + j) * H;
-    double2 *ex = s + (local * 2 + odd) * R1 * S::ROW;
+    double2 *ex = s + (min(local, S::PAIRS - 1) * 2 + odd) * R1 * S::ROW;
     // E and O from the two lines
     double2 v[R1];
 #pragma unroll
@@ -243,7 +343,7 @@ k_fft_pairs(double2 *__restrict__ data, const double *__restrict__ table,
 #pragma unroll
     for (int q = 0; q < R1; ++q) {
         if (q > 0) v[q] = cmul<false>(v[q], __ldg(tw + 2 * t * q));
-        ex[q * S::ROW + t] = v[q];
+        if (held) ex[q * S::ROW + t] = v[q];
     }
     __syncthreads();
     // modes m (even lane) and m + H (odd lane): F = E + w O, E - w O
@@ -253,7 +353,7 @@ k_fft_pairs(double2 *__restrict__ data, const double *__restrict__ table,
     double2 w[M][R2];
 #pragma unroll
     for (int u = 0; u < M; ++u) {
-        const int q = t + R2 * u;
+        const int q = min(t + R2 * u, R1 - 1);   // threads without one repeat the last
 #pragma unroll
         for (int c = 0; c < R2; ++c) w[u][c] = ex[q * S::ROW + c];
         Dft<R2, false>::run(w[u]);
@@ -277,11 +377,11 @@ k_fft_pairs(double2 *__restrict__ data, const double *__restrict__ table,
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < M; ++u) {
-        const int q = t + R2 * u;
+        const int q = min(t + R2 * u, R1 - 1);
 #pragma unroll
         for (int c = 0; c < R2; ++c) {
             if (c > 0) w[u][c] = cmul<true>(w[u][c], __ldg(tw + 2 * c * q));
-            ex[q * S::ROW + c] = w[u][c];
+            if (held && t + R2 * u < R1) ex[q * S::ROW + c] = w[u][c];
         }
     }
     __syncthreads();
@@ -312,20 +412,44 @@ void convolve(double2 *data, const double *table, const double2 *tw, cudaStream_
 {
     constexpr unsigned H = G / 2;
     constexpr int threads = LINES * Split<G>::R2;
-    constexpr unsigned grid = G * H / LINES;
+    constexpr unsigned slabs = G * ((H + LINES - 1) / LINES), planes = (G * H + LINES - 1) / LINES;
     using S = PairShape<G>;
-    k_fft_lines<G, false><<<grid, threads, 0, s>>>(data, H, (size_t)G * H, H, tw);
-    k_fft_lines<G, false><<<grid, threads, 0, s>>>(data, G * H, 0, G * H, tw);
+    k_fft_lines<G, false><<<slabs, threads, 0, s>>>(data, H, (size_t)G * H, H, tw);
+    k_fft_lines<G, false><<<planes, threads, 0, s>>>(data, G * H, 0, G * H, tw);
     k_fft_pairs<G><<<(S::COUNT + S::PAIRS - 1) / S::PAIRS, 128, 0, s>>>(data, table, tw);
-    k_fft_lines<G, true><<<grid, threads, 0, s>>>(data, G * H, 0, G * H, tw);
-    k_fft_lines<G, true><<<grid, threads, 0, s>>>(data, H, (size_t)G * H, H, tw);
+    k_fft_lines<G, true><<<planes, threads, 0, s>>>(data, G * H, 0, G * H, tw);
+    k_fft_lines<G, true><<<slabs, threads, 0, s>>>(data, H, (size_t)G * H, H, tw);
 }
 
 }  // namespace
 
-// Powers of two with two radix steps of at most 16 per axis; other sizes go to the
-// library's transforms.
-bool convolve_supports(int g) { return g == 32 || g == 64 || g == 128 || g == 256; }
+using Convolve = void (*)(double2 *, const double *, const double2 *, cudaStream_t);
+
+// Even sizes of small prime factors whose lines and half lines have two factors
+// of at most 16; other sizes go to the library's transforms.
+static Convolve convolve_for(int g)
+{
+    switch (g) {
+    case 32: return convolve<32>;
+    case 40: return convolve<40>;
+    case 48: return convolve<48>;
+    case 60: return convolve<60>;
+    case 64: return convolve<64>;
+    case 72: return convolve<72>;
+    case 80: return convolve<80>;
+    case 96: return convolve<96>;
+    case 100: return convolve<100>;
+    case 120: return convolve<120>;
+    case 128: return convolve<128>;
+    case 144: return convolve<144>;
+    case 160: return convolve<160>;
+    case 192: return convolve<192>;
+    case 256: return convolve<256>;
+    default: return nullptr;
+    }
+}
+
+bool convolve_supports(int g) { return convolve_for(g) != nullptr; }
 
 ErrorStatus convolve_table(int g, double2 *tw, cudaStream_t s)
 {
@@ -337,14 +461,9 @@ ErrorStatus convolve_table(int g, double2 *tw, cudaStream_t s)
 ErrorStatus convolve_mesh(double *mesh, int g, const double *table, const double2 *tw,
                           cudaStream_t s)
 {
-    double2 *data = reinterpret_cast<double2 *>(mesh);
-    switch (g) {
-    case 32: convolve<32>(data, table, tw, s); break;
-    case 64: convolve<64>(data, table, tw, s); break;
-    case 128: convolve<128>(data, table, tw, s); break;
-    case 256: convolve<256>(data, table, tw, s); break;
-    default: return GS_RAISE(GRAV_VALUE_ERROR, "no convolution of a mesh of %d cells a side", g);
-    }
+    const Convolve run = convolve_for(g);
+    if (!run) return GS_RAISE(GRAV_VALUE_ERROR, "no convolution of a mesh of %d cells a side", g);
+    run(reinterpret_cast<double2 *>(mesh), table, tw, s);
     GS_CUDA(cudaGetLastError());
     return ok();
 }

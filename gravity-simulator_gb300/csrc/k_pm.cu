@@ -8,8 +8,8 @@
 //                  unsynchronised += here), which makes the mesh the density
 //                  contrast rho / (V_cell rho_mean) - 1;
 //   the potential  the mesh convolved with -1/k^2 (0 at k = 0), from a table by
-//                  the integer |n|^2: for g = 32, 64, 128 and 256 in place by
-//                  k_fft.cu, otherwise cuFFT D2Z (FFTW's layout:
+//                  the integer |n|^2: for the sizes of k_fft.cu (even, of small
+//                  factors, 32 to 256) in place, otherwise cuFFT D2Z (FFTW's layout:
 //                  g x g x (g/2+1)), k_pm_green, and cuFFT Z2D, unnormalised;
 //   k_pm_gradient  fourth-order central differences of phi into the
 //                  acceleration mesh, without their constant factor;

@@ -76,9 +76,10 @@ def mesh_reference(x, m, c, bw, H0, om, rho, grid, sf):
     return a
 
 
-@pytest.mark.parametrize("grid", [16, 31, 32, 64, 66, 128, 256])
+@pytest.mark.parametrize("grid", [16, 31, 32, 40, 48, 60, 64, 66, 72, 75, 80, 96, 100, 120, 128, 144,
+                                  160, 192, 256])
 def test_acceleration_pm_mesh_sizes(lib, g, grid):
-    """Sizes of the mesh's own transforms (32, 64, 128, 256) and, around them, the library's."""
+    """Every size of the own transforms and, around them, the library's (16, 31, 66, 75)."""
     rng = np.random.default_rng(grid)
     c, bw = np.array([1.0, -2.0, 3.0]), 7.0
     x = c + np.clip(rng.standard_normal((20000, 3)) * 2.0, -0.999 * bw, 0.999 * bw)
