@@ -19,7 +19,10 @@
 // evaluations (k_pm_particles): interpolation, the kick that ends a step, the kick
 // and the drift that begin the next, the periodic wrap, and the deposit at the
 // new positions.  As five kernels these took 463 us a step at 128^3 particles, with
-// the accelerations and momenta written and read in between; fused, 409 us.
+// the accelerations and momenta written and read in between; fused, 409 us; with
+// the cells and fractions of the deposit kept for the interpolation at the same
+// positions, and the two kicks in one, 336 us (80 FP64 operations a particle, 98
+// before).
 // Every kernel computes the reference's quantity in FP64.  The FP64 pipe of
 // this GPU runs at 1/64 of the FP32 rate and bounds the particle kernels, so
 // they use algebraically equal forms with fewer FP64 operations than the
@@ -119,6 +122,36 @@ __device__ __forceinline__ void cic_cell(const double xi[3], const PmGeom &G, in
     }
 }
 
+// Cells and fractions of every particle at its last deposit, which are those of
+// the interpolation that follows at the same positions: 15 of its 54 FP64
+// operations for 32 bytes a particle (null: not kept).
+struct CicKept {
+    double *w;       // 3n: the weight of the upper cell on each axis
+    ushort4 *cell;   // n: the lower cell (a mesh has at most 1,290 cells a side)
+};
+
+__device__ __forceinline__ void keep_cic(const CicKept &K, int i, const int idx[2][3],
+                                         const double w[2][3])
+{
+#pragma unroll
+    for (int d = 0; d < 3; ++d) K.w[3 * (size_t)i + d] = w[1][d];
+    K.cell[i] = make_ushort4(idx[0][0], idx[0][1], idx[0][2], 0);
+}
+
+__device__ __forceinline__ void kept_cic(const CicKept &K, int i, int g, int idx[2][3], double w[2][3])
+{
+    const ushort4 c = K.cell[i];
+    idx[0][0] = c.x;
+    idx[0][1] = c.y;
+    idx[0][2] = c.z;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        w[1][d] = K.w[3 * (size_t)i + d];
+        w[0][d] = 1.0 - w[1][d];
+        idx[1][d] = idx[0][d] + 1 < g ? idx[0][d] + 1 : 0;
+    }
+}
+
 // Corner order of the reference's eight terms: bit 0 x, bit 1 y, bit 2 z
 // (a constant in unrolled loops, so the per-corner arrays stay in registers).
 __host__ __device__ constexpr int corner_bits(int c)
@@ -127,11 +160,12 @@ __host__ __device__ constexpr int corner_bits(int c)
 }
 
 __device__ __forceinline__ void deposit_one(const double xi[3], double mi, const PmGeom &G,
-                                            double *__restrict__ delta)
+                                            double *__restrict__ delta, const CicKept &K, int i)
 {
     int idx[2][3];
     double w[2][3];
     cic_cell(xi, G, idx, w);
+    if (K.w) keep_cic(K, i, idx, w);
     const long long g = G.g, g2 = g * g;
     double mx[2], mxy[2][2];
 #pragma unroll
@@ -150,12 +184,9 @@ __device__ __forceinline__ void deposit_one(const double xi[3], double mi, const
 }
 
 // src/acceleration_PM.c:112-210, in units of the gradient mesh
-__device__ __forceinline__ void interp_one(const double xi[3], const PmGeom &G,
+__device__ __forceinline__ void interp_one(const int idx[2][3], const double w[2][3], const PmGeom &G,
                                            const double *__restrict__ acc, double s[3])
 {
-    int idx[2][3];
-    double w[2][3];
-    cic_cell(xi, G, idx, w);
     const long long g = G.g, g2 = g * g;
     double wxy[2][2];
 #pragma unroll
@@ -186,12 +217,12 @@ __global__ void k_pm_fill(double *__restrict__ mesh, long long cells, double val
 }
 
 __global__ void k_pm_deposit(const double *__restrict__ x, const double *__restrict__ mn, int n,
-                             PmGeom G, double *__restrict__ delta)
+                             PmGeom G, double *__restrict__ delta, CicKept K)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double xi[3] = {x[3 * (size_t)i], x[3 * (size_t)i + 1], x[3 * (size_t)i + 2]};
-    deposit_one(xi, mn[i], G, delta);
+    deposit_one(xi, mn[i], G, delta, K, i);
 }
 
 // -1 / (|n|^2 (2 pi / L)^2) by the integer |n|^2 of a mode (src/acceleration_PM.c:
@@ -259,7 +290,10 @@ __global__ void k_pm_interp(const double *__restrict__ x, int n, PmGeom G,
     if (i >= n) return;
     const double xi[3] = {x[3 * (size_t)i], x[3 * (size_t)i + 1], x[3 * (size_t)i + 2]};
     double s[3];
-    interp_one(xi, G, acc, s);
+    int idx[2][3];
+    double w[2][3];
+    cic_cell(xi, G, idx, w);
+    interp_one(idx, w, G, acc, s);
 #pragma unroll
     for (int d = 0; d < 3; ++d) a[3 * (size_t)i + d] = s[d] * scale;
 }
@@ -359,39 +393,42 @@ __global__ void k_cosmo_velocity(double *__restrict__ v, const double *__restric
 // gradient mesh (GATHER) or read from `a`, the kick that ends a step,
 // p -= k1 a (:176-183), and with MOVE the kick and the drift that begin the next,
 // p -= k2 a (:142-149), x += c p (:152-160), wrapped (:163), and its deposit.
+// Both kicks have the same accelerations and are one, p -= (k1 + k2) a.
 // k1 and k2 carry 0.5 dt / da and the acceleration's constant factor,
 // c = dt / (a^2 da).  Without MOVE the accelerations are kept in `a`.
 template <bool GATHER, bool MOVE>
 __global__ void k_pm_particles(double *__restrict__ x, double *__restrict__ p,
                                const double *__restrict__ mn, double *__restrict__ a, int n,
                                PmGeom G, const double *__restrict__ acc, double k1, double k2,
-                               double c, double bw, double *__restrict__ delta)
+                               double c, double bw, double *__restrict__ delta, CicKept K)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const size_t q = 3 * (size_t)i;
-    double xi[3] = {x[q], x[q + 1], x[q + 2]};
     double s[3];
     if (GATHER) {
-        interp_one(xi, G, acc, s);
+        int idx[2][3];
+        double w[2][3];
+        kept_cic(K, i, G.g, idx, w);
+        interp_one(idx, w, G, acc, s);
     } else {
         for (int d = 0; d < 3; ++d) s[d] = a[q + d];
     }
     const double centre[3] = {G.cx, G.cy, G.cz};
+    const double kick = -((GATHER ? k1 : 0.0) + (MOVE ? k2 : 0.0));
+    double xi[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        double pd = p[q + d];
-        if (GATHER) pd = fma(-k1, s[d], pd);
+        const double pd = fma(kick, s[d], p[q + d]);
         if (MOVE) {
-            pd = fma(-k2, s[d], pd);
-            xi[d] = periodic(fma(c, pd, xi[d]), centre[d], bw);
+            xi[d] = periodic(fma(c, pd, x[q + d]), centre[d], bw);
             x[q + d] = xi[d];
         } else {
             a[q + d] = s[d];
         }
         p[q + d] = pd;
     }
-    if (MOVE) deposit_one(xi, mn[i], G, delta);
+    if (MOVE) deposit_one(xi, mn[i], G, delta, K, i);
 }
 
 }  // namespace
@@ -595,7 +632,7 @@ ErrorStatus pm_acceleration_host(double *a, int n, const double *x, const double
     GS_TRY(pm.scale_masses(c->m.as<double>(), n, box_width, true, mean_bkg_density, c->stream));
     GS_TRY(pm.clear(c->stream));
     k_pm_deposit<<<blocks(n), TPB, 0, c->stream>>>(c->x.as<double>(), pm.masses(), n, pm.geom(),
-                                                   pm.mesh());
+                                                   pm.mesh(), CicKept{nullptr, nullptr});
     GS_CUDA(cudaGetLastError());
     GS_TRY(pm.solve(c->stream));
     k_pm_interp<<<blocks(n), TPB, 0, c->stream>>>(c->x.as<double>(), n, pm.geom(), pm.acc(),
@@ -625,10 +662,13 @@ ErrorStatus pm_leapfrog_cosmology(CosmologicalSystem *system, SimulationStatus *
     cudaStream_t s = pc->stream;
     const int L = 3 * n;
     const size_t b3 = (size_t)L * sizeof(double);
-    DBuf x, v, m, p, a;
+    DBuf x, v, m, p, a, w, cell;
     GS_TRY(x.reserve(b3));
     GS_TRY(v.reserve(b3));
     GS_TRY(p.reserve(b3));
+    GS_TRY(w.reserve(b3));
+    GS_TRY(cell.reserve((size_t)n * sizeof(ushort4)));
+    const CicKept kept = {w.as<double>(), cell.as<ushort4>()};
     GS_TRY(a.reserve(b3));
     GS_TRY(m.reserve((size_t)n * sizeof(double)));
     GS_CUDA(cudaMemcpyAsync(x.p, system->x, b3, cudaMemcpyHostToDevice, s));
@@ -648,7 +688,7 @@ ErrorStatus pm_leapfrog_cosmology(CosmologicalSystem *system, SimulationStatus *
     k_cosmo_momentum<<<blocks(L), TPB, 0, s>>>(p.as<double>(), v.as<double>(), L, t);
     GS_CUDA(cudaGetLastError());
     GS_TRY(pm.clear(s));
-    k_pm_deposit<<<blocks(n), TPB, 0, s>>>(x.as<double>(), pm.masses(), n, pm.geom(), pm.mesh());
+    k_pm_deposit<<<blocks(n), TPB, 0, s>>>(x.as<double>(), pm.masses(), n, pm.geom(), pm.mesh(), kept);
     GS_CUDA(cudaGetLastError());
     GS_TRY(pm.solve(s));
     double factor = pm.scale(H0, omega_m, t);   // of the accelerations now in the mesh
@@ -673,7 +713,7 @@ ErrorStatus pm_leapfrog_cosmology(CosmologicalSystem *system, SimulationStatus *
         auto move = gather ? k_pm_particles<true, true> : k_pm_particles<false, true>;
         move<<<blocks(n), TPB, 0, s>>>(x.as<double>(), p.as<double>(), pm.masses(), a.as<double>(),
                                        n, pm.geom(), pm.acc(), k1, k2, dt / (t * t * da), bw,
-                                       pm.mesh());
+                                       pm.mesh(), kept);
         GS_CUDA(cudaGetLastError());
         GS_TRY(pm.solve(s));
         factor = pm.scale(H0, omega_m, t);
@@ -692,7 +732,7 @@ ErrorStatus pm_leapfrog_cosmology(CosmologicalSystem *system, SimulationStatus *
             // accelerations
             k_pm_particles<true, false><<<blocks(n), TPB, 0, s>>>(
                 x.as<double>(), p.as<double>(), pm.masses(), a.as<double>(), n, pm.geom(), pm.acc(),
-                k1, 0.0, 0.0, bw, pm.mesh());
+                k1, 0.0, 0.0, bw, pm.mesh(), kept);
             GS_CUDA(cudaGetLastError());
         }
         if (snap) {
