@@ -21,7 +21,7 @@
 //
 // Bound: the FP64 pipe (an FP64 warp instruction holds its SM sub-partition for
 // 64 cycles): at g = 128, 1.38e8 operations, 221 us.  The library's transforms
-// took 490 us there and the multiplication 8; these five launches take 312 (51 for
+// took 490 us there and the multiplication 8; these five launches take 292 (46 for
 // each pass of lines, 108 for the pairs).  A step with 24^3 particles, before and
 // now: g = 32 104 and 60 us, 48 104 and 72, 60 145 and 86, 96 297 and 173, 160 1311
 // and 867, 256 4195 and 2729.  Accelerations differ from an extended
@@ -236,17 +236,25 @@ struct Split {
     static_assert(R1 * R2 == N, "two radices");
 };
 
+// Lines of 128 points take 8 x 16: twice as many threads of half the work fill the
+// sub-partitions more evenly (46 us a pass instead of 51 at g = 128).  The second
+// step then needs half the threads; neighbouring blocks take different halves.
+template <int N>
+struct LineSplit {
+    static constexpr int R1 = N == 128 ? 8 : Split<N>::R1, R2 = N / R1;
+};
+
 // Lines along one of the first two axes.  A CTA takes LINES neighbouring lines
 // (128-byte rows) of one slab; line l of slab o starts at o outer + l, its points
 // are `stride` apart.  tw: exp(-2 pi i k / N).
 constexpr int LINES = 8;
 
 template <int N, bool INV>
-__global__ void __launch_bounds__(LINES *Split<N>::R2)
+__global__ void __launch_bounds__(LINES *LineSplit<N>::R2)
 k_fft_lines(double2 *__restrict__ data, unsigned lines_per_slab, size_t outer, unsigned stride,
             const double2 *__restrict__ tw)
 {
-    constexpr int R1 = Split<N>::R1, R2 = Split<N>::R2, M = (R1 + R2 - 1) / R2;
+    constexpr int R1 = LineSplit<N>::R1, R2 = LineSplit<N>::R2, M = (R1 + R2 - 1) / R2;
     __shared__ double2 s[N * LINES];
     const unsigned tiles = (lines_per_slab + LINES - 1) / LINES;
     const unsigned slab = blockIdx.x / tiles, tile = blockIdx.x - slab * tiles;
@@ -266,7 +274,7 @@ k_fft_lines(double2 *__restrict__ data, unsigned lines_per_slab, size_t outer, u
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < M; ++u) {
-        const int q = t + R2 * u;
+        const int q = (R1 < R2 ? (t + (blockIdx.x & 1) * R1) % R2 : t) + R2 * u;
         if (R1 % R2 != 0 && q >= R1) break;
         double2 w[R2];
 #pragma unroll
@@ -411,7 +419,7 @@ template <int G>
 void convolve(double2 *data, const double *table, const double2 *tw, cudaStream_t s)
 {
     constexpr unsigned H = G / 2;
-    constexpr int threads = LINES * Split<G>::R2;
+    constexpr int threads = LINES * LineSplit<G>::R2;
     constexpr unsigned slabs = G * ((H + LINES - 1) / LINES), planes = (G * H + LINES - 1) / LINES;
     using S = PairShape<G>;
     k_fft_lines<G, false><<<slabs, threads, 0, s>>>(data, H, (size_t)G * H, H, tw);
