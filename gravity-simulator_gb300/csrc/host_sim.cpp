@@ -174,7 +174,7 @@ struct gsgpu_sim {
     // which sees the masses).  One CTA forms 128 pairs at a time, so a force costs
     // it about as many rounds of them, and the pairwise force by launches does not
     // grow below 48 bodies.  Microseconds in one block against by launches: a
-    // leapfrog step 5.5 and 8.8 (9 bodies), 7.8 and 9.0 (23), 11.0 and 9.1 (24, a
+    // leapfrog step 4.1 and 8.8 (9 bodies), 7.8 and 9.0 (23), 11.0 and 9.1 (24, a
     // third round); a Runge-Kutta run of 300 days 19,100 and 20,700 (32 bodies, 496
     // pairs), 27,100 and 22,800 (40); IAS15, a dozen forces a step in one launch, 94
     // and 120 thousand (40 bodies, 780 pairs), 140 and 122 thousand (48).  The

@@ -21,13 +21,24 @@ constexpr int TY_THREADS = 128;   // a warp per SM sub-partition
 constexpr int TY_L = 3 * kTinyMax;
 constexpr int TY_PAIRS = kTinyMax * (kTinyMax - 1) / 2;
 
-// Force state: t (x_i - x_j) of every interacting pair, and the lists of the
+constexpr int TY_FEW = TY_THREADS / 3;   // pairs with a thread per component
+
+// Force state: t (x_i - x_j) of every interacting pair, or, of at most TY_FEW
+// pairs, its products with the masses (of the first body, negated, and of the
+// second; of a light body's pair with the heavy one's), and the lists of the
 // massless variant.
 struct TinyForce {
-    double tr[TY_PAIRS][3];
+    union {
+        double tr[TY_PAIRS][3];
+        struct {
+            double pr[2][TY_FEW][3];
+            int i[TY_FEW], j[TY_FEW], mi[TY_FEW];   // bodies of a pair, index of its first mass
+        } few;
+    };
     double m[kTinyMax];
     int heavy[kTinyMax], light[kTinyMax];
     int nh, nl;
+    bool is_few;
 };
 
 __device__ void tiny_lists(TinyForce &f, const double *__restrict__ m, int n, bool massless)
@@ -44,17 +55,77 @@ __device__ void tiny_lists(TinyForce &f, const double *__restrict__ m, int n, bo
         }
         f.nh = nh;
         f.nl = nl;
+        f.is_few = nh * (nh - 1) / 2 + nl * nh <= TY_FEW && 3 * n <= TY_THREADS;
     }
     __syncthreads();
+    const int nh = f.nh, np = nh * (nh - 1) / 2;
+    const int e = threadIdx.x;
+    if (f.is_few && e < np + f.nl * nh) {
+        if (e < np) {
+            int q = 1;
+            while ((q + 1) * q / 2 <= e) ++q;
+            f.few.i[e] = f.few.mi[e] = f.heavy[e - q * (q - 1) / 2];
+            f.few.j[e] = f.heavy[q];
+        } else {
+            f.few.i[e] = f.heavy[(e - np) % nh];
+            f.few.mi[e] = (e - np) % nh;
+            f.few.j[e] = f.light[(e - np) / nh];
+        }
+    }
+    __syncthreads();
+}
+
+// t (x_i - x_j) of a pair, t = G / (|x_i - x_j|^2 + eps^2)^(3/2).
+__device__ __forceinline__ void tiny_pair(const double *x, int i, int j, double G, double eps2, double r[3],
+                                          double &t)
+{
+#pragma unroll
+    for (int c = 0; c < 3; ++c) r[c] = __dsub_rn(x[3 * i + c], x[3 * j + c]);
+    const double rn = __dsqrt_rn(__dadd_rn(
+        __dadd_rn(__dadd_rn(__dmul_rn(r[0], r[0]), __dmul_rn(r[1], r[1])), __dmul_rn(r[2], r[2])), eps2));
+    t = __ddiv_rn(G, __dmul_rn(__dmul_rn(rn, rn), rn));
 }
 
 // Accelerations at x (shared, 3 n) into a (shared): src/acceleration.c:177-234,
 // and :236-367 when massless bodies are listed apart (weighted by the mass at the
 // loop index, as there).  Entered and left in step.
+//
+// What bounds it is the chain of FP64 operations (65 cycles each).  With at most
+// TY_FEW pairs a thread per pair and component forms the component's two products
+// with the masses, so that the ordered sums are additions alone (IAS15 step of the
+// Sun and eight planets 280 -> 235 us together with the kept quotients below,
+// leapfrog step 5.5 -> 4.1).
 __device__ void tiny_force(TinyForce &f, const double *x, double *a, double G, double eps2)
 {
     const int nh = f.nh, nl = f.nl;
     const int np = nh * (nh - 1) / 2;
+    if (f.is_few) {
+        const int e = threadIdx.x / 3, c = threadIdx.x % 3;
+        if (e < np + nl * nh) {
+            double r[3], t;
+            tiny_pair(x, f.few.i[e], f.few.j[e], G, eps2, r, t);
+            const double tr = __dmul_rn(t, c == 0 ? r[0] : c == 1 ? r[1] : r[2]);
+            const double mi = f.m[f.few.mi[e]];
+            f.few.pr[0][e][c] = __dmul_rn(e < np ? -tr : tr, mi);
+            if (e < np) f.few.pr[1][e][c] = __dmul_rn(tr, f.m[f.few.j[e]]);
+        }
+        __syncthreads();
+        if (threadIdx.x < 3 * (nh + nl)) {
+            const int b = e;
+            double acc = 0.0;
+            if (b < nh) {
+                for (int q = 0; q < b; ++q) acc = __dsub_rn(acc, f.few.pr[0][b * (b - 1) / 2 + q][c]);
+                for (int q = b + 1; q < nh; ++q) acc = __dsub_rn(acc, f.few.pr[1][q * (q - 1) / 2 + b][c]);
+                a[3 * f.heavy[b] + c] = acc;
+            } else {
+                const int first = np + (b - nh) * nh;
+                for (int p = 0; p < nh; ++p) acc = __dadd_rn(acc, f.few.pr[0][first + p][c]);
+                a[3 * f.light[b - nh] + c] = acc;
+            }
+        }
+        __syncthreads();
+        return;
+    }
     // pair (p, q), p < q in list order, at q (q - 1) / 2 + p, then (light l, heavy p)
     for (int e = threadIdx.x; e < np + nl * nh; e += TY_THREADS) {
         int i, j;
@@ -67,14 +138,10 @@ __device__ void tiny_force(TinyForce &f, const double *x, double *a, double G, d
             i = f.heavy[(e - np) % nh];
             j = f.light[(e - np) / nh];
         }
-        const double r0 = __dsub_rn(x[3 * i], x[3 * j]), r1 = __dsub_rn(x[3 * i + 1], x[3 * j + 1]),
-                     r2 = __dsub_rn(x[3 * i + 2], x[3 * j + 2]);
-        const double rn = __dsqrt_rn(__dadd_rn(
-            __dadd_rn(__dadd_rn(__dmul_rn(r0, r0), __dmul_rn(r1, r1)), __dmul_rn(r2, r2)), eps2));
-        const double t = __ddiv_rn(G, __dmul_rn(__dmul_rn(rn, rn), rn));
-        f.tr[e][0] = __dmul_rn(t, r0);
-        f.tr[e][1] = __dmul_rn(t, r1);
-        f.tr[e][2] = __dmul_rn(t, r2);
+        double r[3], t;
+        tiny_pair(x, i, j, G, eps2, r, t);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) f.tr[e][c] = __dmul_rn(t, r[c]);
     }
     __syncthreads();
     for (int e = threadIdx.x; e < 3 * (nh + nl); e += TY_THREADS) {
@@ -362,16 +429,19 @@ k_tiny_ias15(TinySystem S, TinyIas I, bool accept, bool refine, bool step, doubl
     }
     if (!step) return;
     tiny_lists(w.f, S.m, S.n, S.massless);
+    // The predictor's quotients, b_r over its divisor (b_6 times the spacing): kept
+    // up to date where b or the spacing changes, beside other work, instead of all
+    // formed again at every spacing (650 of 6,800 cycles).
+    for (int e = t; e < 7 * L; e += TY_THREADS) {
+        const int r = e / L, k = e % L;
+        w.q[r][k] = quotient(s_px[r], r == 6 ? __dmul_rn(I.spacing[0], w.b[6][k]) : w.b[r][k]);
+    }
+    __syncthreads();
     for (int it = 0; it < 12; ++it) {
         for (int i = 0; i < 8; ++i) {
             // predictor at spacing hi (:808-919); the velocities are not needed,
             // the force depends on positions alone
-            const double hi = I.spacing[i];
-            for (int e = t; e < 7 * L; e += TY_THREADS) {
-                const int r = e / L, k = e % L;
-                w.q[r][k] = quotient(s_px[r], r == 6 ? __dmul_rn(hi, w.b[6][k]) : w.b[r][k]);
-            }
-            __syncthreads();
+            const double hi = I.spacing[i], next = I.spacing[(i + 1) & 7];
             const double dth = __dmul_rn(h, hi);
             bool same = it > 0 && i == 0;
             for (int k = t; k < L; k += TY_THREADS) {
@@ -389,7 +459,11 @@ k_tiny_ias15(TinySystem S, TinyIas I, bool accept, bool refine, bool step, doubl
             }
             if (i == 0) {
                 // spacing 0: the same positions in every iteration
-                if (!__syncthreads_and(same)) tiny_force(w.f, w.x1, w.f0, S.G, eps2);
+                const bool again = __syncthreads_and(same);
+                for (int k = t; k < L; k += TY_THREADS)
+                    w.q[6][k] = quotient(s_px[6], __dmul_rn(next, w.b[6][k]));
+                if (!again) tiny_force(w.f, w.x1, w.f0, S.G, eps2);
+                __syncthreads();
                 continue;
             }
             __syncthreads();
@@ -402,21 +476,25 @@ k_tiny_ias15(TinySystem S, TinyIas I, bool accept, bool refine, bool step, doubl
                 w.g[i - 1][k] = q;
             }
             __syncthreads();
-            // b from g (:985-1115)
-            for (int e = t; e < i * L; e += TY_THREADS) {
-                const int r = e / L, k = e % L;
-                double q = __dmul_rn(I.c[r][r], w.g[r][k]);
-                for (int j = r + 1; j < 7; ++j) q = __dadd_rn(q, __dmul_rn(I.c[j][r], w.g[j][k]));
-                w.b[r][k] = q;
+            // b from g (:985-1115), and the quotients at the next spacing
+            for (int e = t; e < min(i + 1, 7) * L; e += TY_THREADS) {
+                const int r = e < i * L ? e / L : 6, k = e % L;
+                double q = w.b[r][k];
+                if (e < i * L) {
+                    q = __dmul_rn(I.c[r][r], w.g[r][k]);
+                    for (int j = r + 1; j < 7; ++j) q = __dadd_rn(q, __dmul_rn(I.c[j][r], w.g[j][k]));
+                    w.b[r][k] = q;
+                }
+                w.q[r][k] = quotient(s_px[r], r == 6 ? __dmul_rn(next, q) : q);
             }
             __syncthreads();
         }
         for (int k = t; k < L; k += TY_THREADS) {
-            w.q[0][k] = __dsub_rn(w.b[6][k], w.b6_old[k]);
+            w.q[13][k] = __dsub_rn(w.b[6][k], w.b6_old[k]);
             w.b6_old[k] = w.b[6][k];
         }
         __syncthreads();
-        tiny_absmax(w, w.q[0], w.fi, L);
+        tiny_absmax(w, w.q[13], w.fi, L);
         const double ratio = __ddiv_rn(__longlong_as_double((long long)w.top[0]),
                                        __longlong_as_double((long long)w.top[1]));
         if (ratio < 1e-16) break;   // CTA-uniform
