@@ -93,7 +93,8 @@ __device__ __forceinline__ void tiny_pair(const double *x, int i, int j, double 
 // What bounds it is the chain of FP64 operations (65 cycles each).  With at most
 // TY_FEW pairs a thread per pair and component forms the component's two products
 // with the masses, so that the ordered sums are additions alone (IAS15 step of the
-// Sun and eight planets 280 -> 235 us together with the kept quotients below,
+// Sun and eight planets 280 -> 235 us together with the kept quotients below, 225 with
+// the kept products of b,
 // leapfrog step 5.5 -> 4.1).
 __device__ void tiny_force(TinyForce &f, const double *x, double *a, double G, double eps2)
 {
@@ -333,6 +334,7 @@ struct IasShared {
     double x[TY_L], v[TY_L], a[TY_L], xe[TY_L], ve[TY_L], x1[TY_L], x1_first[TY_L];
     double f0[TY_L], fi[TY_L], b6_old[TY_L];
     double b[7][TY_L], g[7][TY_L], q[14][TY_L];
+    double cg[28][TY_L];   // c_jr g_j, j >= r, at j (j + 1) / 2 + r
     unsigned long long top[2];
 };
 
@@ -436,6 +438,14 @@ k_tiny_ias15(TinySystem S, TinyIas I, bool accept, bool refine, bool step, doubl
         const int r = e / L, k = e % L;
         w.q[r][k] = quotient(s_px[r], r == 6 ? __dmul_rn(I.spacing[0], w.b[6][k]) : w.b[r][k]);
     }
+    // Products of b = sum_j c_jr g_j: at a spacing only g_{i-1} changes, so one of
+    // the seven is formed and the chain of b is additions.
+    for (int e = t; e < 28 * L; e += TY_THREADS) {
+        const int row = e / L, k = e % L;
+        int j = 0;
+        while ((j + 1) * (j + 2) / 2 <= row) ++j;
+        w.cg[row][k] = __dmul_rn(I.c[j][row - j * (j + 1) / 2], w.g[j][k]);
+    }
     __syncthreads();
     for (int it = 0; it < 12; ++it) {
         for (int i = 0; i < 8; ++i) {
@@ -481,8 +491,12 @@ k_tiny_ias15(TinySystem S, TinyIas I, bool accept, bool refine, bool step, doubl
                 const int r = e < i * L ? e / L : 6, k = e % L;
                 double q = w.b[r][k];
                 if (e < i * L) {
-                    q = __dmul_rn(I.c[r][r], w.g[r][k]);
-                    for (int j = r + 1; j < 7; ++j) q = __dadd_rn(q, __dmul_rn(I.c[j][r], w.g[j][k]));
+                    const int j0 = i - 1;   // r <= j0
+                    const double fresh = __dmul_rn(I.c[j0][r], w.g[j0][k]);
+                    w.cg[j0 * (j0 + 1) / 2 + r][k] = fresh;
+                    q = r == j0 ? fresh : w.cg[r * (r + 1) / 2 + r][k];
+                    for (int j = r + 1; j < 7; ++j)
+                        q = __dadd_rn(q, j == j0 ? fresh : w.cg[j * (j + 1) / 2 + r][k]);
                     w.b[r][k] = q;
                 }
                 w.q[r][k] = quotient(s_px[r], r == 6 ? __dmul_rn(next, q) : q);
