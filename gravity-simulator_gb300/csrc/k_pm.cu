@@ -662,14 +662,13 @@ ErrorStatus pm_leapfrog_cosmology(CosmologicalSystem *system, SimulationStatus *
     cudaStream_t s = pc->stream;
     const int L = 3 * n;
     const size_t b3 = (size_t)L * sizeof(double);
-    DBuf x, v, m, p, a, w, cell;
+    DBuf x, v, m, p, a;
     GS_TRY(x.reserve(b3));
     GS_TRY(v.reserve(b3));
     GS_TRY(p.reserve(b3));
-    GS_TRY(w.reserve(b3));
-    GS_TRY(cell.reserve((size_t)n * sizeof(ushort4)));
-    const CicKept kept = {w.as<double>(), cell.as<ushort4>()};
-    GS_TRY(a.reserve(b3));
+    // the kept cells and fractions in the accelerations' allocation
+    GS_TRY(a.reserve(2 * b3 + (size_t)n * sizeof(ushort4)));
+    const CicKept kept = {a.as<double>() + L, reinterpret_cast<ushort4 *>(a.as<double>() + 2 * (size_t)L)};
     GS_TRY(m.reserve((size_t)n * sizeof(double)));
     GS_CUDA(cudaMemcpyAsync(x.p, system->x, b3, cudaMemcpyHostToDevice, s));
     GS_CUDA(cudaMemcpyAsync(v.p, system->v, b3, cudaMemcpyHostToDevice, s));
