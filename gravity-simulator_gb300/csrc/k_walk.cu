@@ -101,6 +101,7 @@ struct WalkShared {
     float4 sC[WK_LIST / 2];      // (x, x', y, y')    lo
     float2 sZ[WK_LIST / 2];      // (z, z')
     uint2 sM[WK_LIST / 2];       // lanes
+    // negated quadrupole (xx, xx', xy, xy'), (xz, xz', yy, yy'), (yz, yz', zz, zz'); 0 for a particle
     float4 qA[QUAD ? WK_LIST / 2 : 1], qB[QUAD ? WK_LIST / 2 : 1], qC[QUAD ? WK_LIST / 2 : 1];
     float4 a[32], b[32];         // nodes to test lane by lane: com (hi, mass), (lo, cell side^2)
     int4 c[32];                  // (node, -, first particle, particles)
@@ -140,13 +141,13 @@ __device__ __forceinline__ void put_entry(WalkShared<QUAD, COMPAT> &w, int at, c
     put(w.sC, at, 1, l.y);
     reinterpret_cast<float *>(w.sZ)[at] = l.z;
     reinterpret_cast<unsigned *>(w.sM)[at] = lanes;
-    if (QUAD) {
-        put(w.qA, at, 0, q0.x);
-        put(w.qA, at, 1, q0.y);
-        put(w.qB, at, 0, q0.z);
-        put(w.qB, at, 1, q0.w);
-        put(w.qC, at, 0, q1.x);
-        put(w.qC, at, 1, q1.y);
+    if (QUAD) {   // negated, as the evaluation expects
+        put(w.qA, at, 0, -q0.x);
+        put(w.qA, at, 1, -q0.y);
+        put(w.qB, at, 0, -q0.z);
+        put(w.qB, at, 1, -q0.w);
+        put(w.qC, at, 0, -q1.x);
+        put(w.qC, at, 1, -q1.y);
     }
 }
 
@@ -197,22 +198,25 @@ __device__ __forceinline__ void eval_list(WalkShared<QUAD, COMPAT> &w, int count
                                           lanes.y & bit[k] ? rsqrt_approx(r2.y) : 0.0f);
             const float2 ri2 = __fmul2_rn(ri, ri);
             const float2 ri3 = __fmul2_rn(ri2, ri);
-            float2 sc = __fmul2_rn(wk_hi2(vB), ri3);
-            float2 p[3];
+            float2 sc, p[3];
             if (QUAD) {
-                // d = com - x = -R:  G [-Q d / r^5 + 2.5 (d.Q.d) d / r^7]
+                // d = com - x = -R, P = -Q:  G [m d / r^3 + P d / r^5 - 2.5 (d.P.d) d / r^7], as
+                // r^-3 [d (m - 2.5 (d.t) r^-2) + t] with t = P d / r^2.  t is at most m s^2 / r
+                // for a cell of extent s, so no term leaves the range before m r^-3 does (r^-7
+                // is infinite below 3e-6, r^-5 below 2e-8, and a particle's P = 0 then gives
+                // NaN; above 3e6 r^-7 is 0).  The same number of operations.
                 const float2 xx = wk_lo2(qa), xy = wk_hi2(qa), xz = wk_lo2(qb);
                 const float2 yy = wk_hi2(qb), yz = wk_lo2(qc), zz = wk_hi2(qc);
-                const float2 qx = __ffma2_rn(xx, dx, __ffma2_rn(xy, dy, __fmul2_rn(xz, dz)));
-                const float2 qy = __ffma2_rn(xy, dx, __ffma2_rn(yy, dy, __fmul2_rn(yz, dz)));
-                const float2 qz = __ffma2_rn(xz, dx, __ffma2_rn(yz, dy, __fmul2_rn(zz, dz)));
-                const float2 dqd = __ffma2_rn(dx, qx, __ffma2_rn(dy, qy, __fmul2_rn(dz, qz)));
-                const float2 ri5 = __fmul2_rn(ri3, ri2), nri5 = __fmul2_rn(ri5, minus);
-                sc = __ffma2_rn(wk_splat(2.5f), __fmul2_rn(dqd, __fmul2_rn(ri5, ri2)), sc);
-                p[0] = __ffma2_rn(qx, nri5, __fmul2_rn(dx, sc));
-                p[1] = __ffma2_rn(qy, nri5, __fmul2_rn(dy, sc));
-                p[2] = __ffma2_rn(qz, nri5, __fmul2_rn(dz, sc));
+                const float2 tx = __fmul2_rn(__ffma2_rn(xx, dx, __ffma2_rn(xy, dy, __fmul2_rn(xz, dz))), ri2);
+                const float2 ty = __fmul2_rn(__ffma2_rn(xy, dx, __ffma2_rn(yy, dy, __fmul2_rn(yz, dz))), ri2);
+                const float2 tz = __fmul2_rn(__ffma2_rn(xz, dx, __ffma2_rn(yz, dy, __fmul2_rn(zz, dz))), ri2);
+                const float2 dt = __ffma2_rn(dx, tx, __ffma2_rn(dy, ty, __fmul2_rn(dz, tz)));
+                sc = __fmul2_rn(__ffma2_rn(wk_splat(-2.5f), __fmul2_rn(dt, ri2), wk_hi2(vB)), ri3);
+                p[0] = __ffma2_rn(tx, ri3, __fmul2_rn(dx, sc));
+                p[1] = __ffma2_rn(ty, ri3, __fmul2_rn(dy, sc));
+                p[2] = __ffma2_rn(tz, ri3, __fmul2_rn(dz, sc));
             } else {
+                sc = __fmul2_rn(wk_hi2(vB), ri3);
                 p[0] = __fmul2_rn(dx, sc);
                 p[1] = __fmul2_rn(dy, sc);
                 p[2] = __fmul2_rn(dz, sc);

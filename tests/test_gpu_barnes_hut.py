@@ -452,3 +452,25 @@ def test_width_division_matches_ddiv(lib):
     for seed in (1, 2):
         assert lib.gsgpu_width_division_selftest(1 << 26, seed, ctypes.byref(bad)) == 0
         assert bad.value == 0
+
+
+@pytest.mark.parametrize("method", [103, 105])
+@pytest.mark.parametrize("case", ["pair", 1e-7, 1.0, 1e6, 1e8])
+def test_walk_at_close_pairs_and_scales(lib, g, orc, wl, method, case):
+    """Distances far from one, unsoftened: two particles 1e-7 apart among 1,000 others, and a
+    galaxy pair scaled as a whole.  No power of the distance in a term may leave the FP32 range
+    before m / r^3 does; the bounds are those of the walk at any scale."""
+    if case == "pair":
+        x, v, m = wl.plummer(1002, 6)
+        x[501] = x[500] + np.array([6e-8, -8e-8, 0.0])
+    else:
+        x, v, m = wl.galaxy_pair(4096, 17)
+        x = x * case
+    a = g.acceleration(lib, x, m, 1.0, method, opening_angle=0.5, softening_length=0.0,
+                       max_num_particles_per_leaf=1)
+    assert np.isfinite(a).all()
+    if method == 105:
+        a_o, mag, _ = orc.bh_quad(x, m, 1.0, 0.0, 0.5, 1)
+    else:
+        a_o, _, mag = orc.bh_counts(x, m, 1.0, 0.0, 0.5, 1, False)
+    check_terms(a, a_o, mag)
