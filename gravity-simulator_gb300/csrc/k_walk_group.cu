@@ -253,6 +253,7 @@ struct GroupWalkArgs {
     const float4 *pa;       // sorted particles (x_hi, m)
     const float4 *pb;       // (x_lo, 0)
     const int *sidx;
+    const double *frame;    // cx, cy, cz, width, box_length
     float eps2;
     float theta2;
     double G;
@@ -276,8 +277,11 @@ struct GroupShared {
     float4 qB[GW_CELLS / 2];   // (xz, xz', yy, yy')
     float4 qC[GW_CELLS / 2];   // (yz, yz', zz, zz')
     float4 pA[16], pB[16];     // a tile of leaf particles, in the same way
-    float4 oh, ol;             // origin: the group's first particle (double-float)
-    float4 lo, hi;             // the group's box from it
+    float4 oh, ol;             // origin: the group's first particle (double-float);
+                               // oh.w: -unit^2, ol.w: 1 / unit
+    float4 nol;                // ol times -unit
+    float4 lo, hi;             // the group's box from it, times unit (length_unit); lo.w: unit,
+                               // hi.w: theta^2 / unit^2
     float sum[6 * GW_ROWS][32];   // (sum, error) of x, y, z of every lane's particles
     int parts[GW_PARTS + 32];  // particles of opened leaves (sorted positions)
 };
@@ -301,14 +305,29 @@ __device__ __forceinline__ float2 splat(float v) { return make_float2(v, v); }
 // A lane's particles.  Lane l holds the particles l % GW_COLS + k GW_COLS
 // (k < GW_ROWS) of the group and takes the pairs of a list that are
 // l / GW_COLS modulo GW_ROWS, so one shared load serves GW_ROWS particles.
-struct LaneRows {
+struct LaneRows {   // times unit
     float rx[GW_ROWS], ry[GW_ROWS], rz[GW_ROWS];
 };
 
-// Adds a list's partial sums to the compensated sums.
+// With quadrupoles the lengths of a group's walk are times this power of two, which
+// makes the box about 2^10 long: accepted cells are then 2^-11 to 2^12 away at an
+// angle of 1, and r^-5 stays in the middle of the FP32 range whatever the units of the
+// positions (as they come it is infinite below 2e-8 and subnormal above 3e7).  The
+// scaling is exact, and fused multiply-adds take it along without an instruction.
+// Terms of particles, which go to shorter distances and have no power beyond r^-3,
+// are in the units of the positions.
+template <bool QUAD>
+__device__ __forceinline__ float length_unit(double box_length)
+{
+    if (!QUAD) return 1.0f;
+    const int e = ((__double2hiint(box_length) >> 20) & 0x7ff) - 1023;
+    return __int_as_float((127 + max(-50, min(50, 10 - e))) << 23);
+}
+
+// Adds a list's partial sums, whose lengths were times unit, to the compensated sums.
 template <int K>
 __device__ __forceinline__ void add_sums(GroupShared &g, int lane, const float2 *ax, const float2 *ay,
-                                         const float2 *az)
+                                         const float2 *az, float unit2)
 {
 #pragma unroll
     for (int k = 0; k < K; ++k) {
@@ -316,7 +335,7 @@ __device__ __forceinline__ void add_sums(GroupShared &g, int lane, const float2 
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             float s = g.sum[6 * k + 2 * d][lane], c = g.sum[6 * k + 2 * d + 1][lane];
-            kahan_add(s, c, v[d].x + v[d].y);
+            kahan_add(s, c, (v[d].x + v[d].y) * unit2);
             g.sum[6 * k + 2 * d][lane] = s;
             g.sum[6 * k + 2 * d + 1][lane] = c;
         }
@@ -326,13 +345,15 @@ __device__ __forceinline__ void add_sums(GroupShared &g, int lane, const float2 
 // Evaluates the accepted cells for the first K particles of every lane.  The
 // list is filled up to whole turns of the lanes with copies of its last cell
 // without mass or quadrupole, which add zero.  With P = -Q and d = com - x:
-//     a = d [m / r^3 - 2.5 (d.P.d) / r^7] + P d / r^5
-// (the monopole plus G [-Q d / r^5 + 2.5 (d.Q.d) d / r^7], G applied last).
+//     a = d [m / r^3 - 2.5 ((d.P.d) / r^2) / r^5] + P d / r^5
+// (the monopole plus G [-Q d / r^5 + 2.5 (d.Q.d) d / r^7], G applied last; r^-7 by
+// itself would leave the FP32 range).
 template <bool QUAD, int K>
 __device__ __forceinline__ void eval_cells(GroupShared &g, int count, int lane, float eps2,
                                            const LaneRows &L)
 {
-    const float2 e2 = splat(eps2);
+    const float unit2 = -g.oh.w;
+    const float2 e2 = splat(eps2 * unit2);
     float2 ax[K], ay[K], az[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) ax[k] = ay[k] = az[k] = splat(0.f);
@@ -364,7 +385,7 @@ __device__ __forceinline__ void eval_cells(GroupShared &g, int count, int lane, 
                 const float2 pz = __ffma2_rn(xz, dx, __ffma2_rn(yz, dy, __fmul2_rn(zz, dz)));
                 const float2 dpd = __ffma2_rn(dx, px, __ffma2_rn(dy, py, __fmul2_rn(dz, pz)));
                 const float2 ri5 = __fmul2_rn(ri3, ri2);
-                sc = __ffma2_rn(splat(-2.5f), __fmul2_rn(dpd, __fmul2_rn(ri5, ri2)), sc);
+                sc = __ffma2_rn(splat(-2.5f), __fmul2_rn(__fmul2_rn(dpd, ri2), ri5), sc);
                 ax[k] = __ffma2_rn(dx, sc, __ffma2_rn(px, ri5, ax[k]));
                 ay[k] = __ffma2_rn(dy, sc, __ffma2_rn(py, ri5, ay[k]));
                 az[k] = __ffma2_rn(dz, sc, __ffma2_rn(pz, ri5, az[k]));
@@ -375,7 +396,7 @@ __device__ __forceinline__ void eval_cells(GroupShared &g, int count, int lane, 
             }
         }
     }
-    add_sums<K>(g, lane, ax, ay, az);
+    add_sums<K>(g, lane, ax, ay, az, unit2);
 }
 
 // Evaluates the first `count` leaf particles (count > 0).  They are gathered 32
@@ -388,9 +409,16 @@ __device__ __forceinline__ void eval_parts(const GroupWalkArgs &A, GroupShared &
                                            const LaneRows &L)
 {
     const float2 e2 = splat(A.eps2);
+    const float back = g.ol.w;
     float2 ax[K], ay[K], az[K];
+    float mx[K], my[K], mz[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) ax[k] = ay[k] = az[k] = splat(0.f);
+    for (int k = 0; k < K; ++k) {
+        ax[k] = ay[k] = az[k] = splat(0.f);
+        mx[k] = -L.rx[k] * back;
+        my[k] = -L.ry[k] * back;
+        mz[k] = -L.rz[k] * back;
+    }
     const float4 oh = g.oh, ol = g.ol;
     int p = g.parts[min(lane, count - 1)];
     float4 ph = A.pa[p], pl = A.pb[p];
@@ -412,9 +440,9 @@ __device__ __forceinline__ void eval_parts(const GroupWalkArgs &A, GroupShared &
             const float4 va = g.pA[j], vb = g.pB[j];
 #pragma unroll
             for (int k = 0; k < K; ++k) {
-                const float2 dx = __fadd2_rn(lo2(va), splat(-L.rx[k]));
-                const float2 dy = __fadd2_rn(hi2(va), splat(-L.ry[k]));
-                const float2 dz = __fadd2_rn(lo2(vb), splat(-L.rz[k]));
+                const float2 dx = __fadd2_rn(lo2(va), splat(mx[k]));
+                const float2 dy = __fadd2_rn(hi2(va), splat(my[k]));
+                const float2 dz = __fadd2_rn(lo2(vb), splat(mz[k]));
                 const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
                 float2 ri = make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
                 if (!SOFT) {   // own term without softening: r2 = 0 contributes nothing
@@ -428,7 +456,7 @@ __device__ __forceinline__ void eval_parts(const GroupWalkArgs &A, GroupShared &
             }
         }
     }
-    add_sums<K>(g, lane, ax, ay, az);
+    add_sums<K>(g, lane, ax, ay, az, 1.0f);
 }
 
 // A group of at most GW_COLS particles leaves the second row empty and skips
@@ -507,10 +535,12 @@ __device__ __forceinline__ void walk_group(const GroupWalkArgs &A, GroupShared &
     const bool two = gend - g0 > GW_COLS;
     LaneRows L;
     {
-        const float4 oh = A.pa[g0], ol = A.pb[g0];
+        float4 oh = A.pa[g0];
+        const float4 ol = A.pb[g0];
         const float4 ph = A.pa[s], pl = A.pb[s];
-        float lo[3] = {(ph.x - oh.x) + (pl.x - ol.x), (ph.y - oh.y) + (pl.y - ol.y),
-                       (ph.z - oh.z) + (pl.z - ol.z)};
+        const float unit = length_unit<QUAD>(A.frame[4]);
+        float lo[3] = {((ph.x - oh.x) + (pl.x - ol.x)) * unit, ((ph.y - oh.y) + (pl.y - ol.y)) * unit,
+                       ((ph.z - oh.z) + (pl.z - ol.z)) * unit};
         float hi[3] = {lo[0], lo[1], lo[2]};
 #pragma unroll
         for (int k = 0; k < GW_ROWS; ++k) {
@@ -525,10 +555,13 @@ __device__ __forceinline__ void walk_group(const GroupWalkArgs &A, GroupShared &
                 hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
             }
         if (lane == 0) {
+            const float back = __int_as_float((254 << 23) - __float_as_int(unit));   // 1 / unit
+            oh.w = -unit * unit;
             g.oh = oh;
-            g.ol = ol;
-            g.lo = make_float4(lo[0], lo[1], lo[2], 0.f);
-            g.hi = make_float4(hi[0], hi[1], hi[2], 0.f);
+            g.ol = make_float4(ol.x, ol.y, ol.z, back);
+            g.nol = make_float4(-ol.x * unit, -ol.y * unit, -ol.z * unit, 0.f);
+            g.lo = make_float4(lo[0], lo[1], lo[2], unit);
+            g.hi = make_float4(hi[0], hi[1], hi[2], A.theta2 * back * back);
             if (part == 0) stack[0] = make_int2(0, 1);   // root
         }
 #pragma unroll
@@ -559,17 +592,18 @@ __device__ __forceinline__ void walk_group(const GroupWalkArgs &A, GroupShared &
                 q0 = A.nq[2 * node];
                 q1 = A.nq[2 * node + 1];
             }
-            const float4 oh = g.oh, ol = g.ol, lo = g.lo, hi = g.hi;
-            nx = (ca.x - oh.x) + (cb.x - ol.x);
-            ny = (ca.y - oh.y) + (cb.y - ol.y);
-            nz = (ca.z - oh.z) + (cb.z - ol.z);
+            const float4 oh = g.oh, nol = g.nol, lo = g.lo, hi = g.hi;
+            // ((com_hi - origin_hi) + (com_lo - origin_lo)) unit
+            nx = fmaf(ca.x - oh.x, lo.w, fmaf(cb.x, lo.w, nol.x));
+            ny = fmaf(ca.y - oh.y, lo.w, fmaf(cb.y, lo.w, nol.y));
+            nz = fmaf(ca.z - oh.z, lo.w, fmaf(cb.z, lo.w, nol.z));
             nm = ca.w;
             const float ex = fmaxf(fmaxf(lo.x - nx, nx - hi.x), 0.f);
             const float ey = fmaxf(fmaxf(lo.y - ny, ny - hi.y), 0.f);
             const float ez = fmaxf(fmaxf(lo.z - nz, nz - hi.z), 0.f);
             const float d2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
             // cb.w: (cell side)^2 of the node's depth
-            const bool far = !(ci.z < gend && ci.z + ci.w > g0) && cb.w < A.theta2 * d2;
+            const bool far = !(ci.z < gend && ci.z + ci.w > g0) && cb.w < hi.w * d2;
             accept = far && nm > 0.f;   // a far cell without mass adds nothing
             open = !far && ci.y > 0;
             leaf = !far && ci.y <= 0 && ci.w > 0;
@@ -610,12 +644,13 @@ __device__ __forceinline__ void walk_group(const GroupWalkArgs &A, GroupShared &
                 put(g.cB, at, 0, nz);
                 put(g.cB, at, 1, nm);
                 if (QUAD) {   // negated, as the evaluation expects
-                    put(g.qA, at, 0, -q0.x);
-                    put(g.qA, at, 1, -q0.y);
-                    put(g.qB, at, 0, -q0.z);
-                    put(g.qB, at, 1, -q0.w);
-                    put(g.qC, at, 0, -q1.x);
-                    put(g.qC, at, 1, -q1.y);
+                    const float nu2 = g.oh.w;
+                    put(g.qA, at, 0, q0.x * nu2);
+                    put(g.qA, at, 1, q0.y * nu2);
+                    put(g.qB, at, 0, q0.z * nu2);
+                    put(g.qB, at, 1, q0.w * nu2);
+                    put(g.qC, at, 0, q1.x * nu2);
+                    put(g.qC, at, 1, q1.y * nu2);
                 }
             }
             ncell += __popc(accepted);
@@ -756,6 +791,7 @@ ErrorStatus launch_bh_group_walk(const OctreeDevice &t, double theta, double eps
     w.pa = t.w_pa.as<float4>();
     w.pb = t.w_pb.as<float4>();
     w.sidx = t.sidx.as<int>();
+    w.frame = t.frame.as<double>();
     w.eps2 = (float)(eps * eps);
     w.theta2 = (float)(theta * theta);
     w.G = G;

@@ -474,3 +474,18 @@ def test_walk_at_close_pairs_and_scales(lib, g, orc, wl, method, case):
     else:
         a_o, _, mag = orc.bh_counts(x, m, 1.0, 0.0, 0.5, 1, False)
     check_terms(a, a_o, mag)
+
+
+@pytest.mark.parametrize("log2_scale", [-10, 23, 27])
+def test_group_walk_scales(lib, g, wl, log2_scale):
+    """Scaling every position by a power of two scales each FP32 operation of the walk exactly
+    while nothing leaves the range, so the accelerations scale by its inverse square.  (r^-7,
+    once a factor of the quadrupole term, leaves it at each of these scales; below 2^-100 of
+    the largest the terms are subnormal and round differently: 1e-6.)"""
+    x, v, m = wl.galaxy_pair(20000, 23)
+    kw = dict(opening_angle=0.5, softening_length=0.0, max_num_particles_per_leaf=1)
+    scale = 2.0 ** log2_scale
+    a = g.acceleration(lib, x, m, 1.0, g.METHOD_GPU_BARNES_HUT_GROUP, **kw)
+    b = g.acceleration(lib, x * scale, m, 1.0, g.METHOD_GPU_BARNES_HUT_GROUP, **kw) * scale ** 2
+    assert np.isfinite(b).all()
+    assert (np.linalg.norm(a - b, axis=1) <= 1e-6 * np.linalg.norm(a, axis=1)).all()
