@@ -17,8 +17,8 @@
 //   * the j-particles are divided in granules of 128 (the length of a plain
 //     partial sum), and a row tile's granules into units so that the last wave of
 //     resident CTAs is as full as it gets (choose_per); the units' Kahan pairs go
-//     to scratch [split][3][N], which a second kernel adds in fixed order with the
-//     FP32 rounding errors kept, and scales by G;
+//     to scratch [split][3][N], which a second kernel adds in fixed order, to the
+//     precision of an FP64 sum, and scales by G;
 //   * up to 20,480 particles the units are 64 rows by 1,024 or 2,048 terms
 //     (k_direct_run).
 //   Measured at N = 100,000: 3.76 -> 3.51 ms (57 TFLOP/s at 20 per pair term, 0.74
@@ -30,6 +30,7 @@
 // the same operations as the reference's symmetric loop applies to that
 // particle, so the result equals the reference's bit for bit where the
 // reference is not FMA-contracted.
+#include "gs_fp64.cuh"
 #include "gs_internal.h"
 #include "gs_ptx.cuh"
 
@@ -255,15 +256,22 @@ __device__ __forceinline__ void direct_sum_unit(const float4 *__restrict__ pi_ti
     }
 }
 
-// A unit's Kahan pair (s, c), whose value is s - c, added to the running sum
-// h + l by Knuth's two-sum (exact), the small parts gathered in l.
-__device__ __forceinline__ void add_pair(float &h, float &l, const float2 sc)
+// a + b = sum + err exactly (Knuth's two-sum).
+__device__ __forceinline__ float two_sum(float a, float b, float &err)
 {
-    const float t = __fadd_rn(h, sc.x);
-    const float b = __fsub_rn(t, h);
-    const float e = __fadd_rn(__fsub_rn(h, __fsub_rn(t, b)), __fsub_rn(sc.x, b));
-    l = __fadd_rn(l, __fsub_rn(e, sc.y));
-    h = t;
+    const float t = __fadd_rn(a, b), v = __fsub_rn(t, a);
+    err = __fadd_rn(__fsub_rn(a, __fsub_rn(t, v)), __fsub_rn(b, v));
+    return t;
+}
+
+// A unit's Kahan pair (s, c), whose value is s - c, added to the running sum
+// h + l + t: h and l exactly, t holds what they leave (72 bits in all).
+__device__ __forceinline__ void add_pair(float &h, float &l, float &t, const float2 sc)
+{
+    float e, f, g;
+    h = two_sum(h, sc.x, e);
+    l = two_sum(l, two_sum(e, -sc.y, f), g);
+    t = __fadd_rn(t, __fadd_rn(f, g));
 }
 
 // Work units: unit (itile, split) takes granules [split * per, (split + 1) * per).
@@ -372,18 +380,27 @@ k_direct_rows(const float4 *__restrict__ pi, int ni_pad, const float4 *__restric
                           reinterpret_cast<float4 *>(ds_smem), full_bar);
 }
 
-// Sum over the splits, in split order, of component k of row i.  The pairs
-// are added in FP32 with their rounding errors kept: FP64 conversions and adds
-// cost a whole warp's time on a pipe of 1/64 of the FP32 rate (72 of them per
-// thread in a unit's epilogue took 4 us of a 65 us launch at N = 12,000).
+// Sum over the splits, in split order, of component k of row i: in FP32 with the
+// rounding errors kept, which is an FP64 sum's precision and more.  FP64
+// conversions and adds cost a whole warp's time on a pipe of 1/64 of the FP32 rate:
+// 72 of them per thread in a unit's epilogue took 4 us of a 65 us launch at
+// N = 12,000.  A sum that leaves the FP32 range (or is not finite) is one of FP64.
 __device__ __forceinline__ double reduce_row(const float2 *__restrict__ partial, int splits,
                                              size_t plane, int k, int i)
 {
     const float2 *p = partial + k * plane + i;
-    float h = 0.0f, l = 0.0f;
+    float h = 0.0f, l = 0.0f, t = 0.0f;
 #pragma unroll 8
-    for (int q = 0; q < splits; ++q) add_pair(h, l, p[(size_t)q * 3 * plane]);
-    return (double)h + (double)l;
+    for (int q = 0; q < splits; ++q) add_pair(h, l, t, p[(size_t)q * 3 * plane]);
+    const double sum = (double)h + ((double)l + (double)t);
+    if (finite_bits(sum)) return sum;
+    double wide = 0.0;
+#pragma unroll 1
+    for (int q = 0; q < splits; ++q) {
+        const float2 sc = p[(size_t)q * 3 * plane];
+        wide += (double)sc.x - (double)sc.y;
+    }
+    return wide;
 }
 
 // a_i = G * sum_s partial[s][.][i]; a thread per component.

@@ -164,3 +164,24 @@ def test_softened_energy_against_fp64(lib, n):
                                      m.ctypes.data_as(dp), n, 1.0, 0.01, ctypes.byref(e)) == 0
     want = _softened_energy_fp64(x, v, m, 1.0, 0.01) if n else 0.0
     assert abs(e.value - want) <= 1e-6 * max(abs(want), 1e-300), (e.value, want)
+
+
+@pytest.mark.parametrize("n", [12000, 20000, 24000])
+def test_fp32_partial_sums_added_as_in_fp64(lib, g, n):
+    """Sums over the units of a direct sum keep an FP64 sum's precision.  Particle 0 is at the
+    origin, all others at (1, 0, 0), so its terms are their masses exactly: one in the first
+    unit, one in the middle, one in the last.  The exact sum has 50 bits, and an FP64 addition
+    of the three gives it."""
+    x = np.zeros((n, 3))
+    x[1:, 0] = 1.0
+    m = np.zeros(n)
+    m[5] = 1.0
+    m[n // 2] = 2.0 ** -25 * (1.0 + 2.0 ** -23)
+    m[n - 3] = 2.0 ** -26 * (1.0 + 2.0 ** -23)
+    exact = float(m.sum())
+    assert exact - 1.0 == m[n // 2] + m[n - 3]   # representable
+    a = g.acceleration(lib, x, m, 1.0, g.METHOD_GPU_PAIRWISE, softening_length=0.0)
+    assert a[0, 0] == exact and a[0, 1] == 0.0 and a[0, 2] == 0.0
+    m[[5, n // 2, n - 3]] = 2.0 ** 127   # each in the FP32 range, their sum not
+    a = g.acceleration(lib, x, m, 1.0, g.METHOD_GPU_PAIRWISE, softening_length=0.0)
+    assert a[0, 0] == 3.0 * 2.0 ** 127 and a[0, 1] == 0.0 and a[0, 2] == 0.0
