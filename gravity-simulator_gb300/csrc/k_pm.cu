@@ -81,7 +81,7 @@ struct PmGeom {
     double cx, cy, cz;   // box centre
     double half;         // box_length / 2
     double inv_cell;     // 1 / (box_length / g)
-    double shift[3];     // half - centre
+    double half_cells;   // g / 2
     int g;
 };
 
@@ -94,15 +94,16 @@ __device__ __forceinline__ int wrap_index(int n, int g)
 }
 
 // Cell indices and weights of one particle (src/acceleration_PM.c:44-58).  Inside
-// the box the cell is the integer part of u = (x - c + half) / cell, taken by
-// adding 2^52 rounded down: six FP64 operations a dimension.
+// the box the cell is the integer part of u = (x - c + half) / cell, formed as
+// (x - c) / cell + g / 2 (x - c first, so that a box far from the origin loses
+// nothing) and taken by adding 2^52 rounded down: six FP64 operations a dimension.
 __device__ __forceinline__ void cic_cell(const double xi[3], const PmGeom &G, int idx[2][3],
                                          double w[2][3])
 {
     const double c[3] = {G.cx, G.cy, G.cz};
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        const double u = (xi[d] + G.shift[d]) * G.inv_cell;
+        const double u = fma(xi[d] - c[d], G.inv_cell, G.half_cells);
         if ((unsigned)__double2hiint(u) < 0x41d00000u) {   // 0 <= u < 2^30
             const double t = __dadd_rd(u, 0x1p52);
             const int nd = __double2loint(t);
@@ -475,7 +476,7 @@ class PmSolver {
         geom_.cz = box_center[2];
         geom_.half = box_length / 2.0;
         geom_.inv_cell = 1.0 / cell_length_;
-        for (int d = 0; d < 3; ++d) geom_.shift[d] = geom_.half - box_center[d];
+        geom_.half_cells = 0.5 * g;
         geom_.g = g;
         const int top = g / 2;
         const int len = 3 * top * top + 1;

@@ -119,3 +119,19 @@ def test_cosmological_simulation_golden(lib, g):
     lo = np.array(kw["box_center"]) - kw["box_width"]
     hi = np.array(kw["box_center"]) + kw["box_width"]
     assert ((x >= lo) & (x <= hi)).all()
+
+
+@pytest.mark.parametrize("grid", [32, 30])
+@pytest.mark.parametrize("centre", [1e6, -3e9])
+def test_acceleration_pm_box_far_from_origin(lib, g, grid, centre):
+    """A box far from the origin gives the accelerations of the same box at the origin: the
+    positions are multiples of 2^-20, so x - centre is exact, and nothing else may depend on the
+    centre (its half width of 1/3 is no such multiple)."""
+    rng = np.random.default_rng(grid)
+    bw = 1.0 / 3.0
+    x = np.round(np.clip(rng.standard_normal((5000, 3)) * 0.1, -0.3, 0.3) * 2.0 ** 20) / 2.0 ** 20
+    m = rng.uniform(0.5, 1.5, len(x))
+    c = np.array([centre, 0.0, -centre])
+    rest = (bw, 70.0, 0.3, m.sum() / (2 * bw) ** 3, grid, 0.25)
+    _close(g.acceleration_pm(lib, x + c, m, c, *rest),
+           g.acceleration_pm(lib, x, m, np.zeros(3), *rest), 1e-12)
