@@ -246,13 +246,14 @@ struct LineSplit {
 
 // Lines along one of the first two axes.  A CTA takes LINES neighbouring lines
 // (128-byte rows) of one slab; line l of slab o starts at o outer + l, its points
-// are `stride` apart.  tw: exp(-2 pi i k / N).
+// are `stride` apart.  tw: exp(-2 pi i k / N).  FIRST: the mesh holds densities,
+// read as their contrast.
 constexpr int LINES = 8;
 
-template <int N, bool INV>
+template <int N, bool INV, bool FIRST = false>
 __global__ void __launch_bounds__(LINES *LineSplit<N>::R2)
 k_fft_lines(double2 *__restrict__ data, unsigned lines_per_slab, size_t outer, unsigned stride,
-            const double2 *__restrict__ tw)
+            const double2 *__restrict__ tw, MeshScale scale = {nullptr, 1.0})
 {
     constexpr int R1 = LineSplit<N>::R1, R2 = LineSplit<N>::R2, M = (R1 + R2 - 1) / R2;
     __shared__ double2 s[N * LINES];
@@ -265,6 +266,11 @@ k_fft_lines(double2 *__restrict__ data, unsigned lines_per_slab, size_t outer, u
 #pragma unroll
     for (int r = 0; r < R1; ++r)
         v[r] = live ? base[(size_t)(t + R2 * r) * stride] : make_double2(0.0, 0.0);
+    if (FIRST) {
+        const double f = scale.device ? *scale.device : scale.value;
+#pragma unroll
+        for (int r = 0; r < R1; ++r) v[r] = make_double2(contrast(v[r].x, f), contrast(v[r].y, f));
+    }
     Dft<R1, INV>::run(v);
 #pragma unroll
     for (int q = 0; q < R1; ++q) {
@@ -416,13 +422,14 @@ __global__ void k_fft_table(int g, double2 *__restrict__ tw)
 }
 
 template <int G>
-void convolve(double2 *data, const double *table, const double2 *tw, cudaStream_t s)
+void convolve(double2 *data, const MeshScale &scale, const double *table, const double2 *tw,
+              cudaStream_t s)
 {
     constexpr unsigned H = G / 2;
     constexpr int threads = LINES * LineSplit<G>::R2;
     constexpr unsigned slabs = G * ((H + LINES - 1) / LINES), planes = (G * H + LINES - 1) / LINES;
     using S = PairShape<G>;
-    k_fft_lines<G, false><<<slabs, threads, 0, s>>>(data, H, (size_t)G * H, H, tw);
+    k_fft_lines<G, false, true><<<slabs, threads, 0, s>>>(data, H, (size_t)G * H, H, tw, scale);
     k_fft_lines<G, false><<<planes, threads, 0, s>>>(data, G * H, 0, G * H, tw);
     k_fft_pairs<G><<<(S::COUNT + S::PAIRS - 1) / S::PAIRS, 128, 0, s>>>(data, table, tw);
     k_fft_lines<G, true><<<planes, threads, 0, s>>>(data, G * H, 0, G * H, tw);
@@ -431,7 +438,7 @@ void convolve(double2 *data, const double *table, const double2 *tw, cudaStream_
 
 }  // namespace
 
-using Convolve = void (*)(double2 *, const double *, const double2 *, cudaStream_t);
+using Convolve = void (*)(double2 *, const MeshScale &, const double *, const double2 *, cudaStream_t);
 
 // Even sizes of small prime factors whose lines and half lines have two factors
 // of at most 16; other sizes go to the library's transforms.
@@ -466,12 +473,12 @@ ErrorStatus convolve_table(int g, double2 *tw, cudaStream_t s)
     return ok();
 }
 
-ErrorStatus convolve_mesh(double *mesh, int g, const double *table, const double2 *tw,
-                          cudaStream_t s)
+ErrorStatus convolve_mesh(double *mesh, int g, const MeshScale &scale, const double *table,
+                          const double2 *tw, cudaStream_t s)
 {
     const Convolve run = convolve_for(g);
     if (!run) return GS_RAISE(GRAV_VALUE_ERROR, "no convolution of a mesh of %d cells a side", g);
-    run(reinterpret_cast<double2 *>(mesh), table, tw, s);
+    run(reinterpret_cast<double2 *>(mesh), scale, table, tw, s);
     GS_CUDA(cudaGetLastError());
     return ok();
 }

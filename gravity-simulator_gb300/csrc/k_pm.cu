@@ -2,12 +2,11 @@
 // cosmological leapfrog (src/integrator_cosmology_leapfrog.c:24-255).
 //
 // One evaluation on a g^3 periodic mesh:
-//   k_pm_fill      the mesh at -1;
-//   deposit        cloud-in-cell deposit of m / (V_cell rho_mean), eight FP64
-//                  atomic adds per particle (the reference's OpenMP loop has
-//                  unsynchronised += here), which makes the mesh the density
-//                  contrast rho / (V_cell rho_mean) - 1;
-//   the potential  the mesh convolved with -1/k^2 (0 at k = 0), from a table by
+//   deposit        cloud-in-cell deposit of the masses, eight FP64 atomic adds per
+//                  particle (the reference's OpenMP loop has unsynchronised += here);
+//   the potential  the density contrast rho / (V_cell rho_mean) - 1, formed where
+//                  the mesh is first read (a deposit into a mesh of -1 would round
+//                  every addition to the contrast's last bit), convolved with -1/k^2 (0 at k = 0), from a table by
 //                  the integer |n|^2: for the sizes of k_fft.cu (even, of small
 //                  factors, 32 to 256) in place, otherwise cuFFT D2Z (FFTW's layout:
 //                  g x g x (g/2+1)), k_pm_green, and cuFFT Z2D, unnormalised;
@@ -208,22 +207,20 @@ __device__ __forceinline__ void interp_one(const int idx[2][3], const double w[2
     }
 }
 
-__global__ void k_pm_fill(double *__restrict__ mesh, long long cells, double value)
-{
-    const long long i = 2 * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
-    if (i + 1 < cells)
-        *reinterpret_cast<double2 *>(mesh + i) = make_double2(value, value);
-    else if (i < cells)
-        mesh[i] = value;
-}
-
-__global__ void k_pm_deposit(const double *__restrict__ x, const double *__restrict__ mn, int n,
+__global__ void k_pm_deposit(const double *__restrict__ x, const double *__restrict__ m, int n,
                              PmGeom G, double *__restrict__ delta, CicKept K)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double xi[3] = {x[3 * (size_t)i], x[3 * (size_t)i + 1], x[3 * (size_t)i + 2]};
-    deposit_one(xi, mn[i], G, delta, K, i);
+    deposit_one(xi, m[i], G, delta, K, i);
+}
+
+// The contrast where the library's transforms read the mesh.
+__global__ void k_pm_contrast(double *__restrict__ mesh, long long cells, MeshScale scale)
+{
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < cells) mesh[i] = contrast(mesh[i], scale.device ? *scale.device : scale.value);
 }
 
 // -1 / (|n|^2 (2 pi / L)^2) by the integer |n|^2 of a mode (src/acceleration_PM.c:
@@ -337,15 +334,6 @@ k_pm_mass_inv(const double *__restrict__ part, double volume, double cell_volume
     if (threadIdx.x == 0) *inv = 1.0 / (cell_volume * (total / volume));
 }
 
-// mn = m * inv, inv given or read from *d_inv
-__global__ void k_pm_mass_scale(const double *__restrict__ m, int n,
-                                const double *__restrict__ d_inv, double inv,
-                                double *__restrict__ mn)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) mn[i] = m[i] * (d_inv ? *d_inv : inv);
-}
-
 // ---- cosmological leapfrog (src/integrator_cosmology_leapfrog.c) -----------
 // src/system.c:1337-1375 for one coordinate.
 __device__ __forceinline__ double periodic(double xv, double c, double bw)
@@ -399,7 +387,7 @@ __global__ void k_cosmo_velocity(double *__restrict__ v, const double *__restric
 // c = dt / (a^2 da).  Without MOVE the accelerations are kept in `a`.
 template <bool GATHER, bool MOVE>
 __global__ void k_pm_particles(double *__restrict__ x, double *__restrict__ p,
-                               const double *__restrict__ mn, double *__restrict__ a, int n,
+                               const double *__restrict__ m, double *__restrict__ a, int n,
                                PmGeom G, const double *__restrict__ acc, double k1, double k2,
                                double c, double bw, double *__restrict__ delta, CicKept K)
 {
@@ -429,7 +417,7 @@ __global__ void k_pm_particles(double *__restrict__ x, double *__restrict__ p,
         }
         p[q + d] = pd;
     }
-    if (MOVE) deposit_one(xi, mn[i], G, delta, K, i);
+    if (MOVE) deposit_one(xi, m[i], G, delta, K, i);
 }
 
 }  // namespace
@@ -488,34 +476,30 @@ class PmSolver {
         return ok();
     }
 
-    // Masses as the deposit takes them: m / (V_cell rho_mean), with rho_mean given
-    // or the total mass over the box's volume.
-    ErrorStatus scale_masses(const double *d_m, int n, double box_width, bool given, double rho_mean,
-                             cudaStream_t s)
+    // 1 / (V_cell rho_mean) with rho_mean given.
+    void set_mean_density(double rho_mean)
     {
-        GS_TRY(mn_.reserve((size_t)n * sizeof(double)));
-        const double cell_volume = cell_length_ * cell_length_ * cell_length_;
-        double *inv = nullptr;
-        if (!given) {
-            GS_TRY(part_.reserve((MS_BLOCKS + 1) * sizeof(double)));
-            inv = part_.as<double>() + MS_BLOCKS;
-            k_pm_mass_parts<<<MS_BLOCKS, MS_THREADS, 0, s>>>(d_m, n, part_.as<double>());
-            k_pm_mass_inv<<<1, MS_THREADS, 0, s>>>(
-                part_.as<double>(), (box_width * 2) * (box_width * 2) * (box_width * 2), cell_volume,
-                inv);
-        }
-        k_pm_mass_scale<<<blocks(n), TPB, 0, s>>>(d_m, n, inv, given ? 1.0 / (cell_volume * rho_mean)
-                                                                     : 0.0, mn_.as<double>());
+        scale_ = {nullptr, 1.0 / (cell_length_ * cell_length_ * cell_length_ * rho_mean)};
+    }
+
+    // The same with rho_mean the total mass over the box's volume.
+    ErrorStatus mean_density_of(const double *d_m, int n, double box_width, cudaStream_t s)
+    {
+        GS_TRY(part_.reserve((MS_BLOCKS + 1) * sizeof(double)));
+        double *inv = part_.as<double>() + MS_BLOCKS;
+        k_pm_mass_parts<<<MS_BLOCKS, MS_THREADS, 0, s>>>(d_m, n, part_.as<double>());
+        k_pm_mass_inv<<<1, MS_THREADS, 0, s>>>(
+            part_.as<double>(), (box_width * 2) * (box_width * 2) * (box_width * 2),
+            cell_length_ * cell_length_ * cell_length_, inv);
         GS_CUDA(cudaGetLastError());
+        scale_ = {inv, 0.0};
         return ok();
     }
 
     // The mesh ready for a deposit.
     ErrorStatus clear(cudaStream_t s)
     {
-        const long long cells = (long long)g_ * g_ * g_;
-        k_pm_fill<<<blocks((cells + 1) / 2), TPB, 0, s>>>(mesh_.as<double>(), cells, -1.0);
-        GS_CUDA(cudaGetLastError());
+        GS_CUDA(cudaMemsetAsync(mesh_.p, 0, (size_t)g_ * g_ * g_ * sizeof(double), s));
         return ok();
     }
 
@@ -523,9 +507,12 @@ class PmSolver {
     ErrorStatus solve(cudaStream_t s)
     {
         double *mesh = mesh_.as<double>();
+        const long long cells = (long long)g_ * g_ * g_;
         if (convolve_supports(g_)) {
-            GS_TRY(convolve_mesh(mesh, g_, green_.as<double>(), tw_.as<double2>(), s));
+            GS_TRY(convolve_mesh(mesh, g_, scale_, green_.as<double>(), tw_.as<double2>(), s));
         } else {
+            k_pm_contrast<<<blocks(cells), TPB, 0, s>>>(mesh, cells, scale_);
+            GS_CUDA(cudaGetLastError());
             GS_CUFFT(cufftSetStream(fwd_, s));
             GS_CUFFT(cufftExecD2Z(fwd_, mesh, spec_.as<cufftDoubleComplex>()));
             const long long half = (long long)g_ * g_ * (g_ / 2 + 1);
@@ -534,15 +521,14 @@ class PmSolver {
             GS_CUFFT(cufftSetStream(inv_, s));
             GS_CUFFT(cufftExecZ2D(inv_, spec_.as<cufftDoubleComplex>(), mesh));
         }
-        const long long cells = (long long)g_ * g_ * g_;
         k_pm_gradient<<<blocks(cells), TPB, 0, s>>>(mesh, g_, acc_.as<double>());
         GS_CUDA(cudaGetLastError());
         return ok();
     }
 
-    // Kernels of this library in a step: the fill, the particles, the potential and
-    // the gradient.
-    int kernels_per_step() const { return 3 + (convolve_supports(g_) ? kConvolveLaunches : 1); }
+    // Kernels of this library in a step: the particles, the potential (the contrast
+    // and the Green's function beside cuFFT) and the gradient.
+    int kernels_per_step() const { return 2 + (convolve_supports(g_) ? kConvolveLaunches : 2); }
 
     // The gradient mesh's constant factor.
     double scale(double H0, double omega_m, double scale_factor) const
@@ -554,14 +540,14 @@ class PmSolver {
     const PmGeom &geom() const { return geom_; }
     double *mesh() const { return mesh_.as<double>(); }
     const double *acc() const { return acc_.as<double>(); }
-    const double *masses() const { return mn_.as<double>(); }
 
   private:
     int g_ = 0;
     double cell_length_ = 1.0;
     PmGeom geom_{};
     cufftHandle fwd_ = 0, inv_ = 0;
-    DBuf mesh_, spec_, acc_, green_, tw_, mn_, part_;
+    MeshScale scale_{nullptr, 1.0};
+    DBuf mesh_, spec_, acc_, green_, tw_, part_;
 };
 
 namespace {
@@ -630,9 +616,9 @@ ErrorStatus pm_acceleration_host(double *a, int n, const double *x, const double
                             c->stream));
     PmSolver &pm = c->solver;
     GS_TRY(pm.prepare(box_center, box_width, g, c->stream));
-    GS_TRY(pm.scale_masses(c->m.as<double>(), n, box_width, true, mean_bkg_density, c->stream));
+    pm.set_mean_density(mean_bkg_density);
     GS_TRY(pm.clear(c->stream));
-    k_pm_deposit<<<blocks(n), TPB, 0, c->stream>>>(c->x.as<double>(), pm.masses(), n, pm.geom(),
+    k_pm_deposit<<<blocks(n), TPB, 0, c->stream>>>(c->x.as<double>(), c->m.as<double>(), n, pm.geom(),
                                                    pm.mesh(), CicKept{nullptr, nullptr});
     GS_CUDA(cudaGetLastError());
     GS_TRY(pm.solve(c->stream));
@@ -683,12 +669,12 @@ ErrorStatus pm_leapfrog_cosmology(CosmologicalSystem *system, SimulationStatus *
     if (is_output && op->output_initial) GS_TRY(output_snapshot_cosmology(op, system, t));
     PmSolver &pm = pc->solver;
     GS_TRY(pm.prepare(c, bw, g, s));
-    GS_TRY(pm.scale_masses(m.as<double>(), n, bw, false, 0.0, s));
+    GS_TRY(pm.mean_density_of(m.as<double>(), n, bw, s));
     k_cosmo_wrap<<<blocks(L), TPB, 0, s>>>(x.as<double>(), L, c[0], c[1], c[2], bw);
     k_cosmo_momentum<<<blocks(L), TPB, 0, s>>>(p.as<double>(), v.as<double>(), L, t);
     GS_CUDA(cudaGetLastError());
     GS_TRY(pm.clear(s));
-    k_pm_deposit<<<blocks(n), TPB, 0, s>>>(x.as<double>(), pm.masses(), n, pm.geom(), pm.mesh(), kept);
+    k_pm_deposit<<<blocks(n), TPB, 0, s>>>(x.as<double>(), m.as<double>(), n, pm.geom(), pm.mesh(), kept);
     GS_CUDA(cudaGetLastError());
     GS_TRY(pm.solve(s));
     double factor = pm.scale(H0, omega_m, t);   // of the accelerations now in the mesh
@@ -711,7 +697,7 @@ ErrorStatus pm_leapfrog_cosmology(CosmologicalSystem *system, SimulationStatus *
         da = compute_da(t, H0, omega_m, omega_lambda);
         GS_TRY(pm.clear(s));
         auto move = gather ? k_pm_particles<true, true> : k_pm_particles<false, true>;
-        move<<<blocks(n), TPB, 0, s>>>(x.as<double>(), p.as<double>(), pm.masses(), a.as<double>(),
+        move<<<blocks(n), TPB, 0, s>>>(x.as<double>(), p.as<double>(), m.as<double>(), a.as<double>(),
                                        n, pm.geom(), pm.acc(), k1, k2, dt / (t * t * da), bw,
                                        pm.mesh(), kept);
         GS_CUDA(cudaGetLastError());
@@ -731,7 +717,7 @@ ErrorStatus pm_leapfrog_cosmology(CosmologicalSystem *system, SimulationStatus *
             // the step's last kick by itself; the next step's takes the stored
             // accelerations
             k_pm_particles<true, false><<<blocks(n), TPB, 0, s>>>(
-                x.as<double>(), p.as<double>(), pm.masses(), a.as<double>(), n, pm.geom(), pm.acc(),
+                x.as<double>(), p.as<double>(), m.as<double>(), a.as<double>(), n, pm.geom(), pm.acc(),
                 k1, 0.0, 0.0, bw, pm.mesh(), kept);
             GS_CUDA(cudaGetLastError());
         }

@@ -135,3 +135,21 @@ def test_acceleration_pm_box_far_from_origin(lib, g, grid, centre):
     rest = (bw, 70.0, 0.3, m.sum() / (2 * bw) ** 3, grid, 0.25)
     _close(g.acceleration_pm(lib, x + c, m, c, *rest),
            g.acceleration_pm(lib, x, m, np.zeros(3), *rest), 1e-12)
+
+
+@pytest.mark.parametrize("grid", [32, 30])
+def test_acceleration_pm_light_deposits(lib, g, grid):
+    """Deposits far below the mean density add up: 200,000 particles in a blob, each less than
+    half of the last bit of a contrast of -1 (5e-17 of the mean).  The accelerations are those
+    of the usual mean over the ratio of the means, to the contrast's own rounding (1e-16 of
+    1e-13 a cell, and the transforms' of a mesh near -1): within 5 % of the largest."""
+    rng = np.random.default_rng(grid)
+    bw, n = 1.0, 200_000
+    x = np.clip(rng.standard_normal((n, 3)) * 0.05, -0.9, 0.9)
+    m = np.ones(n)
+    c = np.zeros(3)
+    cell = (2 * bw / grid) ** 3
+    usual, high = n / (2 * bw) ** 3, 1.0 / (cell * 5e-17)
+    a = g.acceleration_pm(lib, x, m, c, bw, 70.0, 0.3, usual, grid, 0.25)
+    b = g.acceleration_pm(lib, x, m, c, bw, 70.0, 0.3, high, grid, 0.25)
+    _close(b * (high / usual), a, 0.05)
