@@ -731,7 +731,9 @@ ErrorStatus pm_leapfrog_cosmology(CosmologicalSystem *system, SimulationStatus *
             GS_TRY(output_snapshot_cosmology(op, system, t));
             next_output_time = op->output_count_ * op->output_interval;
         }
-        if (stop) break;
+        // the flag may have been set while the snapshot was written, after which the
+        // step is complete
+        if (stop || (snap && is_exit && *is_exit)) break;
     }
     GS_CUDA(cudaEventRecord(pc->ev[1], s));
     GS_CUDA(cudaMemcpyAsync(system->x, x.p, b3, cudaMemcpyDeviceToHost, s));

@@ -12,7 +12,10 @@ uninitialised; this library writes t = 0 and the integrator's dt there, so
 those two lines of snapshot_00000.csv are not compared when output_initial
 is set.
 """
+import ctypes
 import json
+import os
+import threading
 
 import numpy as np
 import pytest
@@ -165,3 +168,42 @@ def test_cosmological_csv_output_is_refused(lib, g, tmp_path):
         g.launch_cosmological_simulation(lib, cs["x0"].copy(), cs["v0"].copy(), cs["m"], **kw,
                                          output_method=g.OUTPUT_METHOD_CSV,
                                          output_dir=str(tmp_path) + "/")
+
+
+def test_exit_flag_set_during_a_cosmological_snapshot(lib, g, tmp_path):
+    """A flag set while a snapshot is written ends the run at that snapshot's step.  The first
+    snapshot (step 3) goes to a pipe, smaller than the file, whose reader sets the flag before it
+    takes a byte."""
+    rng = np.random.default_rng(3)
+    n, da = 100_000, 1.0 / 256
+    x, v, m = rng.uniform(-1.0, 1.0, (n, 3)), np.zeros((n, 3)), np.ones(n)
+    ids = np.arange(n, dtype=np.int32)
+    out_dir = tmp_path / "run"
+    out_dir.mkdir()
+    pipe = out_dir / "snapshot_00000.hdf5"
+    os.mkfifo(pipe)
+    flag = ctypes.c_bool(False)
+
+    def read():
+        with open(pipe, "rb") as f:
+            flag.value = True
+            f.read()
+
+    reader = threading.Thread(target=read, daemon=True)
+    reader.start()
+    system = g.CosmologicalSystem(n, ids.ctypes.data_as(ctypes.POINTER(ctypes.c_int)),
+                                  *[a.ctypes.data_as(g.c_double_p) for a in (x, v, m)],
+                                  0.7, 0.3, 0.7, 0.0, (ctypes.c_double * 3)(0.0, 0.0, 0.0), 1.0,
+                                  1.0, 1.0, 1.0)
+    op = g.OutputParam(g.OUTPUT_METHOD_HDF5, (str(out_dir) + "/").encode(), False, 0.5 + 2.5 * da,
+                       *[g.OUTPUT_DTYPE_DOUBLE] * 3, 0)
+    status = g.SimulationStatus(0.0, 0.0, 0)
+    settings = g.Settings(0, False, ctypes.pointer(flag))
+    lib.launch_cosmological_simulation.restype = g.ErrorStatus
+    st = lib.launch_cosmological_simulation(
+        ctypes.byref(system), ctypes.byref(op), ctypes.byref(status), ctypes.byref(settings),
+        ctypes.c_double(da), ctypes.c_double(0.5), ctypes.c_double(0.5 + 8 * da), ctypes.c_int(16))
+    assert st.return_code == 0, g.take_traceback(lib, st)
+    reader.join(10.0)
+    assert status.num_steps == 3 and status.t == 0.5 + 3 * da
+    assert sorted(p.name for p in out_dir.iterdir()) == [pipe.name]
