@@ -229,7 +229,9 @@ __global__ void k_pm_contrast(double *__restrict__ mesh, long long cells, MeshSc
 __global__ void k_pm_green_table(double *__restrict__ table, int len, double two_pi_over_l2)
 {
     const int k2 = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k2 < len) table[k2] = k2 == 0 ? 0.0 : -1.0 / ((double)k2 * two_pi_over_l2);
+    if (k2 >= len) return;
+    const double k_sq = (double)k2 * two_pi_over_l2;   // 0 also where it underflows
+    table[k2] = k_sq == 0.0 ? 0.0 : -1.0 / k_sq;
 }
 
 __global__ void k_pm_green(double2 *__restrict__ spec, int g, const double *__restrict__ table)

@@ -153,3 +153,12 @@ def test_acceleration_pm_light_deposits(lib, g, grid):
     a = g.acceleration_pm(lib, x, m, c, bw, 70.0, 0.3, usual, grid, 0.25)
     b = g.acceleration_pm(lib, x, m, c, bw, 70.0, 0.3, high, grid, 0.25)
     _close(b * (high / usual), a, 0.05)
+
+
+@pytest.mark.parametrize("grid", [32, 30])
+def test_acceleration_pm_huge_box(lib, g, grid):
+    """A box so wide that its squared wave numbers underflow has no potential: zeros."""
+    rng = np.random.default_rng(grid)
+    x = rng.uniform(-1.0, 1.0, (100, 3)) * 1e165
+    a = g.acceleration_pm(lib, x, np.ones(100), np.zeros(3), 1e165, 70.0, 0.3, 1.0, grid, 0.25)
+    assert (a == 0.0).all()
