@@ -112,6 +112,7 @@ struct WalkShared {
     int2 part[64];               // particles of opened leaves, lanes
     float pos[6][32];            // negated particle positions: hi x y z, lo x y z
     float4 oh, ol, lo, hi;       // origin (the first particle) and the particles' box from it
+    unsigned poison;             // lanes that a particle that is not finite acts on
 };
 
 // Compensated sums of a lane's two particles, the even and the odd list entries
@@ -233,6 +234,32 @@ __device__ __forceinline__ void eval_list(WalkShared<QUAD, COMPAT> &w, int count
     __syncwarp();   // the list is read
 }
 
+// The particles w.part[0 .. count) (at most 32) of opened leaves become list entries
+// from `at` on; returns the lanes that this lane's one acts on (not the particle
+// itself).  Lanes an entry does not act on add its terms times zero, so a particle
+// with a coordinate or mass that is not finite acts on no lane: the sums of those it
+// should act on become NaN at the end (w.poison).
+template <bool QUAD, bool COMPAT>
+__device__ __forceinline__ unsigned put_parts(const WalkArgs &A, WalkShared<QUAD, COMPAT> &w, int at,
+                                              int count, int s0, int lane)
+{
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (lane >= count) return 0u;
+    const int2 e = w.part[lane];
+    const int own = e.x - s0;
+    const unsigned lanes = (unsigned)e.y & ~((unsigned)own < 32u ? 1u << own : 0u);
+    float4 h = A.pa[e.x], l = A.pb[e.x];
+    unsigned on = lanes;
+    // zero unless one of them is infinite or NaN
+    if (!(fmaf(h.x, 0.f, fmaf(h.y, 0.f, fmaf(h.z, 0.f, h.w * 0.f))) == 0.f)) {
+        atomicOr(&w.poison, lanes);
+        h = l = zero;
+        on = 0;
+    }
+    put_entry<QUAD, COMPAT>(w, at + lane, h, l, on, zero, zero);
+    return lanes;
+}
+
 template <int TEAM>
 __device__ __forceinline__ void walk_sync()
 {
@@ -298,6 +325,7 @@ k_bh_walk(WalkArgs A)
             w.ol = ol;
             w.lo = make_float4(lo[0], lo[1], lo[2], 0.f);
             w.hi = make_float4(hi[0], hi[1], hi[2], 0.f);
+            w.poison = 0;
         }
     }
     if (COMPAT) {   // each key goes to its rank; lanes past the end behind all keys
@@ -480,12 +508,8 @@ k_bh_walk(WalkArgs A)
                     eval_list<QUAD, COMPAT>(w, nlist, lane, A.eps2, acc);
                     nlist = 0;
                 }
-                const int2 e = w.part[lane];
-                const int own = e.x - s0;
-                const unsigned lanes = (unsigned)e.y & ~((unsigned)own < 32u ? 1u << own : 0u);
-                put_entry<QUAD, COMPAT>(w, nlist + lane, A.pa[e.x], A.pb[e.x], lanes, zero4, zero4);
+                n_pp += __popc(put_parts<QUAD, COMPAT>(A, w, nlist, 32, s0, lane));
                 nlist += 32;
-                n_pp += __popc(lanes);
                 npart -= 32;
                 int2 rest = make_int2(0, 0);
                 if (lane < npart) rest = w.part[32 + lane];
@@ -514,13 +538,7 @@ k_bh_walk(WalkArgs A)
             eval_list<QUAD, COMPAT>(w, nlist, lane, A.eps2, acc);
             nlist = 0;
         }
-        if (lane < npart) {
-            const int2 e = w.part[lane];
-            const int own = e.x - s0;
-            const unsigned lanes = (unsigned)e.y & ~((unsigned)own < 32u ? 1u << own : 0u);
-            put_entry<QUAD, COMPAT>(w, nlist + lane, A.pa[e.x], A.pb[e.x], lanes, zero4, zero4);
-            n_pp += __popc(lanes);
-        }
+        n_pp += __popc(put_parts<QUAD, COMPAT>(A, w, nlist, npart, s0, lane));
         nlist += npart;
     }
     if (nlist > 0) eval_list<QUAD, COMPAT>(w, nlist, lane, A.eps2, acc);
@@ -537,6 +555,7 @@ k_bh_walk(WalkArgs A)
         const bool second = lane >= WK_COLS;
         a[d] = (second ? row[1] : row[0]) +
                __shfl_xor_sync(0xffffffffu, second ? row[0] : row[1], WK_COLS);
+        if ((w.poison >> lane) & 1u) a[d] = __longlong_as_double(0x7ff8000000000000ll);
     }
     if (TEAM > 1) {   // the other warps' sums, in their order
         double *out = reinterpret_cast<double *>(w.sA);

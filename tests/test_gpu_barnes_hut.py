@@ -489,3 +489,24 @@ def test_group_walk_scales(lib, g, wl, log2_scale):
     b = g.acceleration(lib, x * scale, m, 1.0, g.METHOD_GPU_BARNES_HUT_GROUP, **kw) * scale ** 2
     assert np.isfinite(b).all()
     assert (np.linalg.norm(a - b, axis=1) <= 1e-6 * np.linalg.norm(a, axis=1)).all()
+
+
+@pytest.mark.parametrize("method,what", [(113, "position"), (103, "mass"), (105, "mass")])
+def test_walk_with_a_particle_that_is_not_finite(lib, g, orc, wl, method, what):
+    """A particle that is not finite reaches those that its leaf is opened for, and no others of
+    their warps: with the reference's walk (113), where far leaves weigh nothing, the rest stay
+    finite, and the particle with an infinite mass itself feels the others alone."""
+    x, v, m = wl.galaxy_pair(3000, 19)
+    k = 1234
+    if what == "position":
+        x[k, 1] = np.nan
+    else:
+        m[k] = np.inf
+    a = g.acceleration(lib, x, m, 1.0, method, opening_angle=0.5, softening_length=0.01,
+                       max_num_particles_per_leaf=1)
+    a_o, _, mag = orc.bh_counts(x, m, 1.0, 0.01, 0.5, 1, method == 113)
+    finite = np.isfinite(a_o).all(axis=1)
+    assert finite.any() and not finite.all() and (what == "position" or finite[k])
+    assert np.array_equal(np.isfinite(a).all(axis=1), finite)
+    if method != 105:
+        check_terms(a[finite], a_o[finite], mag[finite])
