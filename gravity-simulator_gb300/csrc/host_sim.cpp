@@ -212,6 +212,7 @@ struct gsgpu_sim {
     // Enqueue `steps` fixed steps of h of a small system.
     ErrorStatus run_tiny(int64_t steps, double h)
     {
+        if (steps <= 0) return ok();          // last_dt stays that of the last step
         constexpr int64_t kPerLaunch = 256;   // about a millisecond
         for (; steps > 0; steps -= kPerLaunch)
             launch_tiny_fixed(tiny(), integrator, (int)std::min(steps, kPerLaunch), h, stream);

@@ -274,3 +274,34 @@ def test_small_system_is_exit_and_single_body(lib, g, orc, wl):
     _, xo, vo, _ = g.launch_simulation(lib, x1, v1, m1, 1.0, integrator=4, dt=1e-3, tf=0.05,
                                        method=g.METHOD_GPU_PAIRWISE_FP64)
     assert np.array_equal(xo, xr) and np.array_equal(vo, vr)
+
+
+@pytest.mark.parametrize("n", [9, 60])
+def test_run_of_no_steps_changes_nothing(lib, g, wl, n):
+    """gsgpu_sim_run(0) after a run whose last step was clamped leaves the state, and the
+    velocities a download synchronises with the last step, as they are; a system of one block and
+    one of several launches."""
+    x, v, m = wl.plummer(n, 70)
+    dp = ctypes.POINTER(ctypes.c_double)
+    lib.gsgpu_sim_create.argtypes = [
+        ctypes.POINTER(ctypes.c_void_p), ctypes.c_int, ctypes.c_double,
+        ctypes.POINTER(g.AccelerationParam), ctypes.c_int, ctypes.c_double, ctypes.c_void_p]
+    lib.gsgpu_sim_upload.argtypes = [ctypes.c_void_p, dp, dp, dp]
+    lib.gsgpu_sim_run.argtypes = [ctypes.c_void_p, ctypes.c_int64]
+    lib.gsgpu_sim_run_until.argtypes = [ctypes.c_void_p, ctypes.c_double]
+    lib.gsgpu_sim_download.argtypes = [ctypes.c_void_p, dp, dp]
+    lib.gsgpu_sim_destroy.argtypes = [ctypes.c_void_p]
+    lib.gsgpu_sim_destroy.restype = None
+    p = g.AccelerationParam(g.METHOD_GPU_PAIRWISE_FP64, 1.0, 0.05, 1)
+    sim = ctypes.c_void_p()
+    assert lib.gsgpu_sim_create(ctypes.byref(sim), n, 1.0, ctypes.byref(p), 4, 4e-3, None) == 0
+    state = [np.empty((n, 3)) for _ in range(4)]
+    try:
+        assert lib.gsgpu_sim_upload(sim, *[a.ctypes.data_as(dp) for a in (x, v, m)]) == 0
+        assert lib.gsgpu_sim_run_until(sim, 0.0101) == 0
+        assert lib.gsgpu_sim_download(sim, *[a.ctypes.data_as(dp) for a in state[:2]]) == 0
+        assert lib.gsgpu_sim_run(sim, 0) == 0
+        assert lib.gsgpu_sim_download(sim, *[a.ctypes.data_as(dp) for a in state[2:]]) == 0
+    finally:
+        lib.gsgpu_sim_destroy(sim)
+    assert np.array_equal(state[0], state[2]) and np.array_equal(state[1], state[3])
