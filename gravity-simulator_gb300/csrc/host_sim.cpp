@@ -4,7 +4,8 @@
 // The integrator loops follow src/integrator.c (euler :281-454,
 // euler_cromer :456-628, rk4 :630-892, leapfrog :894-1121): the same step
 // count ceil(tf/dt), the same last-step dt clamp (all but rk4), t = steps*dt,
-// one is_exit check per step.  The state (x, v, compensation terms) stays in
+// is_exit read before each enqueued step (or batch of a small system).  The
+// state (x, v, compensation terms) stays in
 // HBM for the whole run; only the initial state goes host->device and the
 // final state device->host.  A step's kernels are captured once in a CUDA
 // graph and replayed; a clamped last step is launched directly.
@@ -874,7 +875,8 @@ ErrorStatus sim_download(gsgpu_sim *s, double *x, double *v)
     return ok();
 }
 
-// Run the reference's step loop for time tf with an is_exit check per step.
+// Run the reference's step loop for time tf; is_exit is read before each step is
+// enqueued, or before each batch of a small system.
 ErrorStatus sim_run_until(gsgpu_sim *s, double tf, SimulationStatus *status, const bool *is_exit,
                           OutputContext *out)
 {
@@ -898,8 +900,11 @@ ErrorStatus sim_run_until(gsgpu_sim *s, double tf, SimulationStatus *status, con
         if (status) status->dt = dt;
         int64_t batch = 1;
         if (s->tiny_fixed()) {
-            // Up to 32 steps (a tenth of a millisecond) at once, not past a step
-            // that is clamped or takes a snapshot; one when the run is to end.
+            // Up to 32 steps at once, not past a step that is clamped or takes a
+            // snapshot; one when the run is to end.  A flag set meanwhile ends the
+            // run after them: 0.12 ms for 9 bodies under leapfrog, 0.5 ms under RK4,
+            // 3.5 ms for 48 bodies of method 102 under RK4.  (The loop by launches
+            // runs up to 32 steps ahead of the device as well.)
             while (batch < 32 && steps + batch < total && !(is_exit && *is_exit) &&
                    !(oc && oc->due((double)(steps + batch) * dt)) &&
                    !(clamp && (double)(steps + batch) * dt + dt > tf))

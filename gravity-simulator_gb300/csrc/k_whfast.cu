@@ -1613,8 +1613,9 @@ ErrorStatus ensemble_run_until(gsgpu_ensemble *e, double tf, SimulationStatus *s
         if (t + dt > tf) dt = tf - t;
         if (status) status->dt = dt;
         if (e->batched()) {
-            // Up to 32 steps (half a millisecond) at once, not past a step that
-            // is clamped or takes a snapshot; one when the run is to end.
+            // Up to 32 steps at once, not past a step that is clamped or takes a
+            // snapshot; one when the run is to end.  A flag set meanwhile ends the
+            // run after them (0.6 ms for 9 bodies, 1.2 ms for 16 massive ones).
             int64_t k = 1;
             while (k < 32 && steps + k < total && !(is_exit && *is_exit) &&
                    !(oc && oc->due((double)(steps + k) * dt)) &&

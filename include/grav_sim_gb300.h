@@ -137,7 +137,8 @@ typedef struct SimulationStatus {
 typedef struct Settings {
     int verbose;
     bool enable_progress_bar;
-    bool *is_exit_ptr;
+    bool *is_exit_ptr;   /* read between steps; a system of at most 48 bodies takes up
+                          * to 32 steps (0.1 to 4 ms) between two reads */
 } Settings;
 
 /* src/system.h:28 */

@@ -7,6 +7,8 @@ With the compensated-FP32 force (101) the final state agrees to the
 accuracy of the force, and the energy drift matches the reference's.
 """
 import ctypes
+import threading
+import time
 
 import numpy as np
 import pytest
@@ -305,3 +307,47 @@ def test_run_of_no_steps_changes_nothing(lib, g, wl, n):
     finally:
         lib.gsgpu_sim_destroy(sim)
     assert np.array_equal(state[0], state[2]) and np.array_equal(state[1], state[3])
+
+
+class IntegratorParam(ctypes.Structure):
+    _fields_ = [("integrator", ctypes.c_int), ("dt", ctypes.c_double),
+                ("tolerance", ctypes.c_double), ("initial_dt", ctypes.c_double),
+                ("whfast_remove_invalid_particles", ctypes.c_bool)]
+
+
+@pytest.mark.parametrize("integ", [4, 10])
+def test_exit_flag_set_during_a_small_systems_run(lib, g, wl, integ):
+    """A flag that another thread sets while a system of one block runs (up to 32 steps a
+    launch) ends the run within a second, at a step that num_steps, t and the state agree on: the
+    same as a run of num_steps steps."""
+    G, dt = wl.G_AU_MSUN_DAY, 1.0
+    x, v, m = (a[:9].copy() for a in next(s for s in wl.planetary_ensemble(8, 3) if s[2].size >= 9))
+
+    def run(tf, after):
+        xs, vs, ms = x.copy(), v.copy(), m.copy()
+        system, keep = g.make_system(xs, ms, G, vs)
+        flag = ctypes.c_bool(False)
+        status = g.SimulationStatus(0.0, 0.0, 0)
+        settings = g.Settings(0, False, ctypes.pointer(flag))
+        ip = IntegratorParam(integ, dt, -1.0, -1.0, True)
+        ap = g.AccelerationParam(g.METHOD_GPU_MASSLESS, 1.0, 0.0, 1)
+        op = g.OutputParam(g.OUTPUT_METHOD_DISABLED, None, False, 0.0, 2, 2, 2, 0)
+        lib.launch_simulation.restype = g.ErrorStatus
+        timer = threading.Timer(after, setattr, (flag, "value", True))
+        if after > 0:
+            timer.start()
+        t0 = time.perf_counter()
+        st = lib.launch_simulation(ctypes.byref(system), ctypes.byref(ip), ctypes.byref(ap),
+                                   ctypes.byref(op), ctypes.byref(status), ctypes.byref(settings),
+                                   ctypes.c_double(tf))
+        wall = time.perf_counter() - t0
+        assert st.return_code == 0, g.take_traceback(lib, st)
+        assert system.num_particles == 9
+        return status, xs, vs, wall
+
+    run(64 * dt, 0.0)   # the library is loaded and the GPU awake
+    status, xs, vs, wall = run(1e9 * dt, 0.2)
+    assert 32 < status.num_steps < 1e9 and status.t == status.num_steps * dt and wall < 1.2
+    again, xr, vr, _ = run(status.num_steps * dt, 0.0)
+    assert again.num_steps == status.num_steps
+    assert xs.tobytes() == xr.tobytes() and vs.tobytes() == vr.tobytes()
