@@ -1,6 +1,6 @@
 // k_fft.cu -- FP64 convolution of a real g^3 mesh with a real, even kernel given
-// by its transform, for even g of small prime factors from 32 to 256 (the
-// particle-mesh potential).
+// by its transform (the particle-mesh potential), for the 15 sizes g of convolve_for:
+// 32, 40, 48, 60, 64, 72, 80, 96, 100, 120, 128, 144, 160, 192 and 256.
 //
 // The mesh is read as g x g x g/2 complex numbers, two neighbours on the last
 // axis in one: C = E + i O with E the even and O the odd planes.  Transforms
@@ -23,8 +23,8 @@
 // 64 cycles): at g = 128, 1.38e8 operations, 221 us.  The library's transforms
 // took 490 us there and the multiplication 8; these five launches take 292 (46 for
 // each pass of lines, 108 for the pairs).  A step with 24^3 particles, before and
-// now: g = 32 104 and 60 us, 48 104 and 72, 60 145 and 86, 96 297 and 173, 160 1311
-// and 867, 256 4195 and 2729.  Accelerations differ from an extended
+// now: g = 32 104 and 54 us, 48 104 and 70, 60 145 and 84, 96 297 and 174, 160 1311
+// and 825, 256 4195 and 2762.  Accelerations differ from an extended
 // precision computation by as much with either (1e-14 at g = 32 to 256).
 #include "gs_fft.h"
 
@@ -236,12 +236,20 @@ struct Split {
     static_assert(R1 * R2 == N, "two radices");
 };
 
-// Lines of 128 points take 8 x 16: twice as many threads of half the work fill the
-// sub-partitions more evenly (46 us a pass instead of 51 at g = 128).  The second
-// step then needs half the threads; neighbouring blocks take different halves.
+// Lines take the smaller radix first: a line is then shared by as many threads as
+// the larger one, each with less work, which fills the sub-partitions more evenly (in
+// the second step as many are busy as the smaller one; neighbouring blocks take
+// different ones).  Unless only the other order fills whole warps: a block is eight
+// lines, so its threads are a multiple of 32 where the second radix is one of 4.
+// Step with 24^3 particles, the larger radix first and the smaller one: g = 32 61.8
+// and 53.6 us, 40 68.1 and 62.2, 60 86.3 and 84.3, 72 115 and 108, 80 (10 x 8) 132
+// and 142, 96 173 and 174, 120 382 and 347, 128 371 and 351, 160 877 and 825, 192 both
+// 1240.
 template <int N>
 struct LineSplit {
-    static constexpr int R1 = N == 128 ? 8 : Split<N>::R1, R2 = N / R1;
+    static constexpr int A = Split<N>::R1, B = Split<N>::R2;
+    static constexpr int SMALL = A < B ? A : B, LARGE = A < B ? B : A;
+    static constexpr int R1 = LARGE % 4 != 0 && SMALL % 4 == 0 ? LARGE : SMALL, R2 = N / R1;
 };
 
 // Lines along one of the first two axes.  A CTA takes LINES neighbouring lines
@@ -440,8 +448,9 @@ void convolve(double2 *data, const MeshScale &scale, const double *table, const 
 
 using Convolve = void (*)(double2 *, const MeshScale &, const double *, const double2 *, cudaStream_t);
 
-// Even sizes of small prime factors whose lines and half lines have two factors
-// of at most 16; other sizes go to the library's transforms.
+// The sizes that are built: multiples of four whose lines and half lines are products
+// of two of the radices above, each measured faster than the library's transforms.
+// Every other size goes to the library, also 36 and 50, whose factors would fit.
 static Convolve convolve_for(int g)
 {
     switch (g) {
