@@ -205,16 +205,17 @@ constexpr int TC_ITEMS = 8;
 constexpr int TC_TILE = OT_THREADS * TC_ITEMS;   // particles per scan tile
 constexpr int TN_ROUND = OT_THREADS / 8;         // internal nodes a CTA works on at once
 constexpr int TN_ROUNDS = 8;                     // rounds per scan tile at most
-constexpr int TN_MANY = 1216;                    // scan tiles from which a tile takes more rounds
+constexpr int TN_GRID = 4;                       // CTAs per SM of the kernels over nodes
+constexpr int TN_MANY = 2;                       // tiles per CTA from which a tile takes more rounds
 
-// Internal nodes per scan tile of a tree with ni of them.  A round is a chain
-// of dependent loads (the searches of the octants' ends), so a small tree takes
-// one round per tile: eight rounds left 8 of 152 SMs with work at 60,000 particles
-// and 16 per leaf (38 us, now 11).  Tiles grow with the tree so
-// that their scan, by one CTA, stays short.
-__device__ __forceinline__ int node_tile(int ni)
+// Internal nodes per scan tile of a tree with ni of them, on a grid of `ctas`.  A
+// round is a chain of dependent loads (the searches of the octants' ends), so a small
+// tree takes one round per tile: eight rounds left 8 of 152 SMs with work at 60,000
+// particles and 16 per leaf (38 us, now 11).  With more than TN_MANY tiles a CTA (eight
+// an SM) tiles grow with the tree, so that their scan, by one CTA, stays short.
+__device__ __forceinline__ int node_tile(int ni, int ctas)
 {
-    return TN_ROUND * min(TN_ROUNDS, 1 + ni / (TN_ROUND * TN_MANY));
+    return TN_ROUND * min(TN_ROUNDS, 1 + ni / (TN_ROUND * TN_MANY * ctas));
 }
 
 // Levels (octant digits) shared by two 63-bit keys.
@@ -385,7 +386,7 @@ k_tree_children(const uint64_t *__restrict__ keys, int n, int cap, const int2 *_
 {
     const int ni = ctr[CTR_SAFE_INTERNAL];
     const int lane = threadIdx.x & 31, o = lane & 7, g0 = lane & ~7;
-    const int size = node_tile(ni), tiles = (ni + size - 1) / size;
+    const int size = node_tile(ni, gridDim.x), tiles = (ni + size - 1) / size;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         unsigned mine = 0;
         for (int q = 0; q < size; q += TN_ROUND) {
@@ -438,7 +439,7 @@ k_tree_nodes(int n, int leaf_max, const unsigned *__restrict__ tile_off,
     __shared__ int s_fc[TN_ROUND * TN_ROUNDS];
     const int ni = ctr[CTR_SAFE_INTERNAL];
     const int lane = threadIdx.x & 31, o = lane & 7, g0 = lane & ~7;
-    const int size = node_tile(ni), tiles = (ni + size - 1) / size;
+    const int size = node_tile(ni, gridDim.x), tiles = (ni + size - 1) / size;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int mine = tile * size + (int)threadIdx.x;
         unsigned sum;
@@ -895,8 +896,11 @@ ErrorStatus OctreeDevice::setup(int n_, int leaf_max_, bool compat_, bool quad_)
     GS_TRY(in_sd.reserve((size_t)cap * sizeof(int2)));
     GS_TRY(in_end.reserve((size_t)cap * 8 * sizeof(int)));
     GS_TRY(in_rec.reserve((size_t)cap * sizeof(int4)));
+    const DeviceInfo *dev = nullptr;
+    GS_TRY(device_info(&dev));
+    const int small_tiles = TN_MANY * TN_GRID * dev->sm_count + TN_ROUNDS;
     GS_TRY(scan_tiles.reserve(
-        (size_t)(std::max(std::max((n + TC_TILE - 1) / TC_TILE, TN_MANY + TN_ROUNDS),
+        (size_t)(std::max(std::max((n + TC_TILE - 1) / TC_TILE, small_tiles),
                           cap / (TN_ROUND * TN_ROUNDS) + 1) +
                  1) *
         sizeof(unsigned)));
@@ -954,7 +958,7 @@ ErrorStatus OctreeDevice::build(const double *d_x, const double *d_m, cudaStream
     GS_TRY(device_info(&dev));
     // Kernels over internal nodes or nodes, whose count only the device knows,
     // stride over them: a grid for the capacity would be mostly empty CTAs.
-    const int grid = dev->sm_count * 4;
+    const int grid = dev->sm_count * TN_GRID;
     const int ptiles = (n + TC_TILE - 1) / TC_TILE;
     unsigned *tiles = scan_tiles.as<unsigned>();
     k_tree_count<<<ptiles, OT_THREADS, 0, s>>>(keys.as<uint64_t>(), n, leaf_max, cap_nodes, tiles,
