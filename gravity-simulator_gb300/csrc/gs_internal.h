@@ -99,8 +99,6 @@ struct ForceTimer {
 };
 
 // ---- force engines -----------------------------------------------------
-// One engine per (method, N); it owns its scratch memory.  compute() reads
-// FP64 positions and masses on the device and writes FP64 accelerations.
 // State of n bodies on the device, 3n values each, with its compensation terms.
 struct StepState {
     double *x, *xe, *v, *ve;
@@ -113,6 +111,8 @@ struct Kick {
     double h;
 };
 
+// One engine per (method, N); it owns its scratch memory.  compute() reads
+// FP64 positions and masses on the device and writes FP64 accelerations.
 class Engine {
   public:
     virtual ~Engine() {}

@@ -96,15 +96,10 @@ struct OctreeDevice {
     ErrorStatus clear_status(cudaStream_t s);
 };
 
-// Barnes-Hut walk of a built tree (k_walk.cu).  counters (2 x u64) receive
-// cell and particle terms (added); gate (device int, may be null) makes the
-// launch return at once when *gate == 0.
-ErrorStatus launch_bh_walk(const OctreeDevice &t, const double *d_x, double theta, double eps,
-                           double G, double *d_a, const int *gate,
-                           unsigned long long *counters, cudaStream_t s);
-
-// Group walk with interaction lists (k_walk_group.cu): same counters and
-// gate as launch_bh_walk; needs a tree with true leaf multipoles (not compat).
+// Group walk with interaction lists (k_walk_group.cu) of a tree with true leaf
+// multipoles (not compat).  counters (2 x u64) receive cell and particle terms
+// (added); gate (device int, may be null) makes the launch return at once when
+// *gate == 0.
 // The groups depend on the tree alone: a second walk of the same tree (another
 // angle) passes reuse_groups and keeps the first walk's list.
 ErrorStatus launch_bh_group_walk(const OctreeDevice &t, double theta, double eps, double G,

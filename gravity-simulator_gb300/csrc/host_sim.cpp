@@ -5,10 +5,10 @@
 // euler_cromer :456-628, rk4 :630-892, leapfrog :894-1121): the same step
 // count ceil(tf/dt), the same last-step dt clamp (all but rk4), t = steps*dt,
 // is_exit read before each enqueued step (or batch of a small system).  The
-// state (x, v, compensation terms) stays in
-// HBM for the whole run; only the initial state goes host->device and the
-// final state device->host.  A step's kernels are captured once in a CUDA
-// graph and replayed; a clamped last step is launched directly.
+// state (x, v, compensation terms) stays in HBM for the whole run; only the
+// initial state goes host->device and the final state device->host.  A step's
+// kernels are captured once in a CUDA graph and replayed; a clamped last step is
+// launched directly.
 #include "gs_internal.h"
 
 #include <algorithm>

@@ -48,7 +48,6 @@ constexpr int DS_JTILE = 1024;                 // 16 KiB of float4
 constexpr int DS_STAGES = 3;
 constexpr int DS_SMEM = DS_STAGES * DS_JTILE * 16;
 constexpr int DS_GRANULE = 128;                // plain FP32 partials of 128 terms
-constexpr int DS_SMALL_ITILE = 2 * DS_THREADS; // rows of a unit of k_direct_small
 constexpr int DS_TILE_GRANULES = DS_JTILE / DS_GRANULE;
 constexpr int DR_WARPS = 8;                    // k_direct_run
 constexpr int DR_THREADS = 32 * DR_WARPS;
@@ -607,7 +606,11 @@ class DirectEngine final : public Engine {
         n_pad_ = ((n + DS_ITILE - 1) / DS_ITILE) * DS_ITILE;
         granules_ = (n + DS_GRANULE - 1) / DS_GRANULE;
         if (n <= DS_RUN_N) {
-            // compensated runs of 1,024 terms, 2,048 from 17,409 particles on
+            // Compensated runs of 1,024 terms; of 2,048 from 17,409 particles on,
+            // where both take the same time and half the partial sums are stored.
+            // Leapfrog step with runs of 1,024 and 2,048: N = 12,000 68.3 and 72.4 us,
+            // 16,000 110 and 115, 17,000 121.9 and 121.6, 18,000 136 and 137, 19,000
+            // 150 and 149, 20,480 173 and 175.
             per_ = (n <= 17 * DS_JTILE ? 1 : 2) * DS_TILE_GRANULES;
             i_tiles_ = (n + DR_ROWS - 1) / DR_ROWS;
         } else {
@@ -829,9 +832,12 @@ ErrorStatus DirectRows::check(cudaStream_t s)
 // records or replays a fixed plan of work and may not call cudaMalloc
 // (which can synchronise the device) in the middle of it, embedders whose
 // allocator is a pool they own, and real-time loops that must not touch the
-// allocator at all.  This entry point computes the same accelerations as
+// allocator at all.  This entry point computes the accelerations of
 // acceleration() with GRAV_GPU_PAIRWISE, from device arrays the caller
-// owns, using the same kernels; its scratch (the packed float4 particles,
+// owns, to the same accuracy: the pair terms are the same, but the work is
+// always k_direct_sum's, in at most NOALLOC_MAX_SPLITS units of whole tiles per
+// row, so the compensated partial sums are grouped otherwise and last bits
+// differ, and small systems take longer.  Its scratch (the packed float4 particles,
 // the per-split partial sums, the status word and the frame centre) lives
 // in one file-scope device array instead of memory the library allocates.
 // That array is part of the library image: every GPU that loads the library

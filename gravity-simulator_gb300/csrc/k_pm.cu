@@ -4,12 +4,12 @@
 // One evaluation on a g^3 periodic mesh:
 //   deposit        cloud-in-cell deposit of the masses, eight FP64 atomic adds per
 //                  particle (the reference's OpenMP loop has unsynchronised += here);
-//   the potential  the density contrast rho / (V_cell rho_mean) - 1, formed where
-//                  the mesh is first read (a deposit into a mesh of -1 would round
-//                  every addition to the contrast's last bit), convolved with -1/k^2 (0 at k = 0), from a table by
-//                  the integer |n|^2: for the sizes of k_fft.cu (even, of small
-//                  factors, 32 to 256) in place, otherwise cuFFT D2Z (FFTW's layout:
-//                  g x g x (g/2+1)), k_pm_green, and cuFFT Z2D, unnormalised;
+//   the potential  the density contrast rho / (V_cell rho_mean) - 1, formed where the
+//                  mesh is first read (a deposit into a mesh of -1 would round every
+//                  addition to the contrast's last bit), convolved with -1/k^2 (0 at
+//                  k = 0), from a table by the integer |n|^2: in place for the sizes
+//                  of k_fft.cu, otherwise cuFFT D2Z (FFTW's layout: g x g x (g/2+1)),
+//                  k_pm_green, and cuFFT Z2D, unnormalised;
 //   k_pm_gradient  fourth-order central differences of phi into the
 //                  acceleration mesh, without their constant factor;
 //   interpolation  cloud-in-cell, back to the particles; the caller's multiplier

@@ -92,10 +92,9 @@ __device__ __forceinline__ void tiny_pair(const double *x, int i, int j, double 
 //
 // What bounds it is the chain of FP64 operations (65 cycles each).  With at most
 // TY_FEW pairs a thread per pair and component forms the component's two products
-// with the masses, so that the ordered sums are additions alone (IAS15 step of the
-// Sun and eight planets 280 -> 235 us together with the kept quotients below, 225 with
-// the kept products of b,
-// leapfrog step 5.5 -> 4.1).
+// with the masses, so that the ordered sums are additions alone (the Sun and eight
+// planets, with products formed inside the sums and so: leapfrog step 5.5 and 4.1 us;
+// an IAS15 step takes 225).
 __device__ void tiny_force(TinyForce &f, const double *x, double *a, double G, double eps2)
 {
     const int nh = f.nh, nl = f.nl;

@@ -87,7 +87,6 @@ struct WalkArgs {
     double *a;
     unsigned long long *counters;   // [0] accepted cells, [1] leaf pair terms
     unsigned *status;
-    const int *gate;                // when set, the launch runs only if *gate != 0
 };
 
 // One warp's state.  List entries (accepted cells and particles of opened
@@ -284,7 +283,6 @@ k_bh_walk(WalkArgs A)
     __shared__ unsigned char children_all[WK_WARPS * WK_STACK];    // children
     __shared__ int counts[WK_WARPS];
 
-    if (A.gate && *A.gate == 0) return;   // block-uniform
     if (*A.status & ST_TREE_OVERFLOW) return;   // the build overflowed: no tree to walk
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int part = TEAM == 1 ? 0 : warp;
@@ -651,7 +649,6 @@ class BarnesHutEngine final : public Engine {
         w.a = d_a;
         w.counters = counters_.as<unsigned long long>();
         w.status = reinterpret_cast<unsigned *>(tree_.ctr.as<int>() + CTR_STATUS);
-        w.gate = nullptr;
         GS_CUDA(cudaMemsetAsync(counters_.p, 0, 2 * sizeof(unsigned long long), s));
         if (group_) {
             if (timer) GS_TRY(timer->begin(s));
@@ -715,41 +712,6 @@ class BarnesHutEngine final : public Engine {
 std::unique_ptr<Engine> make_barnes_hut_engine(bool compat, bool quad, bool group)
 {
     return std::unique_ptr<Engine>(new BarnesHutEngine(compat, quad, group));
-}
-
-// Walk of a built (non-compat) tree, for engines that walk one tree several
-// times (the learned method's cheap walk and its gated fallback).
-ErrorStatus launch_bh_walk(const OctreeDevice &t, const double *d_x, double theta, double eps,
-                           double G, double *d_a, const int *gate,
-                           unsigned long long *counters, cudaStream_t s)
-{
-    WalkArgs w;
-    w.na = t.w_na.as<float4>();
-    w.nb = t.w_nb.as<float4>();
-    w.nq = t.quad ? t.w_nq.as<float4>() : nullptr;
-    w.nc = t.w_nc.as<int4>();
-    w.nkey = t.w_nkey.as<uint64_t>();
-    w.ncom = t.t_com.as<double>();
-    w.depth = t.t_depth.as<int>();
-    w.pa = t.w_pa.as<float4>();
-    w.pb = t.w_pb.as<float4>();
-    w.sidx = t.sidx.as<int>();
-    w.skeys = t.keys.as<uint64_t>();
-    w.x = d_x;
-    w.frame = t.frame.as<double>();
-    w.n = t.n;
-    w.eps2 = (float)(eps * eps);
-    w.theta2 = theta * theta;
-    w.G = G;
-    w.a = d_a;
-    w.counters = counters;
-    w.status = reinterpret_cast<unsigned *>(t.ctr.as<int>() + CTR_STATUS);
-    w.gate = gate;
-    const DeviceInfo *dev = nullptr;
-    GS_TRY(device_info(&dev));
-    launch_walk_kernel(w, t.quad, t.compat, dev->sm_count, s);
-    GS_CUDA(cudaGetLastError());
-    return ok();
 }
 
 ErrorStatus accel_host(double *a, const System *system, const AccelerationParam *param_in);

@@ -250,24 +250,6 @@ struct SeqRuns {
     int nruns;
 };
 
-// One exact chain step of src/integrator_whfast.c:744-760 for particle i;
-// y[6] receives the offsets added to jx_i / jv_i.
-__device__ __forceinline__ void jac_step(double xc[3], double vc[3], double mi, double ei,
-                                         double ep, const double *jxi, const double *jvi,
-                                         double *xi, double *vi, double y[6])
-{
-    for (int k = 0; k < 3; ++k) {
-        xc[k] = __ddiv_rn(__dsub_rn(xc[k], __dmul_rn(mi, jxi[k])), ei);
-        vc[k] = __ddiv_rn(__dsub_rn(vc[k], __dmul_rn(mi, jvi[k])), ei);
-        y[k] = xc[k];
-        y[3 + k] = vc[k];
-        xi[k] = __dadd_rn(jxi[k], xc[k]);
-        vi[k] = __dadd_rn(jvi[k], vc[k]);
-        xc[k] = __dmul_rn(ep, xc[k]);
-        vc[k] = __dmul_rn(ep, vc[k]);
-    }
-}
-
 __device__ void wh_massive_list_warp(const EnsDev &E, int base, int n, int s, int lane)
 {
     int k = 0;
