@@ -111,7 +111,7 @@ struct WalkShared {
     int2 part[64];               // particles of opened leaves, lanes
     float pos[6][32];            // negated particle positions: hi x y z, lo x y z
     float4 oh, ol, lo, hi;       // origin (the first particle) and the particles' box from it
-    unsigned poison;             // lanes that a particle that is not finite acts on
+    unsigned poison;             // lanes that a term that is not finite acts on
 };
 
 // Compensated sums of a lane's two particles, the even and the odd list entries
@@ -233,6 +233,11 @@ __device__ __forceinline__ void eval_list(WalkShared<QUAD, COMPAT> &w, int count
     __syncwarp();   // the list is read
 }
 
+__device__ __forceinline__ bool all_finite(const float4 v)
+{
+    return fmaf(v.x, 0.f, fmaf(v.y, 0.f, fmaf(v.z, 0.f, v.w * 0.f))) == 0.f;
+}
+
 // The particles w.part[0 .. count) (at most 32) of opened leaves become list entries
 // from `at` on; returns the lanes that this lane's one acts on (not the particle
 // itself).  Lanes an entry does not act on add its terms times zero, so a particle
@@ -249,8 +254,7 @@ __device__ __forceinline__ unsigned put_parts(const WalkArgs &A, WalkShared<QUAD
     const unsigned lanes = (unsigned)e.y & ~((unsigned)own < 32u ? 1u << own : 0u);
     float4 h = A.pa[e.x], l = A.pb[e.x];
     unsigned on = lanes;
-    // zero unless one of them is infinite or NaN
-    if (!(fmaf(h.x, 0.f, fmaf(h.y, 0.f, fmaf(h.z, 0.f, h.w * 0.f))) == 0.f)) {
+    if (!all_finite(h)) {
         atomicOr(&w.poison, lanes);
         h = l = zero;
         on = 0;
@@ -488,7 +492,15 @@ k_bh_walk(WalkArgs A)
             eval_list<QUAD, COMPAT>(w, nlist, lane, A.eps2, acc);
             nlist = 0;
         }
-        if (takers) put_entry<QUAD, COMPAT>(w, nlist + __popc(taken & lt), ca, cb, takers, q0, q1);
+        if (takers) {
+            unsigned on = takers;
+            if (!all_finite(ca) || (QUAD && !(all_finite(q0) && all_finite(q1)))) {
+                atomicOr(&w.poison, takers);   // as in put_parts
+                ca = cb = q0 = q1 = zero4;
+                on = 0;
+            }
+            put_entry<QUAD, COMPAT>(w, nlist + __popc(taken & lt), ca, cb, on, q0, q1);
+        }
         nlist += __popc(taken);
         n_cell += __popc(takers);
         // particles of opened leaves: leaves of one particle together, the others

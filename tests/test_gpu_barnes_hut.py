@@ -510,3 +510,42 @@ def test_walk_with_a_particle_that_is_not_finite(lib, g, orc, wl, method, what):
     assert np.array_equal(np.isfinite(a).all(axis=1), finite)
     if method != 105:
         check_terms(a[finite], a_o[finite], mag[finite])
+
+
+@pytest.mark.parametrize("method,what", [(103, "mass"), (105, "mass"), (105, "quadrupole")])
+def test_walk_with_cells_beyond_fp32(lib, g, orc, method, what):
+    """A cell whose mass or quadrupole is infinite in FP32 reaches the particles that accept it,
+    and not those of their warps that open it; which ones follows from the oracle's tree.  Among
+    light particles a tight clump of 64 masses of 1e37, or a pair of 1e34 a thousand apart, whose
+    other terms stay in range."""
+    rng = np.random.default_rng(8)
+    n, theta = 500, 0.7
+    scale, k, heavy = (100.0, 64, 1e37) if what == "mass" else (1e5, 2, 1e34)
+    x = rng.uniform(-scale, scale, (n, 3))
+    x[:k] = 0.4 * scale
+    x[:k] += rng.uniform(-0.002, 0.002, (k, 3)) if what == "mass" else [[-500.0] * 3, [500.0] * 3]
+    x[k:k + 64] = 0.4 * scale + rng.uniform(-0.09 * scale, 0.09 * scale, (64, 3))
+    m = np.ones(n)
+    m[:k] = heavy
+    t = orc.build_tree(x, m, 1, False)
+    q = orc.bh_quad(x, m, 1.0, 0.0, theta, 1)[2]
+    first, num, side = t["first_particle"], t["num_particles"], t["box_width"] / 2.0 ** t["depth"]
+    big = t["mass"] if what == "mass" else np.abs(q).max(axis=1)
+    big = big > 3.4028236e38
+    place = np.empty(n, int)
+    place[t["sorted_indices"]] = np.arange(n)
+    expect = np.zeros(n, bool)
+    for i in range(n):
+        stack = [0]
+        while stack:
+            c = stack.pop()
+            inside = first[c] <= place[i] < first[c] + num[c]
+            if c and not inside and side[c] ** 2 < theta ** 2 * ((t["com"][c] - x[i]) ** 2).sum():
+                expect[i] |= big[c]
+            elif t["num_children"][c]:
+                stack += range(t["first_child"][c], t["first_child"][c] + t["num_children"][c])
+    assert 20 < expect.sum() < n - 20
+    a = g.acceleration(lib, x, m, 1.0, method, opening_angle=theta,
+                       softening_length=1.0 if what == "mass" else 0.0,
+                       max_num_particles_per_leaf=1)
+    assert np.array_equal(~np.isfinite(a).all(axis=1), expect)
