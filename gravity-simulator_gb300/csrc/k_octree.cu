@@ -727,7 +727,8 @@ __device__ __forceinline__ void multipole_node4(const int4 rec, int j, unsigned 
         float Q[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int k = 0; k < 2; ++k)
-            if (j + 4 * k < nch) {
+            // a massless child (no centre of mass: 0 / 0) adds nothing
+            if (j + 4 * k < nch && !(ca[k].w == 0.0f && isnan(ca[k].x))) {
                 add_quad(Q, ca[k].w, df_offset(ca[k].x, cb[k].x, h[0], l[0]),
                          df_offset(ca[k].y, cb[k].y, h[1], l[1]),
                          df_offset(ca[k].z, cb[k].z, h[2], l[2]));

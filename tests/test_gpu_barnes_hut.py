@@ -549,3 +549,21 @@ def test_walk_with_cells_beyond_fp32(lib, g, orc, method, what):
                        softening_length=1.0 if what == "mass" else 0.0,
                        max_num_particles_per_leaf=1)
     assert np.array_equal(~np.isfinite(a).all(axis=1), expect)
+
+
+@pytest.mark.parametrize("n", [400, 20000])
+def test_quadrupole_walks_with_massless_particles(lib, g, orc, wl, n):
+    """Massless particles (cells of them have no centre of mass) add nothing to the quadrupoles
+    of the cells above: 105 against the oracle, whose quadrupoles are sums over a node's
+    particles, and 106 at least about as accurate."""
+    x, v, m = wl.galaxy_pair(n, 29)
+    m = np.where(np.random.default_rng(1).random(n) < 0.7, 0.0, m)
+    kw = dict(opening_angle=0.5, softening_length=0.01, max_num_particles_per_leaf=1)
+    a = g.acceleration(lib, x, m, 1.0, g.METHOD_GPU_BARNES_HUT_QUAD, **kw)
+    b = g.acceleration(lib, x, m, 1.0, g.METHOD_GPU_BARNES_HUT_GROUP, **kw)
+    assert np.isfinite(a).all() and np.isfinite(b).all()
+    a_o, mag, _ = orc.bh_quad(x, m, 1.0, 0.01, 0.5, 1)
+    check_terms(a, a_o, mag)
+    rows = np.arange(0, n, max(1, n // 400), dtype=np.int32)
+    exact = orc.direct_rows(x, m, 1.0, 0.01, rows)
+    assert np.median(orc.rel_err(b[rows], exact)) <= 1.1 * np.median(orc.rel_err(a[rows], exact))
