@@ -410,7 +410,8 @@ k_bh_walk(WalkArgs A)
             if (around || cb.w > 1.00002f * th2f * far2)
                 opened = reach;
             else
-                test = !(away && 1.00002f * cb.w < th2f * near2);
+                // (far2 is NaN where any coordinate of the centre is, near2 is not)
+                test = !(away && 1.00002f * cb.w < th2f * fmaf(far2, 0.f, near2));
         }
         // the other nodes lane by lane
         const unsigned tests = __ballot_sync(0xffffffffu, test);

@@ -567,3 +567,21 @@ def test_quadrupole_walks_with_massless_particles(lib, g, orc, wl, n):
     rows = np.arange(0, n, max(1, n // 400), dtype=np.int32)
     exact = orc.direct_rows(x, m, 1.0, 0.01, rows)
     assert np.median(orc.rel_err(b[rows], exact)) <= 1.1 * np.median(orc.rel_err(a[rows], exact))
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("theta", [0.5, 1.5, 5.0])
+def test_compat_walk_with_a_lost_coordinate(lib, g, orc, axis, theta):
+    """One coordinate of one particle is NaN, and of the centres of the cells it is in: no
+    particle accepts those, however far away they are in the other coordinates."""
+    rng = np.random.default_rng(12)
+    x = rng.integers(-4, 5, (1500, 3)).astype(float) + rng.uniform(-0.2, 0.2, (1500, 3))
+    m = np.ones(len(x))
+    x[777, axis] = np.nan
+    a = g.acceleration(lib, x, m, 1.0, g.METHOD_GPU_BARNES_HUT_COMPAT, opening_angle=theta,
+                       softening_length=0.05, max_num_particles_per_leaf=1)
+    a_o, _, mag = orc.bh_counts(x, m, 1.0, 0.05, theta, 1, True)
+    finite = np.isfinite(a_o).all(axis=1)
+    assert finite.any() and not finite.all()
+    assert np.array_equal(np.isfinite(a).all(axis=1), finite)
+    check_terms(a[finite], a_o[finite], mag[finite])
